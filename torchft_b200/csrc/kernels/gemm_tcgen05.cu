@@ -115,18 +115,18 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        int m0, n0;
-        tile_coords(t, m0, n0);
-        for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      int m0, n0;
+      tile_coords(t, m0, n0);
+      for (int kb = 0; kb < num_k; ++kb) {
+        if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           const uint32_t sa = smem_base + stage * STAGE_BYTES;
           const uint32_t sb = sa + A_BYTES;
           const int k0 = kb * BK;
@@ -143,45 +143,46 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * (BK * 128), &tmB, full_bar(stage), n0 + 64 * j, k0);
           }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      if (!ok) {
-        // give copies that are still in flight time to land before the CTA retires
-        const uint64_t t0 = ftb200::globaltimer_ns();
-        while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-      }
+    }
+    if (!ok) {
+      // give copies that are still in flight time to land before the CTA retires
+      const uint64_t t0 = ftb200::globaltimer_ns();
+      while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.a_mn) << 15) |
-                             (static_cast<uint32_t>(p.b_mn) << 16) | (static_cast<uint32_t>(BN >> 3) << 17) |
-                             (static_cast<uint32_t>(BM >> 4) << 24);
-      // K-major: 8-row groups 1024 B apart, step 32 B along K inside the swizzle row.
-      // MN-major: 64-element column blocks BK*128 B apart, 8-deep K groups 1024 B apart,
-      //           step 16 K rows = 2048 B.
-      const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, a_step = p.a_mn ? 2048 : 32;
-      const uint32_t b_lbo = p.b_mn ? BK * 128 : 16, b_step = p.b_mn ? 2048 : 32;
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.a_mn) << 15) |
+                           (static_cast<uint32_t>(p.b_mn) << 16) | (static_cast<uint32_t>(BN >> 3) << 17) |
+                           (static_cast<uint32_t>(BM >> 4) << 24);
+    // K-major: 8-row groups 1024 B apart, step 32 B along K inside the swizzle row.
+    // MN-major: 64-element column blocks BK*128 B apart, 8-deep K groups 1024 B apart,
+    //           step 16 K rows = 2048 B.
+    const uint32_t a_lbo = p.a_mn ? BK * 128 : 16, a_step = p.a_mn ? 2048 : 32;
+    const uint32_t b_lbo = p.b_mn ? BK * 128 : 16, b_step = p.b_mn ? 2048 : 32;
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      if (!mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = 0; kb < num_k; ++kb) {
+        if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) {
+          ok = false;
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
           const uint32_t sa = smem_base + stage * STAGE_BYTES;
           const uint32_t sb = sa + A_BYTES;
 #pragma unroll
@@ -191,17 +192,18 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             umma_bf16(d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
           }
           umma_commit(empty_bar(stage));
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          if (kb == num_k - 1) umma_commit(tfull_bar(acc));
         }
-        if (!ok) break;
-        umma_commit(tfull_bar(acc));
-        if (++acc == 2) {
-          acc = 0;
-          acc_phase ^= 1u;
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
+      }
+      if (!ok) break;
+      if (++acc == 2) {
+        acc = 0;
+        acc_phase ^= 1u;
       }
     }
     __syncwarp();

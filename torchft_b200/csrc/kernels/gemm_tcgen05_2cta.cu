@@ -223,28 +223,28 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
-        int m0, n0;
-        tile_coords(t, m0, n0);
-        const int nb = n0 + static_cast<int>(rank) * BNH;  // this CTA's half of the B tile
-        if (p.ga_world > 0 && nb < p.N) {
-          // these 128 rows of B are local once all their pieces are counted; the loads below go through the
-          // async proxy, the pieces were written through the generic one
-          if (!count_wait(p.ga_sync + 1 + nb / BNH, static_cast<unsigned int>(p.K / 64), abort_flag)) {
-            ok = false;
-            break;
-          }
-          asm volatile("fence.proxy.async.global;" ::: "memory");
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
+      int m0, n0;
+      tile_coords(t, m0, n0);
+      const int nb = n0 + static_cast<int>(rank) * BNH;  // this CTA's half of the B tile
+      if (p.ga_world > 0 && nb < p.N) {
+        // these 128 rows of B are local once all their pieces are counted; the loads below go through the
+        // async proxy, the pieces were written through the generic one
+        if (!__all_sync(0xffffffffu, count_wait(p.ga_sync + 1 + nb / BNH, static_cast<unsigned int>(p.K / 64), abort_flag))) {
+          ok = false;
+          break;
         }
-        for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+      }
+      for (int kb = 0; kb < num_k; ++kb) {
+        if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           const uint32_t sa = smem_base + stage * STAGE_BYTES;
           const uint32_t sb = sa + A_BYTES;
           const int k0 = kb * BK;
@@ -262,21 +262,22 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
 #pragma unroll
             for (int j = 0; j < BNH / 64; ++j) tma_load_2d_pair(sb + j * (BK * 128), &tmB, fb, nb + 64 * j, k0);
           }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        __syncwarp();
+        if (++stage == STAGES) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
-      if (!ok) {
-        const uint64_t t0 = ftb200::globaltimer_ns();
-        while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-      }
+    }
+    if (!ok) {
+      const uint64_t t0 = ftb200::globaltimer_ns();
+      while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
-    if (leader && lane == 0) {
+    if (leader) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.a_mn) << 15) |
                              (static_cast<uint32_t>(p.b_mn) << 16) | (static_cast<uint32_t>(BN >> 3) << 17) |
                              (static_cast<uint32_t>((2 * BM) >> 4) << 24);
@@ -288,31 +289,34 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
-        if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < num_k; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
+          if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) {
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t sa = smem_base + stage * STAGE_BYTES;
-          const uint32_t sb = sa + A_BYTES;
+          if (elect_one()) {
+            const uint32_t sa = smem_base + stage * STAGE_BYTES;
+            const uint32_t sb = sa + A_BYTES;
 #pragma unroll
-          for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-            const uint64_t adesc = make_smem_desc(sa + kk * a_step, a_lbo, 1024);
-            const uint64_t bdesc = make_smem_desc(sb + kk * b_step, b_lbo, 1024);
-            umma_bf16_pair(d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
+            for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+              const uint64_t adesc = make_smem_desc(sa + kk * a_step, a_lbo, 1024);
+              const uint64_t bdesc = make_smem_desc(sb + kk * b_step, b_lbo, 1024);
+              umma_bf16_pair(d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
+            }
+            umma_commit_pair(empty_bar(stage));
+            if (kb == num_k - 1) umma_commit_pair(tfull_bar(acc));
           }
-          umma_commit_pair(empty_bar(stage));
+          __syncwarp();
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1u;
           }
         }
         if (!ok) break;
-        umma_commit_pair(tfull_bar(acc));
         if (++acc == 2) {
           acc = 0;
           acc_phase ^= 1u;
