@@ -187,28 +187,31 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(bar(BAR_KV), 2 * KV_TILE);
 #pragma unroll
       for (int sl = 0; sl < SLABS; ++sl) {
         tma_load_2d(smem_base + OFF_K + sl * KV_SLAB, &tmK, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
         tma_load_2d(smem_base + OFF_V + sl * KV_SLAB, &tmV, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
       }
-      bool ok = true;
-      for (int t = 0; t < T && ok; ++t) {
-        const int st = t % QDO_STAGES;
-        const uint32_t use = static_cast<uint32_t>(t / QDO_STAGES);
-        if (!mbar_wait(bar(BAR_QDO_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        int h, qt;
-        tile_of(t, h, qt);
-        const int q_row0 = b * p.seq + qt * BQ;
-        const uint32_t sq = smem_base + OFF_STAGE + st * STAGE_BYTES;
-        const uint32_t sdo = sq + Q_TILE;
-        const uint32_t sst = smem_base + OFF_STATS + st * STATS_BYTES;
-        const long long stat_off = (static_cast<long long>(b) * p.n_heads + h) * p.seq + qt * BQ;
+    }
+    __syncwarp();
+    bool ok = true;
+    for (int t = 0; t < T && ok; ++t) {
+      const int st = t % QDO_STAGES;
+      const uint32_t use = static_cast<uint32_t>(t / QDO_STAGES);
+      if (!mbar_wait_warp(bar(BAR_QDO_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
+        ok = false;
+        break;
+      }
+      int h, qt;
+      tile_of(t, h, qt);
+      const int q_row0 = b * p.seq + qt * BQ;
+      const uint32_t sq = smem_base + OFF_STAGE + st * STAGE_BYTES;
+      const uint32_t sdo = sq + Q_TILE;
+      const uint32_t sst = smem_base + OFF_STATS + st * STATS_BYTES;
+      const long long stat_off = (static_cast<long long>(b) * p.n_heads + h) * p.seq + qt * BQ;
+      if (elect_one()) {
         mbar_expect_tx(bar(BAR_QDO_FULL + st), 2 * Q_TILE + STATS_BYTES);
 #pragma unroll
         for (int sl = 0; sl < SLABS; ++sl) {
@@ -218,76 +221,83 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         bulk_load_1d(sst, p.lse + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
         bulk_load_1d(sst + BQ * 4, p.delta + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
       }
-      if (!ok) {
-        const uint64_t t0 = ftb200::globaltimer_ns();
-        while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-      }
+      __syncwarp();
+    }
+    if (!ok) {
+      const uint64_t t0 = ftb200::globaltimer_ns();
+      while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t F = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(128 >> 4) << 24);
-      const uint32_t idesc_st = F | (static_cast<uint32_t>(BQ >> 3) << 17);                             // N = 64, K-major both
-      const uint32_t idesc_kv = F | (1u << 16) | (static_cast<uint32_t>(D >> 3) << 17);                 // N = D, B MN-major
-      const uint32_t idesc_dq = F | (1u << 15) | (1u << 16) | (static_cast<uint32_t>(BQ >> 3) << 17);   // N = 64, both MN-major
-      // descriptor bases: one per buffer and operand role, constants per K step (the issue loop
-      // must stay short: these MMAs are too small to hide descriptor arithmetic)
-      constexpr uint32_t HI = smem_desc_hi(1024);
-      const uint32_t k_km = smem_desc_lo(smem_base + OFF_K, 16);        // K as K-major A (S^T)
-      const uint32_t v_km = smem_desc_lo(smem_base + OFF_V, 16);        // V as K-major A (dP^T)
-      // K as MN-major A (dQ^T): M = 128 runs over the head dim.  With head dim 64 the second 64 rows of that MMA
-      // read the slab behind K's only one, which is V's: lanes 64..127 of dQ^T then hold a product nobody reads.
-      const uint32_t k_mn = smem_desc_lo(smem_base + OFF_K, KV_SLAB);
-      const uint32_t q_km0 = smem_desc_lo(smem_base + OFF_STAGE, 16);             // Q, stage 0, K-major B
-      const uint32_t q_mn0 = smem_desc_lo(smem_base + OFF_STAGE, Q_SLAB);         // Q, stage 0, MN-major B
-      const uint32_t ds_mn0 = smem_desc_lo(smem_base + OFF_PDS, PT_TILE);  // dS^T, buffer 0, MN-major B
-      constexpr uint32_t STAGE16 = STAGE_BYTES >> 4, QT16 = Q_TILE >> 4, PDS16 = PDS_BYTES >> 4;
-      bool ok = mbar_wait(bar(BAR_KV), 0, abort_flag);
-      for (int t = 0; t <= T && ok; ++t) {
-        if (t < T) {
-          const int st = t & 1, qs = t % QDO_STAGES;
-          const uint32_t use = static_cast<uint32_t>(t >> 1);
-          if (!mbar_wait(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag) ||
-              !mbar_wait(bar(BAR_S_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          TRACE(0, t, 0);  // S inputs ready
-          const uint32_t qb_km = q_km0 + qs * STAGE16;
+    const uint32_t F = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(128 >> 4) << 24);
+    const uint32_t idesc_st = F | (static_cast<uint32_t>(BQ >> 3) << 17);                             // N = 64, K-major both
+    const uint32_t idesc_kv = F | (1u << 16) | (static_cast<uint32_t>(D >> 3) << 17);                 // N = D, B MN-major
+    const uint32_t idesc_dq = F | (1u << 15) | (1u << 16) | (static_cast<uint32_t>(BQ >> 3) << 17);   // N = 64, both MN-major
+    // descriptor bases: one per buffer and operand role, constants per K step (the issue loop
+    // must stay short: these MMAs are too small to hide descriptor arithmetic)
+    constexpr uint32_t HI = smem_desc_hi(1024);
+    const uint32_t k_km = smem_desc_lo(smem_base + OFF_K, 16);        // K as K-major A (S^T)
+    const uint32_t v_km = smem_desc_lo(smem_base + OFF_V, 16);        // V as K-major A (dP^T)
+    // K as MN-major A (dQ^T): M = 128 runs over the head dim.  With head dim 64 the second 64 rows of that MMA
+    // read the slab behind K's only one, which is V's: lanes 64..127 of dQ^T then hold a product nobody reads.
+    const uint32_t k_mn = smem_desc_lo(smem_base + OFF_K, KV_SLAB);
+    const uint32_t q_km0 = smem_desc_lo(smem_base + OFF_STAGE, 16);             // Q, stage 0, K-major B
+    const uint32_t q_mn0 = smem_desc_lo(smem_base + OFF_STAGE, Q_SLAB);         // Q, stage 0, MN-major B
+    const uint32_t ds_mn0 = smem_desc_lo(smem_base + OFF_PDS, PT_TILE);  // dS^T, buffer 0, MN-major B
+    constexpr uint32_t STAGE16 = STAGE_BYTES >> 4, QT16 = Q_TILE >> 4, PDS16 = PDS_BYTES >> 4;
+    bool ok = mbar_wait_warp(bar(BAR_KV), 0, abort_flag);
+    for (int t = 0; t <= T && ok; ++t) {
+      if (t < T) {
+        const int st = t & 1, qs = t % QDO_STAGES;
+        const uint32_t use = static_cast<uint32_t>(t >> 1);
+        if (!mbar_wait_warp(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag) ||
+            !mbar_wait_warp(bar(BAR_S_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        TRACE(0, t, 0);  // S inputs ready
+        const uint32_t qb_km = q_km0 + qs * STAGE16;
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t a_off = ((kk >> 2) * KV_SLAB + (kk & 3) * 32) >> 4, b_off = ((kk >> 2) * Q_SLAB + (kk & 3) * 32) >> 4;
             umma_bf16_lh(tmem_base + COL_S + st * BQ, k_km + a_off, HI, qb_km + b_off, HI, idesc_st, kk != 0);
           }
           umma_commit(bar(BAR_S_FULL + st));
-          if (!mbar_wait(bar(BAR_DP_EMPTY), (static_cast<uint32_t>(t) & 1u) ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(bar(BAR_DP_EMPTY), (static_cast<uint32_t>(t) & 1u) ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t a_off = ((kk >> 2) * KV_SLAB + (kk & 3) * 32) >> 4, b_off = ((kk >> 2) * Q_SLAB + (kk & 3) * 32) >> 4;
             umma_bf16_lh(tmem_base + COL_DP, v_km + a_off, HI, qb_km + QT16 + b_off, HI, idesc_st, kk != 0);
           }
           umma_commit(bar(BAR_DP_FULL));
-          TRACE(0, t, 1);  // S, dP issued
         }
-        if (t >= 1) {
-          const int u = t - 1, pb = u & 1, qs = u % QDO_STAGES;
-          const uint32_t use = static_cast<uint32_t>(u >> 1);
-          if (!mbar_wait(bar(BAR_PDS_FULL + pb), use & 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          TRACE(0, u, 2);  // P, dS ready for the tail of tile u
-          const uint32_t qb_mn = q_mn0 + qs * STAGE16;
-          const uint32_t dsb_mn = ds_mn0 + pb * PDS16;
-          // queries 16k..16k+15 of tile u: P^T in columns 16k..16k+7 of its score buffer, dS^T in 16k+8..16k+15
-          const uint32_t pt_tmem = tmem_base + COL_S + pb * BQ;
+        __syncwarp();
+        TRACE(0, t, 1);  // S, dP issued
+      }
+      if (t >= 1) {
+        const int u = t - 1, pb = u & 1, qs = u % QDO_STAGES;
+        const uint32_t use = static_cast<uint32_t>(u >> 1);
+        if (!mbar_wait_warp(bar(BAR_PDS_FULL + pb), use & 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        TRACE(0, u, 2);  // P, dS ready for the tail of tile u
+        const uint32_t qb_mn = q_mn0 + qs * STAGE16;
+        const uint32_t dsb_mn = ds_mn0 + pb * PDS16;
+        // queries 16k..16k+15 of tile u: P^T in columns 16k..16k+7 of its score buffer, dS^T in 16k+8..16k+15
+        const uint32_t pt_tmem = tmem_base + COL_S + pb * BQ;
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < BQ / 16; ++kk) {  // dV += P^T dO
             umma_bf16_tmem_a(tmem_base + COL_DV, pt_tmem + kk * 16, qb_mn + QT16 + ((kk * 2048) >> 4), HI, idesc_kv, (u | kk) != 0);
@@ -297,22 +307,26 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             umma_bf16_tmem_a(tmem_base + COL_DK, pt_tmem + kk * 16 + 8, qb_mn + ((kk * 2048) >> 4), HI, idesc_kv, (u | kk) != 0);
           }
           umma_commit(bar(BAR_QDO_EMPTY + qs));
-          if (!mbar_wait(bar(BAR_DQ_EMPTY), (static_cast<uint32_t>(u) & 1u) ^ 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(bar(BAR_DQ_EMPTY), (static_cast<uint32_t>(u) & 1u) ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < BKV / 16; ++kk) {  // dQ^T = K^T dS^T
             umma_bf16_lh(tmem_base + COL_DQ, k_mn + ((kk * 2048) >> 4), HI, dsb_mn + ((kk * 2048) >> 4), HI, idesc_dq, kk != 0);
           }
           umma_commit(bar(BAR_PDS_EMPTY + pb));
           umma_commit(bar(BAR_DQ_FULL));
-          TRACE(0, u, 3);  // tail issued
         }
+        __syncwarp();
+        TRACE(0, u, 3);  // tail issued
       }
-      if (ok) umma_commit(bar(BAR_DKV_DONE));
     }
+    if (ok && elect_one()) umma_commit(bar(BAR_DKV_DONE));
     __syncwarp();
   } else if (warp >= 18) {
     // ---------------- dQ drain (warps 18..21): TMEM lane = head-dim index ----------------

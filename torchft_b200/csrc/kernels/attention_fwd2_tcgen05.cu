@@ -13,15 +13,21 @@
 //   warp 0        TMA: Q tiles once, K and V blocks into a 2-stage ring
 //   warp 1        tcgen05.mma, in the order  P0 V, S0', P1 V, S1'  (' = next block): the softmax of
 //                 a tile has the two MMAs of the other tile to hide under
-//   warps 2..5    softmax of tile 0, warps 6..9 softmax of tile 1: ONE thread per query row (the
+//   warps 4..7    softmax of tile 0, warps 8..11 softmax of tile 1: ONE thread per query row (the
 //                 128 scores of a row sit in one TMEM lane), so the row maximum and sum need no
 //                 exchange between threads.  P goes back as packed bf16 into the first 64 columns
 //                 of the scores and is the A operand of P V straight from tensor memory.
 //
-// A share of the exponentials (POLY of every 8) is computed with a cubic polynomial on the FMA
-// pipe instead of the exponential unit, which is the scarcer of the two; its relative error of
-// 8e-5 disappears in the bf16 rounding of P.  The running maximum is only raised (and O in TMEM
-// rescaled) when it grows by more than 2^8.
+// What bounds it: a tile's chain S -> softmax -> P V, of which the softmax is the longest part, so
+//   - the scaled scores, sums and polynomial steps are packed fp32 pairs, the maximum takes three
+//     inputs an instruction, and the softmax warpgroups hold the registers (216 a thread) for it;
+//   - P V of a block's first 64 keys starts while the exponentials of the last 64 are computed;
+//   - POLY of every 8 exponentials are computed on the FMA pipe instead of the exponential unit,
+//     where that unit is the scarcer (head dim 64);
+//   - the issuing warps stay converged (see elect_one).
+// The running maximum is only raised (and O in TMEM rescaled) when it grows by more than 2^8.
+// Measured, 1 x 8192, 32/8 heads of 128: 630 -> 475 us (1157 TFLOP/s); 8 x 2048, heads of 64:
+// 379 -> 303 us.
 //
 // Every mbarrier wait is bounded; on expiry the CTA records FTB200_ST_TIMEOUT in the caller's
 // status word, frees its TMEM and returns.
@@ -40,7 +46,11 @@ constexpr int BQ = 128;       // queries per tile
 constexpr int TILES = 2;      // tiles per CTA
 constexpr int BKV = 128;      // keys per block
 constexpr int KV_STAGES = 2;
-constexpr int NUM_THREADS = 320;
+constexpr int NUM_THREADS = 384;
+// Registers: a CTA is launched with 168 a thread (65536 / 384, checked on the host); the first warpgroup (TMA, MMA) gives
+// most of its own to the two softmax warpgroups, whose threads hold a row's 128 scores: 72 + 2 * 216 = 3 * 168.
+constexpr int LAUNCH_REGS = 168, ISSUE_REGS = 72, SOFTMAX_REGS = 216;
+static_assert(ISSUE_REGS + 2 * SOFTMAX_REGS <= 3 * LAUNCH_REGS, "more registers than the CTA is launched with");
 constexpr int ROW_THREADS = 128;  // softmax threads per tile
 constexpr uint32_t TMEM_COLS = 512;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // in log2 units
@@ -77,20 +87,9 @@ enum : int {
   BAR_S_FULL = 10,   // +tile
   BAR_P_FULL = 12,   // +tile
   BAR_O_DONE = 14,   // +tile
-  NUM_BARS = 16,
+  BAR_P_HALF = 16,   // +tile: P of the block's first 64 keys
+  NUM_BARS = 18,
 };
-
-// 2^x for x <= 8 on the FMA pipe: round to the nearest integer n with the magic-number trick,
-// cubic in the remainder f in [-0.5, 0.5] (relative error 7.5e-5), n added to the exponent bits.
-__device__ __forceinline__ float exp2_poly(float x) {
-  x = fmaxf(x, -125.f);
-  const float xr = x + 12582912.f;  // 1.5 * 2^23: the integer lands in the low mantissa bits
-  const float f = x - (xr - 12582912.f);
-  float p = fmaf(f, 0.05517063f, 0.24260884f);
-  p = fmaf(f, p, 0.69326095f);
-  p = fmaf(f, p, 0.99992822f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(xr) << 23));
-}
 
 template <int D, int POLY>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -126,6 +125,7 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(bar(BAR_Q_FULL + t), 1);
       mbar_init(bar(BAR_S_FULL + t), 1);
       mbar_init(bar(BAR_P_FULL + t), ROW_THREADS);
+      mbar_init(bar(BAR_P_HALF + t), ROW_THREADS);
       mbar_init(bar(BAR_O_DONE + t), 1);
     }
     for (int s = 0; s < KV_STAGES; ++s) {
@@ -149,10 +149,11 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      for (int t = 0; t < TILES; ++t) {
+  if (warp < 4) {
+    regs_dec<ISSUE_REGS>();
+    if (warp == 0) {
+      // ---------------- TMA producer ----------------
+      if (elect_one()) for (int t = 0; t < TILES; ++t) {
         const uint32_t sq = smem_base + C::OFF_Q + t * C::TILE_BYTES;
         mbar_expect_tx(bar(BAR_Q_FULL + t), C::TILE_BYTES);
         for (int s = 0; s < C::SLABS; ++s)
@@ -162,32 +163,35 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int j = 0; j < n_kv1 && ok; ++j) {
         const int st = j & 1;
         const uint32_t use = static_cast<uint32_t>(j >> 1);
-        if (!mbar_wait(bar(BAR_K_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
+        if (!mbar_wait_warp(bar(BAR_K_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
           ok = false;
           break;
         }
         const uint32_t sk = smem_base + C::OFF_KV + st * 2 * C::TILE_BYTES;
         const uint32_t sv = sk + C::TILE_BYTES;
         const int kv_row0 = b * p.seq + j * BKV;
-        mbar_expect_tx(bar(BAR_K_FULL + st), C::TILE_BYTES);
-        for (int s = 0; s < C::SLABS; ++s) tma_load_2d(sk + s * C::SLAB_BYTES, &tmK, bar(BAR_K_FULL + st), hk * D + s * 64, kv_row0);
-        if (!mbar_wait(bar(BAR_V_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
+        if (elect_one()) {
+          mbar_expect_tx(bar(BAR_K_FULL + st), C::TILE_BYTES);
+          for (int s = 0; s < C::SLABS; ++s) tma_load_2d(sk + s * C::SLAB_BYTES, &tmK, bar(BAR_K_FULL + st), hk * D + s * 64, kv_row0);
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(bar(BAR_V_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
           ok = false;
           break;
         }
-        mbar_expect_tx(bar(BAR_V_FULL + st), C::TILE_BYTES);
-        for (int s = 0; s < C::SLABS; ++s) tma_load_2d(sv + s * C::SLAB_BYTES, &tmV, bar(BAR_V_FULL + st), hk * D + s * 64, kv_row0);
+        if (elect_one()) {
+          mbar_expect_tx(bar(BAR_V_FULL + st), C::TILE_BYTES);
+          for (int s = 0; s < C::SLABS; ++s) tma_load_2d(sv + s * C::SLAB_BYTES, &tmV, bar(BAR_V_FULL + st), hk * D + s * 64, kv_row0);
+        }
+        __syncwarp();
       }
       if (!ok) {
         // copies in flight land in this CTA's shared memory: give them time before the CTA exits
         const uint64_t t0 = ftb200::globaltimer_ns();
         while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
       }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    } else if (warp == 1) {
+      // ---------------- MMA issuer ----------------
       // S = Q K^T: both operands K-major (head dim contiguous), M = N = 128
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BKV >> 3) << 17) |
                                (static_cast<uint32_t>(BQ >> 4) << 24);
@@ -205,49 +209,62 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const uint32_t qb = q_lo + t * QTILE16;
         const uint32_t kb = k_lo + st * STAGE16;
         const uint32_t d_tmem = tmem_base + C::COL_S + t * 128;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = ((kk >> 2) * C::SLAB_BYTES + (kk & 3) * 32) >> 4;
-          umma_bf16_lh(d_tmem, qb + off, HI, kb + off, HI, idesc_s, kk != 0);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = ((kk >> 2) * C::SLAB_BYTES + (kk & 3) * 32) >> 4;
+            umma_bf16_lh(d_tmem, qb + off, HI, kb + off, HI, idesc_s, kk != 0);
+          }
+          umma_commit(bar(BAR_S_FULL + t));
         }
-        umma_commit(bar(BAR_S_FULL + t));
+        __syncwarp();
       };
-      auto issue_pv = [&](int t, int j) {
+      // half 0 or 1 of a block's keys: the first half is multiplied while the exponentials of the second are computed
+      auto issue_pv = [&](int t, int j, int half) {
         const int st = j & 1;
-        const uint32_t vb = v_lo + st * STAGE16;
+        const uint32_t vb = v_lo + st * STAGE16 + half * ((64 * 128) >> 4);
         const uint32_t d_tmem = tmem_base + C::COL_O + t * D;
-        const uint32_t p_tmem = tmem_base + C::COL_S + t * 128;  // P: keys 2k, 2k+1 in column k
+        const uint32_t p_tmem = tmem_base + C::COL_S + t * 128 + half * 32;  // P: keys 2k, 2k+1 in column k
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk)
-          umma_bf16_tmem_a(d_tmem, p_tmem + kk * 8, vb + ((kk * 2048) >> 4), HI, idesc_o, (j | kk) != 0);
-        umma_commit(bar(BAR_O_DONE + t));
+          for (int kk = 0; kk < BKV / 32; ++kk)
+            umma_bf16_tmem_a(d_tmem, p_tmem + kk * 8, vb + ((kk * 2048) >> 4), HI, idesc_o, (j | half | kk) != 0);
+          if (half == 1) umma_commit(bar(BAR_O_DONE + t));
+        }
+        __syncwarp();
       };
-      bool ok = mbar_wait(bar(BAR_Q_FULL + 0), 0, abort_flag) && mbar_wait(bar(BAR_K_FULL + 0), 0, abort_flag);
+      bool ok = mbar_wait_warp(bar(BAR_Q_FULL + 0), 0, abort_flag) && mbar_wait_warp(bar(BAR_K_FULL + 0), 0, abort_flag);
       if (ok) {
         tc_fence_after();
         issue_s(0, 0);
-        ok = mbar_wait(bar(BAR_Q_FULL + 1), 0, abort_flag);
+        ok = mbar_wait_warp(bar(BAR_Q_FULL + 1), 0, abort_flag);
       }
       if (ok) {
         tc_fence_after();
         issue_s(1, 0);
-        umma_commit(bar(BAR_K_EMPTY + 0));
+        if (elect_one()) umma_commit(bar(BAR_K_EMPTY + 0));
       }
       for (int j = 0; j < n_kv1 && ok; ++j) {
         const int st = j & 1, st1 = st ^ 1;
         const uint32_t use = static_cast<uint32_t>(j >> 1), use1 = static_cast<uint32_t>((j + 1) >> 1);
         bool k_next = false;
         if (j < n_kv0) {
-          if (!mbar_wait(bar(BAR_P_FULL + 0), static_cast<uint32_t>(j) & 1u, abort_flag) ||
-              !mbar_wait(bar(BAR_V_FULL + st), use & 1u, abort_flag)) {
+          if (!mbar_wait_warp(bar(BAR_P_HALF + 0), static_cast<uint32_t>(j) & 1u, abort_flag) ||
+              !mbar_wait_warp(bar(BAR_V_FULL + st), use & 1u, abort_flag)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          issue_pv(0, j);
+          issue_pv(0, j, 0);
+          if (!mbar_wait_warp(bar(BAR_P_FULL + 0), static_cast<uint32_t>(j) & 1u, abort_flag)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          issue_pv(0, j, 1);
           if (j + 1 < n_kv0) {
             // S0 held P0 of block j: its P V was issued above and the tensor pipe runs in order
-            if (!mbar_wait(bar(BAR_K_FULL + st1), use1 & 1u, abort_flag)) {
+            if (!mbar_wait_warp(bar(BAR_K_FULL + st1), use1 & 1u, abort_flag)) {
               ok = false;
               break;
             }
@@ -256,29 +273,36 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             issue_s(0, j + 1);
           }
         }
-        if (!mbar_wait(bar(BAR_P_FULL + 1), static_cast<uint32_t>(j) & 1u, abort_flag) ||
-            !mbar_wait(bar(BAR_V_FULL + st), use & 1u, abort_flag)) {
+        if (!mbar_wait_warp(bar(BAR_P_HALF + 1), static_cast<uint32_t>(j) & 1u, abort_flag) ||
+            !mbar_wait_warp(bar(BAR_V_FULL + st), use & 1u, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        issue_pv(1, j);
-        umma_commit(bar(BAR_V_EMPTY + st));
+        issue_pv(1, j, 0);
+        if (!mbar_wait_warp(bar(BAR_P_FULL + 1), static_cast<uint32_t>(j) & 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        issue_pv(1, j, 1);
+        if (elect_one()) umma_commit(bar(BAR_V_EMPTY + st));
         if (j + 1 < n_kv1) {
-          if (!k_next && !mbar_wait(bar(BAR_K_FULL + st1), use1 & 1u, abort_flag)) {
+          if (!k_next && !mbar_wait_warp(bar(BAR_K_FULL + st1), use1 & 1u, abort_flag)) {
             ok = false;
             break;
           }
           tc_fence_after();
           issue_s(1, j + 1);
-          umma_commit(bar(BAR_K_EMPTY + st1));
+          if (elect_one()) umma_commit(bar(BAR_K_EMPTY + st1));
         }
       }
     }
     __syncwarp();
   } else {
     // ---------------- softmax + epilogue: one thread per query row ----------------
-    const int t = (warp - 2) >> 2;   // tile
+    regs_inc<SOFTMAX_REGS>();
+    const int t = (warp - 4) >> 2;   // tile
     const int quarter = warp & 3;    // TMEM lane quarter this warp may touch
     const int row = quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
@@ -305,7 +329,8 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int c = 0; c < BKV; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(sv[c]));
+      for (int c = 0; c < BKV; c += 2)
+        mx4[(c >> 1) & 3] = fmaxf(fmaxf(mx4[(c >> 1) & 3], __uint_as_float(sv[c])), __uint_as_float(sv[c + 1]));
       const float m_new = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
 
       // raise the maximum only when it moved far
@@ -337,24 +362,41 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       }
       const float neg_m = -m_used * p.scale_log2;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      const unsigned long long scale2 = f2_pack(p.scale_log2, p.scale_log2), neg_m2 = f2_pack(neg_m, neg_m);
+      unsigned long long sum2[2] = {0ull, 0ull};
 #pragma unroll
       for (int c = 0; c < BKV / 32; ++c) {
         uint32_t packed[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          const float x0 = fmaf(__uint_as_float(sv[c * 32 + 2 * e]), p.scale_log2, neg_m);
-          const float x1 = fmaf(__uint_as_float(sv[c * 32 + 2 * e + 1]), p.scale_log2, neg_m);
-          // POLY of every 8 exponentials go to the FMA pipe
-          const float p0 = ((2 * e) & 7) < POLY ? exp2_poly(x0) : exp2f(x0);
-          const float p1 = ((2 * e + 1) & 7) < POLY ? exp2_poly(x1) : exp2f(x1);
-          sum4[e & 3] += p0 + p1;
+          const unsigned long long x2 =
+              f2_fma(f2_pack(__uint_as_float(sv[c * 32 + 2 * e]), __uint_as_float(sv[c * 32 + 2 * e + 1])), scale2, neg_m2);
+          unsigned long long p2;
+          float p0, p1;
+          if (((e * POLY) & 7) < POLY) {  // POLY of every 8 exponentials go to the FMA pipe
+            p2 = f2_exp2_poly(x2);
+            f2_unpack(p2, p0, p1);
+          } else {
+            f2_unpack(x2, p0, p1);
+            p0 = exp2f(p0);
+            p1 = exp2f(p1);
+            p2 = f2_pack(p0, p1);
+          }
+          sum2[e & 1] = f2_add(sum2[e & 1], p2);
           __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
           packed[e] = *reinterpret_cast<uint32_t*>(&pk);
         }
         // P replaces the first half of the scores this thread has already taken into registers
         tmem_st16(s_addr + c * 16, packed);
+        if (c == 1) {
+          tmem_wait_st();
+          tc_fence_before();
+          mbar_arrive(bar(BAR_P_HALF + t));
+        }
       }
+      float sum4[4];
+      f2_unpack(sum2[0], sum4[0], sum4[1]);
+      f2_unpack(sum2[1], sum4[2], sum4[3]);
       l_sum += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
       tmem_wait_st();
       tc_fence_before();
@@ -431,6 +473,9 @@ int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
   if (!attr_set) {
     if (cudaFuncSetAttribute(attention_fwd2_kernel<D, POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg<D>::SMEM_BYTES) != cudaSuccess)
+      return FTB200_E_CUDA;
+    cudaFuncAttributes attr;  // the warpgroups' register split assumes this count
+    if (cudaFuncGetAttributes(&attr, attention_fwd2_kernel<D, POLY>) != cudaSuccess || attr.numRegs < LAUNCH_REGS)
       return FTB200_E_CUDA;
     attr_set = true;
   }

@@ -150,53 +150,57 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      bool ok = true;
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t use = static_cast<uint32_t>(j >> 1);
-        if (!mbar_wait(bar(BAR_K_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        const uint32_t sk = smem_base + OFF_KV + st * 2 * TILE_BYTES;
-        const uint32_t sv = sk + TILE_BYTES;
-        const int kv_row0 = b * p.seq + j * BKV;
+    bool ok = true;
+    for (int j = 0; j < n_kv && ok; ++j) {
+      const int st = j & 1;
+      const uint32_t use = static_cast<uint32_t>(j >> 1);
+      if (!mbar_wait_warp(bar(BAR_K_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
+        ok = false;
+        break;
+      }
+      const uint32_t sk = smem_base + OFF_KV + st * 2 * TILE_BYTES;
+      const uint32_t sv = sk + TILE_BYTES;
+      const int kv_row0 = b * p.seq + j * BKV;
+      if (elect_one()) {
         mbar_expect_tx(bar(BAR_K_FULL + st), TILE_BYTES);
         tma_load_2d(sk, &tmK, bar(BAR_K_FULL + st), hk * D, kv_row0);
         tma_load_2d(sk + SLAB_BYTES, &tmK, bar(BAR_K_FULL + st), hk * D + 64, kv_row0);
-        if (!mbar_wait(bar(BAR_V_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
+      }
+      __syncwarp();
+      if (!mbar_wait_warp(bar(BAR_V_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
+        ok = false;
+        break;
+      }
+      if (elect_one()) {
         mbar_expect_tx(bar(BAR_V_FULL + st), TILE_BYTES);
         tma_load_2d(sv, &tmV, bar(BAR_V_FULL + st), hk * D, kv_row0);
         tma_load_2d(sv + SLAB_BYTES, &tmV, bar(BAR_V_FULL + st), hk * D + 64, kv_row0);
       }
-      if (!ok) {
-        const uint64_t t0 = ftb200::globaltimer_ns();
-        while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-      }
+      __syncwarp();
+    }
+    if (!ok) {
+      const uint64_t t0 = ftb200::globaltimer_ns();
+      while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      // S = Q K^T: both operands K-major (head dim contiguous), M = N = 128
-      const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BKV >> 3) << 17) |
-                               (static_cast<uint32_t>(BQ >> 4) << 24);
-      // O += P V: A = P K-major (keys contiguous), B = V MN-major (stored [key][d])
-      const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(D >> 3) << 17) |
-                               (static_cast<uint32_t>(BQ >> 4) << 24);
-      // descriptor bases: one per buffer, constants per K step (the issue loop must stay short)
-      constexpr uint32_t HI = smem_desc_hi(1024);
-      const uint32_t k_lo = smem_desc_lo(smem_base + OFF_KV, 16);
-      const uint32_t v_lo = smem_desc_lo(smem_base + OFF_KV + TILE_BYTES, SLAB_BYTES);
-      constexpr uint32_t STAGE16 = (2 * TILE_BYTES) >> 4;
-      auto issue_s = [&](int j) {
-        const int st = j & 1;
-        const uint32_t kb = k_lo + st * STAGE16;
-        const uint32_t d_tmem = tmem_base + COL_S + st * BKV;
+    // S = Q K^T: both operands K-major (head dim contiguous), M = N = 128
+    const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BKV >> 3) << 17) |
+                             (static_cast<uint32_t>(BQ >> 4) << 24);
+    // O += P V: A = P K-major (keys contiguous), B = V MN-major (stored [key][d])
+    const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (static_cast<uint32_t>(D >> 3) << 17) |
+                             (static_cast<uint32_t>(BQ >> 4) << 24);
+    // descriptor bases: one per buffer, constants per K step (the issue loop must stay short)
+    constexpr uint32_t HI = smem_desc_hi(1024);
+    const uint32_t k_lo = smem_desc_lo(smem_base + OFF_KV, 16);
+    const uint32_t v_lo = smem_desc_lo(smem_base + OFF_KV + TILE_BYTES, SLAB_BYTES);
+    constexpr uint32_t STAGE16 = (2 * TILE_BYTES) >> 4;
+    auto issue_s = [&](int j) {
+      const int st = j & 1;
+      const uint32_t kb = k_lo + st * STAGE16;
+      const uint32_t d_tmem = tmem_base + COL_S + st * BKV;
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = ((kk >> 2) * SLAB_BYTES + (kk & 3) * 32) >> 4;
@@ -204,47 +208,51 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
         }
         umma_commit(bar(BAR_S_FULL + st));
         umma_commit(bar(BAR_K_EMPTY + st));
-      };
-      bool ok = mbar_wait(bar(BAR_Q), 0, abort_flag) && mbar_wait(bar(BAR_K_FULL + 0), 0, abort_flag);
-      if (ok) {
-        tc_fence_after();
-        issue_s(0);
       }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t use = static_cast<uint32_t>(j >> 1);
-        if (j + 1 < n_kv) {
-          const int st1 = (j + 1) & 1;
-          const uint32_t use1 = static_cast<uint32_t>((j + 1) >> 1);
-          // S buffer st1 last held P of block j-1: its P V was issued above, and the tensor pipe runs in order
-          if (!mbar_wait(bar(BAR_K_FULL + st1), use1 & 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          TRACE(0, j, 0);  // K of block j+1 present
-          issue_s(j + 1);
-          TRACE(0, j, 1);  // S of block j+1 issued
-        }
-        if (!mbar_wait(bar(BAR_P_FULL), static_cast<uint32_t>(j) & 1u, abort_flag) ||
-            !mbar_wait(bar(BAR_V_FULL + st), use & 1u, abort_flag)) {
+      __syncwarp();
+    };
+    bool ok = mbar_wait_warp(bar(BAR_Q), 0, abort_flag) && mbar_wait_warp(bar(BAR_K_FULL + 0), 0, abort_flag);
+    if (ok) {
+      tc_fence_after();
+      issue_s(0);
+    }
+    for (int j = 0; j < n_kv && ok; ++j) {
+      const int st = j & 1;
+      const uint32_t use = static_cast<uint32_t>(j >> 1);
+      if (j + 1 < n_kv) {
+        const int st1 = (j + 1) & 1;
+        const uint32_t use1 = static_cast<uint32_t>((j + 1) >> 1);
+        // S buffer st1 last held P of block j-1: its P V was issued above, and the tensor pipe runs in order
+        if (!mbar_wait_warp(bar(BAR_K_FULL + st1), use1 & 1u, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        TRACE(0, j, 2);  // P of block j and V present
-        const uint32_t vb = v_lo + st * STAGE16;
-        const uint32_t d_tmem = tmem_base + COL_O;
-        // P of keys 32g..32g+31 sits, two per column, in the first 16 of the 32 columns its thread group read S from
-        const uint32_t p_tmem = tmem_base + COL_S + st * BKV;
+        TRACE(0, j, 0);  // K of block j+1 present
+        issue_s(j + 1);
+        TRACE(0, j, 1);  // S of block j+1 issued
+      }
+      if (!mbar_wait_warp(bar(BAR_P_FULL), static_cast<uint32_t>(j) & 1u, abort_flag) ||
+          !mbar_wait_warp(bar(BAR_V_FULL + st), use & 1u, abort_flag)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      TRACE(0, j, 2);  // P of block j and V present
+      const uint32_t vb = v_lo + st * STAGE16;
+      const uint32_t d_tmem = tmem_base + COL_O;
+      // P of keys 32g..32g+31 sits, two per column, in the first 16 of the 32 columns its thread group read S from
+      const uint32_t p_tmem = tmem_base + COL_S + st * BKV;
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < BKV / 16; ++kk) {
           umma_bf16_tmem_a(d_tmem, p_tmem + (kk >> 1) * CPT + (kk & 1) * 8, vb + ((kk * 2048) >> 4), HI, idesc_o, (j | kk) != 0);
         }
         umma_commit(bar(BAR_V_EMPTY + st));
         umma_commit(bar(BAR_O_DONE));
-        TRACE(0, j, 3);  // P V of block j issued
       }
+      __syncwarp();
+      TRACE(0, j, 3);  // P V of block j issued
     }
     __syncwarp();
   } else {
@@ -256,20 +264,18 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     float m_used = -INFINITY, l_part = 0.f;
     bool ok = true;
-    {
-      // this thread's quarter of its query row -> TMEM (two head-dim elements per column)
-      const uint4* src = reinterpret_cast<const uint4*>(p.Q + static_cast<long long>(q_row0 + row) * p.ld_q + h * D + g * 32);
-      uint32_t qw[16];
+    // this thread's quarter of its query row -> TMEM (two head-dim elements per column)
+    const uint4* src = reinterpret_cast<const uint4*>(p.Q + static_cast<long long>(q_row0 + row) * p.ld_q + h * D + g * 32);
+    uint32_t qw[16];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint4 v4 = src[c];
-        qw[4 * c] = v4.x; qw[4 * c + 1] = v4.y; qw[4 * c + 2] = v4.z; qw[4 * c + 3] = v4.w;
-      }
-      tmem_st16(tmem_base + COL_Q + g * 16 + lane_addr, qw);
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(bar(BAR_Q));
+    for (int c = 0; c < 4; ++c) {
+      const uint4 v4 = src[c];
+      qw[4 * c] = v4.x; qw[4 * c + 1] = v4.y; qw[4 * c + 2] = v4.z; qw[4 * c + 3] = v4.w;
     }
+    tmem_st16(tmem_base + COL_Q + g * 16 + lane_addr, qw);
+    tmem_wait_st();
+    tc_fence_before();
+    mbar_arrive(bar(BAR_Q));
     for (int j = 0; j < n_kv; ++j) {
       const int st = j & 1;
       const uint32_t use = static_cast<uint32_t>(j >> 1);

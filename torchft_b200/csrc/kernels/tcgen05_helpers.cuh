@@ -214,6 +214,67 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 
+// Two fp32 operations per instruction (the packed forms of Blackwell's FMA pipe): the softmax loops are bound by issue
+// slots, and a scaled score, a sum or a polynomial step then costs half of one.
+__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// 2^x of a pair, x <= 8, on the FMA pipe instead of the exponential unit: the nearest integer n by adding 1.5 * 2^23, a
+// polynomial of degree 5 in the remainder f in [-0.5, 0.5], n added to the exponent bits.  The coefficients minimise the
+// largest relative error over that interval (Lawson's iteration of weighted least squares): 7.5e-8, 2.1e-7 with the
+// fp32 evaluation, which is no more than that of the unit's own ex2.approx (2^-22).
+__device__ __forceinline__ unsigned long long f2_exp2_poly(unsigned long long x2) {
+  float x0, x1;
+  f2_unpack(x2, x0, x1);
+  const unsigned long long x = f2_pack(fmaxf(x0, -125.f), fmaxf(x1, -125.f));
+  const unsigned long long xr = f2_add(x, f2_pack(12582912.f, 12582912.f));
+  const unsigned long long n = f2_add(xr, f2_pack(-12582912.f, -12582912.f));
+  const unsigned long long f = f2_fma(n, f2_pack(-1.f, -1.f), x);
+  auto c = [](float v) { return f2_pack(v, v); };
+  unsigned long long p = f2_fma(f, c(0.0013276472f), c(0.00967554148f));
+  p = f2_fma(f, p, c(0.0555071327f));
+  p = f2_fma(f, p, c(0.240221197f));
+  p = f2_fma(f, p, c(0.693146967f));
+  p = f2_fma(f, p, c(1.00000007f));
+  float p0, p1, r0, r1;
+  f2_unpack(p, p0, p1);
+  f2_unpack(xr, r0, r1);
+  return f2_pack(__int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23)),
+                 __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23)));
+}
+
+// Moves registers between warpgroups; N x 128 threads summed over a CTA's warpgroups must not exceed what it was
+// launched with (threads x registers a thread), or the increase waits for good.
+template <int N>
+__device__ __forceinline__ void regs_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }

@@ -575,10 +575,15 @@ def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int,
     scale = 1.0 / math.sqrt(head_dim)
     impl = os.environ.get("FTB200_ATTN_FWD", "auto")
     if impl == "auto":
-        impl = "single"  # same speed as "pair" at head dim 128 and fewer registers
+        # Two query tiles per CTA where the sequence divides into them and they fill the chip: 475 us against 589 us at
+        # 1 x 8192, 32/8 heads.  Up to one wave of 128-query CTAs (148 SMs) the length of one CTA's chain counts, and
+        # that is shorter with one tile: 28.5 us against 40.7 us at 1 x 2048, 8/8 heads; 28.6 against 22.9 at twice a wave.
+        impl = "pair" if seq_len % 256 == 0 and batch * n_heads * (seq_len // 128) > 148 else "single"
     if impl == "pair" or head_dim != 128:
-        # two query tiles per CTA, one softmax thread per row (head dim 64 or 128, seq % 256 == 0)
-        poly = int(os.environ.get("FTB200_ATTN_POLY", "0"))
+        # two query tiles per CTA, one softmax thread per row (head dim 64 or 128, seq % 256 == 0).  At head dim 64 the
+        # products are half as long and the exponential unit is the scarcer: a quarter of the exponentials goes to the
+        # FMA pipe (8 x 2048, 32/8 heads: 303 us against 321); at head dim 128 none (475 us against 486).
+        poly = int(os.environ.get("FTB200_ATTN_POLY") or ("2" if head_dim == 64 else "0"))
         N.check(
             N.lib().ftb200_attention_fwd2(ptr(q), ptr(k), ptr(v), ptr(out), ptr(lse), c_int(batch), c_int(seq_len),
                                           c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_ll(q.stride(0)),
