@@ -198,6 +198,38 @@ def test_kernels_match_reference_gpu(dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("numels", [
+    [1], [128], [127, 1, 0, 129], [16] * 7, [5, 7, 11, 13, 4096, 3], [1] * 300,   # more tensors than one launch takes
+    [128 * 1000 + 8, 64, 128 * 333], [100_003, 128 * 517, 40],
+])
+def test_list_kernels_match_flat_kernels_gpu(numels, dtype):
+    """The list kernels give, bit for bit, what packing into a flat tensor and the flat kernels give, whatever the
+    tensors' sizes, alignments and strides."""
+    world = 3
+    ts = [with_outliers(k, i).to(dtype).cuda() if k else torch.empty(0, dtype=dtype, device="cuda") for i, k in enumerate(numels)]
+    ts.append(torch.randn(64, 48, device="cuda").to(dtype).t())           # not contiguous
+    ts.append(torch.randn(1000, device="cuda").to(dtype)[1:])             # not on a 16-byte boundary
+    n = Q.padded_numel(sum(t.numel() for t in ts), world)
+    flat = torch.zeros(n, dtype=dtype, device="cuda")
+    flat[: sum(t.numel() for t in ts)] = torch.cat([t.reshape(-1) for t in ts])
+    want = torch.empty(Q.quantized_nbytes(n), dtype=torch.uint8, device="cuda")
+    Q.quantize_into(flat, want)
+    buf, (got_n,) = Q.fused_quantize_into_fp8(ts, world)
+    assert got_n == n and torch.equal(buf, want)
+    Q.dequantize_from(want, flat)
+    versions = [t._version for t in ts]
+    for t in ts:
+        t.fill_(float("nan"))
+    Q.fused_dequantize_from_fp8(ts, buf, world)
+    assert torch.equal(torch.cat([t.reshape(-1) for t in ts]), flat[: sum(t.numel() for t in ts)])
+    assert all(t._version > v for t, v in zip(ts, versions))
+    leaf = torch.zeros(256, dtype=dtype, device="cuda", requires_grad=True)
+    with pytest.raises(RuntimeError):  # as any write in place to a leaf
+        Q.fused_dequantize_from_fp8([leaf], Q.fused_quantize_into_fp8([leaf], world)[0], world)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("world", [2, 4, 8])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_fused_allreduce_fp8_emulated(world, dtype):

@@ -163,6 +163,205 @@ __global__ void dequantize_kernel(const uint4* __restrict__ codes, const float* 
   }
 }
 
+// ---- lists of tensors -------------------------------------------------------------------------------------------
+//
+// A list is quantised from, and dequantised into, the tensors where they are: the buffer's elements are those of the
+// tensors one after the other, zeros behind the last.  Packing the list into a flat tensor first (zero-fill, one copy
+// per tensor, quantise, and the way back) moved 3.9 GB for 243 M bf16 elements and 1028 us; read and written once they
+// are 1.47 GB.  Memory-bound: a block that lies in one tensor on a 16-byte boundary is read and written 16 bytes a lane,
+// lane after lane, several blocks in flight; in any other block the lanes take its elements in turn.
+constexpr int LIST_MAX = 128;  // tensors per launch; at least one block's worth of elements, so every launch advances
+
+struct TensorList {
+  void* data[LIST_MAX];
+  long long begin[LIST_MAX + 1];  // element of the buffer where each tensor begins; begin[count]: end of the last
+  int count;
+  long long blk_lo, blk_hi;  // blocks of the buffer that this launch handles
+};
+
+// The tensor that holds element `e` (begin[0] <= e < begin[count]); no tensor of the list is empty.
+__device__ __forceinline__ int list_find(const TensorList& l, long long e) {
+  int lo = 0, hi = l.count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (l.begin[mid] <= e)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  return lo;
+}
+
+template <typename T>
+__device__ __forceinline__ T* list_at(const TensorList& l, int t, long long e) {
+  return reinterpret_cast<T*>(l.data[t]) + (e - l.begin[t]);
+}
+
+// Whether the block that begins at element `e` lies in tensor `t` and starts on a 16-byte boundary there.
+template <typename T>
+__device__ __forceinline__ bool list_whole(const TensorList& l, int t, long long e) {
+  return e + QB <= l.begin[t + 1] && (reinterpret_cast<uintptr_t>(list_at<T>(l, t, e)) & 15) == 0;
+}
+
+// A lane's share of a block is read and written 16 bytes at a time, lane after lane: piece k of lane `sub` begins at
+// element (8 k + sub) * LV of the block.
+template <typename T>
+constexpr int LV = 16 / static_cast<int>(sizeof(T));
+
+__device__ __forceinline__ void load_piece(const float* p, float* f) { load4<float>(p, f); }
+__device__ __forceinline__ void load_piece(const __nv_bfloat16* p, float* f) {
+  ftb200::unpack8(*reinterpret_cast<const ftb200::bf16x8*>(p), f);
+}
+__device__ __forceinline__ void store_piece(float* p, const float* f) { store4<float>(p, f); }
+__device__ __forceinline__ void store_piece(__nv_bfloat16* p, const float* f) {
+  *reinterpret_cast<ftb200::bf16x8*>(p) = ftb200::pack8(f);
+}
+// A piece's codes: LV bytes.
+template <typename T>
+struct PieceCodes;
+template <>
+struct PieceCodes<float> {
+  using type = uint32_t;
+  static __device__ __forceinline__ uint32_t get(const uint32_t* w) { return w[0]; }
+  static __device__ __forceinline__ void put(uint32_t v, uint32_t* w) { w[0] = v; }
+};
+template <>
+struct PieceCodes<__nv_bfloat16> {
+  using type = uint2;
+  static __device__ __forceinline__ uint2 get(const uint32_t* w) { return make_uint2(w[0], w[1]); }
+  static __device__ __forceinline__ void put(uint2 v, uint32_t* w) { w[0] = v.x; w[1] = v.y; }
+};
+__device__ __forceinline__ float to_f32(float v) { return v; }
+__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
+__device__ __forceinline__ void from_f32(float* p, float v) { *p = v; }
+__device__ __forceinline__ void from_f32(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
+
+template <typename T, int GROUPS>
+__global__ void __launch_bounds__(256) quantize_list_kernel(const __grid_constant__ TensorList l, uint8_t* __restrict__ codes,
+                                                            float* __restrict__ scales) {
+  using PC = PieceCodes<T>;
+  constexpr int V = LV<T>, NP = EPL / V;
+  const int lane = threadIdx.x & 31, sub = lane & (LPB - 1), bw = lane / LPB;
+  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  const long long end = l.begin[l.count];
+  int t = -1;  // tensor of the block's first element: blocks only move forward
+  for (long long blk0 = l.blk_lo + warp * (BPW * GROUPS); blk0 < l.blk_hi; blk0 += nwarps * (BPW * GROUPS)) {
+    float f[GROUPS][EPL];
+    bool whole[GROUPS];
+#pragma unroll
+    for (int u = 0; u < GROUPS; ++u) {
+      const long long blk = blk0 + u * BPW + bw, e0 = blk * QB;
+      const bool live = blk < l.blk_hi && e0 < end;
+      if (live) {
+        if (t < 0) t = list_find(l, e0);
+        while (e0 >= l.begin[t + 1]) ++t;
+      }
+      whole[u] = live && list_whole<T>(l, t, e0);
+      if (whole[u]) {
+        const T* src = list_at<T>(l, t, e0);
+#pragma unroll
+        for (int k = 0; k < NP; ++k) load_piece(src + (k * LPB + sub) * V, f[u] + k * V);
+      } else {
+        // element i of this lane is e0 + 8 i + sub
+        int s = live ? t : 0;
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) {
+          const long long x = e0 + i * LPB + sub;
+          f[u][i] = 0.f;
+          if (live && x < end) {
+            while (x >= l.begin[s + 1]) ++s;
+            f[u][i] = to_f32(*list_at<T>(l, s, x));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < GROUPS; ++u) {
+      const long long blk = blk0 + u * BPW + bw;
+      const float amax = group8_max(absmax16(f[u]));
+      if (blk < l.blk_hi) {
+        const float scale = amax > 0.f ? amax / FP8_MAX : 1.f;
+        const uint4 q = encode16(f[u], 1.f / scale);
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        uint8_t* dst = codes + blk * QB;
+        if (whole[u]) {
+#pragma unroll
+          for (int k = 0; k < NP; ++k)
+            *reinterpret_cast<typename PC::type*>(dst + (k * LPB + sub) * V) = PC::get(w + k * V / 4);
+        } else {
+#pragma unroll
+          for (int i = 0; i < EPL; ++i) dst[i * LPB + sub] = static_cast<uint8_t>(w[i >> 2] >> (8 * (i & 3)));
+        }
+        if (sub == 0) scales[blk] = scale;
+      }
+    }
+  }
+}
+
+template <typename T, int GROUPS>
+__global__ void __launch_bounds__(256) dequantize_list_kernel(const __grid_constant__ TensorList l,
+                                                              const uint8_t* __restrict__ codes,
+                                                              const float* __restrict__ scales) {
+  using PC = PieceCodes<T>;
+  constexpr int V = LV<T>, NP = EPL / V;
+  const int lane = threadIdx.x & 31, sub = lane & (LPB - 1), bw = lane / LPB;
+  const long long warp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const long long nwarps = (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
+  const long long end = l.begin[l.count];
+  int t = -1;
+  for (long long blk0 = l.blk_lo + warp * (BPW * GROUPS); blk0 < l.blk_hi; blk0 += nwarps * (BPW * GROUPS)) {
+    typename PC::type q[GROUPS][NP];
+    float sc[GROUPS];
+#pragma unroll
+    for (int u = 0; u < GROUPS; ++u) {
+      const long long blk = blk0 + u * BPW + bw;
+      if (blk < l.blk_hi) {
+#pragma unroll
+        for (int k = 0; k < NP; ++k)
+          q[u][k] = *reinterpret_cast<const typename PC::type*>(codes + blk * QB + (k * LPB + sub) * V);
+        sc[u] = scales[blk];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < GROUPS; ++u) {
+      const long long blk = blk0 + u * BPW + bw, e0 = blk * QB;
+      if (blk >= l.blk_hi || e0 >= end) continue;
+      if (t < 0) t = list_find(l, e0);
+      while (e0 >= l.begin[t + 1]) ++t;
+      if (list_whole<T>(l, t, e0)) {
+        T* dst = list_at<T>(l, t, e0);
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+          uint32_t w[V / 4];
+          float f[V];
+          PC::put(q[u][k], w);
+#pragma unroll
+          for (int i = 0; i < V / 4; ++i) decode4(w[i], sc[u], f + 4 * i);
+          store_piece(dst + (k * LPB + sub) * V, f);
+        }
+      } else {
+        int s = t;
+        const uint8_t* c = codes + e0 + sub;
+#pragma unroll
+        for (int i = 0; i < EPL; i += 4) {
+          float f[4];
+          decode4(c[i * LPB] | (c[(i + 1) * LPB] << 8) | (c[(i + 2) * LPB] << 16) | (static_cast<uint32_t>(c[(i + 3) * LPB]) << 24),
+                  sc[u], f);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const long long x = e0 + (i + k) * LPB + sub;
+            if (x < end) {
+              while (x >= l.begin[s + 1]) ++s;
+              from_f32(list_at<T>(l, s, x), f[k]);
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
 struct QuantAllreduceArgs {
   uint8_t* arena[MAX_RANKS];  // every rank's quantised buffer: [n codes][n/128 scales]
   const void* in_a;           // local input (or the "global" operand of a pseudo-gradient)
@@ -366,6 +565,79 @@ FTB200_API int ftb200_dequantize_fp8(const void* codes, const float* scales, voi
   else
     dequantize_kernel<float><<<grid_for_blocks(nb), 512, 0, st>>>((const uint4*)codes, scales, (float*)out, nb);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+}
+
+namespace {
+
+// Cuts a list of tensors (data[i], numel[i] elements, empty ones allowed) into launches of at most LIST_MAX tensors and
+// whole blocks of the buffer's n elements, and calls launch(list) for each.  The blocks behind the last tensor belong
+// to the last launch.
+template <typename F>
+int for_list(void* const* data, const long long* numel, int count, long long n, F launch) {
+  if (n <= 0 || n % QB || count < 0) return FTB200_E_ALIGN;
+  long long total = 0;
+  for (int i = 0; i < count; ++i) {
+    if (numel[i] < 0 || (numel[i] > 0 && data[i] == nullptr)) return FTB200_E_BADARG;
+    total += numel[i];
+  }
+  if (total <= 0 || total > n) return FTB200_E_BADARG;
+  int first = 0;            // tensor that holds the first element of the next launch
+  long long first_off = 0;  // where it begins in the buffer
+  TensorList l;
+  for (long long blk = 0; blk < n / QB;) {
+    l.count = 0;
+    long long off = first_off;
+    int i = first;
+    for (; i < count && l.count < LIST_MAX; ++i) {
+      if (numel[i] == 0) continue;
+      l.data[l.count] = data[i];
+      l.begin[l.count++] = off;
+      off += numel[i];
+    }
+    l.begin[l.count] = off;
+    l.blk_lo = blk;
+    l.blk_hi = off == total ? n / QB : off / QB;
+    launch(l);
+    if (cudaGetLastError() != cudaSuccess) return FTB200_E_CUDA;
+    blk = l.blk_hi;
+    while (first < count && first_off + numel[first] <= blk * QB) first_off += numel[first++];
+  }
+  return 0;
+}
+
+// Block groups in flight per warp.  Quantising keeps 16 floats a lane for each: two groups 5130 GB/s for bf16, four 4029.
+constexpr int QUANT_GROUPS = 2;
+constexpr int DEQUANT_GROUPS = 4;
+
+int grid_for_list(const TensorList& l, int groups) {
+  const long long per_cta = 8LL * BPW * groups;  // 8 warps, each BPW * groups blocks at a time
+  const long long g = (l.blk_hi - l.blk_lo + per_cta - 1) / per_cta;
+  return static_cast<int>(std::max<long long>(1, std::min<long long>(g, ftb200::sm_count() * 8LL)));
+}
+
+}  // namespace
+
+// Quantises count tensors (contiguous, numel[i] elements of the type) as one buffer of n elements, zeros behind them.
+FTB200_API int ftb200_quantize_list_fp8(void* const* data, const long long* numel, int count, void* codes, float* scales,
+                                        long long n, int dtype, cudaStream_t st) {
+  return for_list(data, numel, count, n, [&](const TensorList& l) {
+    const int grid = grid_for_list(l, QUANT_GROUPS);
+    if (dtype == 0)
+      quantize_list_kernel<__nv_bfloat16, QUANT_GROUPS><<<grid, 256, 0, st>>>(l, (uint8_t*)codes, scales);
+    else
+      quantize_list_kernel<float, QUANT_GROUPS><<<grid, 256, 0, st>>>(l, (uint8_t*)codes, scales);
+  });
+}
+
+FTB200_API int ftb200_dequantize_list_fp8(void* const* data, const long long* numel, int count, const void* codes,
+                                          const float* scales, long long n, int dtype, cudaStream_t st) {
+  return for_list(data, numel, count, n, [&](const TensorList& l) {
+    const int grid = grid_for_list(l, DEQUANT_GROUPS);
+    if (dtype == 0)
+      dequantize_list_kernel<__nv_bfloat16, DEQUANT_GROUPS><<<grid, 256, 0, st>>>(l, (const uint8_t*)codes, scales);
+    else
+      dequantize_list_kernel<float, DEQUANT_GROUPS><<<grid, 256, 0, st>>>(l, (const uint8_t*)codes, scales);
+  });
 }
 
 // arena[i]: rank i's quantised buffer (n + n/128*4 bytes, 16-byte aligned) inside its exported arena.

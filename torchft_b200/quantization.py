@@ -109,6 +109,17 @@ def reduce_quantized(bufs: List[torch.Tensor], n: int, scale: float, out: torch.
 # --------------------------------------------------------------------------- list-of-tensors API
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _list_call(name: str, tensors: List[torch.Tensor], codes: torch.Tensor, scales: torch.Tensor, n: int) -> None:
+    count = len(tensors)
+    data = (ctypes.c_void_p * count)(*[t.data_ptr() for t in tensors])
+    numel = (ctypes.c_longlong * count)(*[t.numel() for t in tensors])
+    N.check(getattr(N.lib(), name)(data, numel, ctypes.c_int(count), N.ptr(codes), N.ptr(scales), ctypes.c_longlong(n),
+                                   ctypes.c_int(_DT[tensors[0].dtype]), N.stream_ptr()), name)
+
+
 def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tuple[torch.Tensor, List[int]]:
     """Pack ``tensors`` (same dtype/device) into one flat quantised buffer whose element
     count is padded to ``128 * world_size`` so it splits evenly across ranks.  Returns the
@@ -119,6 +130,14 @@ def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tup
     assert dtype in _DT, f"unsupported dtype {dtype}"
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
+    if device.type == "cuda" and total > 0 and all(type(t) in _PLAIN for t in tensors):
+        for t in tensors:
+            assert t.dtype == dtype and t.device == device
+        buf = torch.empty(quantized_nbytes(n), dtype=torch.uint8, device=device)
+        # the kernel reads the tensors where they are; only a non-contiguous one is copied
+        flats = [t.detach().resolve_neg().reshape(-1) for t in tensors]
+        _list_call("ftb200_quantize_list_fp8", flats, *split_quantized(buf, n), n)
+        return buf, [n]
     flat = torch.zeros(n, dtype=dtype, device=device)
     off = 0
     for t in tensors:
@@ -130,11 +149,28 @@ def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tup
     return buf, [n]
 
 
+def _written_in_place(t: torch.Tensor, dtype: torch.dtype, device: torch.device) -> bool:
+    """Whether a kernel may write ``t`` directly; the rest takes ``copy_`` with its checks and conversions (other types
+    and devices, strides, leaves that require grad, inference tensors, tensor subclasses)."""
+    return (type(t) in _PLAIN and t.dtype == dtype and t.device == device and t.is_contiguous()
+            and not (t.requires_grad and torch.is_grad_enabled()) and not t.is_inference() and not t.is_neg())
+
+
 def fused_dequantize_from_fp8(tensors: List[torch.Tensor], buf: torch.Tensor, world_size: int) -> None:
     """Inverse of :func:`fused_quantize_into_fp8`: write the values back into ``tensors``."""
     dtype, device = tensors[0].dtype, tensors[0].device
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
+    if device.type == "cuda" and total > 0 and buf.is_cuda:
+        direct = [_written_in_place(t, dtype, device) for t in tensors]
+        targets = [t if ok else torch.empty(t.shape, dtype=dtype, device=device) for t, ok in zip(tensors, direct)]
+        _list_call("ftb200_dequantize_list_fp8", targets, *split_quantized(buf, n), n)
+        for t, target, ok in zip(tensors, targets, direct):
+            if ok:
+                torch.autograd.graph.increment_version(t)
+            else:
+                t.copy_(target)
+        return
     flat = torch.empty(n, dtype=dtype, device=device)
     dequantize_from(buf, flat)
     off = 0
