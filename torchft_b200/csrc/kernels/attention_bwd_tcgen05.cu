@@ -14,13 +14,22 @@
 // P^T and dS^T go back, as packed bf16, into the TMEM columns their scores came from and are the
 // A operands of the dV and dK MMAs straight from tensor memory; dS^T is also written to shared
 // memory (128-byte swizzle) as the MN-major B operand of the dQ^T MMA.  dK and dV stay in TMEM for the
-// whole CTA; dQ^T is drained every tile and added to an fp32 accumulator in global memory with
-// coalesced reductions (one query row, 32 consecutive head-dim elements per warp instruction).
+// whole CTA; dQ^T is drained every tile and added to an fp32 accumulator in global memory (four
+// queries of a head-dim element per reduction, 512 consecutive bytes per warp instruction).
 //
-// Warps: 0 = TMA (K, V once; Q, dO, lse, delta per tile, 3 stages), 1 = MMA issue, 2..17 =
-// softmax and the final dK, dV store, 18..21 = dQ drain (so that the reductions of tile t-1 run
-// beside the softmax of tile t).  The tail MMAs of tile t-1 are issued after S and dP
-// of tile t, so the tensor cores work under the softmax of tile t.  All waits are bounded.
+// Warps: 0 = TMA (K, V once; Q, dO, lse, delta per tile, 3 stages), 1 = MMA issue, 2..9 and 10..17 =
+// two softmax groups that take the tiles in turn (and together store dK, dV at the end), 18..21 = dQ
+// drain.  S^T and dP^T have two buffers each, and dQ^T of a tile takes the place of its dP^T, which fills
+// the 512 TMEM columns:
+//   issue order   dQ(t-1) dV(t-1) dK(t-1) | S(t+1) dP(t+1) | dQ(t) ...
+// so that the softmax of one tile runs beside that of the other, and dQ(t-1) is drained under dV(t-1),
+// dK(t-1) and S(t+1), before dP(t+1) needs its columns.  All waits are bounded.
+//
+// What bounds it: a tile's MMAs take 1650 cycles by themselves, a tile 3300; the difference is the
+// instruction stream of the MMA warp (commits of about 230 cycles, waits) next to 20 others, not the
+// exponentials, the stores of dS^T or the reductions, each of which can be taken out for 0 to 3 %.
+// 8 x 2048, 32/8 heads of 64: 930 us with one softmax group of 16 warps and scalar reductions, 777 us with
+// two (442 TFLOP/s); 1 x 8192, heads of 128: 1706 us either way.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <math.h>
@@ -35,26 +44,27 @@ using namespace ftb200::tc;
 // Optional event trace for tuning (compiled in with -DFTB200_ATTN_TRACE): CTA 0 records clock64()
 // at pipeline events of its first tiles into p.trace[role][tile][event].
 #ifdef FTB200_ATTN_TRACE
-#define TRACE(role, tile, ev)                                                                       \
+#define TRACE(tile, ev)                                                                              \
   do {                                                                                              \
-    if (p.trace != nullptr && blockIdx.x == 0 && (tile) < 32)                                       \
-      p.trace[((role) * 32 + (tile)) * 8 + (ev)] = clock64();                                       \
+    if (p.trace != nullptr && blockIdx.x == 0 && (tile) < 32 && (threadIdx.x & 31) == 0)            \
+      p.trace[((threadIdx.x >> 5) * 32 + (tile)) * 4 + (ev)] = clock64();                           \
   } while (0)
 #else
-#define TRACE(role, tile, ev) \
-  do {                        \
+#define TRACE(tile, ev) \
+  do {                  \
   } while (0)
 #endif
 
 constexpr int BKV = 128;
 constexpr int BQ = 64;
 constexpr int NUM_THREADS = 704;
-constexpr int SOFTMAX_THREADS = 512;
-constexpr int DRAIN_THREADS = 128;
-constexpr int GROUPS = 4;          // threads per key row
-constexpr int CPT = BQ / GROUPS;   // query columns per thread
+constexpr int SOFTMAX_WARPS = 16;
+constexpr int DRAIN_WARPS = 4;
+constexpr int GROUP_WARPS = SOFTMAX_WARPS / 2;  // softmax warps per tile
+constexpr int CPT = BQ / 2;        // query columns per thread: two threads per key row and tile
+constexpr int CHUNK = 16;          // of them at a time
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DQ = 192, COL_DV = 256, COL_DK = 384;
+constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 384;  // dQ^T where dP^T was
 constexpr uint32_t KV_SLAB = BKV * 128;        // 16 KB: [128 rows x 128 B], 64 head-dim elements per row
 constexpr uint32_t Q_SLAB = BQ * 128;          // 8 KB: [64 rows x 128 B]
 constexpr uint32_t PT_TILE = BKV * BQ * 2;     // 16 KB, one slab of [128 key rows x 64 q]
@@ -84,24 +94,21 @@ enum : int {
   BAR_QDO_FULL = 1,   // +stage (3)
   BAR_QDO_EMPTY = 4,  // +stage (3)
   BAR_S_FULL = 7,     // +buf
-  BAR_S_EMPTY = 9,    // +buf
-  BAR_DP_FULL = 11,
-  BAR_DP_EMPTY = 12,
-  BAR_PDS_FULL = 13,  // +buf
-  BAR_PDS_EMPTY = 15, // +buf
-  BAR_DQ_FULL = 17,
-  BAR_DQ_EMPTY = 18,
-  BAR_DKV_DONE = 19,
-  NUM_BARS = 20,
+  BAR_DP_FULL = 9,    // +buf
+  BAR_PDS_FULL = 11,  // +buf
+  BAR_DQ_FULL = 13,   // +buf
+  BAR_DQ_EMPTY = 15,  // +buf
+  BAR_DKV_DONE = 17,
+  NUM_BARS = 18,
 };
 
 struct BwdParams {
   int batch, seq, n_heads, n_kv_heads;
   int causal;
   float scale, scale_log2;
-  const float* lse;    // [batch, n_heads, seq], natural log
-  const float* delta;  // [batch, n_heads, seq]
-  float* dq_acc;       // [batch*seq, n_heads*128] fp32, zeroed by the caller
+  const float* neg_lse2;   // [batch, n_heads, seq], -log2(e) times the forward's log-sum-exp
+  const float* neg_delta;  // [batch, n_heads, seq]
+  float* dq_acc;           // fp32, zeroed; per 64-query tile and head: [16][D][4 queries]
   __nv_bfloat16* dK;   // rows batch*seq, row stride ld_dk
   __nv_bfloat16* dV;
   long long ld_dk, ld_dv;
@@ -113,6 +120,10 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
+}
+
+__device__ __forceinline__ void red_add_v4(float* dst, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
 template <int D>
@@ -144,13 +155,18 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int b = bh / p.n_kv_heads, hk = bh % p.n_kv_heads;
   const int rep = p.n_heads / p.n_kv_heads;
   const int n_qtiles = p.seq / BQ;
-  const int first_q = (p.causal & 1) ? (jb * BKV) / BQ : 0;
-  const int tiles_per_head = n_qtiles - first_q;
-  const int T = rep * tiles_per_head;
+  const int first_q = p.causal ? (jb * BKV) / BQ : 0;
+  const int T = rep * (n_qtiles - first_q);
   const int kv_row0 = b * p.seq + jb * BKV;
-  auto tile_of = [&](int t, int& h, int& qt) {
-    h = hk * rep + t / tiles_per_head;
-    qt = first_q + t % tiles_per_head;
+  // tiles in order: the queries of a head that see the block, then the next head of the group
+  struct TileWalk {
+    int h, qt;
+  };
+  auto next_tile = [&](TileWalk& w) {
+    if (++w.qt == n_qtiles) {
+      w.qt = first_q;
+      ++w.h;
+    }
   };
 
   if (threadIdx.x == 0) {
@@ -161,14 +177,11 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(bar(BAR_S_FULL + s), 1);
-      mbar_init(bar(BAR_S_EMPTY + s), SOFTMAX_THREADS);
-      mbar_init(bar(BAR_PDS_FULL + s), SOFTMAX_THREADS);
-      mbar_init(bar(BAR_PDS_EMPTY + s), 1);
+      mbar_init(bar(BAR_DP_FULL + s), 1);
+      mbar_init(bar(BAR_PDS_FULL + s), GROUP_WARPS);
+      mbar_init(bar(BAR_DQ_FULL + s), 1);
+      mbar_init(bar(BAR_DQ_EMPTY + s), DRAIN_WARPS);
     }
-    mbar_init(bar(BAR_DP_FULL), 1);
-    mbar_init(bar(BAR_DP_EMPTY), SOFTMAX_THREADS);
-    mbar_init(bar(BAR_DQ_FULL), 1);
-    mbar_init(bar(BAR_DQ_EMPTY), DRAIN_THREADS);
     mbar_init(bar(BAR_DKV_DONE), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -197,15 +210,15 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     __syncwarp();
     bool ok = true;
-    for (int t = 0; t < T && ok; ++t) {
+    TileWalk w{hk * rep, first_q};
+    for (int t = 0; t < T && ok; ++t, next_tile(w)) {
       const int st = t % QDO_STAGES;
       const uint32_t use = static_cast<uint32_t>(t / QDO_STAGES);
       if (!mbar_wait_warp(bar(BAR_QDO_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
         ok = false;
         break;
       }
-      int h, qt;
-      tile_of(t, h, qt);
+      const int h = w.h, qt = w.qt;
       const int q_row0 = b * p.seq + qt * BQ;
       const uint32_t sq = smem_base + OFF_STAGE + st * STAGE_BYTES;
       const uint32_t sdo = sq + Q_TILE;
@@ -218,8 +231,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           tma_load_2d(sq + sl * Q_SLAB, &tmQ, bar(BAR_QDO_FULL + st), h * D + 64 * sl, q_row0);
           tma_load_2d(sdo + sl * Q_SLAB, &tmDO, bar(BAR_QDO_FULL + st), h * D + 64 * sl, q_row0);
         }
-        bulk_load_1d(sst, p.lse + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
-        bulk_load_1d(sst + BQ * 4, p.delta + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
+        bulk_load_1d(sst, p.neg_lse2 + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
+        bulk_load_1d(sst + BQ * 4, p.neg_delta + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
       }
       __syncwarp();
     }
@@ -249,15 +262,15 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     bool ok = mbar_wait_warp(bar(BAR_KV), 0, abort_flag);
     for (int t = 0; t <= T && ok; ++t) {
       if (t < T) {
+        // S and dP of tile t; the MMAs that read P and dS of tile t - 2 from the same S buffer were issued before
         const int st = t & 1, qs = t % QDO_STAGES;
         const uint32_t use = static_cast<uint32_t>(t >> 1);
-        if (!mbar_wait_warp(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag) ||
-            !mbar_wait_warp(bar(BAR_S_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
+        if (!mbar_wait_warp(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        TRACE(0, t, 0);  // S inputs ready
+        TRACE(t, 0);  // S inputs ready
         const uint32_t qb_km = q_km0 + qs * STAGE16;
         if (elect_one()) {
 #pragma unroll
@@ -268,7 +281,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           umma_commit(bar(BAR_S_FULL + st));
         }
         __syncwarp();
-        if (!mbar_wait_warp(bar(BAR_DP_EMPTY), (static_cast<uint32_t>(t) & 1u) ^ 1u, abort_flag)) {
+        if (!mbar_wait_warp(bar(BAR_DQ_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {  // dQ of tile t - 2 drained
           ok = false;
           break;
         }
@@ -277,12 +290,12 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t a_off = ((kk >> 2) * KV_SLAB + (kk & 3) * 32) >> 4, b_off = ((kk >> 2) * Q_SLAB + (kk & 3) * 32) >> 4;
-            umma_bf16_lh(tmem_base + COL_DP, v_km + a_off, HI, qb_km + QT16 + b_off, HI, idesc_st, kk != 0);
+            umma_bf16_lh(tmem_base + COL_DP + st * BQ, v_km + a_off, HI, qb_km + QT16 + b_off, HI, idesc_st, kk != 0);
           }
-          umma_commit(bar(BAR_DP_FULL));
+          umma_commit(bar(BAR_DP_FULL + st));
         }
         __syncwarp();
-        TRACE(0, t, 1);  // S, dP issued
+        TRACE(t, 1);  // S, dP issued
       }
       if (t >= 1) {
         const int u = t - 1, pb = u & 1, qs = u % QDO_STAGES;
@@ -292,12 +305,17 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           break;
         }
         tc_fence_after();
-        TRACE(0, u, 2);  // P, dS ready for the tail of tile u
+        TRACE(u, 2);  // P, dS ready for the tail of tile u
         const uint32_t qb_mn = q_mn0 + qs * STAGE16;
         const uint32_t dsb_mn = ds_mn0 + pb * PDS16;
         // queries 16k..16k+15 of tile u: P^T in columns 16k..16k+7 of its score buffer, dS^T in 16k+8..16k+15
         const uint32_t pt_tmem = tmem_base + COL_S + pb * BQ;
         if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < BKV / 16; ++kk) {  // dQ^T = K^T dS^T, over dP^T of the tile (read by the softmax)
+            umma_bf16_lh(tmem_base + COL_DP + pb * BQ, k_mn + ((kk * 2048) >> 4), HI, dsb_mn + ((kk * 2048) >> 4), HI, idesc_dq, kk != 0);
+          }
+          umma_commit(bar(BAR_DQ_FULL + pb));
 #pragma unroll
           for (int kk = 0; kk < BQ / 16; ++kk) {  // dV += P^T dO
             umma_bf16_tmem_a(tmem_base + COL_DV, pt_tmem + kk * 16, qb_mn + QT16 + ((kk * 2048) >> 4), HI, idesc_kv, (u | kk) != 0);
@@ -309,21 +327,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           umma_commit(bar(BAR_QDO_EMPTY + qs));
         }
         __syncwarp();
-        if (!mbar_wait_warp(bar(BAR_DQ_EMPTY), (static_cast<uint32_t>(u) & 1u) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk) {  // dQ^T = K^T dS^T
-            umma_bf16_lh(tmem_base + COL_DQ, k_mn + ((kk * 2048) >> 4), HI, dsb_mn + ((kk * 2048) >> 4), HI, idesc_dq, kk != 0);
-          }
-          umma_commit(bar(BAR_PDS_EMPTY + pb));
-          umma_commit(bar(BAR_DQ_FULL));
-        }
-        __syncwarp();
-        TRACE(0, u, 3);  // tail issued
+        TRACE(u, 3);  // tail issued
       }
     }
     if (ok && elect_one()) umma_commit(bar(BAR_DKV_DONE));
@@ -333,124 +337,148 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int quarter = warp & 3;
     const int dcol = quarter * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const long long ldq = static_cast<long long>(p.n_heads) * D;
-    for (int u = 0; u < T; ++u) {
-      if (!mbar_wait(bar(BAR_DQ_FULL), static_cast<uint32_t>(u) & 1u, abort_flag)) break;
+    TileWalk w{hk * rep, first_q};
+    for (int u = 0; u < T; ++u, next_tile(w)) {
+      const int buf = u & 1;
+      if (!mbar_wait_warp(bar(BAR_DQ_FULL + buf), static_cast<uint32_t>(u >> 1) & 1u, abort_flag)) break;
       tc_fence_after();
+      TRACE(u, 0);  // dQ complete
       uint32_t v[BQ];
       const bool mine = quarter * 32 < D;  // head dim 64: only lanes 0..63 of dQ^T are real
       if (mine) {
-        tmem_ld32(tmem_base + COL_DQ + lane_addr, v);
-        tmem_ld32(tmem_base + COL_DQ + 32 + lane_addr, v + 32);
+        tmem_ld32(tmem_base + COL_DP + buf * BQ + lane_addr, v);
+        tmem_ld32(tmem_base + COL_DP + buf * BQ + 32 + lane_addr, v + 32);
         tmem_wait_ld();
       }
       tc_fence_before();
-      mbar_arrive(bar(BAR_DQ_EMPTY));
-      int h, qt;
-      tile_of(u, h, qt);
-      float* dst = p.dq_acc + (static_cast<long long>(b) * p.seq + qt * BQ) * ldq + h * D + dcol;
-      if (mine && !(p.causal & 2))
+      mbar_arrive_warp(bar(BAR_DQ_EMPTY + buf));
+      TRACE(u, 1);  // dQ in registers
+      if (mine) {
+        // four queries of one head-dim element lie together: a warp adds 512 consecutive bytes per instruction
+        const long long tile = (static_cast<long long>(b) * n_qtiles + w.qt) * p.n_heads + w.h;
+        float* dst = p.dq_acc + tile * (BQ * D) + dcol * 4;
 #pragma unroll
-        for (int c = 0; c < BQ; ++c) atomicAdd(dst + c * ldq, __uint_as_float(v[c]));
+        for (int c = 0; c < BQ / 4; ++c)
+          red_add_v4(dst + c * (D * 4), __uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]), __uint_as_float(v[4 * c + 2]),
+                     __uint_as_float(v[4 * c + 3]));
+      }
+      TRACE(u, 2);  // added
     }
   } else {
     // ---------------- softmax, dK/dV store (warps 2..17) ----------------
     const int quarter = warp & 3;
-    const int g = (warp - 2) >> 2;  // which 16 of the tile's 64 queries (32 of 128 columns at the end)
-    const int row = quarter * 32 + lane;  // key within the block; head-dim index when draining dQ^T
+    const int sw = (warp - 2) >> 2;       // four warps with the same columns
+    const int grp = sw >> 1, g = sw & 1;  // which tiles (even or odd), which 32 of the tile's 64 queries
+    const int row = quarter * 32 + lane;  // key within the block
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    const float log2e = 1.4426950408889634f;
     bool ok = true;
-
-    for (int t = 0; t < T; ++t) {
-      const int st = t & 1;
+    const unsigned long long scale2 = f2_pack(p.scale_log2, p.scale_log2);
+    const int key = jb * BKV + row;
+    TileWalk w{hk * rep, first_q};
+    if (grp == 1) next_tile(w);
+    const uint32_t s_addr = tmem_base + COL_S + grp * BQ + g * CPT + lane_addr;
+    const uint32_t dp_addr = tmem_base + COL_DP + grp * BQ + g * CPT + lane_addr;
+    uint8_t* drow = smem + OFF_PDS + grp * PDS_BYTES + row * 128;
+    for (int t = grp; t < T; t += 2, next_tile(w), next_tile(w)) {
       const uint32_t use = static_cast<uint32_t>(t >> 1);
-      int h, qt;
-      tile_of(t, h, qt);
-      if (!mbar_wait(bar(BAR_S_FULL + st), use & 1u, abort_flag) ||
-          !mbar_wait(bar(BAR_DP_FULL), static_cast<uint32_t>(t) & 1u, abort_flag)) {
+      const int qs = t % QDO_STAGES;
+      // the tile's statistics arrived with Q and dO
+      if (!mbar_wait_warp(bar(BAR_S_FULL + grp), use & 1u, abort_flag) ||
+          !mbar_wait_warp(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag)) {
         ok = false;
         break;
       }
       tc_fence_after();
-      if (threadIdx.x == 64) TRACE(1, t, 0);  // S and dP complete
-      uint32_t sv[CPT], dp[CPT];
-      tmem_ld16(tmem_base + COL_S + st * BQ + g * CPT + lane_addr, sv);
-      tmem_ld16(tmem_base + COL_DP + g * CPT + lane_addr, dp);
-      tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive(bar(BAR_S_EMPTY + st));
-      mbar_arrive(bar(BAR_DP_EMPTY));
-      if (threadIdx.x == 64) TRACE(1, t, 1);  // scores in registers
-      // the tile's statistics arrived with Q and dO
-      const int qs = t % QDO_STAGES;
-      if (!mbar_wait(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag)) {
-        ok = false;
-        break;
-      }
-      const float4* stats4 = reinterpret_cast<const float4*>(smem + OFF_STATS + qs * STATS_BYTES);
-      float lse_q[CPT], del_q[CPT];
+      TRACE(t, 0);  // S complete
+      // pairs of -log2(e) lse and -delta, as the packed arithmetic takes them
+      const ulonglong2* stats2 = reinterpret_cast<const ulonglong2*>(smem + OFF_STATS + qs * STATS_BYTES) + g * (CPT / 4);
+      const int q0 = w.qt * BQ + g * CPT;
+      const bool diag = (p.causal != 0) && (q0 < jb * BKV + BKV);
 #pragma unroll
-      for (int c = 0; c < CPT / 4; ++c) {
-        const float4 a = stats4[g * (CPT / 4) + c];
-        const float4 d4 = stats4[BQ / 4 + g * (CPT / 4) + c];
-        lse_q[4 * c] = a.x; lse_q[4 * c + 1] = a.y; lse_q[4 * c + 2] = a.z; lse_q[4 * c + 3] = a.w;
-        del_q[4 * c] = d4.x; del_q[4 * c + 1] = d4.y; del_q[4 * c + 2] = d4.z; del_q[4 * c + 3] = d4.w;
-      }
-      const int key = jb * BKV + row;
-      const int q0 = qt * BQ + g * CPT;
-      const bool diag = (p.causal & 1) && (q0 < jb * BKV + BKV);
-      uint32_t pk[CPT / 2], dk[CPT / 2];
+      for (int cc = 0; cc < CPT / CHUNK; ++cc) {
+        uint32_t sv[CHUNK], dp[CHUNK];
+        tmem_ld16(s_addr + cc * CHUNK, sv);
+        if (cc > 0) tmem_ld16(dp_addr + cc * CHUNK, dp);
+        tmem_wait_ld();
+        float pe[CHUNK];
 #pragma unroll
-      for (int c = 0; c < CPT / 2; ++c) {
-        float pv[2], dv[2];
+        for (int c = 0; c < CHUNK / 4; ++c) {
+          const ulonglong2 l4 = stats2[cc * (CHUNK / 4) + c];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int qi = 2 * c + e;
-          float pe = exp2f(fmaf(__uint_as_float(sv[qi]), p.scale_log2, -lse_q[qi] * log2e));
-          if (diag && key > q0 + qi) pe = 0.f;
-          pv[e] = pe;
-          dv[e] = pe * (__uint_as_float(dp[qi]) - del_q[qi]) * p.scale;
+          for (int e = 0; e < 2; ++e) {
+            const int qi = 4 * c + 2 * e;
+            const unsigned long long x2 =
+                f2_fma(f2_pack(__uint_as_float(sv[qi]), __uint_as_float(sv[qi + 1])), scale2, e == 0 ? l4.x : l4.y);
+            f2_unpack(x2, pe[qi], pe[qi + 1]);
+            pe[qi] = exp2f(pe[qi]);
+            pe[qi + 1] = exp2f(pe[qi + 1]);
+          }
         }
-        __nv_bfloat162 a = __floats2bfloat162_rn(pv[0], pv[1]);
-        __nv_bfloat162 d2 = __floats2bfloat162_rn(dv[0], dv[1]);
-        pk[c] = *reinterpret_cast<uint32_t*>(&a);
-        dk[c] = *reinterpret_cast<uint32_t*>(&d2);
-      }
-      if (!mbar_wait(bar(BAR_PDS_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
-        ok = false;
-        break;
-      }
-      if (threadIdx.x == 64) TRACE(1, t, 2);  // math done, P/dS buffer free
-      // P^T and dS^T replace the scores this thread has just read (its own 16 columns)
-      uint32_t pds[CPT];
+        if (diag) {
 #pragma unroll
-      for (int c = 0; c < CPT / 2; ++c) {
-        pds[c] = pk[c];
-        pds[CPT / 2 + c] = dk[c];
-      }
-      tmem_st16(tmem_base + COL_S + st * BQ + g * CPT + lane_addr, pds);
-      uint8_t* drow = smem + OFF_PDS + st * PDS_BYTES + row * 128;
+          for (int c = 0; c < CHUNK; ++c)
+            if (key > q0 + cc * CHUNK + c) pe[c] = 0.f;
+        }
+        if (cc == 0) {
+          if (!mbar_wait_warp(bar(BAR_DP_FULL + grp), use & 1u, abort_flag)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          TRACE(t, 1);  // dP complete
+          tmem_ld16(dp_addr, dp);
+          tmem_wait_ld();
+        }
+        uint32_t pds[CHUNK];  // P^T, dS^T
 #pragma unroll
-      for (int c = 0; c < CPT / 8; ++c) {
-        const int chunk = ((g * (CPT / 8) + c) ^ (row & 7)) << 4;
-        *reinterpret_cast<uint4*>(drow + chunk) = make_uint4(dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
+        for (int c = 0; c < CHUNK / 4; ++c) {
+          const ulonglong2 d4 = stats2[BQ / 4 + cc * (CHUNK / 4) + c];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int qi = 4 * c + 2 * e;
+            // dS without the softmax scale, which the stores of dQ and dK apply
+            const unsigned long long ds2 =
+                f2_mul(f2_pack(pe[qi], pe[qi + 1]),
+                       f2_add(f2_pack(__uint_as_float(dp[qi]), __uint_as_float(dp[qi + 1])), e == 0 ? d4.x : d4.y));
+            float s0, s1;
+            f2_unpack(ds2, s0, s1);
+            __nv_bfloat162 a = __floats2bfloat162_rn(pe[qi], pe[qi + 1]);
+            __nv_bfloat162 d2 = __floats2bfloat162_rn(s0, s1);
+            pds[qi / 2] = *reinterpret_cast<uint32_t*>(&a);
+            pds[CHUNK / 2 + qi / 2] = *reinterpret_cast<uint32_t*>(&d2);
+          }
+        }
+        // the dS^T buffer is free once dQ^T of the group's tile before is complete
+        if (cc == 0 && !mbar_wait_warp(bar(BAR_DQ_FULL + grp), (use & 1u) ^ 1u, abort_flag)) {
+          ok = false;
+          break;
+        }
+        // P^T and dS^T replace the scores this thread has just read (its own 16 columns)
+        tmem_st16(s_addr + cc * CHUNK, pds);
+#pragma unroll
+        for (int c = 0; c < CHUNK / 8; ++c) {
+          const int chunk = ((g * (CPT / 8) + cc * (CHUNK / 8) + c) ^ (row & 7)) << 4;
+          *reinterpret_cast<uint4*>(drow + chunk) = make_uint4(pds[CHUNK / 2 + 4 * c], pds[CHUNK / 2 + 4 * c + 1],
+                                                               pds[CHUNK / 2 + 4 * c + 2], pds[CHUNK / 2 + 4 * c + 3]);
+        }
       }
+      if (!ok) break;
+      TRACE(t, 2);  // math done
       fence_async_smem();
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(bar(BAR_PDS_FULL + st));
-      if (threadIdx.x == 64) TRACE(1, t, 3);  // P/dS published
+      mbar_arrive_warp(bar(BAR_PDS_FULL + grp));
+      TRACE(t, 3);  // P/dS published
     }
-    if (ok && mbar_wait(bar(BAR_DKV_DONE), 0, abort_flag)) {
+    if (ok && mbar_wait_warp(bar(BAR_DKV_DONE), 0, abort_flag)) {
       tc_fence_after();
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
-        constexpr int CW = D / GROUPS;  // head-dim columns per thread
-        const uint32_t col = (which == 0 ? COL_DV : COL_DK) + g * CW;
+        constexpr int CW = D / 4;  // head-dim columns per thread
+        const uint32_t col = (which == 0 ? COL_DV : COL_DK) + sw * CW;
         __nv_bfloat16* base = which == 0 ? p.dV : p.dK;
         const long long ld = which == 0 ? p.ld_dv : p.ld_dk;
-        __nv_bfloat16* dst = base + static_cast<long long>(kv_row0 + row) * ld + hk * D + g * CW;
+        __nv_bfloat16* dst = base + static_cast<long long>(kv_row0 + row) * ld + hk * D + sw * CW;
         uint32_t v[CW];
         if constexpr (CW == 32)
           tmem_ld32(tmem_base + col + lane_addr, v);
@@ -461,7 +489,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int c = 0; c < CW / 8; ++c) {
           float f[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * c + e]);
+          for (int e = 0; e < 8; ++e) f[e] = which == 0 ? __uint_as_float(v[8 * c + e]) : __uint_as_float(v[8 * c + e]) * p.scale;
           reinterpret_cast<ftb200::bf16x8*>(dst)[c] = ftb200::pack8(f);
         }
       }
@@ -477,51 +505,63 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d]; one warp per (row, head)
+// Before the main kernel, one pass over O and dO: neg_delta[b, h, s] = -sum_d dO O, neg_lse2 = -log2(e) lse, and the dQ
+// accumulator zeroed.  A thread takes 8 elements (16 bytes of each), D / 8 neighbouring lanes a (row, head).
 template <int D>
-__global__ void attention_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                       float* __restrict__ delta, int batch, int seq, int n_heads, long long ld_o,
-                                       long long ld_do) {
-  const long long w = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const long long total = static_cast<long long>(batch) * seq * n_heads;
-  if (w >= total) return;
-  const long long r = w / n_heads;
-  const int h = static_cast<int>(w % n_heads);
-  constexpr int PAIRS = D / 64;  // bf16 pairs per lane
-  __nv_bfloat162 a2[PAIRS], c2[PAIRS];
-  if constexpr (PAIRS == 2) {
-    *reinterpret_cast<uint2*>(a2) = *reinterpret_cast<const uint2*>(o + r * ld_o + h * D + lane * 4);
-    *reinterpret_cast<uint2*>(c2) = *reinterpret_cast<const uint2*>(d_o + r * ld_do + h * D + lane * 4);
-  } else {
-    *reinterpret_cast<uint32_t*>(a2) = *reinterpret_cast<const uint32_t*>(o + r * ld_o + h * D + lane * 2);
-    *reinterpret_cast<uint32_t*>(c2) = *reinterpret_cast<const uint32_t*>(d_o + r * ld_do + h * D + lane * 2);
-  }
+__global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
+                                                                 const __nv_bfloat16* __restrict__ d_o,
+                                                                 const float* __restrict__ lse, float* __restrict__ neg_lse2,
+                                                                 float* __restrict__ neg_delta, float4* __restrict__ dq_acc,
+                                                                 int seq, int n_heads, long long pieces, long long ld_o,
+                                                                 long long ld_do) {
+  constexpr int LANES = D / 8;
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const bool live = i < pieces;
+  const int per_row = n_heads * LANES;
+  const int r = static_cast<int>((live ? i : 0) / per_row);  // batch * seq rows fit an int (the host checks)
+  const int c = static_cast<int>((live ? i : 0) - static_cast<long long>(r) * per_row);
   float s = 0.f;
+  if (live) {
+    float x[8], y[8];
+    ftb200::unpack8(*reinterpret_cast<const ftb200::bf16x8*>(o + r * ld_o + c * 8), x);
+    ftb200::unpack8(*reinterpret_cast<const ftb200::bf16x8*>(d_o + r * ld_do + c * 8), y);
+    dq_acc[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    dq_acc[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < PAIRS; ++i) {
-    const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(c2[i]);
-    s += x.x * y.x + x.y * y.y;
+    for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
   }
-  s = ftb200::warp_sum(s);
-  if (lane == 0) {
-    const long long bb = r / seq, ss = r % seq;
-    delta[(bb * n_heads + h) * seq + ss] = s;
+#pragma unroll
+  for (int k = LANES / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+  if (live && c % LANES == 0) {
+    const long long at = (static_cast<long long>(r / seq) * n_heads + c / LANES) * seq + r % seq;
+    neg_delta[at] = -s;
+    neg_lse2[at] = lse[at] * -1.4426950408889634f;
   }
 }
 
-// dq[rows, cols] (bf16, row stride ld) = dq_acc[rows, cols] (fp32, dense)
-__global__ void attention_dq_cast_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long rows,
-                                         int cols, long long ld) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;  // one 8-element piece each
-  const int per_row = cols / 8;
-  if (i >= rows * per_row) return;
-  const long long r = i / per_row;
-  const int c = static_cast<int>(i % per_row) * 8;
-  const float4 a = *reinterpret_cast<const float4*>(acc + r * cols + c);
-  const float4 b2 = *reinterpret_cast<const float4*>(acc + r * cols + c + 4);
-  const float f[8] = {a.x, a.y, a.z, a.w, b2.x, b2.y, b2.z, b2.w};
-  *reinterpret_cast<ftb200::bf16x8*>(dq + r * ld + c) = ftb200::pack8(f);
+// dq (bf16, row stride ld) = scale * accumulator (fp32, per 64-query tile and head [16][D][4 queries]); a thread takes 8
+// head-dim elements of 4 queries.
+template <int D>
+__global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
+                                                                long long pieces, int n_heads, long long ld, float scale) {
+  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= pieces) return;
+  const int d8 = static_cast<int>(i % (D / 8));
+  const long long g = i / (D / 8);  // (tile, head, group of 4 queries)
+  const int q4 = static_cast<int>(g & 15);
+  const long long th = g >> 4;
+  const int h = static_cast<int>(th % n_heads);
+  const long long row0 = th / n_heads * 64 + q4 * 4;
+  float4 v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) v[e] = acc[g * D + d8 * 8 + e];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float f[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = scale * (k == 0 ? v[e].x : k == 1 ? v[e].y : k == 2 ? v[e].z : v[e].w);
+    *reinterpret_cast<ftb200::bf16x8*>(dq + (row0 + k) * ld + h * D + d8 * 8) = ftb200::pack8(f);
+  }
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -556,11 +596,11 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 }  // namespace
 
-// Scratch the backward pass needs, in bytes: fp32 dQ accumulator followed by delta.
+// Scratch the backward pass needs, in bytes: fp32 dQ accumulator, -delta, -log2(e) lse.
 // (sized for head dim 128; enough for 64 as well)
 FTB200_API long long ftb200_attention_bwd_scratch_bytes(int batch, int seq, int n_heads) {
   const long long rows = static_cast<long long>(batch) * seq;
-  return rows * n_heads * 128 * 4 + rows * n_heads * 4;
+  return rows * n_heads * 128 * 4 + 2 * rows * n_heads * 4;
 }
 
 namespace {
@@ -573,7 +613,9 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   constexpr uint32_t SMEM_BYTES = Lay<D>::SMEM_BYTES;
   const long long rows = static_cast<long long>(batch) * seq;
   float* dq_acc = reinterpret_cast<float*>(scratch);
-  float* delta = dq_acc + rows * n_heads * D;
+  float* neg_delta = dq_acc + rows * n_heads * D;
+  float* neg_lse2 = neg_delta + rows * n_heads;
+  if (rows > 0x7fffffffLL) return FTB200_E_TOOBIG;
   CUtensorMap tq, tk, tv, tdo;
   int rc = encode_rows(&tq, q, rows, static_cast<long long>(n_heads) * D, ld_q, BQ);
   if (rc == 0) rc = encode_rows(&tdo, d_o, rows, static_cast<long long>(n_heads) * D, ld_do, BQ);
@@ -587,32 +629,26 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
       return FTB200_E_CUDA;
     attr_set = true;
   }
-  if (cudaMemsetAsync(dq_acc, 0, rows * n_heads * D * 4, stream) != cudaSuccess) return FTB200_E_CUDA;
-  {
-    const long long warps = rows * n_heads;
-    const long long blocks = (warps * 32 + 255) / 256;
-    attention_delta_kernel<D><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), delta, batch, seq, n_heads,
-        ld_o, ld_do);
-  }
+  const long long pieces = rows * n_heads * (D / 8);
+  if ((pieces + 255) / 256 > 0x7fffffffLL) return FTB200_E_TOOBIG;
+  attention_bwd_prep_kernel<D><<<static_cast<unsigned>((pieces + 255) / 256), 256, 0, stream>>>(
+      reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), lse, neg_lse2, neg_delta,
+      reinterpret_cast<float4*>(dq_acc), seq, n_heads, pieces, ld_o, ld_do);
   BwdParams p;
   p.batch = batch; p.seq = seq; p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.causal = causal;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
-  p.lse = lse; p.delta = delta; p.dq_acc = dq_acc;
+  p.neg_lse2 = neg_lse2; p.neg_delta = neg_delta; p.dq_acc = dq_acc;
   p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
   p.ld_dk = ld_dk; p.ld_dv = ld_dv; p.status = status;
   p.trace = nullptr;
 #ifdef FTB200_ATTN_TRACE
-  p.trace = reinterpret_cast<long long*>(delta + rows * n_heads);  // the caller sized the scratch for it
+  p.trace = reinterpret_cast<long long*>(neg_lse2 + rows * n_heads);  // the caller sized the scratch for it
 #endif
   const long long grid = static_cast<long long>(batch) * n_kv_heads * (seq / BKV);
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_bwd_kernel<D><<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
-  {
-    const long long pieces = rows * (static_cast<long long>(n_heads) * D / 8);
-    attention_dq_cast_kernel<<<static_cast<unsigned>((pieces + 255) / 256), 256, 0, stream>>>(
-        dq_acc, reinterpret_cast<__nv_bfloat16*>(dq), rows, n_heads * D, ld_dq);
-  }
+  attention_dq_cast_kernel<D><<<static_cast<unsigned>((pieces / 4 + 255) / 256), 256, 0, stream>>>(
+      reinterpret_cast<const float4*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), pieces / 4, n_heads, ld_dq, scale);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 

@@ -51,7 +51,7 @@ constexpr int NUM_THREADS = 384;
 // most of its own to the two softmax warpgroups, whose threads hold a row's 128 scores: 72 + 2 * 216 = 3 * 168.
 constexpr int LAUNCH_REGS = 168, ISSUE_REGS = 72, SOFTMAX_REGS = 216;
 static_assert(ISSUE_REGS + 2 * SOFTMAX_REGS <= 3 * LAUNCH_REGS, "more registers than the CTA is launched with");
-constexpr int ROW_THREADS = 128;  // softmax threads per tile
+constexpr int ROW_WARPS = 4;  // softmax warps per tile
 constexpr uint32_t TMEM_COLS = 512;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // in log2 units
 
@@ -124,8 +124,8 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int t = 0; t < TILES; ++t) {
       mbar_init(bar(BAR_Q_FULL + t), 1);
       mbar_init(bar(BAR_S_FULL + t), 1);
-      mbar_init(bar(BAR_P_FULL + t), ROW_THREADS);
-      mbar_init(bar(BAR_P_HALF + t), ROW_THREADS);
+      mbar_init(bar(BAR_P_FULL + t), ROW_WARPS);
+      mbar_init(bar(BAR_P_HALF + t), ROW_WARPS);
       mbar_init(bar(BAR_O_DONE + t), 1);
     }
     for (int s = 0; s < KV_STAGES; ++s) {
@@ -312,7 +312,7 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     float m_used = -INFINITY, l_sum = 0.f;
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
-      if (!mbar_wait(bar(BAR_S_FULL + t), static_cast<uint32_t>(j) & 1u, abort_flag)) {
+      if (!mbar_wait_warp(bar(BAR_S_FULL + t), static_cast<uint32_t>(j) & 1u, abort_flag)) {
         ok = false;
         break;
       }
@@ -346,7 +346,7 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       if (any_raise) {
         // O may only be touched once P V of the previous block is done; P V of this block waits for P
-        if (!mbar_wait(bar(BAR_O_DONE + t), static_cast<uint32_t>(j - 1) & 1u, abort_flag)) {
+        if (!mbar_wait_warp(bar(BAR_O_DONE + t), static_cast<uint32_t>(j - 1) & 1u, abort_flag)) {
           ok = false;
           break;
         }
@@ -391,7 +391,7 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (c == 1) {
           tmem_wait_st();
           tc_fence_before();
-          mbar_arrive(bar(BAR_P_HALF + t));
+          mbar_arrive_warp(bar(BAR_P_HALF + t));
         }
       }
       float sum4[4];
@@ -400,10 +400,10 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       l_sum += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(bar(BAR_P_FULL + t));
+      mbar_arrive_warp(bar(BAR_P_FULL + t));
     }
 
-    if (ok && mbar_wait(bar(BAR_O_DONE + t), static_cast<uint32_t>(n_kv - 1) & 1u, abort_flag)) {
+    if (ok && mbar_wait_warp(bar(BAR_O_DONE + t), static_cast<uint32_t>(n_kv - 1) & 1u, abort_flag)) {
       tc_fence_after();
       const float inv = 1.f / l_sum;
       const long long grow = static_cast<long long>(q_row0 + t * BQ + row);

@@ -55,7 +55,7 @@ constexpr uint32_t TILE_BYTES = 128 * 128 * 2;  // every operand tile: 128 x 128
 constexpr uint32_t SLAB_BYTES = TILE_BYTES / 2;  // 128 rows x 64 elements, one swizzle atom wide
 constexpr int KV_STAGES = 2;
 constexpr int NUM_THREADS = 576;
-constexpr int SOFTMAX_THREADS = 512;
+constexpr int SOFTMAX_WARPS = 16;
 constexpr int GROUPS = 4;   // threads per query row
 constexpr int CPT = BKV / GROUPS;  // score columns per thread
 constexpr uint32_t TMEM_COLS = 512;
@@ -122,16 +122,16 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
   const int q_row0 = b * p.seq + qb * BQ;
 
   if (threadIdx.x == 0) {
-    mbar_init(bar(BAR_Q), SOFTMAX_THREADS);
+    mbar_init(bar(BAR_Q), SOFTMAX_WARPS);
     for (int s = 0; s < KV_STAGES; ++s) {
       mbar_init(bar(BAR_K_FULL + s), 1);
       mbar_init(bar(BAR_V_FULL + s), 1);
       mbar_init(bar(BAR_K_EMPTY + s), 1);
       mbar_init(bar(BAR_V_EMPTY + s), 1);
       mbar_init(bar(BAR_S_FULL + s), 1);
-      mbar_init(bar(BAR_XCHG + s), SOFTMAX_THREADS);
+      mbar_init(bar(BAR_XCHG + s), SOFTMAX_WARPS);
     }
-    mbar_init(bar(BAR_P_FULL), SOFTMAX_THREADS);
+    mbar_init(bar(BAR_P_FULL), SOFTMAX_WARPS);
     mbar_init(bar(BAR_O_DONE), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -275,11 +275,11 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
     tmem_st16(tmem_base + COL_Q + g * 16 + lane_addr, qw);
     tmem_wait_st();
     tc_fence_before();
-    mbar_arrive(bar(BAR_Q));
+    mbar_arrive_warp(bar(BAR_Q));
     for (int j = 0; j < n_kv; ++j) {
       const int st = j & 1;
       const uint32_t use = static_cast<uint32_t>(j >> 1);
-      if (!mbar_wait(bar(BAR_S_FULL + st), use & 1u, abort_flag)) {
+      if (!mbar_wait_warp(bar(BAR_S_FULL + st), use & 1u, abort_flag)) {
         ok = false;
         break;
       }
@@ -302,8 +302,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       float* xc = xchg + (st * GROUPS) * BQ;
       xc[g * BQ + row] = mx;
-      mbar_arrive(bar(BAR_XCHG + st));
-      if (!mbar_wait(bar(BAR_XCHG + st), use & 1u, abort_flag)) {
+      mbar_arrive_warp(bar(BAR_XCHG + st));
+      if (!mbar_wait_warp(bar(BAR_XCHG + st), use & 1u, abort_flag)) {
         ok = false;
         break;
       }
@@ -339,7 +339,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
       tmem_st16(tmem_base + COL_S + st * BKV + g * CPT + lane_addr, packed);
       if (any_raise) {
         // O may only be touched once P V of the previous block is done
-        if (!mbar_wait(bar(BAR_O_DONE), static_cast<uint32_t>(j - 1) & 1u, abort_flag)) {
+        if (!mbar_wait_warp(bar(BAR_O_DONE), static_cast<uint32_t>(j - 1) & 1u, abort_flag)) {
           ok = false;
           break;
         }
@@ -354,18 +354,18 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
       }
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(bar(BAR_P_FULL));
+      mbar_arrive_warp(bar(BAR_P_FULL));
       if (threadIdx.x == 64) TRACE(1, j, 4);  // P published
     }
 
-    if (ok && mbar_wait(bar(BAR_O_DONE), static_cast<uint32_t>(n_kv - 1) & 1u, abort_flag)) {
+    if (ok && mbar_wait_warp(bar(BAR_O_DONE), static_cast<uint32_t>(n_kv - 1) & 1u, abort_flag)) {
       tc_fence_after();
       // total row sum: the threads of a row hold partial sums over their keys
       float* xc = xchg;  // both parities are free again
       xc[g * BQ + row] = l_part;
       const uint32_t xuse = static_cast<uint32_t>((n_kv + 1) >> 1);  // completed phases of XCHG+0 so far
-      mbar_arrive(bar(BAR_XCHG + 0));
-      if (mbar_wait(bar(BAR_XCHG + 0), xuse & 1u, abort_flag)) {
+      mbar_arrive_warp(bar(BAR_XCHG + 0));
+      if (mbar_wait_warp(bar(BAR_XCHG + 0), xuse & 1u, abort_flag)) {
         const float l = (xc[row] + xc[BQ + row]) + (xc[2 * BQ + row] + xc[3 * BQ + row]);
         const float inv = 1.f / l;
         __nv_bfloat16* dst = p.O + static_cast<long long>(q_row0 + row) * p.ld_o + h * D + g * 32;

@@ -45,6 +45,12 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// One arrival for the whole warp, after what its lanes did before.
+__device__ __forceinline__ void mbar_arrive_warp(uint32_t bar) {
+  __syncwarp();
+  if (elect_one()) mbar_arrive(bar);
+}
+
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -59,16 +65,17 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  Returns false when the CTA is aborting (limit hit here or elsewhere).
+// Bounded wait.  Returns false when the CTA is aborting (limit hit here or elsewhere).  The clock is only read after
+// 1024 failed polls.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_test(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  uint32_t spins = 0;
-  for (;;) {
+  uint64_t t0 = 0;
+  for (uint32_t polls = 1;; ++polls) {
     if (mbar_test(bar, parity)) return true;
-    if ((++spins & 63u) == 0) {
+    if ((polls & 1023u) == 0) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > WAIT_LIMIT_NS) {
         *abort_flag = 1;
         return false;
       }
