@@ -95,5 +95,8 @@ def ptr(t: Optional[torch.Tensor]) -> c_void_p:
 
 
 def stream_ptr(stream: Optional[torch.cuda.Stream] = None) -> c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return c_void_p(s.cuda_stream)
+    """The CUDA stream to launch on: ``stream``, or the current one of the current device.  The latter is read without
+    building a ``torch.cuda.Stream``, which took a third of the host's time per launch."""
+    if stream is not None:
+        return c_void_p(stream.cuda_stream)
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))

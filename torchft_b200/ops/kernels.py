@@ -59,6 +59,9 @@ def _check_2d_bf16(t: torch.Tensor, name: str) -> None:
 GEMM_IMPL = os.environ.get("FTB200_GEMM", "2cta")
 
 
+_GEMM_ARGS = (N.c_void_p,) * 3 + (c_int,) * 5 + (c_ll,) * 3 + (c_int, N.c_void_p, c_int, N.c_void_p)
+
+
 def gemm(
     a: torch.Tensor,
     b: torch.Tensor,
@@ -104,10 +107,11 @@ def gemm(
         return out
     flags = (1 if out.dtype == torch.float32 else 0) | (2 if accumulate else 0)
     fn = N.lib().ftb200_gemm_bf16_2cta if (impl or GEMM_IMPL) == "2cta" else N.lib().ftb200_gemm_bf16
+    if fn.argtypes is None:
+        fn.argtypes = _GEMM_ARGS  # plain Python numbers from here on: no ctypes object per argument
     rc = fn(
-        ptr(a), ptr(b), ptr(out), c_int(M), c_int(Nn), c_int(K), c_int(int(a_mn_major)), c_int(int(b_mn_major)),
-        c_ll(a.stride(0)), c_ll(b.stride(0)), c_ll(out.stride(0)), c_int(flags), ptr(status_word(a.device)),
-        c_int(max_ctas), stream_ptr(),
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, int(a_mn_major), int(b_mn_major), a.stride(0), b.stride(0),
+        out.stride(0), flags, status_word(a.device).data_ptr(), max_ctas, stream_ptr(),
     )
     N.check(rc, "gemm_bf16")
     return out
@@ -631,7 +635,7 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
     lib = N.lib()
     lib.ftb200_attention_bwd_scratch_bytes.restype = ctypes.c_longlong
     need = int(lib.ftb200_attention_bwd_scratch_bytes(c_int(batch), c_int(seq_len), c_int(n_heads)))
-    key = (q.device.index, torch.cuda.current_stream().cuda_stream)
+    key = (q.device.index, stream_ptr().value)
     scratch = _attn_scratch.get(key)
     if scratch is None or scratch.numel() < need:
         scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
