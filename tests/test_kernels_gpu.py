@@ -34,6 +34,25 @@ def test_gemm_layouts(a_mn, b_mn, M, N, K_, impl):
     assert rel_err(acc, ref + 1.0) < 1e-2
 
 
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("N", [128 * 74 - 8, 128 * 74, 128 * 74 + 8, 128 * 75 + 136])
+def test_gemm_tile_width(a_mn, b_mn, N):
+    """On both sides of the line between 128- and 256-column tiles (74 CTA pairs on 148 SMs), with remainders in every
+    dimension.  Same sums in the same order either way: bf16 rounding of the result is the whole error (2^-9 relative)."""
+    torch.manual_seed(9)
+    M, K_ = 200, 328
+    a = torch.randn((K_, M) if a_mn else (M, K_), device=DEV).bfloat16()
+    b = torch.randn((K_, N) if b_mn else (N, K_), device=DEV).bfloat16()
+    ref = (a.float().t() if a_mn else a.float()) @ (b.float() if b_mn else b.float().t())
+    out = torch.full((M, N + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    K.gemm(a, b, a_mn, b_mn, out=out[:, :N])
+    assert rel_err(out[:, :N], ref) < 4e-3 and bool((out[:, N:] == 7.0).all())
+    acc = torch.ones(M, N, device=DEV, dtype=torch.float32)
+    K.gemm(a, b, a_mn, b_mn, out=acc, accumulate=True)
+    assert rel_err(acc, ref + 1.0) < 1e-5
+    K.check_status(out.device)
+
+
 @pytest.mark.parametrize("impl", ["1cta", "2cta"])
 def test_gemm_many_tiles_persistent(impl):
     torch.manual_seed(2)

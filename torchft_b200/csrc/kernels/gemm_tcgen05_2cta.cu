@@ -1,7 +1,7 @@
 // bf16 GEMM with 2-SM tensor-core instructions (tcgen05.mma.cta_group::2).
 //
 // Same contract as the 1-CTA kernel in gemm_tcgen05.cu.  Two CTAs of a cluster share
-// one 256x256 output tile: each stages its own 128 rows of A and its own 128 of the 256
+// one 256x256 output tile (256x128 where the output is small, see tile_columns): each stages its own 128 rows of A and its own 128 of the 256
 // B columns (32 KiB per 64-deep K slab instead of 48 KiB), the pair's leader issues one
 // M=256 MMA that reads both halves of B, and each CTA's TMEM receives the accumulator of
 // its own 128 rows.  Per SM that is a third less shared-memory fill traffic per FLOP and
@@ -36,20 +36,28 @@
 namespace {
 
 constexpr int BM = 128;  // rows per CTA (256 per pair)
-constexpr int BN = 256;  // columns per pair
-constexpr int BNH = BN / 2;
 constexpr int BK = 64;
-constexpr int STAGES = 6;
 constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
-constexpr uint32_t B_BYTES = BNH * BK * 2;
-constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+
+// A pair's tile has 256 or 128 columns; the K ring fills the same 192 KB with 6 or 8 stages.
+template <int BN_>
+struct Tile {
+  static constexpr int BN = BN_;        // columns per pair
+  static constexpr int BNH = BN / 2;    // of B's rows, per CTA
+  static constexpr int STAGES = BN == 256 ? 6 : 8;
+  static constexpr uint32_t B_BYTES = BNH * BK * 2;
+  static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+  static_assert(STAGES * STAGE_BYTES == 196608, "the epilogue's staging area follows the ring");
+};
+constexpr uint32_t RING_BYTES = 196608;
+constexpr int GATHER_BLOCK = 128;  // B rows whose pieces the all-gather counts together: a CTA's half of a 256-column tile
 constexpr int NUM_THREADS = 192;
 constexpr int GATHER_WARPS = 4;  // only launched by the all-gather variant
 constexpr int NUM_THREADS_GATHER = NUM_THREADS + 32 * GATHER_WARPS;
 constexpr int GATHER_PIECE_V = 1024;  // 16-byte vectors per piece (16 KiB)
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+constexpr uint32_t SMEM_BYTES = RING_BYTES + 1024 + 256;
 constexpr uint32_t SC_STAGE_WARP_BYTES = 32 * 256;  // scatter epilogue: 32 rows x 128 bf16 per warp
 constexpr uint32_t SMEM_BYTES_SCATTER = SMEM_BYTES + 4 * SC_STAGE_WARP_BYTES;
 constexpr int GROUP_M = 8;  // in 256-row pair tiles (the all-gather variant uses twice that)
@@ -157,9 +165,13 @@ __device__ __forceinline__ bool count_wait(const unsigned int* p, unsigned int w
   }
 }
 
+template <int BN_>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS_GATHER, 1)
 gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                               const GemmParams p) {
+  using TL = Tile<BN_>;
+  constexpr int BN = TL::BN, BNH = TL::BNH, STAGES = TL::STAGES;
+  constexpr uint32_t STAGE_BYTES = TL::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -230,10 +242,10 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       int m0, n0;
       tile_coords(t, m0, n0);
       const int nb = n0 + static_cast<int>(rank) * BNH;  // this CTA's half of the B tile
-      if (p.ga_world > 0 && nb < p.N) {
+      if (BNH == GATHER_BLOCK && p.ga_world > 0 && nb < p.N) {
         // these 128 rows of B are local once all their pieces are counted; the loads below go through the
         // async proxy, the pieces were written through the generic one
-        if (!__all_sync(0xffffffffu, count_wait(p.ga_sync + 1 + nb / BNH, static_cast<unsigned int>(p.K / 64), abort_flag))) {
+        if (!__all_sync(0xffffffffu, count_wait(p.ga_sync + 1 + nb / GATHER_BLOCK, static_cast<unsigned int>(p.K / 64), abort_flag))) {
           ok = false;
           break;
         }
@@ -587,6 +599,42 @@ struct GatherSpec {
   unsigned int* sync = nullptr;
 };
 
+// Columns of a pair's tile: 128 where the narrow tiles of the whole output fit the pairs at once, 256 elsewhere.  A narrow
+// tile takes about 0.7 of a wide one's time (it asks the L2 for 96 bytes a cycle and SM instead of 64), so it pays where
+// it only puts idle pairs to work: 1024 x 1024 x 3000 26.0 -> 17.3 us, 256 x 1024 x 256 9.8 -> 6.3 us; but 3000 x 5632 x
+// 1024 36.0 -> 40.6 us, 1536 x 4096 x 14336 146 -> 169 us.
+static int tile_columns(int M, int N, int pairs) {
+  const long long rows = (M + 2 * BM - 1) / (2 * BM);
+  return rows * ((N + 127) / 128) <= pairs ? 128 : 256;
+}
+
+template <int BN>
+static int launch_2cta(const void* A, const void* B, long long lda, long long ldb, int ctas, int threads, const GemmParams& p,
+                       cudaStream_t stream) {
+  CUtensorMap tmA, tmB;
+  int rc;
+  if (!p.a_mn)
+    rc = encode_2d(&tmA, A, p.M, p.K, lda, BK, BM);
+  else
+    rc = encode_2d(&tmA, A, p.K, p.M, lda, 64, BK);
+  if (rc) return rc;
+  if (!p.b_mn)
+    rc = encode_2d(&tmB, B, p.N, p.K, ldb, BK, BN / 2);
+  else
+    rc = encode_2d(&tmB, B, p.K, p.N, ldb, 64, BK);
+  if (rc) return rc;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(gemm_bf16_tcgen05_2cta_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SMEM_BYTES_SCATTER) != cudaSuccess)
+      return FTB200_E_CUDA;
+    attr_set = true;
+  }
+  const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
+  gemm_bf16_tcgen05_2cta_kernel<BN><<<std::min(2 * tiles, ctas), threads, SMEM_BYTES_SCATTER, stream>>>(tmA, tmB, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+}
+
 static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, int b_mn_major,
                           long long lda, long long ldb, long long ldc, int flags, int* status, int max_ctas, void* aux,
                           long long ld_aux, cudaStream_t stream, const ScatterSpec* sc = nullptr,
@@ -595,26 +643,6 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
     return FTB200_E_ALIGN;
   if ((reinterpret_cast<uintptr_t>(C) & 15)) return FTB200_E_ALIGN;
-  CUtensorMap tmA, tmB;
-  int rc;
-  if (!a_mn_major)
-    rc = encode_2d(&tmA, A, M, K, lda, BK, BM);
-  else
-    rc = encode_2d(&tmA, A, K, M, lda, 64, BK);
-  if (rc) return rc;
-  if (!b_mn_major)
-    rc = encode_2d(&tmB, B, N, K, ldb, BK, BNH);
-  else
-    rc = encode_2d(&tmB, B, K, N, ldb, 64, BK);
-  if (rc) return rc;
-
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_bf16_tcgen05_2cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SMEM_BYTES_SCATTER) != cudaSuccess)
-      return FTB200_E_CUDA;
-    attr_set = true;
-  }
   GemmParams p;
   p.M = M; p.N = N; p.K = K;
   p.a_mn = a_mn_major ? 1 : 0;
@@ -657,16 +685,14 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
     // a quarter, which halves the link bandwidth the gather needs to stay ahead, and costs ~2.5 % of the GEMM's
     // speed in L2 locality (measured; all of M per B tile costs ~9 %).
     p.group_m = 2 * GROUP_M;
-    if (cudaMemsetAsync(ga->sync, 0, sizeof(unsigned int) * (1 + static_cast<size_t>(N) / BNH), stream) != cudaSuccess)
+    if (cudaMemsetAsync(ga->sync, 0, sizeof(unsigned int) * (1 + static_cast<size_t>(N) / GATHER_BLOCK), stream) != cudaSuccess)
       return FTB200_E_CUDA;
   }
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
   int ctas = ftb200::sm_count() & ~1;
   if (max_ctas > 0 && max_ctas < ctas) ctas = std::max(2, max_ctas & ~1);
-  if (2 * tiles < ctas) ctas = 2 * tiles;
-  gemm_bf16_tcgen05_2cta_kernel<<<ctas, ga != nullptr ? NUM_THREADS_GATHER : NUM_THREADS, SMEM_BYTES_SCATTER, stream>>>(
-      tmA, tmB, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+  if (ga != nullptr) return launch_2cta<256>(A, B, lda, ldb, ctas, NUM_THREADS_GATHER, p, stream);
+  if (tile_columns(M, N, ctas / 2) == 128) return launch_2cta<128>(A, B, lda, ldb, ctas, NUM_THREADS, p, stream);
+  return launch_2cta<256>(A, B, lda, ldb, ctas, NUM_THREADS, p, stream);
 }
 
 FTB200_API int ftb200_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major,
@@ -718,7 +744,7 @@ FTB200_API int ftb200_gemm_bf16_gather(const void* A, void* B_local, void* C, in
                                        long long unit_off, unsigned int* sync_words, void* aux, long long ld_aux,
                                        int* status, int max_ctas, cudaStream_t stream) {
   if (shard_peers == nullptr || sync_words == nullptr || world < 1 || world > 8) return FTB200_E_BADARG;
-  if ((N % BNH) || (K % 64) || (shard_elems % 8) || (unit_off % 8) || (ldc & 7)) return FTB200_E_ALIGN;
+  if ((N % GATHER_BLOCK) || (K % 64) || (shard_elems % 8) || (unit_off % 8) || (ldc & 7)) return FTB200_E_ALIGN;
   if (shard_elems < 8LL * GATHER_PIECE_V) return FTB200_E_BADARG;  // a piece may cross one shard boundary, not two
   if (unit_off + static_cast<long long>(N) * K > shard_elems * world) return FTB200_E_TOOBIG;
   for (int r = 0; r < world; ++r)
