@@ -609,10 +609,13 @@ int for_list(void* const* data, const long long* numel, int count, long long n, 
 constexpr int QUANT_GROUPS = 2;
 constexpr int DEQUANT_GROUPS = 4;
 
-int grid_for_list(const TensorList& l, int groups) {
+int grid_for_list(const TensorList& l, int groups, bool resident) {
   const long long per_cta = 8LL * BPW * groups;  // 8 warps, each BPW * groups blocks at a time
   const long long g = (l.blk_hi - l.blk_lo + per_cta - 1) / per_cta;
-  return static_cast<int>(std::max<long long>(1, std::min<long long>(g, ftb200::sm_count() * 8LL)));
+  // Blocks that take their part and leave stream best, except where bf16 is quantised, which is bound by its arithmetic
+  // and not by memory (243 M elements, eight looping blocks per SM against this: bf16 quantise 145 / 170 us, dequantise
+  // 133 / 115; fp32 190 / 176 and 213 / 191).
+  return static_cast<int>(std::min<long long>(g, resident ? ftb200::sm_count() * 8LL : 0x7fffffffLL));
 }
 
 }  // namespace
@@ -621,7 +624,7 @@ int grid_for_list(const TensorList& l, int groups) {
 FTB200_API int ftb200_quantize_list_fp8(void* const* data, const long long* numel, int count, void* codes, float* scales,
                                         long long n, int dtype, cudaStream_t st) {
   return for_list(data, numel, count, n, [&](const TensorList& l) {
-    const int grid = grid_for_list(l, QUANT_GROUPS);
+    const int grid = grid_for_list(l, QUANT_GROUPS, dtype == 0);
     if (dtype == 0)
       quantize_list_kernel<__nv_bfloat16, QUANT_GROUPS><<<grid, 256, 0, st>>>(l, (uint8_t*)codes, scales);
     else
@@ -632,7 +635,7 @@ FTB200_API int ftb200_quantize_list_fp8(void* const* data, const long long* nume
 FTB200_API int ftb200_dequantize_list_fp8(void* const* data, const long long* numel, int count, const void* codes,
                                           const float* scales, long long n, int dtype, cudaStream_t st) {
   return for_list(data, numel, count, n, [&](const TensorList& l) {
-    const int grid = grid_for_list(l, DEQUANT_GROUPS);
+    const int grid = grid_for_list(l, DEQUANT_GROUPS, false);
     if (dtype == 0)
       dequantize_list_kernel<__nv_bfloat16, DEQUANT_GROUPS><<<grid, 256, 0, st>>>(l, (const uint8_t*)codes, scales);
     else
