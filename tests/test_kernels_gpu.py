@@ -137,6 +137,21 @@ def test_cross_entropy(T, V):
     assert rel_err(logits, rg) < 1e-2
 
 
+@pytest.mark.parametrize("V", [8, 8 * 1024, 8 * 1024 + 8, 8 * 3 * 1024 - 8, 128256])
+def test_cross_entropy_without_gradient(V):
+    """One to several vectors per thread, with remainders; the logits stay as they are and the loss is the same number."""
+    torch.manual_seed(10)
+    logits = (torch.randn(3, V, device=DEV) * 3).bfloat16()
+    tgt = torch.tensor([0, V - 1, -1], device=DEV)
+    kept = logits.clone()
+    loss = K.cross_entropy_(logits, tgt, 1.0, grad=False)
+    assert torch.equal(logits, kept) and loss[2] == 0
+    want = torch.nn.functional.cross_entropy(kept.double(), tgt.clamp(min=0), reduction="none")[:2]
+    assert rel_err(loss[:2], want) < 1e-5  # fp32 sums of V terms
+    assert torch.equal(K.cross_entropy_(logits, tgt, 1.0), loss)
+    assert rel_err(logits[:2], K.ref_cross_entropy(kept, tgt.clamp(min=0), 1.0)[1][:2]) < 1e-2 and not logits[2].any()
+
+
 @pytest.mark.parametrize("gdt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n", [8, 1000, 1 << 20, (1 << 20) + 3])
 def test_adamw(gdt, n):

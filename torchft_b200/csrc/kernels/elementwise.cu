@@ -265,17 +265,21 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ ds, const bf
 }
 
 // ------------------------------------------------------------------ cross-entropy
-// One block per row.  loss[row] = logsumexp(row) - row[target]; the row is overwritten
-// in place by (softmax - onehot) * grad_scale.
-__global__ void cross_entropy_kernel(bf16x8* __restrict__ logits, const int64_t* __restrict__ target,
-                                     float* __restrict__ loss, int V8, int64_t ld8, float grad_scale) {
+// One block per row.  loss[row] = logsumexp(row) - row[target]; with `grad` the row is overwritten in place by
+// (softmax - onehot) * grad_scale, without it it is only read.  Bound by memory and, next to it, by the exponential
+// unit; CE_LOADS loads in flight per thread and two blocks per SM.
+constexpr int CE_LOADS = 2;
+
+__global__ void __launch_bounds__(1024, 2)
+cross_entropy_kernel(bf16x8* __restrict__ logits, const int64_t* __restrict__ target, float* __restrict__ loss, int V8,
+                     int64_t ld8, float grad_scale, int grad) {
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
   bf16x8* lr = logits + row * ld8;
   float mx = -INFINITY, sum = 0.f;
-  for (int i = threadIdx.x; i < V8; i += blockDim.x) {
+  auto take = [&](const bf16x8& v) {
     float f[8];
-    unpack8(lr[i], f);
+    unpack8(v, f);
     float cm = f[0];
 #pragma unroll
     for (int e = 1; e < 8; ++e) cm = fmaxf(cm, f[e]);
@@ -285,7 +289,17 @@ __global__ void cross_entropy_kernel(bf16x8* __restrict__ logits, const int64_t*
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) sum += __expf(f[e] - mx);
+  };
+  const int step = blockDim.x;
+  int i = threadIdx.x;
+  for (; i + (CE_LOADS - 1) * step < V8; i += CE_LOADS * step) {
+    bf16x8 v[CE_LOADS];
+#pragma unroll
+    for (int u = 0; u < CE_LOADS; ++u) v[u] = lr[i + u * step];
+#pragma unroll
+    for (int u = 0; u < CE_LOADS; ++u) take(v[u]);
   }
+  for (; i < V8; i += step) take(lr[i]);
   const float gmx = ftb200::block_max(mx, scratch);
   sum *= __expf(mx - gmx);
   const float gsum = ftb200::block_sum(sum, scratch);
@@ -298,19 +312,28 @@ __global__ void cross_entropy_kernel(bf16x8* __restrict__ logits, const int64_t*
     const float xt = (tgt >= 0 && tgt < 8 * static_cast<int64_t>(V8)) ? __bfloat162float(flat[tgt]) : 0.f;
     loss[row] = (tgt >= 0) ? (logf(gsum) + gmx - xt) : 0.f;
   }
+  if (!grad) return;
   __syncthreads();  // the target logit is read before any thread overwrites it
   const float gs = (tgt >= 0) ? grad_scale : 0.f;
-  for (int i = threadIdx.x; i < V8; i += blockDim.x) {
+  auto put = [&](const bf16x8& v, int at) {
     float f[8];
-    unpack8(lr[i], f);
+    unpack8(v, f);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       float pr = __expf(f[e] - gmx) * inv;
-      if (static_cast<int64_t>(i) * 8 + e == tgt) pr -= 1.f;
+      if (static_cast<int64_t>(at) * 8 + e == tgt) pr -= 1.f;
       f[e] = pr * gs;
     }
-    lr[i] = pack8(f);
+    lr[at] = pack8(f);
+  };
+  for (i = threadIdx.x; i + (CE_LOADS - 1) * step < V8; i += CE_LOADS * step) {
+    bf16x8 v[CE_LOADS];
+#pragma unroll
+    for (int u = 0; u < CE_LOADS; ++u) v[u] = lr[i + u * step];
+#pragma unroll
+    for (int u = 0; u < CE_LOADS; ++u) put(v[u], i + u * step);
   }
+  for (; i < V8; i += step) put(lr[i], i);
 }
 
 // ------------------------------------------------------------------ AdamW (flat shard)
@@ -493,9 +516,9 @@ FTB200_API int ftb200_swiglu_bwd(const void* ds, const void* gu, void* dgu, long
 }
 
 FTB200_API int ftb200_cross_entropy(void* logits, const int64_t* target, float* loss, int T, int V, long long ld,
-                                    float grad_scale, cudaStream_t st) {
+                                    float grad_scale, int grad, cudaStream_t st) {
   if (V % 8 || ld % 8) return FTB200_E_ALIGN;
-  cross_entropy_kernel<<<T, 1024, 0, st>>>((bf16x8*)logits, target, loss, V / 8, ld / 8, grad_scale);
+  cross_entropy_kernel<<<T, 1024, 0, st>>>((bf16x8*)logits, target, loss, V / 8, ld / 8, grad_scale, grad);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 

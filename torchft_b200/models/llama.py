@@ -416,7 +416,7 @@ class LlamaEngine:
         for ci in range(self.logit_chunks):
             sl = slice(ci * rows, (ci + 1) * rows)
             K.linear_fwd(self.ws_n[sl], W.lm_head, out=self.logits)
-            K.cross_entropy_(self.logits, tgt[sl], self.grad_scale / T, loss=self.loss_rows[sl])
+            K.cross_entropy_(self.logits, tgt[sl], self.grad_scale / T, loss=self.loss_rows[sl], grad=train)
             if train:
                 K.linear_wgrad(self.logits, self.ws_n[sl], out=G.lm_head, accumulate=ci > 0)
                 K.linear_dgrad(self.logits, getattr(W.lm_head, "local", W.lm_head), out=self.ws_dn[sl])

@@ -452,19 +452,20 @@ def ref_cross_entropy(logits, target, grad_scale):
 
 
 def cross_entropy_(logits: torch.Tensor, target: torch.Tensor, grad_scale: float,
-                   loss: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Per-row loss; ``logits`` is overwritten by ``(softmax - onehot) * grad_scale``."""
+                   loss: Optional[torch.Tensor] = None, grad: bool = True) -> torch.Tensor:
+    """Per-row loss; ``logits`` is overwritten by ``(softmax - onehot) * grad_scale`` (left as it is without ``grad``)."""
     T, V = logits.shape
     if loss is None:
         loss = torch.empty(T, dtype=torch.float32, device=logits.device)
     if not logits.is_cuda:
         l, g = ref_cross_entropy(logits, target, grad_scale)
         loss.copy_(l)
-        logits.copy_(g)
+        if grad:
+            logits.copy_(g)
         return loss
     N.check(
         N.lib().ftb200_cross_entropy(ptr(logits), ptr(target), ptr(loss), c_int(T), c_int(V), c_ll(logits.stride(0)),
-                                     c_float(grad_scale), stream_ptr()),
+                                     c_float(grad_scale), c_int(int(grad)), stream_ptr()),
         "cross_entropy",
     )
     return loss
