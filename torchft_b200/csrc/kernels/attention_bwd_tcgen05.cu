@@ -107,7 +107,7 @@ struct BwdParams {
   int causal;
   float scale, scale_log2;
   const float* neg_lse2;   // [batch, n_heads, seq], -log2(e) times the forward's log-sum-exp
-  const float* neg_delta;  // [batch, n_heads, seq]
+  const float* neg_delta;  // [batch, n_heads, seq], -scale times delta
   float* dq_acc;           // fp32, zeroed; per 64-query tile and head: [16][D][4 queries]
   __nv_bfloat16* dK;   // rows batch*seq, row stride ld_dk
   __nv_bfloat16* dV;
@@ -372,7 +372,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int row = quarter * 32 + lane;  // key within the block
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     bool ok = true;
-    const unsigned long long scale2 = f2_pack(p.scale_log2, p.scale_log2);
+    const unsigned long long scale2 = f2_pack(p.scale_log2, p.scale_log2), dscale2 = f2_pack(p.scale, p.scale);
     const int key = jb * BKV + row;
     TileWalk w{hk * rep, first_q};
     if (grp == 1) next_tile(w);
@@ -390,7 +390,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       tc_fence_after();
       TRACE(t, 0);  // S complete
-      // pairs of -log2(e) lse and -delta, as the packed arithmetic takes them
+      // pairs of -log2(e) lse and -scale delta, as the packed arithmetic takes them
       const ulonglong2* stats2 = reinterpret_cast<const ulonglong2*>(smem + OFF_STATS + qs * STATS_BYTES) + g * (CPT / 4);
       const int q0 = w.qt * BQ + g * CPT;
       const bool diag = (p.causal != 0) && (q0 < jb * BKV + BKV);
@@ -436,10 +436,10 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int qi = 4 * c + 2 * e;
-            // dS without the softmax scale, which the stores of dQ and dK apply
+            // dS = P (scale dP - scale delta)
             const unsigned long long ds2 =
                 f2_mul(f2_pack(pe[qi], pe[qi + 1]),
-                       f2_add(f2_pack(__uint_as_float(dp[qi]), __uint_as_float(dp[qi + 1])), e == 0 ? d4.x : d4.y));
+                       f2_fma(f2_pack(__uint_as_float(dp[qi]), __uint_as_float(dp[qi + 1])), dscale2, e == 0 ? d4.x : d4.y));
             float s0, s1;
             f2_unpack(ds2, s0, s1);
             __nv_bfloat162 a = __floats2bfloat162_rn(pe[qi], pe[qi + 1]);
@@ -489,7 +489,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int c = 0; c < CW / 8; ++c) {
           float f[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = which == 0 ? __uint_as_float(v[8 * c + e]) : __uint_as_float(v[8 * c + e]) * p.scale;
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * c + e]);
           reinterpret_cast<ftb200::bf16x8*>(dst)[c] = ftb200::pack8(f);
         }
       }
@@ -505,7 +505,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 }
 
-// Before the main kernel, one pass over O and dO: neg_delta[b, h, s] = -sum_d dO O, neg_lse2 = -log2(e) lse, and the dQ
+// Before the main kernel, one pass over O and dO: neg_delta[b, h, s] = -scale sum_d dO O, neg_lse2 = -log2(e) lse, and the dQ
 // accumulator zeroed.  A thread takes 8 elements (16 bytes of each), D / 8 neighbouring lanes a (row, head).
 template <int D>
 __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bflo
                                                                  const float* __restrict__ lse, float* __restrict__ neg_lse2,
                                                                  float* __restrict__ neg_delta, float4* __restrict__ dq_acc,
                                                                  int seq, int n_heads, long long pieces, long long ld_o,
-                                                                 long long ld_do) {
+                                                                 long long ld_do, float scale) {
   constexpr int LANES = D / 8;
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool live = i < pieces;
@@ -534,16 +534,16 @@ __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bflo
   for (int k = LANES / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
   if (live && c % LANES == 0) {
     const long long at = (static_cast<long long>(r / seq) * n_heads + c / LANES) * seq + r % seq;
-    neg_delta[at] = -s;
+    neg_delta[at] = -s * scale;
     neg_lse2[at] = lse[at] * -1.4426950408889634f;
   }
 }
 
-// dq (bf16, row stride ld) = scale * accumulator (fp32, per 64-query tile and head [16][D][4 queries]); a thread takes 8
+// dq (bf16, row stride ld) = accumulator (fp32, per 64-query tile and head [16][D][4 queries]); a thread takes 8
 // head-dim elements of 4 queries.
 template <int D>
 __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
-                                                                long long pieces, int n_heads, long long ld, float scale) {
+                                                                long long pieces, int n_heads, long long ld) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= pieces) return;
   const int d8 = static_cast<int>(i % (D / 8));
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __
   for (int k = 0; k < 4; ++k) {
     float f[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) f[e] = scale * (k == 0 ? v[e].x : k == 1 ? v[e].y : k == 2 ? v[e].z : v[e].w);
+    for (int e = 0; e < 8; ++e) f[e] = k == 0 ? v[e].x : k == 1 ? v[e].y : k == 2 ? v[e].z : v[e].w;
     *reinterpret_cast<ftb200::bf16x8*>(dq + (row0 + k) * ld + h * D + d8 * 8) = ftb200::pack8(f);
   }
 }
@@ -596,7 +596,7 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 }  // namespace
 
-// Scratch the backward pass needs, in bytes: fp32 dQ accumulator, -delta, -log2(e) lse.
+// Scratch the backward pass needs, in bytes: fp32 dQ accumulator, -scale delta, -log2(e) lse.
 // (sized for head dim 128; enough for 64 as well)
 FTB200_API long long ftb200_attention_bwd_scratch_bytes(int batch, int seq, int n_heads) {
   const long long rows = static_cast<long long>(batch) * seq;
@@ -633,7 +633,7 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   if ((pieces + 255) / 256 > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_bwd_prep_kernel<D><<<static_cast<unsigned>((pieces + 255) / 256), 256, 0, stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), lse, neg_lse2, neg_delta,
-      reinterpret_cast<float4*>(dq_acc), seq, n_heads, pieces, ld_o, ld_do);
+      reinterpret_cast<float4*>(dq_acc), seq, n_heads, pieces, ld_o, ld_do, scale);
   BwdParams p;
   p.batch = batch; p.seq = seq; p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.causal = causal;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
@@ -648,7 +648,7 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_bwd_kernel<D><<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
   attention_dq_cast_kernel<D><<<static_cast<unsigned>((pieces / 4 + 255) / 256), 256, 0, stream>>>(
-      reinterpret_cast<const float4*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), pieces / 4, n_heads, ld_dq, scale);
+      reinterpret_cast<const float4*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), pieces / 4, n_heads, ld_dq);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
