@@ -119,3 +119,52 @@ def test_attention_bwd_matches_reference(B, S, Hq, Hkv, causal, D):
         want = want.reshape(B * S, -1)
         err = (got.float() - want).norm() / want.norm()
         assert err < 2e-2, (name, err)
+
+
+@pytest.mark.parametrize("D,poly", [(64, None), (64, "0"), (64, "4"), (128, "0"), (128, "4")])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("key", [*range(8), 131, 200])
+def test_attention_fwd_keeps_non_finite_scores(monkeypatch, D, poly, bad, key):
+    """A key with a NaN or an infinity spoils the rows that see it, whichever unit its exponentials are computed on
+    (`poly` of every eight on the FMA pipe, None: the default), and no others."""
+    B, S, Hq, Hkv = 1, 256, 2, 1
+    monkeypatch.setenv("FTB200_ATTN_FWD", "pair")
+    if poly is None:
+        monkeypatch.delenv("FTB200_ATTN_POLY", raising=False)
+    else:
+        monkeypatch.setenv("FTB200_ATTN_POLY", poly)
+    _, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=key)
+    k[key, 0] = bad
+    out = torch.empty(B * S, Hq * D, dtype=torch.bfloat16, device="cuda")
+    lse = torch.empty(B, Hq, S, dtype=torch.float32, device="cuda")
+    K.attention_fwd(q, k, v, B, S, Hq, Hkv, D, out, lse)
+    K.check_status(out.device)
+    q4, k4, v4 = (t.reshape(B, S, -1, D) for t in (q, k, v))
+    ref = K.ref_attention(q4.float(), k4.float(), v4.float(), True)
+    got = out.float().reshape(ref.shape)
+    fine = ref.isfinite().all(-1)
+    assert torch.equal(got.isfinite().all(-1), fine) and not got[~fine].isfinite().any()
+    assert torch.equal(lse.isfinite(), fine.transpose(1, 2)) and (~fine).sum() >= (S - key) // 2
+    assert (got[fine] - ref[fine]).norm() <= 1e-2 * ref[fine].norm()  # no row is left where the first key is NaN
+
+
+@pytest.mark.parametrize("D,poly", [(64, None), (64, "4"), (128, "4")])
+@pytest.mark.parametrize("first", [97, 128, 230])
+def test_attention_fwd_masked_keys_have_no_weight(monkeypatch, D, poly, first):
+    """Values behind the mask, however large, leave the rows before them bit for bit as they are: the weight of a masked
+    score is zero on either unit."""
+    B, S, Hq, Hkv = 1, 256, 2, 1
+    monkeypatch.setenv("FTB200_ATTN_FWD", "pair")
+    if poly is None:
+        monkeypatch.delenv("FTB200_ATTN_POLY", raising=False)
+    else:
+        monkeypatch.setenv("FTB200_ATTN_POLY", poly)
+    _, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=first)
+    outs = []
+    for big in (0.0, 3e38):
+        v[first:] = big
+        out = torch.empty(B * S, Hq * D, dtype=torch.bfloat16, device="cuda")
+        K.attention_fwd(q, k, v, B, S, Hq, Hkv, D, out)
+        K.check_status(out.device)
+        outs.append(out[:first])
+    assert torch.equal(*outs)

@@ -247,14 +247,24 @@ __device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsig
   return r;
 }
 
+// max(a, b), NaN if either is (fmaxf would drop it).
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // 2^x of a pair, x <= 8, on the FMA pipe instead of the exponential unit: the nearest integer n by adding 1.5 * 2^23, a
 // polynomial of degree 5 in the remainder f in [-0.5, 0.5], n added to the exponent bits.  The coefficients minimise the
 // largest relative error over that interval (Lawson's iteration of weighted least squares): 7.5e-8, 2.1e-7 with the
 // fp32 evaluation, which is no more than that of the unit's own ex2.approx (2^-22).
+// As on the unit, NaN stays NaN and what is below the normal numbers is zero, -inf (a masked score) with it: x is held at
+// -127, where n = -127 and f >= 0 leave the exponent field zero and the sign bit alone, and the last product (x * 0 + the
+// result) flushes such a result and carries a NaN over the integer addition, which would lose it.
 __device__ __forceinline__ unsigned long long f2_exp2_poly(unsigned long long x2) {
   float x0, x1;
   f2_unpack(x2, x0, x1);
-  const unsigned long long x = f2_pack(fmaxf(x0, -125.f), fmaxf(x1, -125.f));
+  const unsigned long long x = f2_pack(max_nan(x0, -127.f), max_nan(x1, -127.f));
   const unsigned long long xr = f2_add(x, f2_pack(12582912.f, 12582912.f));
   const unsigned long long n = f2_add(xr, f2_pack(-12582912.f, -12582912.f));
   const unsigned long long f = f2_fma(n, f2_pack(-1.f, -1.f), x);
@@ -267,8 +277,9 @@ __device__ __forceinline__ unsigned long long f2_exp2_poly(unsigned long long x2
   float p0, p1, r0, r1;
   f2_unpack(p, p0, p1);
   f2_unpack(xr, r0, r1);
-  return f2_pack(__int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23)),
-                 __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23)));
+  return f2_fma(x, c(0.f),
+                f2_pack(__int_as_float(__float_as_int(p0) + (__float_as_int(r0) << 23)),
+                        __int_as_float(__float_as_int(p1) + (__float_as_int(r1) << 23))));
 }
 
 // Moves registers between warpgroups; N x 128 threads summed over a CTA's warpgroups must not exceed what it was
