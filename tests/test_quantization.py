@@ -229,6 +229,43 @@ def test_list_kernels_match_flat_kernels_gpu(numels, dtype):
         Q.fused_dequantize_from_fp8([leaf], Q.fused_quantize_into_fp8([leaf], world)[0], world)
 
 
+def test_overlapping_targets_are_recognised():
+    def overlaps(*ts):
+        return Q._launch_overlaps(list(ts), [t.is_contiguous() for t in ts])
+
+    x, y = torch.zeros(1000), torch.zeros(64, 48)
+    assert not overlaps(x[:600], x[600:], x[600:600], y, torch.zeros(0))
+    assert not overlaps(y[32:], y[:32], x[1:])
+    assert not overlaps(y[:, :16], x, y[:, 16:])           # interleaved, written by copies one after the other
+    assert overlaps(x, y, x)                               # the same tensor twice
+    assert overlaps(x[:600], y, x[599:])                   # one element in common
+    assert overlaps(x, x[10:20], x[500:600])               # inside
+    assert overlaps(y.t(), y[63:])                         # one of the two is not contiguous
+    assert overlaps(y[60:], y.t())
+    assert overlaps(x[:128].view(torch.uint8)[500:], x[:128])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_overlapping_targets_are_written_in_order_gpu(dtype):
+    """Tensors that share memory end as copies in the list's order leave them: the last one wins."""
+    base = with_outliers(5000, 3).to(dtype).cuda()
+
+    def views(b):
+        return [b[:1000], b[3000:4000].view(40, 25).t(), b[500:1700], b[:1000], b[3500:3777], b[2000:2001]]
+
+    ts = views(base)
+    buf, (n,) = Q.fused_quantize_into_fp8(ts, 2)
+    flat = torch.empty(n, dtype=dtype, device="cuda")
+    Q.dequantize_from(buf, flat)
+    want, off = base.clone(), 0
+    for t in views(want):
+        t.copy_(flat[off : off + t.numel()].view_as(t))
+        off += t.numel()
+    Q.fused_dequantize_from_fp8(ts, buf, 2)
+    assert torch.equal(base, want)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("world", [2, 4, 8])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

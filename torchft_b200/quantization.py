@@ -156,21 +156,42 @@ def _written_in_place(t: torch.Tensor, dtype: torch.dtype, device: torch.device)
             and not (t.requires_grad and torch.is_grad_enabled()) and not t.is_inference() and not t.is_neg())
 
 
+def _launch_overlaps(tensors: List[torch.Tensor], direct: List[bool]) -> bool:
+    """Whether the memory that a ``direct`` tensor spans (from the first element to the last) overlaps another's."""
+    spans = []
+    for t, ok in zip(tensors, direct):
+        if t.numel():
+            last = t.numel() - 1 if ok else sum((n - 1) * s for n, s in zip(t.shape, t.stride()))
+            begin = t.data_ptr()
+            spans.append((begin, begin + (last + 1) * t.element_size(), ok))
+    spans.sort()
+    end_all = end_direct = 0
+    for begin, end, ok in spans:
+        if begin < (end_all if ok else end_direct):
+            return True
+        end_all = max(end_all, end)
+        end_direct = max(end_direct, end) if ok else end_direct
+    return False
+
+
 def fused_dequantize_from_fp8(tensors: List[torch.Tensor], buf: torch.Tensor, world_size: int) -> None:
     """Inverse of :func:`fused_quantize_into_fp8`: write the values back into ``tensors``."""
     dtype, device = tensors[0].dtype, tensors[0].device
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
-    if device.type == "cuda" and total > 0 and buf.is_cuda:
+    if device.type == "cuda" and total > 0 and buf.is_cuda and all(type(t) in _PLAIN for t in tensors):
         direct = [_written_in_place(t, dtype, device) for t in tensors]
-        targets = [t if ok else torch.empty(t.shape, dtype=dtype, device=device) for t, ok in zip(tensors, direct)]
-        _list_call("ftb200_dequantize_list_fp8", targets, *split_quantized(buf, n), n)
-        for t, target, ok in zip(tensors, targets, direct):
-            if ok:
-                torch.autograd.graph.increment_version(t)
-            else:
-                t.copy_(target)
-        return
+        # One launch writes the direct ones in no order.  Where one shares memory with another tensor (listed twice,
+        # overlapping views) or with the buffer, the values go through a flat tensor and are copied in the list's order.
+        if not _launch_overlaps([*tensors, buf], [*direct, False]):
+            targets = [t if ok else torch.empty(t.shape, dtype=dtype, device=device) for t, ok in zip(tensors, direct)]
+            _list_call("ftb200_dequantize_list_fp8", targets, *split_quantized(buf, n), n)
+            for t, target, ok in zip(tensors, targets, direct):
+                if ok:
+                    torch.autograd.graph.increment_version(t)
+                else:
+                    t.copy_(target)
+            return
     flat = torch.empty(n, dtype=dtype, device=device)
     dequantize_from(buf, flat)
     off = 0
