@@ -12,6 +12,7 @@ from torch.distributed.distributed_c10d import ReduceOp
 
 from torchft_b200 import quantization as Q
 from torchft_b200.collectives import allreduce_quantized, reduce_scatter_quantized, allocate_reduce_scatter_output
+from torchft_b200.ops import _native as N
 from torchft_b200.process_group import ProcessGroupGloo
 
 
@@ -227,6 +228,51 @@ def test_list_kernels_match_flat_kernels_gpu(numels, dtype):
     leaf = torch.zeros(256, dtype=dtype, device="cuda", requires_grad=True)
     with pytest.raises(RuntimeError):  # as any write in place to a leaf
         Q.fused_dequantize_from_fp8([leaf], Q.fused_quantize_into_fp8([leaf], world)[0], world)
+
+
+def test_a_buffer_that_is_too_short_is_refused():
+    """A buffer packed for fewer ranks (less padding), cut short, or of another type, before anything reads it."""
+    ts = [torch.randn(1000), torch.randn(77)]
+    buf, (n,) = Q.fused_quantize_into_fp8(ts, 2)
+    for bad in (buf[:-1], buf[: n], buf.view(torch.int16), buf[None], buf[:0]):
+        with pytest.raises(AssertionError):
+            Q.fused_dequantize_from_fp8(ts, bad, 2)
+        with pytest.raises(AssertionError):
+            Q.dequantize_from(bad, torch.empty(n))
+    with pytest.raises(AssertionError):
+        Q.fused_dequantize_from_fp8(ts, buf, 16)
+    Q.fused_dequantize_from_fp8(ts, buf.view(torch.int8), 2)  # bytes are bytes
+
+
+@pytest.mark.parametrize("dtype,step", [(0, 8), (1, 4)])
+def test_misaligned_codes_are_refused_before_the_launch(dtype, step):
+    """The C entries look at the addresses (made up here) before they launch anything."""
+    lib, n = N.lib(), 256
+    bad_arg, align = -1, -2
+    data, numel = (ctypes.c_void_p * 1)(1 << 20), (ctypes.c_longlong * 1)(n + 1)  # one element too many: refused as well
+
+    def both(codes, scales, d=data):
+        return {fn(d, numel, ctypes.c_int(1), ctypes.c_void_p(codes), ctypes.c_void_p(scales), ctypes.c_longlong(n),
+                   ctypes.c_int(dtype), ctypes.c_void_p(0)) for fn in (lib.ftb200_quantize_list_fp8, lib.ftb200_dequantize_list_fp8)}
+
+    assert both(1 << 21, 1 << 22) == both((1 << 21) + step, 1 << 22) == {bad_arg}
+    assert both((1 << 21) + step // 2, 1 << 22) == {align}
+    assert both(1 << 21, (1 << 22) + 2) == {align}
+    assert both(1 << 21, 1 << 22, (ctypes.c_void_p * 1)((1 << 20) + 1)) == {align}
+
+
+@pytest.mark.gpu
+def test_a_buffer_that_is_too_short_is_refused_gpu():
+    ts = [torch.randn(1000, device="cuda")]
+    buf, (n,) = Q.fused_quantize_into_fp8(ts, 2)
+    with pytest.raises(AssertionError):
+        Q.fused_dequantize_from_fp8(ts, buf[:-1], 2)
+    with pytest.raises(AssertionError):
+        Q.fused_dequantize_from_fp8(ts, buf, 16)
+    out = [torch.empty_like(ts[0])]
+    Q.fused_dequantize_from_fp8(out, buf.cpu(), 2)  # a buffer elsewhere comes over first
+    Q.fused_dequantize_from_fp8(ts, buf, 2)
+    assert torch.equal(out[0], ts[0])
 
 
 def test_overlapping_targets_are_recognised():

@@ -536,6 +536,8 @@ __global__ void diloco_outer_kernel(const T* __restrict__ g, float* __restrict__
   }
 }
 
+bool misaligned(const void* p, int bytes) { return reinterpret_cast<uintptr_t>(p) % bytes != 0; }
+
 int grid_for_blocks(long long nblocks) {
   long long g = (nblocks * 8 + 511) / 512;
   return static_cast<int>(std::max<long long>(1, std::min<long long>(g, ftb200::sm_count() * 4LL)));
@@ -546,7 +548,7 @@ int grid_for_blocks(long long nblocks) {
 // dtype: 0 bf16, 1 fp32.  codes: n bytes, scales: n/128 floats.  b (optional) is subtracted.
 FTB200_API int ftb200_quantize_fp8(const void* a, const void* b, void* codes, float* scales, long long n, int dtype,
                                    cudaStream_t st) {
-  if (n <= 0 || n % QB) return FTB200_E_ALIGN;
+  if (n <= 0 || n % QB || misaligned(codes, 16) || misaligned(scales, 4)) return FTB200_E_ALIGN;
   const long long nb = n / QB;
   if (dtype == 0)
     quantize_kernel<__nv_bfloat16><<<grid_for_blocks(nb), 512, 0, st>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
@@ -558,7 +560,7 @@ FTB200_API int ftb200_quantize_fp8(const void* a, const void* b, void* codes, fl
 
 FTB200_API int ftb200_dequantize_fp8(const void* codes, const float* scales, void* out, long long n, int dtype,
                                      cudaStream_t st) {
-  if (n <= 0 || n % QB) return FTB200_E_ALIGN;
+  if (n <= 0 || n % QB || misaligned(codes, 16) || misaligned(scales, 4)) return FTB200_E_ALIGN;
   const long long nb = n / QB;
   if (dtype == 0)
     dequantize_kernel<__nv_bfloat16><<<grid_for_blocks(nb), 512, 0, st>>>((const uint4*)codes, scales, (__nv_bfloat16*)out, nb);
@@ -571,10 +573,15 @@ namespace {
 
 // Cuts a list of tensors (data[i], numel[i] elements, empty ones allowed) into launches of at most LIST_MAX tensors and
 // whole blocks of the buffer's n elements, and calls launch(list) for each.  The blocks behind the last tensor belong
-// to the last launch.
+// to the last launch.  A piece's codes (LV bytes) are read and written at once, so the buffer's codes begin on a multiple
+// of that; the tensors may begin anywhere that their type allows.
 template <typename F>
-int for_list(void* const* data, const long long* numel, int count, long long n, F launch) {
-  if (n <= 0 || n % QB || count < 0) return FTB200_E_ALIGN;
+int for_list(void* const* data, const long long* numel, int count, const void* codes, const float* scales, long long n,
+             int dtype, F launch) {
+  const int size = dtype == 0 ? 2 : 4;
+  if (n <= 0 || n % QB || count < 0 || misaligned(codes, 16 / size) || misaligned(scales, 4)) return FTB200_E_ALIGN;
+  for (int i = 0; i < count; ++i)
+    if (misaligned(data[i], size)) return FTB200_E_ALIGN;
   long long total = 0;
   for (int i = 0; i < count; ++i) {
     if (numel[i] < 0 || (numel[i] > 0 && data[i] == nullptr)) return FTB200_E_BADARG;
@@ -623,7 +630,7 @@ int grid_for_list(const TensorList& l, int groups, bool resident) {
 // Quantises count tensors (contiguous, numel[i] elements of the type) as one buffer of n elements, zeros behind them.
 FTB200_API int ftb200_quantize_list_fp8(void* const* data, const long long* numel, int count, void* codes, float* scales,
                                         long long n, int dtype, cudaStream_t st) {
-  return for_list(data, numel, count, n, [&](const TensorList& l) {
+  return for_list(data, numel, count, codes, scales, n, dtype, [&](const TensorList& l) {
     const int grid = grid_for_list(l, QUANT_GROUPS, dtype == 0);
     if (dtype == 0)
       quantize_list_kernel<__nv_bfloat16, QUANT_GROUPS><<<grid, 256, 0, st>>>(l, (uint8_t*)codes, scales);
@@ -634,7 +641,7 @@ FTB200_API int ftb200_quantize_list_fp8(void* const* data, const long long* nume
 
 FTB200_API int ftb200_dequantize_list_fp8(void* const* data, const long long* numel, int count, const void* codes,
                                           const float* scales, long long n, int dtype, cudaStream_t st) {
-  return for_list(data, numel, count, n, [&](const TensorList& l) {
+  return for_list(data, numel, count, codes, scales, n, dtype, [&](const TensorList& l) {
     const int grid = grid_for_list(l, DEQUANT_GROUPS, false);
     if (dtype == 0)
       dequantize_list_kernel<__nv_bfloat16, DEQUANT_GROUPS><<<grid, 256, 0, st>>>(l, (const uint8_t*)codes, scales);

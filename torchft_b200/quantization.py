@@ -38,6 +38,12 @@ def padded_numel(n: int, world_size: int = 1) -> int:
     return (n + g - 1) // g * g
 
 
+def _check_buffer(buf: torch.Tensor, n: int) -> None:
+    """The kernels go by ``n`` and see pointers only, and a slice that is too long comes out short without a word."""
+    assert buf.dim() == 1 and buf.element_size() == 1 and buf.numel() >= quantized_nbytes(n), (
+        f"{n} elements take a flat byte buffer of {quantized_nbytes(n)}, got {tuple(buf.shape)} of {buf.dtype}")
+
+
 def split_quantized(buf: torch.Tensor, n: int) -> Tuple[torch.Tensor, torch.Tensor]:
     """Views ``(codes uint8 [n], scales fp32 [n/128])`` into a quantised buffer."""
     return buf[:n], buf[n : n + (n // BLOCK) * 4].view(torch.float32)
@@ -85,6 +91,9 @@ def dequantize_from(buf: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """Dequantise the quantised buffer ``buf`` into flat ``out`` (whose length is a multiple of the block size)."""
     n = out.numel()
     assert n % BLOCK == 0
+    _check_buffer(buf, n)
+    if out.is_cuda:
+        buf = buf.to(out.device)
     codes, scales = split_quantized(buf, n)
     if not out.is_cuda:
         out.copy_(ref_dequantize(codes, scales, out.dtype).view_as(out))
@@ -179,7 +188,8 @@ def fused_dequantize_from_fp8(tensors: List[torch.Tensor], buf: torch.Tensor, wo
     dtype, device = tensors[0].dtype, tensors[0].device
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
-    if device.type == "cuda" and total > 0 and buf.is_cuda and all(type(t) in _PLAIN for t in tensors):
+    _check_buffer(buf, n)
+    if device.type == "cuda" and total > 0 and buf.device == device and all(type(t) in _PLAIN for t in tensors):
         direct = [_written_in_place(t, dtype, device) for t in tensors]
         # One launch writes the direct ones in no order.  Where one shares memory with another tensor (listed twice,
         # overlapping views) or with the buffer, the values go through a flat tensor and are copied in the list's order.
