@@ -275,6 +275,16 @@ def test_a_buffer_that_is_too_short_is_refused_gpu():
     assert torch.equal(out[0], ts[0])
 
 
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_tensors_without_storage_are_zeros(device):
+    """Zeros as forward-mode autograd makes them have no memory to read."""
+    x = torch.randn(300).to(device)
+    zero = torch._efficientzerotensor((77,), device=device)
+    got, _ = Q.fused_quantize_into_fp8([x, zero], 2)
+    want, _ = Q.fused_quantize_into_fp8([x, torch.zeros(77, device=device)], 2)
+    assert torch.equal(got, want)
+
+
 def test_overlapping_targets_are_recognised():
     def overlaps(*ts):
         return Q._launch_overlaps(list(ts), [t.is_contiguous() for t in ts])

@@ -118,7 +118,9 @@ def reduce_quantized(bufs: List[torch.Tensor], n: int, scale: float, out: torch.
 # --------------------------------------------------------------------------- list-of-tensors API
 
 
-_PLAIN = (torch.Tensor, torch.nn.Parameter)
+def _plain(t: torch.Tensor) -> bool:
+    """A tensor whose elements lie where ``data_ptr`` says: no subclass, and not one of autograd's zeros without storage."""
+    return type(t) in (torch.Tensor, torch.nn.Parameter) and not t._is_zerotensor()
 
 
 def _list_call(name: str, tensors: List[torch.Tensor], codes: torch.Tensor, scales: torch.Tensor, n: int) -> None:
@@ -139,7 +141,7 @@ def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tup
     assert dtype in _DT, f"unsupported dtype {dtype}"
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
-    if device.type == "cuda" and total > 0 and all(type(t) in _PLAIN for t in tensors):
+    if device.type == "cuda" and total > 0 and all(map(_plain, tensors)):
         for t in tensors:
             assert t.dtype == dtype and t.device == device
         buf = torch.empty(quantized_nbytes(n), dtype=torch.uint8, device=device)
@@ -159,9 +161,9 @@ def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tup
 
 
 def _written_in_place(t: torch.Tensor, dtype: torch.dtype, device: torch.device) -> bool:
-    """Whether a kernel may write ``t`` directly; the rest takes ``copy_`` with its checks and conversions (other types
-    and devices, strides, leaves that require grad, inference tensors, tensor subclasses)."""
-    return (type(t) in _PLAIN and t.dtype == dtype and t.device == device and t.is_contiguous()
+    """Whether a kernel may write the plain tensor ``t`` directly; the rest takes ``copy_`` with its checks and
+    conversions (other types and devices, strides, leaves that require grad, inference tensors)."""
+    return (t.dtype == dtype and t.device == device and t.is_contiguous()
             and not (t.requires_grad and torch.is_grad_enabled()) and not t.is_inference() and not t.is_neg())
 
 
@@ -189,7 +191,7 @@ def fused_dequantize_from_fp8(tensors: List[torch.Tensor], buf: torch.Tensor, wo
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
     _check_buffer(buf, n)
-    if device.type == "cuda" and total > 0 and buf.device == device and all(type(t) in _PLAIN for t in tensors):
+    if device.type == "cuda" and total > 0 and buf.device == device and all(map(_plain, tensors)):
         direct = [_written_in_place(t, dtype, device) for t in tensors]
         # One launch writes the direct ones in no order.  Where one shares memory with another tensor (listed twice,
         # overlapping views) or with the buffer, the values go through a flat tensor and are copied in the list's order.
