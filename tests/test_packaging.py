@@ -3,6 +3,7 @@ console scripts, and an installed copy works away from the source tree (the refe
 maturin-built wheel with a ``torchft_lighthouse`` script, pyproject.toml:43-48)."""
 
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -29,6 +30,17 @@ def clean_setuptools_leftovers():
     for d in (REPO / "build").glob("bdist.*"):
         shutil.rmtree(d, ignore_errors=True)
     shutil.rmtree(REPO / "torchft_b200.egg-info", ignore_errors=True)
+
+
+def test_every_build_switch_of_the_sources_is_built():
+    """A block that only a hand-made build compiles is not seen by any test: the sources ask only for switches that the
+    build driver sets (or the compiler)."""
+    pkg = REPO / "torchft_b200"
+    asked = set()
+    for p in (pkg / "csrc").rglob("*.*"):
+        asked.update(re.findall(r"^\s*#\s*(?:ifn?def|(?:el)?if\s.*?defined)\W+(\w+)", p.read_text(), re.M))
+    asked.discard("__cplusplus")
+    assert asked == set(re.findall(r'"-D(\w+)', (pkg / "_build.py").read_text()))
 
 
 @pytest.mark.timeout(1500)

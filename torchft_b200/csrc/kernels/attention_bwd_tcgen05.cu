@@ -41,20 +41,6 @@ namespace {
 
 using namespace ftb200::tc;
 
-// Optional event trace for tuning (compiled in with -DFTB200_ATTN_TRACE): CTA 0 records clock64()
-// at pipeline events of its first tiles into p.trace[role][tile][event].
-#ifdef FTB200_ATTN_TRACE
-#define TRACE(tile, ev)                                                                              \
-  do {                                                                                              \
-    if (p.trace != nullptr && blockIdx.x == 0 && (tile) < 32 && (threadIdx.x & 31) == 0)            \
-      p.trace[((threadIdx.x >> 5) * 32 + (tile)) * 4 + (ev)] = clock64();                           \
-  } while (0)
-#else
-#define TRACE(tile, ev) \
-  do {                  \
-  } while (0)
-#endif
-
 constexpr int BKV = 128;
 constexpr int BQ = 64;
 constexpr int NUM_THREADS = 704;
@@ -113,7 +99,6 @@ struct BwdParams {
   __nv_bfloat16* dV;
   long long ld_dk, ld_dv;
   int* status;
-  long long* trace;  // tuning aid, null unless built with FTB200_ATTN_TRACE
 };
 
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -270,7 +255,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           break;
         }
         tc_fence_after();
-        TRACE(t, 0);  // S inputs ready
         const uint32_t qb_km = q_km0 + qs * STAGE16;
         if (elect_one()) {
 #pragma unroll
@@ -295,7 +279,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           umma_commit(bar(BAR_DP_FULL + st));
         }
         __syncwarp();
-        TRACE(t, 1);  // S, dP issued
       }
       if (t >= 1) {
         const int u = t - 1, pb = u & 1, qs = u % QDO_STAGES;
@@ -305,7 +288,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           break;
         }
         tc_fence_after();
-        TRACE(u, 2);  // P, dS ready for the tail of tile u
         const uint32_t qb_mn = q_mn0 + qs * STAGE16;
         const uint32_t dsb_mn = ds_mn0 + pb * PDS16;
         // queries 16k..16k+15 of tile u: P^T in columns 16k..16k+7 of its score buffer, dS^T in 16k+8..16k+15
@@ -327,7 +309,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           umma_commit(bar(BAR_QDO_EMPTY + qs));
         }
         __syncwarp();
-        TRACE(u, 3);  // tail issued
       }
     }
     if (ok && elect_one()) umma_commit(bar(BAR_DKV_DONE));
@@ -342,7 +323,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int buf = u & 1;
       if (!mbar_wait_warp(bar(BAR_DQ_FULL + buf), static_cast<uint32_t>(u >> 1) & 1u, abort_flag)) break;
       tc_fence_after();
-      TRACE(u, 0);  // dQ complete
       uint32_t v[BQ];
       const bool mine = quarter * 32 < D;  // head dim 64: only lanes 0..63 of dQ^T are real
       if (mine) {
@@ -352,7 +332,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       tc_fence_before();
       mbar_arrive_warp(bar(BAR_DQ_EMPTY + buf));
-      TRACE(u, 1);  // dQ in registers
       if (mine) {
         // four queries of one head-dim element lie together: a warp adds 512 consecutive bytes per instruction
         const long long tile = (static_cast<long long>(b) * n_qtiles + w.qt) * p.n_heads + w.h;
@@ -362,7 +341,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           red_add_v4(dst + c * (D * 4), __uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]), __uint_as_float(v[4 * c + 2]),
                      __uint_as_float(v[4 * c + 3]));
       }
-      TRACE(u, 2);  // added
     }
   } else {
     // ---------------- softmax, dK/dV store (warps 2..17) ----------------
@@ -389,7 +367,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         break;
       }
       tc_fence_after();
-      TRACE(t, 0);  // S complete
       // pairs of -log2(e) lse and -scale delta, as the packed arithmetic takes them
       const ulonglong2* stats2 = reinterpret_cast<const ulonglong2*>(smem + OFF_STATS + qs * STATS_BYTES) + g * (CPT / 4);
       const int q0 = w.qt * BQ + g * CPT;
@@ -425,7 +402,6 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             break;
           }
           tc_fence_after();
-          TRACE(t, 1);  // dP complete
           tmem_ld16(dp_addr, dp);
           tmem_wait_ld();
         }
@@ -463,12 +439,10 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
       }
       if (!ok) break;
-      TRACE(t, 2);  // math done
       fence_async_smem();
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive_warp(bar(BAR_PDS_FULL + grp));
-      TRACE(t, 3);  // P/dS published
     }
     if (ok && mbar_wait_warp(bar(BAR_DKV_DONE), 0, abort_flag)) {
       tc_fence_after();
@@ -640,10 +614,6 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   p.neg_lse2 = neg_lse2; p.neg_delta = neg_delta; p.dq_acc = dq_acc;
   p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
   p.ld_dk = ld_dk; p.ld_dv = ld_dv; p.status = status;
-  p.trace = nullptr;
-#ifdef FTB200_ATTN_TRACE
-  p.trace = reinterpret_cast<long long*>(neg_lse2 + rows * n_heads);  // the caller sized the scratch for it
-#endif
   const long long grid = static_cast<long long>(batch) * n_kv_heads * (seq / BKV);
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_bwd_kernel<D><<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);

@@ -34,20 +34,6 @@ namespace {
 
 using namespace ftb200::tc;
 
-// Optional event trace for tuning (compiled in with -DFTB200_ATTN_TRACE): the CTA with the most
-// key blocks records clock64() at pipeline events of its first blocks into p.trace[role][block][event].
-#ifdef FTB200_ATTN_TRACE
-#define TRACE(role, blk, ev)                                                                        \
-  do {                                                                                              \
-    if (p.trace != nullptr && blockIdx.x == 0 && (blk) < 32)                                        \
-      p.trace[((role) * 32 + (blk)) * 8 + (ev)] = clock64();                                        \
-  } while (0)
-#else
-#define TRACE(role, blk, ev) \
-  do {                       \
-  } while (0)
-#endif
-
 constexpr int D = 128;       // head dim
 constexpr int BQ = 128;      // queries per CTA
 constexpr int BKV = 128;     // keys per block
@@ -77,7 +63,6 @@ struct AttnParams {
   __nv_bfloat16* O;
   float* lse;        // [batch, n_heads, seq], natural log
   int* status;
-  long long* trace;  // tuning aid, null unless built with FTB200_ATTN_TRACE
 };
 
 // barrier indices
@@ -228,9 +213,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
           break;
         }
         tc_fence_after();
-        TRACE(0, j, 0);  // K of block j+1 present
         issue_s(j + 1);
-        TRACE(0, j, 1);  // S of block j+1 issued
       }
       if (!mbar_wait_warp(bar(BAR_P_FULL), static_cast<uint32_t>(j) & 1u, abort_flag) ||
           !mbar_wait_warp(bar(BAR_V_FULL + st), use & 1u, abort_flag)) {
@@ -238,7 +221,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
         break;
       }
       tc_fence_after();
-      TRACE(0, j, 2);  // P of block j and V present
       const uint32_t vb = v_lo + st * STAGE16;
       const uint32_t d_tmem = tmem_base + COL_O;
       // P of keys 32g..32g+31 sits, two per column, in the first 16 of the 32 columns its thread group read S from
@@ -252,7 +234,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
         umma_commit(bar(BAR_O_DONE));
       }
       __syncwarp();
-      TRACE(0, j, 3);  // P V of block j issued
     }
     __syncwarp();
   } else {
@@ -284,11 +265,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
         break;
       }
       tc_fence_after();
-      if (threadIdx.x == 64) TRACE(1, j, 0);  // S complete
       uint32_t sv[CPT];
       tmem_ld32(tmem_base + COL_S + st * BKV + g * CPT + lane_addr, sv);
       tmem_wait_ld();
-      if (threadIdx.x == 64) TRACE(1, j, 1);  // scores in registers
 
       if (p.causal && j == qb) {
         const int key0 = g * CPT;
@@ -308,7 +287,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
         break;
       }
       const float m_new = fmaxf(fmaxf(xc[row], xc[BQ + row]), fmaxf(xc[2 * BQ + row], xc[3 * BQ + row]));
-      if (threadIdx.x == 64) TRACE(1, j, 2);  // row maximum exchanged
 
       // raise the maximum only when it moved far; all threads of a row see the same numbers
       float alpha = 1.f;
@@ -334,7 +312,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
       }
       l_part += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
 
-      if (threadIdx.x == 64) TRACE(1, j, 3);  // exponentials done
       // P replaces the scores this thread has just read (its own columns: nobody else touches them)
       tmem_st16(tmem_base + COL_S + st * BKV + g * CPT + lane_addr, packed);
       if (any_raise) {
@@ -355,7 +332,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive_warp(bar(BAR_P_FULL));
-      if (threadIdx.x == 64) TRACE(1, j, 4);  // P published
     }
 
     if (ok && mbar_wait_warp(bar(BAR_O_DONE), static_cast<uint32_t>(n_kv - 1) & 1u, abort_flag)) {
@@ -458,10 +434,6 @@ FTB200_API int ftb200_attention_fwd(const void* q, const void* k, const void* v,
   p.scale_log2 = scale * 1.4426950408889634f;
   p.Q = reinterpret_cast<const __nv_bfloat16*>(q); p.ld_q = ld_q;
   p.ld_o = ld_o; p.O = reinterpret_cast<__nv_bfloat16*>(o); p.lse = lse; p.status = status;
-  p.trace = nullptr;
-#ifdef FTB200_ATTN_TRACE
-  p.trace = reinterpret_cast<long long*>(lse) + (static_cast<long long>(batch) * n_heads * seq + 1) / 2;  // caller over-allocates lse
-#endif
   const long long grid = static_cast<long long>(batch) * n_heads * (seq / BQ);
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_fwd_kernel<<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tk, tv, p);
