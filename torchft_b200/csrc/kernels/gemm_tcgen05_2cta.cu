@@ -165,6 +165,14 @@ __device__ __forceinline__ bool count_wait(const unsigned int* p, unsigned int w
   }
 }
 
+// The same for a whole warp whose loop has to stay converged.  One lane polls: 32 of them would load the word that the
+// gather warps add to 32 times as often.  What it acquired is ordered before what the other lanes do next.
+__device__ __forceinline__ bool count_wait_warp(const unsigned int* p, unsigned int want, volatile int* abort_flag) {
+  const bool ok = (threadIdx.x & 31) != 0 || count_wait(p, want, abort_flag);
+  __syncwarp();
+  return __all_sync(0xffffffffu, ok);
+}
+
 template <int BN_>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS_GATHER, 1)
 gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -245,7 +253,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       if (BNH == GATHER_BLOCK && p.ga_world > 0 && nb < p.N) {
         // these 128 rows of B are local once all their pieces are counted; the loads below go through the
         // async proxy, the pieces were written through the generic one
-        if (!__all_sync(0xffffffffu, count_wait(p.ga_sync + 1 + nb / GATHER_BLOCK, static_cast<unsigned int>(p.K / 64), abort_flag))) {
+        if (!count_wait_warp(p.ga_sync + 1 + nb / GATHER_BLOCK, static_cast<unsigned int>(p.K / 64), abort_flag)) {
           ok = false;
           break;
         }
