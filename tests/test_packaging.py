@@ -43,6 +43,16 @@ def test_every_build_switch_of_the_sources_is_built():
     assert asked == set(re.findall(r'"-D(\w+)', (pkg / "_build.py").read_text()))
 
 
+def test_every_error_code_of_the_kernels_has_a_message_of_its_own():
+    from torchft_b200.ops import _native
+
+    header = (REPO / "torchft_b200" / "csrc" / "kernels" / "ftb200_common.cuh").read_text()
+    codes = {name: int(v) for name, v in re.findall(r"#define FTB200_E_(\w+) \((-\d+)\)", header)}
+    assert set(codes.values()) == set(_native.ERRORS) and len(set(_native.ERRORS.values())) == len(codes)
+    # a kernel that cannot share out its registers says so, and not that the launch failed
+    assert "registers" in _native.ERRORS[codes["REGS"]]
+
+
 @pytest.mark.timeout(1500)
 def test_wheel_builds_installs_and_runs(tmp_path, clean_setuptools_leftovers):
     out = tmp_path / "wheel"

@@ -474,9 +474,11 @@ int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     if (cudaFuncSetAttribute(attention_fwd2_kernel<D, POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg<D>::SMEM_BYTES) != cudaSuccess)
       return FTB200_E_CUDA;
-    cudaFuncAttributes attr;  // the warpgroups' register split assumes this count
-    if (cudaFuncGetAttributes(&attr, attention_fwd2_kernel<D, POLY>) != cudaSuccess || attr.numRegs < LAUNCH_REGS)
-      return FTB200_E_CUDA;
+    // The warpgroups' register split assumes this count, which the compiler gives a kernel that moves registers; with fewer
+    // the softmax warpgroups would wait for registers that nobody has.
+    cudaFuncAttributes attr;
+    if (cudaFuncGetAttributes(&attr, attention_fwd2_kernel<D, POLY>) != cudaSuccess) return FTB200_E_CUDA;
+    if (attr.numRegs < LAUNCH_REGS) return FTB200_E_REGS;
     attr_set = true;
   }
   attention_fwd2_kernel<D, POLY><<<static_cast<unsigned>(grid), NUM_THREADS, Cfg<D>::SMEM_BYTES, stream>>>(tq, tk, tv, p);

@@ -30,6 +30,8 @@ ERRORS = {
     -3: "driver entry point unavailable / tensor-map encode failed",
     -4: "size beyond the supported maximum",
     -5: "CUDA launch error",
+    -6: "the kernel was compiled with fewer registers a thread than its warpgroups share out (a debug build, or another "
+        "compiler)",
 }
 
 STATUS = {0: "ok", 1: "timeout", 2: "aborted", 3: "epoch mismatch", 4: "bounds"}
