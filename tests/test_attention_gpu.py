@@ -39,6 +39,28 @@ def test_attention_fwd_matches_reference(B, S, Hq, Hkv, causal, scale):
     torch.testing.assert_close(lse, ref_lse, rtol=1e-3, atol=2e-3)
 
 
+@pytest.mark.parametrize("S,more_heads,two_tiles", [
+    (512, 0, False),   # the last size that one wave of 128-query CTAs takes
+    (512, 1, True),    # one head more
+    (640, 0, False),   # beyond a wave, but no whole number of tile pairs
+    (768, 0, True),
+])
+def test_attention_fwd_dispatch_line(monkeypatch, S, more_heads, two_tiles):
+    """The forward kernel that is chosen on both sides of one wave of CTAs, whatever the number of SMs."""
+    H = torch.cuda.get_device_properties(0).multi_processor_count // 4 + more_heads
+    monkeypatch.delenv("FTB200_ATTN_FWD", raising=False)
+    lib, called = K.N.lib(), []
+
+    class Recorder:
+        def __getattr__(self, name):
+            called.append(name)
+            return getattr(lib, name)
+
+    monkeypatch.setattr(K.N, "lib", Recorder)
+    _check_fwd(1, S, H, H, 128, True, 1.0, seed=S + H)
+    assert called == ["ftb200_attention_fwd2" if two_tiles else "ftb200_attention_fwd"]
+
+
 def _check_fwd(B, S, Hq, Hkv, D, causal, scale, seed):
     _, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=seed, scale=scale)
     out = torch.empty(B * S, Hq * D, dtype=torch.bfloat16, device="cuda")

@@ -111,3 +111,15 @@ def test_shard_pieces_cut_a_field_at_shard_boundaries():
         assert sum(p[3] for p in pieces) == n
         assert pieces[0][2] == off and all(a[2] + a[3] == b[2] for a, b in zip(pieces, pieces[1:]))
         assert all(o * shard + s == u and s + c <= shard for o, s, u, c in pieces)
+
+
+def test_forward_attention_kernel_follows_the_number_of_sms():
+    """Two query tiles per CTA beyond one wave of 128-query CTAs on the device at hand, and only where the sequence
+    divides into tile pairs."""
+    from torchft_b200.ops.kernels import _two_query_tiles
+
+    for sms in (74, 132, 148):
+        assert not _two_query_tiles(1, 256, sms // 2, sms)
+        assert _two_query_tiles(1, 256, sms // 2 + 1, sms)
+        assert _two_query_tiles(sms, 256, 1, sms) and not _two_query_tiles(sms, 128, 2, sms)
+        assert not _two_query_tiles(4, 384, sms, sms)

@@ -12,6 +12,7 @@ Every public function dispatches on the device of its arguments:
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from typing import Optional, Tuple
@@ -561,6 +562,19 @@ def attention_supported(seq_len: int, head_dim: int) -> bool:
     return (head_dim == 128 and seq_len % 128 == 0) or (head_dim == 64 and seq_len % 256 == 0)
 
 
+@functools.lru_cache(maxsize=None)
+def _sm_count(device_index: int) -> int:
+    return torch.cuda.get_device_properties(device_index).multi_processor_count
+
+
+def _two_query_tiles(batch: int, seq_len: int, n_heads: int, sms: int) -> bool:
+    """Whether a CTA of the forward kernel takes two tiles of 128 queries at head dim 128: where the sequence divides into
+    them and they fill the chip (475 us against 589 us at 1 x 8192, 32/8 heads, 148 SMs).  Up to one wave of 128-query
+    CTAs the length of one CTA's chain counts, and that is shorter with one tile: 28.5 us against 40.7 us at 1 x 2048,
+    8/8 heads; at twice a wave 28.6 against 22.9."""
+    return seq_len % 256 == 0 and batch * n_heads * (seq_len // 128) > sms
+
+
 def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int, seq_len: int, n_heads: int,
                   n_kv_heads: int, head_dim: int, out: torch.Tensor, lse: Optional[torch.Tensor] = None,
                   causal: bool = True) -> None:
@@ -580,10 +594,7 @@ def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int,
     scale = 1.0 / math.sqrt(head_dim)
     impl = os.environ.get("FTB200_ATTN_FWD", "auto")
     if impl == "auto":
-        # Two query tiles per CTA where the sequence divides into them and they fill the chip: 475 us against 589 us at
-        # 1 x 8192, 32/8 heads.  Up to one wave of 128-query CTAs (148 SMs) the length of one CTA's chain counts, and
-        # that is shorter with one tile: 28.5 us against 40.7 us at 1 x 2048, 8/8 heads; 28.6 against 22.9 at twice a wave.
-        impl = "pair" if seq_len % 256 == 0 and batch * n_heads * (seq_len // 128) > 148 else "single"
+        impl = "pair" if _two_query_tiles(batch, seq_len, n_heads, _sm_count(q.device.index)) else "single"
     if impl == "pair" or head_dim != 128:
         # two query tiles per CTA, one softmax thread per row (head dim 64 or 128, seq % 256 == 0).  At head dim 64 the
         # products are half as long and the exponential unit is the scarcer: a quarter of the exponentials goes to the
