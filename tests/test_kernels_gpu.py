@@ -35,10 +35,12 @@ def test_gemm_layouts(a_mn, b_mn, M, N, K_, impl):
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
-@pytest.mark.parametrize("N", [128 * 74 - 8, 128 * 74, 128 * 74 + 8, 128 * 75 + 136])
-def test_gemm_tile_width(a_mn, b_mn, N):
-    """On both sides of the line between 128- and 256-column tiles (74 CTA pairs on 148 SMs), with remainders in every
-    dimension.  Same sums in the same order either way: bf16 rounding of the result is the whole error (2^-9 relative)."""
+@pytest.mark.parametrize("past", [-8, 0, 8, 264])
+def test_gemm_tile_width(a_mn, b_mn, past):
+    """On both sides of the line between 128- and 256-column tiles (the narrow ones of a row of tiles fit the CTA pairs),
+    with remainders in every dimension.  Same sums in the same order either way: bf16 rounding of the result is the whole
+    error (2^-9 relative)."""
+    N = 128 * (torch.cuda.get_device_properties(0).multi_processor_count // 2) + past
     torch.manual_seed(9)
     M, K_ = 200, 328
     a = torch.randn((K_, M) if a_mn else (M, K_), device=DEV).bfloat16()
@@ -263,9 +265,10 @@ def test_engine_matches_autograd_at_the_8b_layer_shape():
         assert e < 0.02, (name, errs)
 
 
-def test_linear_swiglu_fused_epilogue():
+@pytest.mark.parametrize("T,Fd", [(384, 352), (1000, 1616)])  # narrow tiles; wide ones (4 x 26 narrow ones would not fit a wave)
+def test_linear_swiglu_fused_epilogue(T, Fd):
     torch.manual_seed(11)
-    T, Kd, Fd = 384, 256, 352  # 2F = 704 = 22 * 32
+    Kd = 256  # 2F is 22 * 32 or 101 * 32
     x = torch.randn(T, Kd, device=DEV).bfloat16()
     w = (torch.randn(2 * Fd, Kd, device=DEV) * 0.1).bfloat16()
     gu = torch.empty(T, 2 * Fd, device=DEV, dtype=torch.bfloat16)
@@ -276,6 +279,31 @@ def test_linear_swiglu_fused_epilogue():
     assert rel_err(gu, ref_gu) < 1e-2
     assert rel_err(s, K.ref_swiglu_fwd(gu)) < 1e-2
     assert rel_err(s, torch.nn.functional.silu(ref_gu[:, 0::2]) * ref_gu[:, 1::2]) < 2e-2
+
+
+@pytest.mark.parametrize("M,N", [(256, 512), (1000, 3232)])  # narrow tiles; wide ones
+@pytest.mark.parametrize("world", [1, 3])
+def test_gemm_scatter_epilogue(world, M, N):
+    """The result as one field of a flat unit that `world` ranks share: every piece lands in its owner's staging area (here
+    all on this GPU: the kernel only sees pointers), in the slice of the rank that computed it, and nothing else changes."""
+    import ctypes
+
+    torch.manual_seed(8)
+    K_, src, unit_off = 328, world - 1, 8 * 77
+    shard = -(-(unit_off + M * N + 8 * 5) // (world * 8)) * 8
+    a = torch.randn(K_, M, device=DEV).bfloat16()  # both operands as a weight gradient has them
+    b = torch.randn(K_, N, device=DEV).bfloat16()
+    stages = [torch.full((world, shard), 7.0, device=DEV, dtype=torch.bfloat16) for _ in range(world)]
+    peers = (ctypes.c_void_p * 8)()
+    for r in range(world):
+        peers[r] = stages[r].data_ptr()
+    K.gemm_scatter(a, b, True, True, K.ScatterField(peers, world, src, shard, unit_off, (M, N)))
+    K.check_status(a.device)
+    unit = torch.cat([s[src] for s in stages])
+    assert torch.equal(unit[unit_off : unit_off + M * N].view(M, N), K.gemm(a, b, True, True))
+    assert rel_err(unit[unit_off : unit_off + M * N].view(M, N), a.float().t() @ b.float()) < 4e-3
+    assert torch.all(unit[:unit_off] == 7.0) and torch.all(unit[unit_off + M * N :] == 7.0)
+    assert all(torch.all(s[r] == 7.0) for s in stages for r in range(world) if r != src)
 
 
 @pytest.mark.parametrize("world", [2, 4])
