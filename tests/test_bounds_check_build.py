@@ -31,6 +31,10 @@ tok = torch.tensor([1, 2, V + 7, 3], device=dev)
 emb = K.embedding_fwd(tok, table)
 torch.cuda.synchronize()
 out["embedding"] = (N.bounds_status(), bool(torch.equal(emb[2], table[0])), bool(torch.equal(emb[1], table[2])))
+# a warp that waits on an mbarrier in vain sees the abort flag of its CTA
+ns = torch.zeros(1, dtype=torch.int64, device=dev)
+assert lib.ftb200_wait_selftest(N.ptr(ns), N.stream_ptr()) == 0
+out["gave_up_ns"] = int(ns.item())
 # ordinary kernels leave the status clean
 x = torch.randn(256, 512, device=dev).bfloat16()
 w = torch.ones(512, device=dev).bfloat16()
@@ -55,4 +59,6 @@ def test_checked_build_records_and_skips():
     assert res["out_of_range"] == [0, [4, 5]]
     assert res["cleared"] == [0, 0]
     assert res["embedding"] == [[4, 64 + 7], True, True]
+    # 64 failed polls of about 2 us each lie between two looks at the flag; a factor of four over that
+    assert 0 <= res["gave_up_ns"] < 512_000, res["gave_up_ns"]
     assert res["clean"] == [0, 0]

@@ -372,3 +372,35 @@ FTB200_API int ftb200_gemm_bf16(const void* A, const void* B, void* C, int M, in
   gemm_bf16_tcgen05_kernel<<<ctas, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
+
+// ---- checked-index debug build: how long (ns) a warp that waits on a barrier nobody arrives at takes to give up once
+// another warp of its CTA has raised the abort flag; -1 if it did not give up
+#ifdef FT_BOUNDS_CHECK
+namespace {
+__global__ void wait_selftest_kernel(long long* ns) {
+  __shared__ alignas(8) uint64_t bar;
+  __shared__ volatile int abort_flag;
+  __shared__ volatile uint64_t raised;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&bar), 1);
+    abort_flag = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const bool ok = mbar_wait_warp(smem_u32(&bar), 0, &abort_flag);
+    if (threadIdx.x == 0) *ns = ok ? -1 : static_cast<long long>(ftb200::globaltimer_ns() - raised);
+  } else if (threadIdx.x == 32) {
+    const uint64_t t0 = ftb200::globaltimer_ns();
+    while (ftb200::globaltimer_ns() - t0 < 20000) {
+    }
+    raised = ftb200::globaltimer_ns();
+    __threadfence_block();
+    abort_flag = 1;
+  }
+}
+}  // namespace
+FTB200_API int ftb200_wait_selftest(long long* ns_dev, cudaStream_t st) {
+  wait_selftest_kernel<<<1, 64, 0, st>>>(ns_dev);
+  return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+}
+#endif

@@ -65,13 +65,13 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  Returns false when the CTA is aborting (limit hit here or elsewhere).  The clock is only read after
-// 1024 failed polls.
+// Bounded wait.  Returns false when the CTA is aborting (limit hit here or elsewhere).  A failed poll suspends the thread
+// for about 2 us; every 64 of them the abort flag and the clock are read, and the limit counts from the first time.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   uint64_t t0 = 0;
   for (uint32_t polls = 1;; ++polls) {
     if (mbar_test(bar, parity)) return true;
-    if ((polls & 1023u) == 0) {
+    if ((polls & 63u) == 0) {
       if (*abort_flag) return false;
       const uint64_t now = globaltimer_ns();
       if (t0 == 0) t0 = now;
