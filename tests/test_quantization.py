@@ -251,7 +251,7 @@ def test_misaligned_codes_are_refused_before_the_launch(dtype, step):
     bad_arg, align = -1, -2
     data, numel = (ctypes.c_void_p * 1)(1 << 20), (ctypes.c_longlong * 1)(n + 1)  # one element too many: refused as well
 
-    def both(codes, scales, d=data):
+    def both(codes, scales, d=data):  # far apart: nothing shares memory
         return {fn(d, numel, ctypes.c_int(1), ctypes.c_void_p(codes), ctypes.c_void_p(scales), ctypes.c_longlong(n),
                    ctypes.c_int(dtype), ctypes.c_void_p(0)) for fn in (lib.ftb200_quantize_list_fp8, lib.ftb200_dequantize_list_fp8)}
 
@@ -277,28 +277,55 @@ def test_a_buffer_that_is_too_short_is_refused_gpu():
 
 @pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
 def test_tensors_without_storage_are_zeros(device):
-    """Zeros as forward-mode autograd makes them have no memory to read."""
+    """Zeros as forward-mode autograd makes them have no memory to read, or to write."""
     x = torch.randn(300).to(device)
     zero = torch._efficientzerotensor((77,), device=device)
     got, _ = Q.fused_quantize_into_fp8([x, zero], 2)
     want, _ = Q.fused_quantize_into_fp8([x, torch.zeros(77, device=device)], 2)
     assert torch.equal(got, want)
+    with pytest.raises(RuntimeError):
+        Q.fused_dequantize_from_fp8([x, zero], got, 2)
 
 
-def test_overlapping_targets_are_recognised():
-    def overlaps(*ts):
-        return Q._launch_overlaps(list(ts), [t.is_contiguous() for t in ts])
+def test_copies_that_overlap_a_direct_target_are_recognised():
+    def overlap(*ts):
+        return Q._copies_overlap(list(ts), [type(t) is torch.Tensor and t.is_contiguous() for t in ts])
 
     x, y = torch.zeros(1000), torch.zeros(64, 48)
-    assert not overlaps(x[:600], x[600:], x[600:600], y, torch.zeros(0))
-    assert not overlaps(y[32:], y[:32], x[1:])
-    assert not overlaps(y[:, :16], x, y[:, 16:])           # interleaved, written by copies one after the other
-    assert overlaps(x, y, x)                               # the same tensor twice
-    assert overlaps(x[:600], y, x[599:])                   # one element in common
-    assert overlaps(x, x[10:20], x[500:600])               # inside
-    assert overlaps(y.t(), y[63:])                         # one of the two is not contiguous
-    assert overlaps(y[60:], y.t())
-    assert overlaps(x[:128].view(torch.uint8)[500:], x[:128])
+    assert not overlap(x[:600], x[600:], y.t(), torch.zeros(0))
+    assert not overlap(y[:, :16], x, y[:, 16:])            # interleaved, written by copies one after the other
+    assert overlap(y.t(), x, y[63:]) and overlap(y[60:], y.t())
+    assert overlap(x[::2], x[999:], y) is False and overlap(x[1::2], x[999:], y)
+    assert overlap(x[100:500:2], x, y)                     # inside
+    assert overlap(y[:, 1:].view(torch.uint8), y[:1].view(torch.uint8)[:, 8:].flatten()[:4])
+    assert overlap(x, y.as_subclass(type("Sub", (torch.Tensor,), {})))
+
+
+@pytest.mark.parametrize("dtype,size", [(0, 2), (1, 4)])
+def test_targets_that_share_memory_are_refused_before_the_launch(dtype, size):
+    """The C entry that writes a list looks at the addresses (made up here) before it launches anything; lists that pass
+    are refused for the elements that they have too many."""
+    lib, n, bad_arg, share = N.lib(), 256, -1, N.E_LIST
+    codes, scales = 1 << 22, (1 << 22) + n
+
+    def call(fn, *spans):
+        data = (ctypes.c_void_p * len(spans))(*[a for a, _ in spans])
+        numel = (ctypes.c_longlong * len(spans))(*[k for _, k in spans])
+        return fn(data, numel, ctypes.c_int(len(spans)), ctypes.c_void_p(codes), ctypes.c_void_p(scales), ctypes.c_longlong(n),
+                  ctypes.c_int(dtype), ctypes.c_void_p(0))
+
+    def dq(*spans):
+        return call(lib.ftb200_dequantize_list_fp8, *spans)
+
+    a = 1 << 20
+    assert dq((a, 200), (a + 200 * size, 200)) == dq((a + 200 * size, 200), (a, 200), (a + 100 * size, 0)) == bad_arg
+    assert dq((a, 200), (a + 199 * size, 200)) == share     # one element in common
+    assert dq((a, 10), (1 << 21, 300), (a, 10)) == share    # listed twice
+    assert dq((a, 300), (a + 50 * size, 10)) == share       # inside
+    assert dq((codes - 300 * size, 300)) == bad_arg and dq((codes - 299 * size, 300)) == share
+    assert dq((scales + n // 128 * 4, 300)) == bad_arg and dq((scales + n // 128 * 4 - size, 300)) == share
+    assert dq((a, 300), (0, 1)) == share and dq((a, 300), (0, 0)) == bad_arg
+    assert call(lib.ftb200_quantize_list_fp8, (a, 200), (a, 200)) == bad_arg  # reading the same twice is fine
 
 
 @pytest.mark.gpu

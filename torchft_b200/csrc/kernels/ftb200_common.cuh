@@ -22,6 +22,7 @@
 #define FTB200_E_TOOBIG (-4)
 #define FTB200_E_CUDA (-5)
 #define FTB200_E_REGS (-6)
+#define FTB200_E_LIST (-7)
 
 // device-side status word values (0 == ok)
 #define FTB200_ST_OK 0

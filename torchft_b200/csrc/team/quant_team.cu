@@ -18,6 +18,8 @@
 #include <cuda_fp8.h>
 
 #include <algorithm>
+#include <memory>
+#include <new>
 #include <vector>
 
 #include "ftb200_common.cuh"
@@ -571,22 +573,48 @@ FTB200_API int ftb200_dequantize_fp8(const void* codes, const float* scales, voi
 
 namespace {
 
+// Whether two of the tensors overlap, or one and the buffer.  Without memory to find out: yes.
+bool share_memory(void* const* data, const long long* numel, int count, int size, const void* codes, const float* scales,
+                  long long n) {
+  struct Span {
+    uintptr_t begin, end;
+  };
+  std::unique_ptr<Span[]> spans(new (std::nothrow) Span[static_cast<size_t>(count) + 2]);
+  if (!spans) return true;
+  int k = 0;
+  auto add = [&](const void* p, long long bytes) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    if (bytes > 0) spans[k++] = {at, at + static_cast<uintptr_t>(bytes)};
+  };
+  for (int i = 0; i < count; ++i) add(data[i], numel[i] * size);
+  add(codes, n);
+  add(scales, n / QB * 4);
+  std::sort(spans.get(), spans.get() + k, [](const Span& a, const Span& b) { return a.begin < b.begin; });
+  for (int i = 1; i < k; ++i)
+    if (spans[i].begin < spans[i - 1].end) return true;
+  return false;
+}
+
 // Cuts a list of tensors (data[i], numel[i] elements, empty ones allowed) into launches of at most LIST_MAX tensors and
 // whole blocks of the buffer's n elements, and calls launch(list) for each.  The blocks behind the last tensor belong
 // to the last launch.  A piece's codes (LV bytes) are read and written at once, so the buffer's codes begin on a multiple
-// of that; the tensors may begin anywhere that their type allows.
+// of that; the tensors may begin anywhere that their type allows.  FTB200_E_LIST, with nothing launched, says that the list
+// is not for these kernels: a tensor without memory, or (`writes`) tensors that share some with each other or with the
+// buffer, which launches that write in no order would leave in any state.
 template <typename F>
 int for_list(void* const* data, const long long* numel, int count, const void* codes, const float* scales, long long n,
-             int dtype, F launch) {
+             int dtype, bool writes, F launch) {
   const int size = dtype == 0 ? 2 : 4;
   if (n <= 0 || n % QB || count < 0 || misaligned(codes, 16 / size) || misaligned(scales, 4)) return FTB200_E_ALIGN;
   for (int i = 0; i < count; ++i)
     if (misaligned(data[i], size)) return FTB200_E_ALIGN;
   long long total = 0;
   for (int i = 0; i < count; ++i) {
-    if (numel[i] < 0 || (numel[i] > 0 && data[i] == nullptr)) return FTB200_E_BADARG;
+    if (numel[i] < 0) return FTB200_E_BADARG;
+    if (numel[i] > 0 && data[i] == nullptr) return FTB200_E_LIST;
     total += numel[i];
   }
+  if (writes && share_memory(data, numel, count, size, codes, scales, n)) return FTB200_E_LIST;
   if (total <= 0 || total > n) return FTB200_E_BADARG;
   int first = 0;            // tensor that holds the first element of the next launch
   long long first_off = 0;  // where it begins in the buffer
@@ -630,7 +658,7 @@ int grid_for_list(const TensorList& l, int groups, bool resident) {
 // Quantises count tensors (contiguous, numel[i] elements of the type) as one buffer of n elements, zeros behind them.
 FTB200_API int ftb200_quantize_list_fp8(void* const* data, const long long* numel, int count, void* codes, float* scales,
                                         long long n, int dtype, cudaStream_t st) {
-  return for_list(data, numel, count, codes, scales, n, dtype, [&](const TensorList& l) {
+  return for_list(data, numel, count, codes, scales, n, dtype, false, [&](const TensorList& l) {
     const int grid = grid_for_list(l, QUANT_GROUPS, dtype == 0);
     if (dtype == 0)
       quantize_list_kernel<__nv_bfloat16, QUANT_GROUPS><<<grid, 256, 0, st>>>(l, (uint8_t*)codes, scales);
@@ -641,7 +669,7 @@ FTB200_API int ftb200_quantize_list_fp8(void* const* data, const long long* nume
 
 FTB200_API int ftb200_dequantize_list_fp8(void* const* data, const long long* numel, int count, const void* codes,
                                           const float* scales, long long n, int dtype, cudaStream_t st) {
-  return for_list(data, numel, count, codes, scales, n, dtype, [&](const TensorList& l) {
+  return for_list(data, numel, count, codes, scales, n, dtype, true, [&](const TensorList& l) {
     const int grid = grid_for_list(l, DEQUANT_GROUPS, false);
     if (dtype == 0)
       dequantize_list_kernel<__nv_bfloat16, DEQUANT_GROUPS><<<grid, 256, 0, st>>>(l, (const uint8_t*)codes, scales);

@@ -24,6 +24,7 @@ c_int = ctypes.c_int
 c_ll = ctypes.c_longlong
 c_float = ctypes.c_float
 
+E_LIST = -7
 ERRORS = {
     -1: "bad argument",
     -2: "misaligned pointer or leading dimension",
@@ -32,6 +33,7 @@ ERRORS = {
     -5: "CUDA launch error",
     -6: "the kernel was compiled with fewer registers a thread than its warpgroups share out (a debug build, or another "
         "compiler)",
+    E_LIST: "tensors of a list share memory or have none",
 }
 
 STATUS = {0: "ok", 1: "timeout", 2: "aborted", 3: "epoch mismatch", 4: "bounds"}

@@ -118,17 +118,21 @@ def reduce_quantized(bufs: List[torch.Tensor], n: int, scale: float, out: torch.
 # --------------------------------------------------------------------------- list-of-tensors API
 
 
-def _plain(t: torch.Tensor) -> bool:
-    """A tensor whose elements lie where ``data_ptr`` says: no subclass, and not one of autograd's zeros without storage."""
-    return type(t) in (torch.Tensor, torch.nn.Parameter) and not t._is_zerotensor()
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
-def _list_call(name: str, tensors: List[torch.Tensor], codes: torch.Tensor, scales: torch.Tensor, n: int) -> None:
+def _list_call(name: str, tensors: List[torch.Tensor], codes: torch.Tensor, scales: torch.Tensor, n: int) -> bool:
+    """Launches a list kernel; False, with nothing launched, where tensors share memory that it would write, or have none
+    (autograd's zeros without storage)."""
     count = len(tensors)
     data = (ctypes.c_void_p * count)(*[t.data_ptr() for t in tensors])
     numel = (ctypes.c_longlong * count)(*[t.numel() for t in tensors])
-    N.check(getattr(N.lib(), name)(data, numel, ctypes.c_int(count), N.ptr(codes), N.ptr(scales), ctypes.c_longlong(n),
-                                   ctypes.c_int(_DT[tensors[0].dtype]), N.stream_ptr()), name)
+    rc = getattr(N.lib(), name)(data, numel, ctypes.c_int(count), N.ptr(codes), N.ptr(scales), ctypes.c_longlong(n),
+                                ctypes.c_int(_DT[tensors[0].dtype]), N.stream_ptr())
+    if rc == N.E_LIST:
+        return False
+    N.check(rc, name)
+    return True
 
 
 def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tuple[torch.Tensor, List[int]]:
@@ -141,14 +145,14 @@ def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tup
     assert dtype in _DT, f"unsupported dtype {dtype}"
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
-    if device.type == "cuda" and total > 0 and all(map(_plain, tensors)):
+    if device.type == "cuda" and total > 0 and all(type(t) in _PLAIN for t in tensors):
         for t in tensors:
             assert t.dtype == dtype and t.device == device
         buf = torch.empty(quantized_nbytes(n), dtype=torch.uint8, device=device)
         # the kernel reads the tensors where they are; only a non-contiguous one is copied
         flats = [t.detach().resolve_neg().reshape(-1) for t in tensors]
-        _list_call("ftb200_quantize_list_fp8", flats, *split_quantized(buf, n), n)
-        return buf, [n]
+        if _list_call("ftb200_quantize_list_fp8", flats, *split_quantized(buf, n), n):
+            return buf, [n]
     flat = torch.zeros(n, dtype=dtype, device=device)
     off = 0
     for t in tensors:
@@ -161,27 +165,29 @@ def fused_quantize_into_fp8(tensors: List[torch.Tensor], world_size: int) -> Tup
 
 
 def _written_in_place(t: torch.Tensor, dtype: torch.dtype, device: torch.device) -> bool:
-    """Whether a kernel may write the plain tensor ``t`` directly; the rest takes ``copy_`` with its checks and
-    conversions (other types and devices, strides, leaves that require grad, inference tensors)."""
-    return (t.dtype == dtype and t.device == device and t.is_contiguous()
+    """Whether a kernel may write ``t`` directly; the rest takes ``copy_`` with its checks and conversions (other types
+    and devices, strides, leaves that require grad, inference tensors, tensor subclasses)."""
+    return (type(t) in _PLAIN and t.dtype == dtype and t.device == device and t.is_contiguous()
             and not (t.requires_grad and torch.is_grad_enabled()) and not t.is_inference() and not t.is_neg())
 
 
-def _launch_overlaps(tensors: List[torch.Tensor], direct: List[bool]) -> bool:
-    """Whether the memory that a ``direct`` tensor spans (from the first element to the last) overlaps another's."""
+def _copies_overlap(tensors: List[torch.Tensor], direct: List[bool]) -> bool:
+    """Whether the memory that a tensor spans which is not ``direct`` (from its first element to its last) overlaps that of
+    a direct one; a subclass need not say where its elements lie, so it does."""
     spans = []
     for t, ok in zip(tensors, direct):
+        if type(t) not in _PLAIN:
+            return True
         if t.numel():
-            last = t.numel() - 1 if ok else sum((n - 1) * s for n, s in zip(t.shape, t.stride()))
             begin = t.data_ptr()
+            last = sum((n - 1) * s for n, s in zip(t.shape, t.stride()))
             spans.append((begin, begin + (last + 1) * t.element_size(), ok))
     spans.sort()
-    end_all = end_direct = 0
+    ends = {True: 0, False: 0}
     for begin, end, ok in spans:
-        if begin < (end_all if ok else end_direct):
+        if begin < ends[not ok]:
             return True
-        end_all = max(end_all, end)
-        end_direct = max(end_direct, end) if ok else end_direct
+        ends[ok] = max(ends[ok], end)
     return False
 
 
@@ -191,19 +197,20 @@ def fused_dequantize_from_fp8(tensors: List[torch.Tensor], buf: torch.Tensor, wo
     total = sum(t.numel() for t in tensors)
     n = padded_numel(total, world_size)
     _check_buffer(buf, n)
-    if device.type == "cuda" and total > 0 and buf.device == device and all(map(_plain, tensors)):
+    if device.type == "cuda" and total > 0 and buf.device == device:
         direct = [_written_in_place(t, dtype, device) for t in tensors]
-        # One launch writes the direct ones in no order.  Where one shares memory with another tensor (listed twice,
-        # overlapping views) or with the buffer, the values go through a flat tensor and are copied in the list's order.
-        if not _launch_overlaps([*tensors, buf], [*direct, False]):
+        # One launch writes the direct ones in no order, the others are copied after it.  Where one of the direct ones
+        # shares memory with another tensor (listed twice, overlapping views) or with the buffer, the values go through a
+        # flat tensor and are copied in the list's order.
+        if all(direct) or not _copies_overlap(tensors, direct):
             targets = [t if ok else torch.empty(t.shape, dtype=dtype, device=device) for t, ok in zip(tensors, direct)]
-            _list_call("ftb200_dequantize_list_fp8", targets, *split_quantized(buf, n), n)
-            for t, target, ok in zip(tensors, targets, direct):
-                if ok:
-                    torch.autograd.graph.increment_version(t)
-                else:
-                    t.copy_(target)
-            return
+            if _list_call("ftb200_dequantize_list_fp8", targets, *split_quantized(buf, n), n):
+                for t, target, ok in zip(tensors, targets, direct):
+                    if ok:
+                        torch.autograd.graph.increment_version(t)
+                    else:
+                        t.copy_(target)
+                return
     flat = torch.empty(n, dtype=dtype, device=device)
     dequantize_from(buf, flat)
     off = 0
