@@ -25,9 +25,11 @@
 // so that the softmax of one tile runs beside that of the other, and dQ(t-1) is drained under dV(t-1),
 // dK(t-1) and S(t+1), before dP(t+1) needs its columns.  All waits are bounded.
 //
-// What bounds it: a tile's MMAs take 1650 cycles by themselves, a tile 3300; the difference is the
-// instruction stream of the MMA warp (commits of about 230 cycles, waits) next to 20 others, not the
-// exponentials, the stores of dS^T or the reductions, each of which can be taken out for 0 to 3 %.
+// What bounds it: a tile's MMAs take 1650 cycles by themselves, a tile 3300.  The exponentials, the stores
+// of dS^T and the reductions can each be taken out for 0 to 3 %, so the difference is taken to be the
+// instruction stream of the MMA warp and its waits next to 21 other warps.  704 threads leave 80 registers a
+// thread, and the softmax spills: 40 bytes of stores and 72 of loads at head dim 128, 48 and 156 at 64
+// (ptxas); what that costs is not measured.
 // 8 x 2048, 32/8 heads of 64: 930 us with one softmax group of 16 warps and scalar reductions, 777 us with
 // two (442 TFLOP/s); 1 x 8192, heads of 128: 1706 us either way.
 #include <cuda.h>
