@@ -143,6 +143,33 @@ def test_attention_bwd_matches_reference(B, S, Hq, Hkv, causal, D):
         assert err < 2e-2, (name, err)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,S,Hq,Hkv,causal,scale", [
+    (1, 256, 1, 1, True, 1.0),      # blocks of two tiles and of one
+    (2, 256, 3, 1, False, 1.0),     # six tiles a block, through the stages of Q and dO
+    (1, 768, 8, 1, True, 3.0),      # eight heads on one; most weights are near 0 or 1
+    (1, 512, 3, 3, False, 1.0),
+    (3, 1280, 2, 2, True, 1.0),     # an odd number of tiles in every other block
+])
+def test_attention_bwd_tiles(B, S, Hq, Hkv, causal, scale, D):
+    """Tiles of 128 queries at the edges of the walk over them.  Three roundings to bf16 lie on the way of every
+    gradient (probabilities or dS, the forward's O behind delta, the result), each at most 2^-9 of its value."""
+    qkv, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=S + D, scale=scale)
+    out = torch.empty(B * S, Hq * D, dtype=torch.bfloat16, device="cuda")
+    lse = torch.empty(B, Hq, S, dtype=torch.float32, device="cuda")
+    K.attention_fwd(q, k, v, B, S, Hq, Hkv, D, out, lse, causal=causal)
+    d_o = torch.randn(B * S, Hq * D, device="cuda", generator=torch.Generator(device="cuda").manual_seed(S)).to(torch.bfloat16)
+    dqkv = torch.full_like(qkv, float("nan"))
+    dq, dk, dv = dqkv[:, : Hq * D], dqkv[:, Hq * D : (Hq + Hkv) * D], dqkv[:, (Hq + Hkv) * D :]
+    for _ in range(2):  # the second call finds the first one's sums in the scratch memory
+        K.attention_bwd(q, k, v, out, d_o, lse, dq, dk, dv, B, S, Hq, Hkv, D, causal=causal)
+    K.check_status(out.device)
+    want = K.ref_attention_bwd(*(t.reshape(B, S, -1, D) for t in (q, k, v, d_o)), causal)
+    for name, got, w in zip(("dq", "dk", "dv"), (dq, dk, dv), want):
+        w = w.reshape(B * S, -1)
+        assert (got.float() - w).norm() <= 3 * 2**-9 * w.norm(), name
+
+
 @pytest.mark.parametrize("D,poly", [(64, None), (64, "0"), (64, "4"), (128, "0"), (128, "4")])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("key", [*range(8), 131, 200])

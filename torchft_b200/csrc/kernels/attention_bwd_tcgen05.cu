@@ -1,7 +1,7 @@
 // Causal grouped-query attention, backward pass, on the 5th-generation tensor cores.
 //
 // One CTA owns one (batch, kv head, 128-key block) and walks over every query head of the
-// group and every 64-query tile that can see the block.  Scores are formed transposed, keys on
+// group and every 128-query tile that can see the block.  Scores are formed transposed, keys on
 // the TMEM lanes and queries on the columns, so every MMA has M = 128:
 //
 //   S^T  = K  Q^T            [keys x q]      A = K   (K-major)      B = Q   (K-major)
@@ -17,21 +17,25 @@
 // whole CTA; dQ^T is drained every tile and added to an fp32 accumulator in global memory (four
 // queries of a head-dim element per reduction, 512 consecutive bytes per warp instruction).
 //
-// Warps: 0 = TMA (K, V once; Q, dO, lse, delta per tile, 3 stages), 1 = MMA issue, 2..9 and 10..17 =
-// two softmax groups that take the tiles in turn (and together store dK, dV at the end), 18..21 = dQ
-// drain.  S^T and dP^T have two buffers each, and dQ^T of a tile takes the place of its dP^T, which fills
-// the 512 TMEM columns:
-//   issue order   dQ(t-1) dV(t-1) dK(t-1) | S(t+1) dP(t+1) | dQ(t) ...
-// so that the softmax of one tile runs beside that of the other, and dQ(t-1) is drained under dV(t-1),
-// dK(t-1) and S(t+1), before dP(t+1) needs its columns.  All waits are bounded.
+// Warps: 0 = TMA (K, V once; Q with lse and delta, dO per tile), 1 = MMA issue, 4..7 = dQ drain, 8..15 = softmax (two
+// threads per key, 64 queries each; together they store dK, dV at the end).  Issue order of a tile t:
+//   dV(t) S(t+1) dK(t) dQ(t) dP(t+1)
+// so that the exponentials of t + 1 run under dK(t), dQ(t) and dP(t+1), and dS(t) is formed under dV(t) and S(t+1).  At head
+// dim 128 the 512 TMEM columns are full and dQ^T takes the place of its dP^T, so dP(t+1) waits until it is drained; at
+// head dim 64 it has columns of its own.
 //
-// What bounds it: a tile's MMAs take 1650 cycles by themselves, a tile 3300.  The exponentials, the stores
-// of dS^T and the reductions can each be taken out for 0 to 3 %, so the difference is taken to be the
-// instruction stream of the MMA warp and its waits next to 21 other warps.  704 threads leave 80 registers a
-// thread, and the softmax spills: 40 bytes of stores and 72 of loads at head dim 128, 48 and 156 at 64
-// (ptxas); what that costs is not measured.
-// 8 x 2048, 32/8 heads of 64: 930 us with one softmax group of 16 warps and scalar reductions, 777 us with
-// two (442 TFLOP/s); 1 x 8192, heads of 128: 1706 us either way.
+// What bounds it: at head dim 128 the sum of dQ^T.  A tile's 64 KB leave an SM at about 21 bytes a cycle as bulk reductions
+// (whatever their size, 4 or 16 KB) and at 25 as red.v4; the latter go through the load/store pipe that the softmax needs
+// for dS^T and the statistics, whose second half then takes 2570 cycles instead of 1020 (800 with no reductions at all).  A
+// tile takes 3750 cycles: 4890 with red.v4, 3250 with no reductions, 2600 for its 40 MMAs, 2048 + 1000 for what they, the
+// TMA and the softmax move through shared memory at 128 bytes a cycle.  dO has one stage there, as the staging of dQ^T takes
+// the second one's place.  At head dim 64 it is the chain of the softmax, 2830 cycles a tile.
+// The warp's index and the TMEM base are read from lane 0 (shfl): then the branch and the addresses are known to be the
+// same in all lanes and the MMAs' descriptors stay in uniform registers (1494 -> 1437 us, 650 -> 605 us).
+// 1 x 8192, 32/8 heads of 128: 1705 us with 64-query tiles, 1290 us (1065 TFLOP/s) with these; 8 x 2048, heads of 64: 785 -> 592 us.
+//
+// Every mbarrier wait is bounded; on expiry the CTA records FTB200_ST_TIMEOUT in the caller's
+// status word, frees its TMEM and returns.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <math.h>
@@ -44,50 +48,60 @@ namespace {
 using namespace ftb200::tc;
 
 constexpr int BKV = 128;
-constexpr int BQ = 64;
-constexpr int NUM_THREADS = 704;
-constexpr int SOFTMAX_WARPS = 16;
+constexpr int BQ = 128;
+constexpr int NUM_THREADS = 512;
+constexpr int SOFTMAX_WARPS = 8;
 constexpr int DRAIN_WARPS = 4;
-constexpr int GROUP_WARPS = SOFTMAX_WARPS / 2;  // softmax warps per tile
-constexpr int CPT = BQ / 2;        // query columns per thread: two threads per key row and tile
-constexpr int CHUNK = 16;          // of them at a time
+// Registers: a CTA is launched with 128 a thread (65536 / 512, checked on the host) and shares them out by warpgroup:
+// TMA and MMA issue, drain (128 elements of dQ^T in flight), two of softmax (a thread keeps 64 probabilities).
+constexpr int LAUNCH_REGS = 128, ISSUE_REGS = 48, DRAIN_REGS = 144, SOFTMAX_REGS = 160;
+static_assert(ISSUE_REGS + DRAIN_REGS + 2 * SOFTMAX_REGS <= 4 * LAUNCH_REGS, "more registers than the CTA is launched with");
+constexpr int CPT = BQ / 2;        // query columns per softmax thread: two threads per key row
+constexpr int CHUNK = 16;          // of them at a time where dP^T is read
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 384;  // dQ^T where dP^T was
-constexpr uint32_t KV_SLAB = BKV * 128;        // 16 KB: [128 rows x 128 B], 64 head-dim elements per row
-constexpr uint32_t Q_SLAB = BQ * 128;          // 8 KB: [64 rows x 128 B]
-constexpr uint32_t PT_TILE = BKV * BQ * 2;     // 16 KB, one slab of [128 key rows x 64 q]
-constexpr int QDO_STAGES = 3;  // a stage is held until the tile's dV/dK MMAs are done, two tiles after its load began
-constexpr uint32_t PDS_BYTES = PT_TILE;        // dS^T only: P^T never leaves tensor memory
-constexpr uint32_t STATS_BYTES = 2 * BQ * 4;   // per stage: lse[64], delta[64]
+constexpr uint32_t SLAB = 128 * 128;           // 16 KB: [128 rows x 128 B], 64 elements per row
+constexpr int STAGES = 2;                      // of Q; of dO as well at head dim 64
+constexpr uint32_t DS_BYTES = BKV * BQ * 2;    // dS^T, two slabs of 64 queries
+constexpr uint32_t STATS_BYTES = 2 * BQ * 4;   // per stage of Q: lse[128], delta[128]
+constexpr int DQ_PARTS = 4;                    // a drain warp's 32 x 128 elements of dQ^T leave in so many bulk reductions,
+constexpr uint32_t DQ_PART_BYTES = 32 * BQ * 4 / DQ_PARTS;  // from two buffers of its own
 
-// Shared-memory layout for head dim D (64 or 128): K and V tiles of D/64 slabs each, then the Q/dO stages, the
-// dS^T buffers, the statistics and the barriers.
+// Shared-memory layout and TMEM columns for head dim D (64 or 128): K and V tiles of D/64 slabs each, then the Q and
+// dO stages, dS^T, the statistics and the barriers.
 template <int D>
 struct Lay {
   static constexpr int SLABS = D / 64;
-  static constexpr uint32_t KV_TILE = SLABS * KV_SLAB;
-  static constexpr uint32_t Q_TILE = SLABS * Q_SLAB;
-  static constexpr uint32_t OFF_K = 0, OFF_V = KV_TILE;
-  static constexpr uint32_t OFF_STAGE = 2 * KV_TILE;    // per stage: Q, dO
-  static constexpr uint32_t STAGE_BYTES = 2 * Q_TILE;
-  static constexpr uint32_t OFF_PDS = OFF_STAGE + QDO_STAGES * STAGE_BYTES;  // per buffer: dS^T
-  static constexpr uint32_t OFF_STATS = OFF_PDS + 2 * PDS_BYTES;
-  static constexpr uint32_t OFF_MISC = OFF_STATS + QDO_STAGES * STATS_BYTES;
-  static constexpr uint32_t SMEM_BYTES = OFF_MISC + 256 + 1024;
+  static constexpr uint32_t TILE = SLABS * SLAB;  // 128 rows of K, V, Q or dO
+  static constexpr uint32_t OFF_K = 0, OFF_V = TILE;
+  static constexpr uint32_t OFF_Q = 2 * TILE;               // per stage: Q
+  static constexpr int DO_STAGES = D == 128 ? 1 : 2;         // one: it is free from dV on and needed again three products later
+  static constexpr uint32_t OFF_DO = OFF_Q + STAGES * TILE;  // per stage: dO
+  static constexpr uint32_t OFF_DS = OFF_DO + DO_STAGES * TILE;
+  static constexpr uint32_t OFF_DQ = OFF_DS + DS_BYTES;      // per drain warp: two parts of dQ^T
+  static constexpr uint32_t OFF_STATS = OFF_DQ + DRAIN_WARPS * 2 * DQ_PART_BYTES;
+  static constexpr uint32_t OFF_MISC = OFF_STATS + STAGES * STATS_BYTES;
+  static constexpr uint32_t SMEM_BYTES = OFF_MISC + 256;
   static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
+  static constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + D;
+  // head dim 128 fills the 512 columns: dQ^T takes the place of its dP^T (and of dS^T, once dK has read it)
+  static constexpr bool DQ_OVER_DP = D == 128;
+  static constexpr uint32_t COL_DQ = DQ_OVER_DP ? COL_DP : 256 + 2 * D;
 };
 
 enum : int {
   BAR_KV = 0,
-  BAR_QDO_FULL = 1,   // +stage (3)
-  BAR_QDO_EMPTY = 4,  // +stage (3)
-  BAR_S_FULL = 7,     // +buf
-  BAR_DP_FULL = 9,    // +buf
-  BAR_PDS_FULL = 11,  // +buf
-  BAR_DQ_FULL = 13,   // +buf
-  BAR_DQ_EMPTY = 15,  // +buf
-  BAR_DKV_DONE = 17,
-  NUM_BARS = 18,
+  BAR_Q_FULL = 1,    // +stage
+  BAR_Q_EMPTY = 3,   // +stage
+  BAR_DO_FULL = 5,   // +stage
+  BAR_DO_EMPTY = 7,  // +stage
+  BAR_S_FULL = 9,
+  BAR_P_READY = 10,
+  BAR_DP_FULL = 11,
+  BAR_DS_READY = 12,
+  BAR_DQ_FULL = 13,
+  BAR_DQ_EMPTY = 14,
+  BAR_DKV_DONE = 15,
+  NUM_BARS = 16,
 };
 
 struct BwdParams {
@@ -96,7 +110,7 @@ struct BwdParams {
   float scale, scale_log2;
   const float* neg_lse2;   // [batch, n_heads, seq], -log2(e) times the forward's log-sum-exp
   const float* neg_delta;  // [batch, n_heads, seq], -scale times delta
-  float* dq_acc;           // fp32, zeroed; per 64-query tile and head: [16][D][4 queries]
+  float* dq_acc;           // fp32, zeroed; per 128 queries and head: [D / 32][32 groups of 4 queries][32][4 queries]
   __nv_bfloat16* dK;   // rows batch*seq, row stride ld_dk
   __nv_bfloat16* dV;
   long long ld_dk, ld_dv;
@@ -109,8 +123,10 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
                : "memory");
 }
 
-__device__ __forceinline__ void red_add_v4(float* dst, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+// Adds `bytes` of shared memory to global memory as fp32.  The calling thread's bulk group has to be committed.
+__device__ __forceinline__ void bulk_add_f32(float* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+               : "memory");
 }
 
 template <int D>
@@ -120,20 +136,23 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                      const BwdParams p) {
   using Ly = Lay<D>;
   constexpr int SLABS = Ly::SLABS;
-  constexpr uint32_t KV_TILE = Ly::KV_TILE, Q_TILE = Ly::Q_TILE, OFF_K = Ly::OFF_K, OFF_V = Ly::OFF_V;
-  constexpr uint32_t OFF_STAGE = Ly::OFF_STAGE, STAGE_BYTES = Ly::STAGE_BYTES, OFF_PDS = Ly::OFF_PDS;
-  constexpr uint32_t OFF_STATS = Ly::OFF_STATS, OFF_MISC = Ly::OFF_MISC;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_MISC);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_MISC + 192);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + 196);
+  constexpr uint32_t TILE = Ly::TILE;
+  extern __shared__ __align__(1024) uint8_t smem[];  // swizzled tiles start at multiples of 1024 (checked)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Ly::OFF_MISC);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Ly::OFF_MISC + 192);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Ly::OFF_MISC + 196);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_u32(bars);
   auto bar = [&](int i) { return bar_base + 8u * i; };
+
+  // tiles have to start at their swizzle atom; there is no room to move them up to it
+  if ((smem_base & 1023u) != 0) {
+    if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, FTB200_ST_BOUNDS);
+    return;
+  }
 
   // early key blocks see the most queries under a causal mask: schedule them first
   const int per_block = p.batch * p.n_kv_heads;
@@ -142,7 +161,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int b = bh / p.n_kv_heads, hk = bh % p.n_kv_heads;
   const int rep = p.n_heads / p.n_kv_heads;
   const int n_qtiles = p.seq / BQ;
-  const int first_q = p.causal ? (jb * BKV) / BQ : 0;
+  const int first_q = p.causal ? jb : 0;
   const int T = rep * (n_qtiles - first_q);
   const int kv_row0 = b * p.seq + jb * BKV;
   // tiles in order: the queries of a head that see the block, then the next head of the group
@@ -158,17 +177,18 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (threadIdx.x == 0) {
     mbar_init(bar(BAR_KV), 1);
-    for (int s = 0; s < QDO_STAGES; ++s) {
-      mbar_init(bar(BAR_QDO_FULL + s), 1);
-      mbar_init(bar(BAR_QDO_EMPTY + s), 1);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(bar(BAR_Q_FULL + s), 1);
+      mbar_init(bar(BAR_Q_EMPTY + s), 1);
+      mbar_init(bar(BAR_DO_FULL + s), 1);
+      mbar_init(bar(BAR_DO_EMPTY + s), 1);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(bar(BAR_S_FULL + s), 1);
-      mbar_init(bar(BAR_DP_FULL + s), 1);
-      mbar_init(bar(BAR_PDS_FULL + s), GROUP_WARPS);
-      mbar_init(bar(BAR_DQ_FULL + s), 1);
-      mbar_init(bar(BAR_DQ_EMPTY + s), DRAIN_WARPS);
-    }
+    mbar_init(bar(BAR_S_FULL), 1);
+    mbar_init(bar(BAR_P_READY), SOFTMAX_WARPS);
+    mbar_init(bar(BAR_DP_FULL), 1);
+    mbar_init(bar(BAR_DS_READY), SOFTMAX_WARPS);
+    mbar_init(bar(BAR_DQ_FULL), 1);
+    mbar_init(bar(BAR_DQ_EMPTY), DRAIN_WARPS);
     mbar_init(bar(BAR_DKV_DONE), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -183,206 +203,221 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-  if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (elect_one()) {
-      mbar_expect_tx(bar(BAR_KV), 2 * KV_TILE);
-#pragma unroll
-      for (int sl = 0; sl < SLABS; ++sl) {
-        tma_load_2d(smem_base + OFF_K + sl * KV_SLAB, &tmK, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
-        tma_load_2d(smem_base + OFF_V + sl * KV_SLAB, &tmV, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
-      }
-    }
-    __syncwarp();
-    bool ok = true;
-    TileWalk w{hk * rep, first_q};
-    for (int t = 0; t < T && ok; ++t, next_tile(w)) {
-      const int st = t % QDO_STAGES;
-      const uint32_t use = static_cast<uint32_t>(t / QDO_STAGES);
-      if (!mbar_wait_warp(bar(BAR_QDO_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
-        ok = false;
-        break;
-      }
-      const int h = w.h, qt = w.qt;
-      const int q_row0 = b * p.seq + qt * BQ;
-      const uint32_t sq = smem_base + OFF_STAGE + st * STAGE_BYTES;
-      const uint32_t sdo = sq + Q_TILE;
-      const uint32_t sst = smem_base + OFF_STATS + st * STATS_BYTES;
-      const long long stat_off = (static_cast<long long>(b) * p.n_heads + h) * p.seq + qt * BQ;
+  if (warp < 4) {
+    regs_dec<ISSUE_REGS>();
+    if (warp == 0) {
+      // ---------------- TMA producer ----------------
       if (elect_one()) {
-        mbar_expect_tx(bar(BAR_QDO_FULL + st), 2 * Q_TILE + STATS_BYTES);
+        mbar_expect_tx(bar(BAR_KV), 2 * TILE);
 #pragma unroll
         for (int sl = 0; sl < SLABS; ++sl) {
-          tma_load_2d(sq + sl * Q_SLAB, &tmQ, bar(BAR_QDO_FULL + st), h * D + 64 * sl, q_row0);
-          tma_load_2d(sdo + sl * Q_SLAB, &tmDO, bar(BAR_QDO_FULL + st), h * D + 64 * sl, q_row0);
+          tma_load_2d(smem_base + Ly::OFF_K + sl * SLAB, &tmK, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
+          tma_load_2d(smem_base + Ly::OFF_V + sl * SLAB, &tmV, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
         }
-        bulk_load_1d(sst, p.neg_lse2 + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
-        bulk_load_1d(sst + BQ * 4, p.neg_delta + stat_off, BQ * 4, bar(BAR_QDO_FULL + st));
       }
       __syncwarp();
-    }
-    if (!ok) {
-      const uint64_t t0 = ftb200::globaltimer_ns();
-      while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    const uint32_t F = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(128 >> 4) << 24);
-    const uint32_t idesc_st = F | (static_cast<uint32_t>(BQ >> 3) << 17);                             // N = 64, K-major both
-    const uint32_t idesc_kv = F | (1u << 16) | (static_cast<uint32_t>(D >> 3) << 17);                 // N = D, B MN-major
-    const uint32_t idesc_dq = F | (1u << 15) | (1u << 16) | (static_cast<uint32_t>(BQ >> 3) << 17);   // N = 64, both MN-major
-    // descriptor bases: one per buffer and operand role, constants per K step (the issue loop
-    // must stay short: these MMAs are too small to hide descriptor arithmetic)
-    constexpr uint32_t HI = smem_desc_hi(1024);
-    const uint32_t k_km = smem_desc_lo(smem_base + OFF_K, 16);        // K as K-major A (S^T)
-    const uint32_t v_km = smem_desc_lo(smem_base + OFF_V, 16);        // V as K-major A (dP^T)
-    // K as MN-major A (dQ^T): M = 128 runs over the head dim.  With head dim 64 the second 64 rows of that MMA
-    // read the slab behind K's only one, which is V's: lanes 64..127 of dQ^T then hold a product nobody reads.
-    const uint32_t k_mn = smem_desc_lo(smem_base + OFF_K, KV_SLAB);
-    const uint32_t q_km0 = smem_desc_lo(smem_base + OFF_STAGE, 16);             // Q, stage 0, K-major B
-    const uint32_t q_mn0 = smem_desc_lo(smem_base + OFF_STAGE, Q_SLAB);         // Q, stage 0, MN-major B
-    const uint32_t ds_mn0 = smem_desc_lo(smem_base + OFF_PDS, PT_TILE);  // dS^T, buffer 0, MN-major B
-    constexpr uint32_t STAGE16 = STAGE_BYTES >> 4, QT16 = Q_TILE >> 4, PDS16 = PDS_BYTES >> 4;
-    bool ok = mbar_wait_warp(bar(BAR_KV), 0, abort_flag);
-    for (int t = 0; t <= T && ok; ++t) {
-      if (t < T) {
-        // S and dP of tile t; the MMAs that read P and dS of tile t - 2 from the same S buffer were issued before
-        const int st = t & 1, qs = t % QDO_STAGES;
-        const uint32_t use = static_cast<uint32_t>(t >> 1);
-        if (!mbar_wait_warp(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag)) {
+      bool ok = true;
+      TileWalk w{hk * rep, first_q};
+      for (int t = 0; t < T && ok; ++t, next_tile(w)) {
+        const int st = t % STAGES;
+        const uint32_t was = static_cast<uint32_t>(t / STAGES) & 1u ^ 1u;
+        const int dst = t % Ly::DO_STAGES;
+        const int q_row0 = b * p.seq + w.qt * BQ;
+        const long long stat_off = (static_cast<long long>(b) * p.n_heads + w.h) * p.seq + w.qt * BQ;
+        const uint32_t sq = smem_base + Ly::OFF_Q + st * TILE, sdo = smem_base + Ly::OFF_DO + dst * TILE;
+        const uint32_t sst = smem_base + Ly::OFF_STATS + st * STATS_BYTES;
+        if (!mbar_wait_warp(bar(BAR_Q_EMPTY + st), was, abort_flag)) {
           ok = false;
           break;
         }
-        tc_fence_after();
-        const uint32_t qb_km = q_km0 + qs * STAGE16;
         if (elect_one()) {
+          mbar_expect_tx(bar(BAR_Q_FULL + st), TILE + STATS_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
-            const uint32_t a_off = ((kk >> 2) * KV_SLAB + (kk & 3) * 32) >> 4, b_off = ((kk >> 2) * Q_SLAB + (kk & 3) * 32) >> 4;
-            umma_bf16_lh(tmem_base + COL_S + st * BQ, k_km + a_off, HI, qb_km + b_off, HI, idesc_st, kk != 0);
-          }
-          umma_commit(bar(BAR_S_FULL + st));
+          for (int sl = 0; sl < SLABS; ++sl)
+            tma_load_2d(sq + sl * SLAB, &tmQ, bar(BAR_Q_FULL + st), w.h * D + 64 * sl, q_row0);
+          bulk_load_1d(sst, p.neg_lse2 + stat_off, BQ * 4, bar(BAR_Q_FULL + st));
+          bulk_load_1d(sst + BQ * 4, p.neg_delta + stat_off, BQ * 4, bar(BAR_Q_FULL + st));
         }
         __syncwarp();
-        if (!mbar_wait_warp(bar(BAR_DQ_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {  // dQ of tile t - 2 drained
+        if (!mbar_wait_warp(bar(BAR_DO_EMPTY + dst), static_cast<uint32_t>(t / Ly::DO_STAGES) & 1u ^ 1u, abort_flag)) {
           ok = false;
           break;
         }
-        tc_fence_after();
         if (elect_one()) {
+          mbar_expect_tx(bar(BAR_DO_FULL + dst), TILE);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) {
-            const uint32_t a_off = ((kk >> 2) * KV_SLAB + (kk & 3) * 32) >> 4, b_off = ((kk >> 2) * Q_SLAB + (kk & 3) * 32) >> 4;
-            umma_bf16_lh(tmem_base + COL_DP + st * BQ, v_km + a_off, HI, qb_km + QT16 + b_off, HI, idesc_st, kk != 0);
-          }
-          umma_commit(bar(BAR_DP_FULL + st));
+          for (int sl = 0; sl < SLABS; ++sl)
+            tma_load_2d(sdo + sl * SLAB, &tmDO, bar(BAR_DO_FULL + dst), w.h * D + 64 * sl, q_row0);
         }
         __syncwarp();
       }
-      if (t >= 1) {
-        const int u = t - 1, pb = u & 1, qs = u % QDO_STAGES;
-        const uint32_t use = static_cast<uint32_t>(u >> 1);
-        if (!mbar_wait_warp(bar(BAR_PDS_FULL + pb), use & 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t qb_mn = q_mn0 + qs * STAGE16;
-        const uint32_t dsb_mn = ds_mn0 + pb * PDS16;
-        // queries 16k..16k+15 of tile u: P^T in columns 16k..16k+7 of its score buffer, dS^T in 16k+8..16k+15
-        const uint32_t pt_tmem = tmem_base + COL_S + pb * BQ;
+      if (!ok) {
+        const uint64_t t0 = ftb200::globaltimer_ns();
+        while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      // ---------------- MMA issuer ----------------
+      const uint32_t F = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(128 >> 4) << 24);
+      const uint32_t idesc_st = F | (static_cast<uint32_t>(BQ >> 3) << 17);                            // N = 128, K-major both
+      const uint32_t idesc_kv = F | (1u << 16) | (static_cast<uint32_t>(D >> 3) << 17);                // N = D, B MN-major
+      const uint32_t idesc_dq = F | (1u << 15) | (1u << 16) | (static_cast<uint32_t>(BQ >> 3) << 17);  // N = 128, both MN-major
+      constexpr uint32_t HI = smem_desc_hi(1024);
+      const uint32_t k_km = smem_desc_lo(smem_base + Ly::OFF_K, 16);  // K as K-major A (S^T)
+      const uint32_t v_km = smem_desc_lo(smem_base + Ly::OFF_V, 16);  // V as K-major A (dP^T)
+      // K as MN-major A (dQ^T): M = 128 runs over the head dim.  With head dim 64 the second 64 rows of that MMA
+      // read the slab behind K's only one, which is V's: lanes 64..127 of dQ^T then hold a product nobody reads.
+      const uint32_t k_mn = smem_desc_lo(smem_base + Ly::OFF_K, SLAB);
+      const uint32_t q_km0 = smem_desc_lo(smem_base + Ly::OFF_Q, 16), q_mn0 = smem_desc_lo(smem_base + Ly::OFF_Q, SLAB);
+      const uint32_t do_km0 = smem_desc_lo(smem_base + Ly::OFF_DO, 16), do_mn0 = smem_desc_lo(smem_base + Ly::OFF_DO, SLAB);
+      const uint32_t ds_mn = smem_desc_lo(smem_base + Ly::OFF_DS, SLAB);
+      constexpr uint32_t TILE16 = TILE >> 4;
+      // queries 16k..16k+15 of P^T (of dS^T): 8 columns at the start of the half of S^T (dP^T) that the writing thread read
+      auto pt_col = [](int kk) { return (kk >> 2) * 64 + (kk & 3) * 8; };
+
+      auto score = [&](uint32_t d_col, uint32_t a_km, uint32_t b_km, int full) {  // S^T or dP^T
         if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < BKV / 16; ++kk) {  // dQ^T = K^T dS^T, over dP^T of the tile (read by the softmax)
-            umma_bf16_lh(tmem_base + COL_DP + pb * BQ, k_mn + ((kk * 2048) >> 4), HI, dsb_mn + ((kk * 2048) >> 4), HI, idesc_dq, kk != 0);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = ((kk >> 2) * SLAB + (kk & 3) * 32) >> 4;
+            umma_bf16_lh(tmem_base + d_col, a_km + off, HI, b_km + off, HI, idesc_st, kk != 0);
           }
-          umma_commit(bar(BAR_DQ_FULL + pb));
-#pragma unroll
-          for (int kk = 0; kk < BQ / 16; ++kk) {  // dV += P^T dO
-            umma_bf16_tmem_a(tmem_base + COL_DV, pt_tmem + kk * 16, qb_mn + QT16 + ((kk * 2048) >> 4), HI, idesc_kv, (u | kk) != 0);
-          }
-#pragma unroll
-          for (int kk = 0; kk < BQ / 16; ++kk) {  // dK += dS^T Q
-            umma_bf16_tmem_a(tmem_base + COL_DK, pt_tmem + kk * 16 + 8, qb_mn + ((kk * 2048) >> 4), HI, idesc_kv, (u | kk) != 0);
-          }
-          umma_commit(bar(BAR_QDO_EMPTY + qs));
+          umma_commit(bar(full));
         }
         __syncwarp();
+      };
+      auto from_tmem = [&](uint32_t d_col, uint32_t a_col, uint32_t b_mn, bool first, int freed) {  // dV or dK
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < BQ / 16; ++kk)
+            umma_bf16_tmem_a(tmem_base + d_col, tmem_base + a_col + pt_col(kk), b_mn + ((kk * 2048) >> 4), HI, idesc_kv,
+                             !first || kk != 0);
+          umma_commit(bar(freed));
+        }
+        __syncwarp();
+      };
+      auto wait = [&](int which, uint32_t parity) {
+        const bool w = mbar_wait_warp(bar(which), parity, abort_flag);
+        tc_fence_after();
+        return w;
+      };
+      // S^T of the next tile is issued ahead of the products that wait for this tile's dS^T, so that its softmax runs
+      // under them; the columns of S^T are free for it as P^T's reader, dV, was issued before.
+      bool ok = wait(BAR_KV, 0) && wait(BAR_Q_FULL, 0);
+      if (ok) score(Ly::COL_S, k_km, q_km0, BAR_S_FULL);
+      ok = ok && wait(BAR_DO_FULL, 0);
+      if (ok) score(Ly::COL_DP, v_km, do_km0, BAR_DP_FULL);
+      for (int t = 0; t < T && ok; ++t) {
+        const int st = t % STAGES, nst = (t + 1) % STAGES;
+        const uint32_t odd = static_cast<uint32_t>(t) & 1u, nph = static_cast<uint32_t>((t + 1) / STAGES) & 1u;
+        const int dst = t % Ly::DO_STAGES, ndst = (t + 1) % Ly::DO_STAGES;
+        if (!(ok = wait(BAR_P_READY, odd))) break;
+        from_tmem(Ly::COL_DV, Ly::COL_S, do_mn0 + dst * TILE16, t == 0, BAR_DO_EMPTY + dst);
+        if (t + 1 < T) {
+          if (!(ok = wait(BAR_Q_FULL + nst, nph))) break;
+          score(Ly::COL_S, k_km, q_km0 + nst * TILE16, BAR_S_FULL);
+        }
+        if (!(ok = wait(BAR_DS_READY, odd))) break;
+        from_tmem(Ly::COL_DK, Ly::COL_DP, q_mn0 + st * TILE16, t == 0, BAR_Q_EMPTY + st);
+        if (!Ly::DQ_OVER_DP && !(ok = wait(BAR_DQ_EMPTY, odd ^ 1u))) break;  // dQ^T of tile t - 1 drained
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < BKV / 16; ++kk)  // dQ^T = K^T dS^T
+            umma_bf16_lh(tmem_base + Ly::COL_DQ, k_mn + ((kk * 2048) >> 4), HI, ds_mn + ((kk * 2048) >> 4), HI, idesc_dq, kk != 0);
+          umma_commit(bar(BAR_DQ_FULL));
+        }
+        __syncwarp();
+        if (t + 1 < T) {
+          if (!(ok = wait(BAR_DO_FULL + ndst, static_cast<uint32_t>((t + 1) / Ly::DO_STAGES) & 1u))) break;
+          if (Ly::DQ_OVER_DP && !(ok = wait(BAR_DQ_EMPTY, odd))) break;  // dQ^T of tile t drained
+          score(Ly::COL_DP, v_km, do_km0 + ndst * TILE16, BAR_DP_FULL);
+        }
       }
+      if (ok && elect_one()) umma_commit(bar(BAR_DKV_DONE));
+      __syncwarp();
     }
-    if (ok && elect_one()) umma_commit(bar(BAR_DKV_DONE));
-    __syncwarp();
-  } else if (warp >= 18) {
-    // ---------------- dQ drain (warps 18..21): TMEM lane = head-dim index ----------------
+  } else if (warp < 8) {
+    // ---------------- dQ drain: TMEM lane = head-dim index ----------------
+    regs_inc<DRAIN_REGS>();
     const int quarter = warp & 3;
-    const int dcol = quarter * 32 + lane;
-    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t dq_addr = tmem_base + Ly::COL_DQ + (static_cast<uint32_t>(quarter * 32) << 16);
+    const bool mine = quarter * 32 < D;  // head dim 64: only lanes 0..63 of dQ^T are real
+    const uint32_t off = Ly::OFF_DQ + quarter * 2 * DQ_PART_BYTES;
+    constexpr int PER = BQ / 4 / DQ_PARTS;  // groups of four queries in a part
     TileWalk w{hk * rep, first_q};
     for (int u = 0; u < T; ++u, next_tile(w)) {
-      const int buf = u & 1;
-      if (!mbar_wait_warp(bar(BAR_DQ_FULL + buf), static_cast<uint32_t>(u >> 1) & 1u, abort_flag)) break;
+      if (!mbar_wait_warp(bar(BAR_DQ_FULL), static_cast<uint32_t>(u) & 1u, abort_flag)) break;
       tc_fence_after();
       uint32_t v[BQ];
-      const bool mine = quarter * 32 < D;  // head dim 64: only lanes 0..63 of dQ^T are real
       if (mine) {
-        tmem_ld32(tmem_base + COL_DP + buf * BQ + lane_addr, v);
-        tmem_ld32(tmem_base + COL_DP + buf * BQ + 32 + lane_addr, v + 32);
+#pragma unroll
+        for (int c = 0; c < BQ / 32; ++c) tmem_ld32(dq_addr + c * 32, v + c * 32);
         tmem_wait_ld();
       }
       tc_fence_before();
-      mbar_arrive_warp(bar(BAR_DQ_EMPTY + buf));
+      mbar_arrive_warp(bar(BAR_DQ_EMPTY));
       if (mine) {
-        // four queries of one head-dim element lie together: a warp adds 512 consecutive bytes per instruction
         const long long tile = (static_cast<long long>(b) * n_qtiles + w.qt) * p.n_heads + w.h;
-        float* dst = p.dq_acc + tile * (BQ * D) + dcol * 4;
+        float* dst = p.dq_acc + tile * (BQ * D) + quarter * (32 * BQ);
 #pragma unroll
-        for (int c = 0; c < BQ / 4; ++c)
-          red_add_v4(dst + c * (D * 4), __uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]), __uint_as_float(v[4 * c + 2]),
-                     __uint_as_float(v[4 * c + 3]));
+        for (int part = 0; part < DQ_PARTS; ++part) {
+          const uint32_t buf = off + (part & 1) * DQ_PART_BYTES;
+          // the reduction that read this buffer last, two before this one, has read it
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+#pragma unroll
+          for (int c = 0; c < PER; ++c) {
+            const uint32_t* x = v + (part * PER + c) * 4;
+            *reinterpret_cast<uint4*>(smem + buf + (c * 32 + lane) * 16) = make_uint4(x[0], x[1], x[2], x[3]);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            bulk_add_f32(dst + part * (DQ_PART_BYTES / 4), smem_base + buf, DQ_PART_BYTES);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
   } else {
-    // ---------------- softmax, dK/dV store (warps 2..17) ----------------
+    // ---------------- softmax, dK/dV store ----------------
+    regs_inc<SOFTMAX_REGS>();
     const int quarter = warp & 3;
-    const int sw = (warp - 2) >> 2;       // four warps with the same columns
-    const int grp = sw >> 1, g = sw & 1;  // which tiles (even or odd), which 32 of the tile's 64 queries
+    const int g = (warp - 8) >> 2;        // which 64 of the tile's queries
     const int row = quarter * 32 + lane;  // key within the block
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     bool ok = true;
     const unsigned long long scale2 = f2_pack(p.scale_log2, p.scale_log2), dscale2 = f2_pack(p.scale, p.scale);
-    const int key = jb * BKV + row;
     TileWalk w{hk * rep, first_q};
-    if (grp == 1) next_tile(w);
-    const uint32_t s_addr = tmem_base + COL_S + grp * BQ + g * CPT + lane_addr;
-    const uint32_t dp_addr = tmem_base + COL_DP + grp * BQ + g * CPT + lane_addr;
-    uint8_t* drow = smem + OFF_PDS + grp * PDS_BYTES + row * 128;
-    for (int t = grp; t < T; t += 2, next_tile(w), next_tile(w)) {
-      const uint32_t use = static_cast<uint32_t>(t >> 1);
-      const int qs = t % QDO_STAGES;
-      // the tile's statistics arrived with Q and dO
-      if (!mbar_wait_warp(bar(BAR_S_FULL + grp), use & 1u, abort_flag) ||
-          !mbar_wait_warp(bar(BAR_QDO_FULL + qs), static_cast<uint32_t>(t / QDO_STAGES) & 1u, abort_flag)) {
+    const uint32_t s_addr = tmem_base + Ly::COL_S + g * CPT + lane_addr;
+    const uint32_t dp_addr = tmem_base + Ly::COL_DP + g * CPT + lane_addr;
+    uint8_t* drow = smem + Ly::OFF_DS + g * SLAB + row * 128;
+    for (int t = 0; t < T && ok; ++t, next_tile(w)) {
+      const uint32_t odd = static_cast<uint32_t>(t) & 1u;
+      const int st = t % STAGES;
+      // the tile's statistics arrived with Q
+      if (!mbar_wait_warp(bar(BAR_Q_FULL + st), static_cast<uint32_t>(t / STAGES) & 1u, abort_flag) ||
+          !mbar_wait_warp(bar(BAR_S_FULL), odd, abort_flag)) {
         ok = false;
         break;
       }
       tc_fence_after();
       // pairs of -log2(e) lse and -scale delta, as the packed arithmetic takes them
-      const ulonglong2* stats2 = reinterpret_cast<const ulonglong2*>(smem + OFF_STATS + qs * STATS_BYTES) + g * (CPT / 4);
-      const int q0 = w.qt * BQ + g * CPT;
-      const bool diag = (p.causal != 0) && (q0 < jb * BKV + BKV);
-#pragma unroll
-      for (int cc = 0; cc < CPT / CHUNK; ++cc) {
-        uint32_t sv[CHUNK], dp[CHUNK];
-        tmem_ld16(s_addr + cc * CHUNK, sv);
-        if (cc > 0) tmem_ld16(dp_addr + cc * CHUNK, dp);
+      const ulonglong2* lse2 = reinterpret_cast<const ulonglong2*>(smem + Ly::OFF_STATS + st * STATS_BYTES) + g * (CPT / 4);
+      const ulonglong2* delta2 = lse2 + BQ / 4;
+      float pe[CPT];
+      {
+        uint32_t sv[CPT];
+        tmem_ld32(s_addr, sv);
+        tmem_ld32(s_addr + 32, sv + 32);
         tmem_wait_ld();
-        float pe[CHUNK];
 #pragma unroll
-        for (int c = 0; c < CHUNK / 4; ++c) {
-          const ulonglong2 l4 = stats2[cc * (CHUNK / 4) + c];
+        for (int c = 0; c < CPT / 4; ++c) {
+          const ulonglong2 l4 = lse2[c];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int qi = 4 * c + 2 * e;
@@ -393,73 +428,79 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             pe[qi + 1] = exp2f(pe[qi + 1]);
           }
         }
-        if (diag) {
+      }
+      if (p.causal != 0 && w.qt == jb) {  // the diagonal tile: queries before the key
 #pragma unroll
-          for (int c = 0; c < CHUNK; ++c)
-            if (key > q0 + cc * CHUNK + c) pe[c] = 0.f;
+        for (int c = 0; c < CPT; ++c)
+          if (row > g * CPT + c) pe[c] = 0.f;
+      }
+      {
+        uint32_t pt[CPT / 2];
+#pragma unroll
+        for (int c = 0; c < CPT / 2; ++c) {
+          __nv_bfloat162 a = __floats2bfloat162_rn(pe[2 * c], pe[2 * c + 1]);
+          pt[c] = *reinterpret_cast<uint32_t*>(&a);
         }
-        if (cc == 0) {
-          if (!mbar_wait_warp(bar(BAR_DP_FULL + grp), use & 1u, abort_flag)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          tmem_ld16(dp_addr, dp);
-          tmem_wait_ld();
-        }
-        uint32_t pds[CHUNK];  // P^T, dS^T
+        tmem_st32(s_addr, pt);  // over scores that this thread has read
+        tmem_wait_st();
+      }
+      tc_fence_before();
+      mbar_arrive_warp(bar(BAR_P_READY));
+
+      if (!mbar_wait_warp(bar(BAR_DP_FULL), odd, abort_flag)) {  // dK and dQ^T of tile t - 1 are complete too: dS^T is free
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      uint32_t dp[2][CHUNK];
+      tmem_ld16(dp_addr, dp[0]);
+      tmem_wait_ld();
+#pragma unroll
+      for (int cc = 0; cc < CPT / CHUNK; ++cc) {
+        if (cc + 1 < CPT / CHUNK) tmem_ld16(dp_addr + (cc + 1) * CHUNK, dp[(cc + 1) & 1]);
+        const uint32_t* d = dp[cc & 1];
+        uint32_t ds[CHUNK / 2];
 #pragma unroll
         for (int c = 0; c < CHUNK / 4; ++c) {
-          const ulonglong2 d4 = stats2[BQ / 4 + cc * (CHUNK / 4) + c];
+          const ulonglong2 d4 = delta2[cc * (CHUNK / 4) + c];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int qi = 4 * c + 2 * e;
             // dS = P (scale dP - scale delta)
             const unsigned long long ds2 =
-                f2_mul(f2_pack(pe[qi], pe[qi + 1]),
-                       f2_fma(f2_pack(__uint_as_float(dp[qi]), __uint_as_float(dp[qi + 1])), dscale2, e == 0 ? d4.x : d4.y));
+                f2_mul(f2_pack(pe[cc * CHUNK + qi], pe[cc * CHUNK + qi + 1]),
+                       f2_fma(f2_pack(__uint_as_float(d[qi]), __uint_as_float(d[qi + 1])), dscale2, e == 0 ? d4.x : d4.y));
             float s0, s1;
             f2_unpack(ds2, s0, s1);
-            __nv_bfloat162 a = __floats2bfloat162_rn(pe[qi], pe[qi + 1]);
-            __nv_bfloat162 d2 = __floats2bfloat162_rn(s0, s1);
-            pds[qi / 2] = *reinterpret_cast<uint32_t*>(&a);
-            pds[CHUNK / 2 + qi / 2] = *reinterpret_cast<uint32_t*>(&d2);
+            __nv_bfloat162 x = __floats2bfloat162_rn(s0, s1);
+            ds[qi / 2] = *reinterpret_cast<uint32_t*>(&x);
           }
         }
-        // the dS^T buffer is free once dQ^T of the group's tile before is complete
-        if (cc == 0 && !mbar_wait_warp(bar(BAR_DQ_FULL + grp), (use & 1u) ^ 1u, abort_flag)) {
-          ok = false;
-          break;
-        }
-        // P^T and dS^T replace the scores this thread has just read (its own 16 columns)
-        tmem_st16(s_addr + cc * CHUNK, pds);
+        if (cc + 1 < CPT / CHUNK) tmem_wait_ld();
+        tmem_st8(dp_addr + cc * (CHUNK / 2), ds);  // over columns that this thread has read
 #pragma unroll
         for (int c = 0; c < CHUNK / 8; ++c) {
-          const int chunk = ((g * (CPT / 8) + cc * (CHUNK / 8) + c) ^ (row & 7)) << 4;
-          *reinterpret_cast<uint4*>(drow + chunk) = make_uint4(pds[CHUNK / 2 + 4 * c], pds[CHUNK / 2 + 4 * c + 1],
-                                                               pds[CHUNK / 2 + 4 * c + 2], pds[CHUNK / 2 + 4 * c + 3]);
+          const int at = ((cc * (CHUNK / 8) + c) ^ (row & 7)) << 4;
+          *reinterpret_cast<uint4*>(drow + at) = make_uint4(ds[4 * c], ds[4 * c + 1], ds[4 * c + 2], ds[4 * c + 3]);
         }
       }
-      if (!ok) break;
       fence_async_smem();
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive_warp(bar(BAR_PDS_FULL + grp));
+      mbar_arrive_warp(bar(BAR_DS_READY));
     }
     if (ok && mbar_wait_warp(bar(BAR_DKV_DONE), 0, abort_flag)) {
       tc_fence_after();
 #pragma unroll
       for (int which = 0; which < 2; ++which) {
-        constexpr int CW = D / 4;  // head-dim columns per thread
-        const uint32_t col = (which == 0 ? COL_DV : COL_DK) + sw * CW;
+        constexpr int CW = D / 2;  // head-dim columns per thread
+        const uint32_t col = (which == 0 ? Ly::COL_DV : Ly::COL_DK) + g * CW;
         __nv_bfloat16* base = which == 0 ? p.dV : p.dK;
         const long long ld = which == 0 ? p.ld_dv : p.ld_dk;
-        __nv_bfloat16* dst = base + static_cast<long long>(kv_row0 + row) * ld + hk * D + sw * CW;
+        __nv_bfloat16* dst = base + static_cast<long long>(kv_row0 + row) * ld + hk * D + g * CW;
         uint32_t v[CW];
-        if constexpr (CW == 32)
-          tmem_ld32(tmem_base + col + lane_addr, v);
-        else
-          tmem_ld16(tmem_base + col + lane_addr, v);
+#pragma unroll
+        for (int c = 0; c < CW / 32; ++c) tmem_ld32(tmem_base + col + c * 32 + lane_addr, v + c * 32);
         tmem_wait_ld();
 #pragma unroll
         for (int c = 0; c < CW / 8; ++c) {
@@ -515,8 +556,8 @@ __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bflo
   }
 }
 
-// dq (bf16, row stride ld) = accumulator (fp32, per 64-query tile and head [16][D][4 queries]); a thread takes 8
-// head-dim elements of 4 queries.
+// dq (bf16, row stride ld) = accumulator (fp32, per 128 queries and head [D / 32][32 groups of 4 queries][32][4 queries]); a
+// thread takes 8 head-dim elements of 4 queries.
 template <int D>
 __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
                                                                 long long pieces, int n_heads, long long ld) {
@@ -524,13 +565,14 @@ __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __
   if (i >= pieces) return;
   const int d8 = static_cast<int>(i % (D / 8));
   const long long g = i / (D / 8);  // (tile, head, group of 4 queries)
-  const int q4 = static_cast<int>(g & 15);
-  const long long th = g >> 4;
+  const int q4 = static_cast<int>(g & 31);
+  const long long th = g >> 5;
   const int h = static_cast<int>(th % n_heads);
-  const long long row0 = th / n_heads * 64 + q4 * 4;
+  const long long row0 = th / n_heads * 128 + q4 * 4;
+  const float4* src = acc + th * (32 * D) + (d8 >> 2) * 1024 + q4 * 32 + (d8 & 3) * 8;
   float4 v[8];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) v[e] = acc[g * D + d8 * 8 + e];
+  for (int e = 0; e < 8; ++e) v[e] = src[e];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     float f[8];
@@ -603,6 +645,10 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
     if (cudaFuncSetAttribute(attention_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
         cudaSuccess)
       return FTB200_E_CUDA;
+    // the warpgroups share out what a CTA is launched with: with fewer registers a thread the increase would wait for good
+    cudaFuncAttributes attr;
+    if (cudaFuncGetAttributes(&attr, attention_bwd_kernel<D>) != cudaSuccess) return FTB200_E_CUDA;
+    if (attr.numRegs < LAUNCH_REGS) return FTB200_E_REGS;
     attr_set = true;
   }
   const long long pieces = rows * n_heads * (D / 8);

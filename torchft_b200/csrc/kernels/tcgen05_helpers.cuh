@@ -207,6 +207,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
 // Two fp32 operations per instruction (the packed forms of Blackwell's FMA pipe): the softmax loops are bound by issue
 // slots, and a scaled score, a sum or a polynomial step then costs half of one.
 __device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
