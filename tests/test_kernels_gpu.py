@@ -55,6 +55,32 @@ def test_gemm_tile_width(a_mn, b_mn, past):
     K.check_status(out.device)
 
 
+@pytest.mark.parametrize("M", [1, 33, 160, 257])
+@pytest.mark.parametrize("N", [8, 72, 200, 328, 12])
+def test_gemm_store_edges(M, N):
+    """Outputs that end inside the epilogue's 32-row, 64-column pieces, with and without the fused activation, and one (12
+    columns) that takes the general path: nothing beyond them is written, and the products are the same bits wherever they
+    lie in a piece."""
+    torch.manual_seed(M + N)
+    a, b = torch.randn(M, 96, device=DEV).bfloat16(), torch.randn(N, 96, device=DEV).bfloat16()
+    out = torch.full((M + 1, N + 12 - N % 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    K.gemm(a, b, out=out[:M, :N])
+    assert bool((out[M:] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+    # further rows and columns of tiles: other pieces, the same values
+    big = K.gemm(torch.cat([a, a]), torch.cat([b, b]))
+    assert torch.equal(out[:M, :N], big[M:, N:] if N % 8 == 0 else big[:M, :N])
+    assert rel_err(out[:M, :N], a.float() @ b.float().t()) < 2**-8
+    if N % 32 == 8:
+        N2 = 32 * (N // 8)
+        w = torch.randn(N2, 96, device=DEV).bfloat16()
+        gu, act = (torch.full((M + 1, n + 8), 7.0, device=DEV, dtype=torch.bfloat16) for n in (N2, N2 // 2))
+        K.linear_swiglu_fwd(a, w, gu[:M, :N2], act[:M, : N2 // 2])
+        assert torch.equal(gu[:M, :N2], K.gemm(a, w)) and torch.equal(act[:M, : N2 // 2], K.swiglu_fwd(gu[:M, :N2].contiguous()))
+        for t, n in ((gu, N2), (act, N2 // 2)):
+            assert bool((t[M:] == 7.0).all()) and bool((t[:, n:] == 7.0).all())
+    K.check_status(a.device)
+
+
 @pytest.mark.parametrize("impl", ["1cta", "2cta"])
 def test_gemm_many_tiles_persistent(impl):
     torch.manual_seed(2)

@@ -12,7 +12,7 @@
 //   full[s]   (leader)  both CTAs' TMA loads complete_tx on the leader's barrier
 //   empty[s]  (each)    the leader's tcgen05.commit arrives on both CTAs' barriers
 //   tfull[a]  (each)    likewise, after the last MMA of a tile
-//   tempty[a] (leader)  the 2 x 128 epilogue threads of the pair arrive (remote arrive
+//   tempty[a] (leader)  the 2 x 4 epilogue warps of the pair arrive (remote arrive
 //                       from the peer)
 // All waits are bounded as in the 1-CTA kernel.
 //
@@ -57,9 +57,10 @@ constexpr int GATHER_WARPS = 4;  // only launched by the all-gather variant
 constexpr int NUM_THREADS_GATHER = NUM_THREADS + 32 * GATHER_WARPS;
 constexpr int GATHER_PIECE_V = 1024;  // 16-byte vectors per piece (16 KiB)
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t SMEM_BYTES = RING_BYTES + 1024 + 256;
-constexpr uint32_t SC_STAGE_WARP_BYTES = 32 * 256;  // scatter epilogue: 32 rows x 128 bf16 per warp
-constexpr uint32_t SMEM_BYTES_SCATTER = SMEM_BYTES + 4 * SC_STAGE_WARP_BYTES;
+constexpr uint32_t STAGE_WARP_BYTES = 32 * 256;  // epilogue: 32 rows x 128 bf16 per warp
+constexpr uint32_t OFF_STAGING = RING_BYTES, OFF_MISC = OFF_STAGING + 4 * STAGE_WARP_BYTES;
+constexpr uint32_t SMEM_BYTES = OFF_MISC + 256 + 1024;
+static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
 constexpr int GROUP_M = 8;  // in 256-row pair tiles (the all-gather variant uses twice that)
 
 using namespace ftb200::tc;
@@ -76,9 +77,10 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   return r;
 }
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+// Orders nothing: with release semantics it would first wait for the kernel's stores to arrive, 1200 cycles at its end.
+__device__ __forceinline__ void cluster_sync_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
@@ -94,6 +96,19 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       "[%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
       : "memory");
+}
+
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
+// Stores a tile of shared memory; what lies beyond the tensor is left out.  The calling thread's bulk group has to be
+// committed.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(src), "r"(c0), "r"(c1)
+               : "memory");
 }
 
 __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -122,6 +137,7 @@ struct GemmParams {
   int a_mn, b_mn;
   int out_fp32;
   int accumulate;
+  int tma_out;                 // bf16 output through tmC (rows and columns beyond M and N are clipped)
   long long ldc;
   void* C;
   int* status;
@@ -173,20 +189,34 @@ __device__ __forceinline__ bool count_wait_warp(const unsigned int* p, unsigned 
   return __all_sync(0xffffffffu, ok);
 }
 
+// silu(gate) * up of four (gate, up) pairs: the activation of the rounded values, so that a later recompute from C agrees.
+__device__ __forceinline__ uint2 silu_mul(const ftb200::bf16x8& packed) {
+  float g[8], sv[4];
+  ftb200::unpack8(packed, g);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) sv[e] = g[2 * e] / (1.f + __expf(-g[2 * e])) * g[2 * e + 1];
+  __nv_bfloat162 lo = __floats2bfloat162_rn(sv[0], sv[1]), hi = __floats2bfloat162_rn(sv[2], sv[3]);
+  uint2 o;
+  o.x = *reinterpret_cast<uint32_t*>(&lo);
+  o.y = *reinterpret_cast<uint32_t*>(&hi);
+  return o;
+}
+
 template <int BN_>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS_GATHER, 1)
 gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                              const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux,
                               const GemmParams p) {
   using TL = Tile<BN_>;
   constexpr int BN = TL::BN, BNH = TL::BNH, STAGES = TL::STAGES;
   constexpr uint32_t STAGE_BYTES = TL::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_MISC);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -198,18 +228,19 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
   auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 + s); };
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
-    }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(tfull_bar(s), 1);
-      mbar_init(tempty_bar(s), 256);
-    }
-    *abort_flag = 0;
+  if (warp == 0) {
+    if (lane < 2 * STAGES) mbar_init(bar_base + 8u * lane, 1);                             // full, empty
+    if (lane >= 16 && lane < 20) mbar_init(tfull_bar(lane - 16), lane < 18 ? 1 : 2 * 4);  // tfull, tempty (one arrival a warp)
+    if (lane == 20) *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (lane == 0) {
+      prefetch_map(&tmA);
+      prefetch_map(&tmB);
+      if (p.tma_out) prefetch_map(&tmC);
+      if (p.tma_out && p.aux != nullptr) prefetch_map(&tmAux);
+    }
+    __syncwarp();
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -217,11 +248,6 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  cluster_sync_all();  // the partner's barriers exist before anything signals them
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
 
   const int num_m = (p.M + 2 * BM - 1) / (2 * BM);
   const int num_n = (p.N + BN - 1) / BN;
@@ -240,6 +266,14 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     m0 = (first_m + r % gsz) * (2 * BM) + static_cast<int>(rank) * BM;  // this CTA's rows
     n0 = (r / gsz) * BN;
   };
+  int m0, n0;
+  tile_coords(cluster_id, m0, n0);  // of the first tile, while the barriers and the TMEM are on their way
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_sync_relaxed();  // the partner's barriers exist (they were fenced) before anything signals them
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
@@ -247,8 +281,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     uint32_t phase = 0;
     bool ok = true;
     for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
-      int m0, n0;
-      tile_coords(t, m0, n0);
+      if (t != cluster_id) tile_coords(t, m0, n0);
       const int nb = n0 + static_cast<int>(rank) * BNH;  // this CTA's half of the B tile
       if (BNH == GATHER_BLOCK && p.ga_world > 0 && nb < p.N) {
         // these 128 rows of B are local once all their pieces are counted; the loads below go through the
@@ -399,18 +432,74 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     uint32_t acc_phase = 0;
     const bool vec_ok = p.out_fp32 ? ((p.ldc & 3) == 0) : ((p.ldc & 7) == 0);
     for (int t = cluster_id; t < num_tiles; t += num_clusters) {
-      int m0, n0;
-      tile_coords(t, m0, n0);
-      if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag)) break;
+      if (t != cluster_id) tile_coords(t, m0, n0);
+      if (!mbar_wait_warp(tfull_bar(acc), acc_phase, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row = m0 + q * 32 + lane;
       const uint32_t taddr0 = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
-      if (p.sc_world > 0 || (!p.out_fp32 && !p.accumulate && vec_ok && (p.N & 7) == 0)) {
-        // Staged epilogue (bf16 output, local or scattered to peers): the tile goes through a
-        // per-warp staging area so that every store instruction covers two 256-byte row segments.
-        // One 16-byte piece per thread and row would touch 32 rows per instruction: half-filled
-        // sectors locally, and an NVLink packet each towards a peer, which throttles the kernel.
-        uint8_t* stg = smem + STAGES * STAGE_BYTES + 256 + q * SC_STAGE_WARP_BYTES;
+      const uint32_t stg = OFF_STAGING + q * STAGE_WARP_BYTES;
+      if (p.tma_out) {
+        // bf16 output: 64 columns at a time go, one row a thread, into a 128-byte-swizzled piece of the warp's staging area
+        // and leave by TMA (which clips what lies beyond M and N), while the next 64 come out of tensor memory.  Nothing hides
+        // the last tile's epilogue: 5800 cycles for 256 columns that leave a row-major staging area as row segments, 4100
+        // this way, all in all 14.2 -> 12.6 us for 3000 x 1536 x 1024, 17.3 -> 14.5 us for 1024 x 1024 x 3000.
+        constexpr int PIECES = BN / 64;
+        uint32_t r[2][64];
+        tmem_ld32(taddr0, r[0]);
+        tmem_ld32(taddr0 + 32, r[0] + 32);
+#pragma unroll
+        for (int c = 0; c < PIECES; ++c) {
+          tmem_wait_ld();
+          if (c + 1 < PIECES) {
+            tmem_ld32(taddr0 + (c + 1) * 64, r[(c + 1) & 1]);
+            tmem_ld32(taddr0 + (c + 1) * 64 + 32, r[(c + 1) & 1] + 32);
+          } else {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+          }
+          const uint32_t* v = r[c & 1];
+          const bool inside = n0 + c * 64 < p.N && m0 + q * 32 < p.M;
+          // With an activation the two halves of the area are one for C and one for 64 columns of aux, which two pieces fill.
+          const bool with_aux = p.aux != nullptr;
+          const uint32_t piece = with_aux ? stg : stg + (c & 1) * (STAGE_WARP_BYTES / 2);
+          if (lane == 0) {  // what was stored from this half last has been read
+            if (with_aux)
+              asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            else
+              asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          }
+          __syncwarp();
+          uint8_t* prow = smem + piece + lane * 128;
+          uint8_t* arow = smem + stg + STAGE_WARP_BYTES / 2 + lane * 128;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * j + e]);
+            const ftb200::bf16x8 packed = ftb200::pack8(f);
+            *reinterpret_cast<ftb200::bf16x8*>(prow + ((j ^ (lane & 7)) << 4)) = packed;
+            if (with_aux) *reinterpret_cast<uint2*>(arow + ((((c & 1) * 4 + (j >> 1)) ^ (lane & 7)) << 4) + (j & 1) * 8) = silu_mul(packed);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0 && inside) {
+            tma_store_2d(&tmC, smem_base + piece, n0 + c * 64, m0 + q * 32);
+            if (with_aux && ((c & 1) || n0 + (c + 1) * 64 >= p.N))
+              tma_store_2d(&tmAux, smem_base + stg + STAGE_WARP_BYTES / 2, (n0 + (c & ~1) * 64) >> 1, m0 + q * 32);
+          }
+          if (lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1u;
+        }
+        continue;
+      }
+      if (p.sc_world > 0) {
+        // Scattered to the owners' memory: the tile goes through a per-warp staging area so that every store instruction
+        // covers two 256-byte row segments.  One 16-byte piece per thread and row would touch 32 rows per instruction: an
+        // NVLink packet each, which throttles the kernel.
         const int half = lane >> 4, ch = lane & 15;
 #pragma unroll 1
         for (int cg = 0; cg < BN / 128; ++cg) {
@@ -424,7 +513,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
               float f[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]);
-              *reinterpret_cast<ftb200::bf16x8*>(stg + lane * 256 + (((cc * 4 + j) ^ (lane & 15)) << 4)) = ftb200::pack8(f);
+              *reinterpret_cast<ftb200::bf16x8*>(smem + stg + lane * 256 + (((cc * 4 + j) ^ (lane & 15)) << 4)) = ftb200::pack8(f);
             }
           }
           __syncwarp();
@@ -433,33 +522,14 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
           for (int it = 0; it < 16; ++it) {
             const int rr = it * 2 + half;
             const int grow = m0 + q * 32 + rr;
-            const ftb200::bf16x8 v = *reinterpret_cast<const ftb200::bf16x8*>(stg + rr * 256 + ((ch ^ (rr & 15)) << 4));
+            const ftb200::bf16x8 v = *reinterpret_cast<const ftb200::bf16x8*>(smem + stg + rr * 256 + ((ch ^ (rr & 15)) << 4));
             if (grow < p.M && gcol + 8 <= p.N) {
-              if (p.sc_world > 0) {
-                const long long flat = p.sc_off + static_cast<long long>(grow) * p.ldc + gcol;
-                const long long owner = flat / p.sc_shard;
-                const long long rem = flat - owner * p.sc_shard;
-                if (!FTB_IN_RANGE(owner, p.sc_world)) continue;
-                __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.sc_peers[owner]);
-                *reinterpret_cast<ftb200::bf16x8*>(base + static_cast<long long>(p.sc_src) * p.sc_shard + rem) = v;
-              } else {
-                __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(grow) * p.ldc;
-                *reinterpret_cast<ftb200::bf16x8*>(crow + gcol) = v;
-                if (p.aux != nullptr) {
-                  // activation of the rounded values, so that a later recompute from C agrees
-                  float g[8];
-                  ftb200::unpack8(v, g);
-                  float sv[4];
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) sv[e] = g[2 * e] / (1.f + __expf(-g[2 * e])) * g[2 * e + 1];
-                  __nv_bfloat162 lo = __floats2bfloat162_rn(sv[0], sv[1]), hi = __floats2bfloat162_rn(sv[2], sv[3]);
-                  uint2 o2;
-                  o2.x = *reinterpret_cast<uint32_t*>(&lo);
-                  o2.y = *reinterpret_cast<uint32_t*>(&hi);
-                  *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.aux) + static_cast<long long>(grow) * p.ld_aux +
-                                            (gcol >> 1)) = o2;
-                }
-              }
+              const long long flat = p.sc_off + static_cast<long long>(grow) * p.ldc + gcol;
+              const long long owner = flat / p.sc_shard;
+              const long long rem = flat - owner * p.sc_shard;
+              if (!FTB_IN_RANGE(owner, p.sc_world)) continue;
+              __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.sc_peers[owner]);
+              *reinterpret_cast<ftb200::bf16x8*>(base + static_cast<long long>(p.sc_src) * p.sc_shard + rem) = v;
             }
           }
           __syncwarp();
@@ -511,21 +581,9 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
                 }
                 const ftb200::bf16x8 packed = ftb200::pack8(f);
                 reinterpret_cast<ftb200::bf16x8*>(dst)[j] = packed;
-                if (p.aux != nullptr) {
-                  // activation of the rounded values, so that a later recompute from C agrees
-                  float g[8];
-                  ftb200::unpack8(packed, g);
-                  float sv[4];
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) sv[e] = g[2 * e] / (1.f + __expf(-g[2 * e])) * g[2 * e + 1];
-                  __nv_bfloat162 lo = __floats2bfloat162_rn(sv[0], sv[1]), hi = __floats2bfloat162_rn(sv[2], sv[3]);
-                  uint2 o2;
-                  o2.x = *reinterpret_cast<uint32_t*>(&lo);
-                  o2.y = *reinterpret_cast<uint32_t*>(&hi);
-                  __nv_bfloat16* adst =
-                      reinterpret_cast<__nv_bfloat16*>(p.aux) + static_cast<long long>(row) * p.ld_aux + (col0 >> 1) + 4 * j;
-                  *reinterpret_cast<uint2*>(adst) = o2;
-                }
+                if (p.aux != nullptr)
+                  *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.aux) + static_cast<long long>(row) * p.ld_aux +
+                                            (col0 >> 1) + 4 * j) = silu_mul(packed);
               }
             } else {
 #pragma unroll
@@ -541,18 +599,20 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
       if (++acc == 2) {
         acc = 0;
         acc_phase ^= 1u;
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // no store reads the staging area any more
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag && p.status != nullptr) atomicExch(p.status, FTB200_ST_TIMEOUT);
-  cluster_sync_all();  // neither CTA retires while its partner may still touch its barriers or operands
+  cluster_sync_relaxed();  // neither CTA retires while its partner may still touch its barriers or operands
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -619,7 +679,7 @@ static int tile_columns(int M, int N, int pairs) {
 template <int BN>
 static int launch_2cta(const void* A, const void* B, long long lda, long long ldb, int ctas, int threads, const GemmParams& p,
                        cudaStream_t stream) {
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmC, tmAux;
   int rc;
   if (!p.a_mn)
     rc = encode_2d(&tmA, A, p.M, p.K, lda, BK, BM);
@@ -631,15 +691,21 @@ static int launch_2cta(const void* A, const void* B, long long lda, long long ld
   else
     rc = encode_2d(&tmB, B, p.K, p.N, ldb, 64, BK);
   if (rc) return rc;
+  tmC = tmAux = tmA;  // not used without tma_out
+  if (p.tma_out) {
+    rc = encode_2d(&tmC, p.C, p.M, p.N, p.ldc, 64, 32);
+    if (rc == 0 && p.aux != nullptr) rc = encode_2d(&tmAux, p.aux, p.M, p.N / 2, p.ld_aux, 64, 32);
+    if (rc) return rc;
+  }
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(gemm_bf16_tcgen05_2cta_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SMEM_BYTES_SCATTER) != cudaSuccess)
+                             SMEM_BYTES) != cudaSuccess)
       return FTB200_E_CUDA;
     attr_set = true;
   }
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
-  gemm_bf16_tcgen05_2cta_kernel<BN><<<std::min(2 * tiles, ctas), threads, SMEM_BYTES_SCATTER, stream>>>(tmA, tmB, p);
+  gemm_bf16_tcgen05_2cta_kernel<BN><<<std::min(2 * tiles, ctas), threads, SMEM_BYTES, stream>>>(tmA, tmB, tmC, tmAux, p);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
@@ -674,6 +740,9 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
     p.sc_off = sc->off;
     for (int i = 0; i < sc->world && i < 8; ++i) p.sc_peers[i] = sc->peers[i];
   }
+  // TMA wants 16-byte rows; what else comes (fp32, accumulation, other strides) takes the general path of the epilogue
+  p.tma_out = sc == nullptr && !p.out_fp32 && !p.accumulate && (ldc & 7) == 0 && ldc >= N && (N & 7) == 0 &&
+              (aux == nullptr || ((ld_aux & 7) == 0 && ld_aux >= N / 2 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0));
   p.group_m = GROUP_M;
   p.ga_world = 0;
   p.ga_shard = 0;
