@@ -55,6 +55,33 @@ def test_gemm_tile_width(a_mn, b_mn, past):
     K.check_status(out.device)
 
 
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("M,N,K_", [
+    (80, 1000, 14400),    # less than a wave of tiles; remainders in M and N
+    (752, 1024, 8200),    # a share of the K slabs each, one slab short
+    (1536, 4096, 9216),   # a whole wave first, then the shared tiles
+    (304, 520, 5000),     # K no multiple of 8 slabs times the pairs
+])
+def test_gemm_split_last_wave(a_mn, b_mn, M, N, K_):
+    """Tiles of the last wave that a cluster of pairs shares along K: bf16, fp32 and accumulated results, the same bits every
+    time.  fp32 sums of K products in another order: sqrt(K) * 2^-24 of the result, plus bf16 rounding where it is stored so."""
+    torch.manual_seed(M)
+    a = torch.randn((K_, M) if a_mn else (M, K_), device=DEV).bfloat16()
+    b = torch.randn((K_, N) if b_mn else (N, K_), device=DEV).bfloat16()
+    ref = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    out = torch.full((M, N + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    K.gemm(a, b, a_mn, b_mn, out=out[:, :N])
+    assert bool((out[:, N:] == 7.0).all()) and rel_err(out[:, :N], ref) < 2**-9
+    assert torch.equal(out[:, :N], K.gemm(a, b, a_mn, b_mn))
+    acc = torch.ones(M, N, device=DEV, dtype=torch.float32)
+    K.gemm(a, b, a_mn, b_mn, out=acc, accumulate=True)
+    assert ((acc - 1.0).double() - ref).norm() <= 4 * K_**0.5 * 2**-24 * ref.norm()
+    both = out[:, :N].clone()
+    K.gemm(a, b, a_mn, b_mn, out=both, accumulate=True)
+    assert rel_err(both, 2 * ref) < 2**-8
+    K.check_status(out.device)
+
+
 @pytest.mark.parametrize("M", [1, 33, 160, 257])
 @pytest.mark.parametrize("N", [8, 72, 200, 328, 12])
 def test_gemm_store_edges(M, N):

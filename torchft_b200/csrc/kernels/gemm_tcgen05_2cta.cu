@@ -1,7 +1,7 @@
 // bf16 GEMM with 2-SM tensor-core instructions (tcgen05.mma.cta_group::2).
 //
 // Same contract as the 1-CTA kernel in gemm_tcgen05.cu.  Two CTAs of a cluster share
-// one 256x256 output tile (256x128 where the output is small, see tile_columns): each stages its own 128 rows of A and its own 128 of the 256
+// one 256x256 output tile (256x128 where the output is small, see plan_tiles): each stages its own 128 rows of A and its own 128 of the 256
 // B columns (32 KiB per 64-deep K slab instead of 48 KiB), the pair's leader issues one
 // M=256 MMA that reads both halves of B, and each CTA's TMEM receives the accumulator of
 // its own 128 rows.  Per SM that is a third less shared-memory fill traffic per FLOP and
@@ -16,6 +16,14 @@
 //                       from the peer)
 // All waits are bounded as in the 1-CTA kernel.
 //
+// A last wave that leaves most pairs idle is split over K (SPLIT, see plan_tiles): a cluster of S pairs takes one of its
+// tiles, each pair a share of the K slabs, and after them the S accumulators meet through distributed shared memory:
+// every CTA owns the 32-column chunks c of its 128 rows with c * S / chunks == its pair and gets the other pairs' values
+// of them copied into its operand ring, which is free by then:
+//   ready     (each)    the S - 1 CTAs with the same rows in the other pairs have finished their products (remote arrive)
+//   got       (each)    their values have arrived (complete_tx of the copies)
+// The values are added in the order of the pairs, so the result does not depend on which one was first.
+//
 // All-gather fused into the GEMM (ftb200_gemm_bf16_gather): B is a weight whose rows lie
 // spread over the ranks of a shard group, as one contiguous piece of a flat parameter unit
 // that the ranks shard evenly.  Four extra warps per CTA pull the weight out of the owners'
@@ -27,6 +35,7 @@
 // handed out through a counter, so the CTAs that are running pull everything whether or
 // not the whole grid is resident.
 #include <algorithm>
+#include <atomic>
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -68,6 +77,12 @@ using namespace ftb200::tc;
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
 
@@ -125,8 +140,8 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t adesc, 
 
 // Arrive (once all MMAs issued so far have completed) on the barrier at the same
 // shared-memory offset in both CTAs of the pair.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-  const uint16_t mask = 3;
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t lead_cta) {
+  const uint16_t mask = static_cast<uint16_t>(3u << lead_cta);
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
                "h"(mask)
                : "memory");
@@ -160,7 +175,33 @@ struct GemmParams {
   const void* ga_peers[8];     // every rank's shard buffer (peer-mapped; [rank] is local)
   void* ga_dst;                // == B
   unsigned int* ga_sync;       // [0] next piece to hand out, [1 + c] pieces done of 128-row block c (zeroed per launch)
+  int whole;                   // SPLIT: this many tiles are worked on by one pair each, the rest by a cluster each
 };
+
+// Bounded mbarrier wait that also acquires what other CTAs of the cluster wrote before they arrived.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  const uint64_t t0 = ftb200::globaltimer_ns();
+  for (uint32_t polls = 1;; ++polls) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
+    if ((polls & 255u) == 0) {
+      const bool give_up = *abort_flag != 0 || ftb200::globaltimer_ns() - t0 > WAIT_LIMIT_NS;
+      if (__any_sync(0xffffffffu, give_up)) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+}
 
 // Bounded wait until *p >= want (device-scope acquire).
 __device__ __forceinline__ bool count_wait(const unsigned int* p, unsigned int want, volatile int* abort_flag) {
@@ -202,8 +243,23 @@ __device__ __forceinline__ uint2 silu_mul(const ftb200::bf16x8& packed) {
   return o;
 }
 
-template <int BN_>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS_GATHER, 1)
+// Asynchronous copy from this CTA's shared memory to another's, counted by a barrier there.
+__device__ __forceinline__ void copy_to_cta(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// Split last wave: a chunk is 32 columns of a CTA's 128 rows, a warp's share of it 32 rows.  With S pairs a CTA gets at
+// most MAX_IN of them (S = 3: two pairs' values of three chunks) and sends at most as many, in a ring of twice that.
+constexpr uint32_t CHUNK_BYTES = 128 * 32 * 4, SHARE_BYTES = CHUNK_BYTES / 4;
+constexpr int MAX_IN = 6;
+constexpr int MAX_SPLIT = 4;  // 8 CTAs: the largest cluster that every part takes
+static_assert(2 * MAX_IN * CHUNK_BYTES <= RING_BYTES, "the ring holds what comes and what goes");
+
+// Clusters of two CTAs (SPLIT: of 2 S), set at the launch.
+template <int BN_, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? NUM_THREADS : NUM_THREADS_GATHER, 1)
 gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                               const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux,
                               const GemmParams p) {
@@ -213,13 +269,17 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_MISC);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 6);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  const uint32_t cluster_rank = cluster_ctarank();
+  const uint32_t rank = cluster_rank & 1u;  // in the pair
+  const uint32_t lead_cta = cluster_rank - rank;
   const bool leader = rank == 0;
+  const int S = SPLIT ? static_cast<int>(cluster_nctarank() >> 1) : 1;  // pairs that share a tile of the last wave
+  const int pair = SPLIT ? static_cast<int>(cluster_rank >> 1) : 0;
 
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_u32(bars);
@@ -227,11 +287,14 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
   auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 + s); };
+  const uint32_t ready_bar = bar_base + 8u * (2 * STAGES + 4), got_bar = bar_base + 8u * (2 * STAGES + 5);
 
   if (warp == 0) {
     if (lane < 2 * STAGES) mbar_init(bar_base + 8u * lane, 1);                             // full, empty
     if (lane >= 16 && lane < 20) mbar_init(tfull_bar(lane - 16), lane < 18 ? 1 : 2 * 4);  // tfull, tempty (one arrival a warp)
     if (lane == 20) *abort_flag = 0;
+    if (SPLIT && lane == 21) mbar_init(ready_bar, S - 1);
+    if (SPLIT && lane == 22) mbar_init(got_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (lane == 0) {
@@ -255,8 +318,27 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   const int num_k = (p.K + BK - 1) / BK;
   const int group_m = p.group_m;
   const int tiles_per_group = group_m * num_n;
-  const int cluster_id = blockIdx.x >> 1;
-  const int num_clusters = gridDim.x >> 1;
+  const int pair_id = blockIdx.x >> 1;
+  const int num_pairs = gridDim.x >> 1;
+  const int whole = SPLIT ? p.whole : num_tiles;
+  // The tiles of this pair in turn: t, and the K slabs of it that are this pair's.
+  struct Work {
+    int t, k0, k1;
+    bool shared;
+  };
+  auto have_work = [&](Work& w) {
+    if (!SPLIT || w.t < whole) return w.t < whole;
+    if (w.shared) return false;  // one shared tile a cluster at most, after its whole ones
+    w.t = whole + pair_id / S;
+    w.k0 = num_k * pair / S;
+    w.k1 = num_k * (pair + 1) / S;
+    w.shared = true;
+    return w.t < num_tiles;
+  };
+  auto next_work = [&](Work& w) {
+    if (!w.shared) w.t += num_pairs;
+  };
+  const Work first{pair_id, 0, num_k, false};
 
   auto tile_coords = [&](int t, int& m0, int& n0) {
     const int g = t / tiles_per_group;
@@ -267,7 +349,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     n0 = (r / gsz) * BN;
   };
   int m0, n0;
-  tile_coords(cluster_id, m0, n0);  // of the first tile, while the barriers and the TMEM are on their way
+  tile_coords(pair_id, m0, n0);  // of the first tile, while the barriers and the TMEM are on their way
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -280,8 +362,8 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
-      if (t != cluster_id) tile_coords(t, m0, n0);
+    for (Work w = first; have_work(w) && ok; next_work(w)) {
+      if (w.t != pair_id) tile_coords(w.t, m0, n0);
       const int nb = n0 + static_cast<int>(rank) * BNH;  // this CTA's half of the B tile
       if (BNH == GATHER_BLOCK && p.ga_world > 0 && nb < p.N) {
         // these 128 rows of B are local once all their pieces are counted; the loads below go through the
@@ -292,7 +374,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         }
         asm volatile("fence.proxy.async.global;" ::: "memory");
       }
-      for (int kb = 0; kb < num_k; ++kb) {
+      for (int kb = w.k0; kb < w.k1; ++kb) {
         if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
           ok = false;
           break;
@@ -302,7 +384,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
           const uint32_t sb = sa + A_BYTES;
           const int k0 = kb * BK;
           if (leader) mbar_expect_tx(full_bar(stage), 2 * STAGE_BYTES);
-          const uint32_t fb = map_to_cta(full_bar(stage), 0);
+          const uint32_t fb = map_to_cta(full_bar(stage), lead_cta);
           if (p.a_mn == 0) {
             tma_load_2d_pair(sa, &tmA, fb, k0, m0);
           } else {
@@ -341,11 +423,11 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int t = cluster_id; t < num_tiles && ok; t += num_clusters) {
+      for (Work w = first; have_work(w) && ok; next_work(w)) {
         if (!mbar_wait_warp(tempty_bar(acc), acc_phase ^ 1u, abort_flag)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_k; ++kb) {
+        for (int kb = w.k0; kb < w.k1; ++kb) {
           if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) {
             ok = false;
             break;
@@ -358,10 +440,10 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
             for (int kk = 0; kk < BK / UMMA_K; ++kk) {
               const uint64_t adesc = make_smem_desc(sa + kk * a_step, a_lbo, 1024);
               const uint64_t bdesc = make_smem_desc(sb + kk * b_step, b_lbo, 1024);
-              umma_bf16_pair(d_tmem, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
+              umma_bf16_pair(d_tmem, adesc, bdesc, idesc, ((kb - w.k0) | kk) != 0 ? 1u : 0u);
             }
-            umma_commit_pair(empty_bar(stage));
-            if (kb == num_k - 1) umma_commit_pair(tfull_bar(acc));
+            umma_commit_pair(empty_bar(stage), lead_cta);
+            if (kb == w.k1 - 1) umma_commit_pair(tfull_bar(acc), lead_cta);
           }
           __syncwarp();
           if (++stage == STAGES) {
@@ -431,14 +513,14 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     int acc = 0;
     uint32_t acc_phase = 0;
     const bool vec_ok = p.out_fp32 ? ((p.ldc & 3) == 0) : ((p.ldc & 7) == 0);
-    for (int t = cluster_id; t < num_tiles; t += num_clusters) {
-      if (t != cluster_id) tile_coords(t, m0, n0);
+    for (Work w = first; have_work(w); next_work(w)) {
+      if (w.t != pair_id) tile_coords(w.t, m0, n0);
       if (!mbar_wait_warp(tfull_bar(acc), acc_phase, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row = m0 + q * 32 + lane;
       const uint32_t taddr0 = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
       const uint32_t stg = OFF_STAGING + q * STAGE_WARP_BYTES;
-      if (p.tma_out) {
+      if (p.tma_out && !(SPLIT && w.shared)) {
         // bf16 output: 64 columns at a time go, one row a thread, into a 128-byte-swizzled piece of the warp's staging area
         // and leave by TMA (which clips what lies beyond M and N), while the next 64 come out of tensor memory.  Nothing hides
         // the last tile's epilogue: 5800 cycles for 256 columns that leave a row-major staging area as row segments, 4100
@@ -456,7 +538,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
           } else {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), lead_cta));
           }
           const uint32_t* v = r[c & 1];
           const bool inside = n0 + c * 64 < p.N && m0 + q * 32 < p.M;
@@ -496,50 +578,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         }
         continue;
       }
-      if (p.sc_world > 0) {
-        // Scattered to the owners' memory: the tile goes through a per-warp staging area so that every store instruction
-        // covers two 256-byte row segments.  One 16-byte piece per thread and row would touch 32 rows per instruction: an
-        // NVLink packet each, which throttles the kernel.
-        const int half = lane >> 4, ch = lane & 15;
-#pragma unroll 1
-        for (int cg = 0; cg < BN / 128; ++cg) {
-#pragma unroll 1
-          for (int cc = 0; cc < 4; ++cc) {
-            uint32_t r[32];
-            tmem_ld32(taddr0 + (cg * 4 + cc) * 32, r);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float f[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]);
-              *reinterpret_cast<ftb200::bf16x8*>(smem + stg + lane * 256 + (((cc * 4 + j) ^ (lane & 15)) << 4)) = ftb200::pack8(f);
-            }
-          }
-          __syncwarp();
-          const int gcol = n0 + cg * 128 + ch * 8;
-#pragma unroll 4
-          for (int it = 0; it < 16; ++it) {
-            const int rr = it * 2 + half;
-            const int grow = m0 + q * 32 + rr;
-            const ftb200::bf16x8 v = *reinterpret_cast<const ftb200::bf16x8*>(smem + stg + rr * 256 + ((ch ^ (rr & 15)) << 4));
-            if (grow < p.M && gcol + 8 <= p.N) {
-              const long long flat = p.sc_off + static_cast<long long>(grow) * p.ldc + gcol;
-              const long long owner = flat / p.sc_shard;
-              const long long rem = flat - owner * p.sc_shard;
-              if (!FTB_IN_RANGE(owner, p.sc_world)) continue;
-              __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.sc_peers[owner]);
-              *reinterpret_cast<ftb200::bf16x8*>(base + static_cast<long long>(p.sc_src) * p.sc_shard + rem) = v;
-            }
-          }
-          __syncwarp();
-        }
-      } else
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld32(taddr0 + c * 32, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      auto store_chunk = [&](int c, const uint32_t* r) {  // 32 columns of the thread's row
         const int col0 = n0 + c * 32;
         if (row < p.M && col0 < p.N) {
           const bool full = vec_ok && (col0 + 32 <= p.N);
@@ -597,10 +636,117 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
             }
           }
         }
+      };
+      if (SPLIT && w.shared) {
+        // A chunk is kept as a share of each warp, four columns of its 32 rows after another.  It is written to this CTA's own
+        // ring and copied from there; remote stores of 16 bytes a thread are no faster and no simpler to count.
+        constexpr int CHUNKS = BN / 32;
+        auto owner = [&](int c) { return c * S / CHUNKS; };
+        auto first_of = [&](int j) { return (j * CHUNKS + S - 1) / S; };
+        const int mine0 = first_of(pair), mine = first_of(pair + 1) - mine0;  // this CTA's chunks
+        const uint32_t in = smem_base + q * SHARE_BYTES + static_cast<uint32_t>(lane) * 16;
+        if (q == 2) {
+          if (lane == 0) mbar_expect_tx(got_bar, (S - 1) * mine * CHUNK_BYTES);
+          __syncwarp();
+          // this CTA's products are done: its ring may be written
+          if (lane < S && lane != pair) mbar_arrive_cluster(map_to_cta(ready_bar, 2 * lane + rank));
+          __syncwarp();
+        }
+        bool told = false;  // the others' rings are free
+        int out = 0;
+        for (int c = 0; c < CHUNKS; ++c) {
+          const int j = owner(c);
+          if (j == pair) continue;
+          uint32_t r[32];
+          tmem_ld32(taddr0 + c * 32, r);
+          const uint32_t from = smem_base + (MAX_IN + out++) * CHUNK_BYTES + q * SHARE_BYTES;
+          tmem_wait_ld();
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<uint4*>(smem + (from - smem_base) + v * 512 + lane * 16) = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+          fence_async_smem();
+          if (!told && !mbar_wait_cluster(ready_bar, 0, abort_flag)) break;
+          told = true;
+          __syncwarp();
+          if (lane == 0) {  // the owner keeps the chunks of the other pairs in their order
+            const int slot = (pair - (pair > j)) * (first_of(j + 1) - first_of(j)) + c - first_of(j);
+            copy_to_cta(map_to_cta(smem_base + slot * CHUNK_BYTES + q * SHARE_BYTES, 2 * j + rank), from, SHARE_BYTES,
+                        map_to_cta(got_bar, 2 * j + rank));
+          }
+        }
+        if (!mbar_wait_warp(got_bar, 0, abort_flag)) break;
+#pragma unroll 1
+        for (int c = mine0; c < mine0 + mine; ++c) {
+          uint32_t own[32], r[32];
+          tmem_ld32(taddr0 + c * 32, own);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < MAX_SPLIT; ++j) {
+            if (j >= S) break;
+            const uint8_t* slot = smem + (in - smem_base) + ((j - (j > pair)) * mine + c - mine0) * CHUNK_BYTES;
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+              float4 x = make_float4(__uint_as_float(own[4 * v]), __uint_as_float(own[4 * v + 1]), __uint_as_float(own[4 * v + 2]),
+                                     __uint_as_float(own[4 * v + 3]));
+              if (j != pair) x = *reinterpret_cast<const float4*>(slot + v * 512);
+              r[4 * v] = __float_as_uint(j == 0 ? x.x : __uint_as_float(r[4 * v]) + x.x);
+              r[4 * v + 1] = __float_as_uint(j == 0 ? x.y : __uint_as_float(r[4 * v + 1]) + x.y);
+              r[4 * v + 2] = __float_as_uint(j == 0 ? x.z : __uint_as_float(r[4 * v + 2]) + x.z);
+              r[4 * v + 3] = __float_as_uint(j == 0 ? x.w : __uint_as_float(r[4 * v + 3]) + x.w);
+            }
+          }
+          store_chunk(c, r);
+        }
+      } else if (p.sc_world > 0) {
+        // Scattered to the owners' memory: the tile goes through a per-warp staging area so that every store instruction
+        // covers two 256-byte row segments.  One 16-byte piece per thread and row would touch 32 rows per instruction: an
+        // NVLink packet each, which throttles the kernel.
+        const int half = lane >> 4, ch = lane & 15;
+#pragma unroll 1
+        for (int cg = 0; cg < BN / 128; ++cg) {
+#pragma unroll 1
+          for (int cc = 0; cc < 4; ++cc) {
+            uint32_t r[32];
+            tmem_ld32(taddr0 + (cg * 4 + cc) * 32, r);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float f[8];
+#pragma unroll
+              for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]);
+              *reinterpret_cast<ftb200::bf16x8*>(smem + stg + lane * 256 + (((cc * 4 + j) ^ (lane & 15)) << 4)) = ftb200::pack8(f);
+            }
+          }
+          __syncwarp();
+          const int gcol = n0 + cg * 128 + ch * 8;
+#pragma unroll 4
+          for (int it = 0; it < 16; ++it) {
+            const int rr = it * 2 + half;
+            const int grow = m0 + q * 32 + rr;
+            const ftb200::bf16x8 v = *reinterpret_cast<const ftb200::bf16x8*>(smem + stg + rr * 256 + ((ch ^ (rr & 15)) << 4));
+            if (grow < p.M && gcol + 8 <= p.N) {
+              const long long flat = p.sc_off + static_cast<long long>(grow) * p.ldc + gcol;
+              const long long owner = flat / p.sc_shard;
+              const long long rem = flat - owner * p.sc_shard;
+              if (!FTB_IN_RANGE(owner, p.sc_world)) continue;
+              __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.sc_peers[owner]);
+              *reinterpret_cast<ftb200::bf16x8*>(base + static_cast<long long>(p.sc_src) * p.sc_shard + rem) = v;
+            }
+          }
+          __syncwarp();
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(taddr0 + c * 32, r);
+          tmem_wait_ld();
+          store_chunk(c, r);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), lead_cta));
       if (++acc == 2) {
         acc = 0;
         acc_phase ^= 1u;
@@ -612,7 +758,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag && p.status != nullptr) atomicExch(p.status, FTB200_ST_TIMEOUT);
-  cluster_sync_relaxed();  // neither CTA retires while its partner may still touch its barriers or operands
+  cluster_sync_relaxed();  // no CTA retires while another may still touch its barriers, operands or ring
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -667,18 +813,95 @@ struct GatherSpec {
   unsigned int* sync = nullptr;
 };
 
+template <int BN, bool SPLIT>
+static cudaError_t prepare_2cta() {
+  static std::atomic<bool> done{false};
+  if (done.load(std::memory_order_acquire)) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+  if (e == cudaSuccess) done.store(true, std::memory_order_release);
+  return e;
+}
+
+static void cluster_launch(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int ctas, int pairs_per_cluster, int threads,
+                           cudaStream_t stream) {
+  cfg = cudaLaunchConfig_t{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = stream;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2 * pairs_per_cluster;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+}
+
+// How many clusters of `split` pairs fit the chip at once (clusters do not span its processing clusters, whose number of
+// SMs is no multiple of every size).
+template <int BN>
+static int resident_clusters(int split) {
+  static std::atomic<int> known[MAX_SPLIT + 1];
+  int n = known[split].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    cluster_launch(cfg, attr, 2 * split, split, NUM_THREADS, nullptr);
+    if (prepare_2cta<BN, true>() != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_bf16_tcgen05_2cta_kernel<BN, true>, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = -1;
+    }
+    known[split].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+struct TilePlan {
+  int columns;  // of a pair's tile
+  int split;    // pairs that share a tile of the last wave (1: none do)
+  int whole;    // tiles before them
+  int ctas;
+};
+
 // Columns of a pair's tile: 128 where the narrow tiles of the whole output fit the pairs at once, 256 elsewhere.  A narrow
 // tile takes about 0.7 of a wide one's time (it asks the L2 for 96 bytes a cycle and SM instead of 64), so it pays where
 // it only puts idle pairs to work: 1024 x 1024 x 3000 26.0 -> 17.3 us, 256 x 1024 x 256 9.8 -> 6.3 us; but 3000 x 5632 x
 // 1024 36.0 -> 40.6 us, 1536 x 4096 x 14336 146 -> 169 us.
-static int tile_columns(int M, int N, int pairs) {
-  const long long rows = (M + 2 * BM - 1) / (2 * BM);
-  return rows * ((N + 127) / 128) <= pairs ? 128 : 256;
+// And whether the last wave (the whole output, where it is less than one) is split over K, by an estimate of the time in
+// units of one 64-deep slab of a 256-column tile (0.3 us): the waves' slabs and, for a shared tile, SPLIT_COST: about
+// 9 us go into the meeting of its accumulators, whatever K is.  1536 x 4096 x 14336 (96 tiles on 74 pairs) 144 -> 123 us,
+// 1536 x 4096 x 28672 290 -> 240, 3072 x 2048 x 8192 84 -> 77, 750 x 1024 x 8192 30 -> 25, 77 x 4096 x 14336 52 -> 44; where the
+// estimate says no: 500 x 4096 x 4096 20 -> 27, 1536 x 1024 x 3000 15 -> 22, 1000 x 2048 x 2048 13 -> 20.
+static TilePlan plan_tiles(int M, int N, int K, int pairs, bool may_split) {
+    constexpr float NARROW = 0.7f, SPLIT_COST = 32.f;
+  const int rows = (M + 2 * BM - 1) / (2 * BM), slabs = (K + BK - 1) / BK;
+  const int wide = rows * ((N + 255) / 256), narrow = rows * ((N + 127) / 128);
+  TilePlan best{narrow <= pairs ? 128 : 256, 1, 0, 2 * pairs};
+  float least = best.columns == 128 ? slabs * NARROW : static_cast<float>((wide + pairs - 1) / pairs) * slabs;
+  if (!may_split || slabs < 16) return best;
+  for (int columns = 128; columns <= 256; columns += 128) {
+    const int tiles = columns == 128 ? narrow : wide;
+    const float slab = columns == 128 ? NARROW : 1.f;
+    for (int split = 2; split <= MAX_SPLIT && 4 * split <= slabs; ++split) {
+      const int clusters = columns == 128 ? resident_clusters<128>(split) : resident_clusters<256>(split);
+      if (clusters <= 0) continue;
+      const int waves = tiles / (clusters * split), rest = tiles - waves * clusters * split;
+      if (rest == 0 || rest > clusters) continue;
+      const float cost = (waves * slabs + (slabs + split - 1) / split) * slab + SPLIT_COST;
+      if (cost < least) {
+        least = cost;
+        best = TilePlan{columns, split, waves * clusters * split, 2 * split * (waves > 0 ? clusters : rest)};
+      }
+    }
+  }
+  return best;
 }
 
-template <int BN>
-static int launch_2cta(const void* A, const void* B, long long lda, long long ldb, int ctas, int threads, const GemmParams& p,
-                       cudaStream_t stream) {
+template <int BN, bool SPLIT>
+static int launch_2cta(const void* A, const void* B, long long lda, long long ldb, int ctas, int split, int threads,
+                       const GemmParams& p, cudaStream_t stream) {
   CUtensorMap tmA, tmB, tmC, tmAux;
   int rc;
   if (!p.a_mn)
@@ -697,16 +920,12 @@ static int launch_2cta(const void* A, const void* B, long long lda, long long ld
     if (rc == 0 && p.aux != nullptr) rc = encode_2d(&tmAux, p.aux, p.M, p.N / 2, p.ld_aux, 64, 32);
     if (rc) return rc;
   }
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_bf16_tcgen05_2cta_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SMEM_BYTES) != cudaSuccess)
-      return FTB200_E_CUDA;
-    attr_set = true;
-  }
+  if (prepare_2cta<BN, SPLIT>() != cudaSuccess) return FTB200_E_CUDA;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
-  gemm_bf16_tcgen05_2cta_kernel<BN><<<std::min(2 * tiles, ctas), threads, SMEM_BYTES, stream>>>(tmA, tmB, tmC, tmAux, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  cluster_launch(cfg, attr, SPLIT ? ctas : std::min(2 * tiles, ctas), split, threads, stream);
+  return cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT>, tmA, tmB, tmC, tmAux, p) == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, int b_mn_major,
@@ -744,6 +963,7 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   p.tma_out = sc == nullptr && !p.out_fp32 && !p.accumulate && (ldc & 7) == 0 && ldc >= N && (N & 7) == 0 &&
               (aux == nullptr || ((ld_aux & 7) == 0 && ld_aux >= N / 2 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0));
   p.group_m = GROUP_M;
+  p.whole = 0;
   p.ga_world = 0;
   p.ga_shard = 0;
   p.ga_off = 0;
@@ -767,9 +987,16 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   }
   int ctas = ftb200::sm_count() & ~1;
   if (max_ctas > 0 && max_ctas < ctas) ctas = std::max(2, max_ctas & ~1);
-  if (ga != nullptr) return launch_2cta<256>(A, B, lda, ldb, ctas, NUM_THREADS_GATHER, p, stream);
-  if (tile_columns(M, N, ctas / 2) == 128) return launch_2cta<128>(A, B, lda, ldb, ctas, NUM_THREADS, p, stream);
-  return launch_2cta<256>(A, B, lda, ldb, ctas, NUM_THREADS, p, stream);
+  if (ga != nullptr) return launch_2cta<256, false>(A, B, lda, ldb, ctas, 1, NUM_THREADS_GATHER, p, stream);
+  // scattered and activated outputs leave through the staging area, which a shared tile does not
+  const TilePlan plan = plan_tiles(M, N, K, ctas / 2, sc == nullptr && aux == nullptr && max_ctas <= 0);
+  p.whole = plan.whole;
+  if (plan.split > 1) {
+    if (plan.columns == 128) return launch_2cta<128, true>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
+    return launch_2cta<256, true>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
+  }
+  if (plan.columns == 128) return launch_2cta<128, false>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+  return launch_2cta<256, false>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
 }
 
 FTB200_API int ftb200_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major,
