@@ -156,6 +156,7 @@ class Tcgen05Attention:
         self.cfg = cfg
         self._saved: Dict[int, Tuple[torch.Tensor, ...]] = {}
         self._lse_pool: List[torch.Tensor] = []
+        self._scratch: Optional[torch.Tensor] = None  # of the backward pass, kept between calls
 
     def _views(self, qkv: torch.Tensor):
         c = self.cfg
@@ -177,7 +178,11 @@ class Tcgen05Attention:
         qkv, out, lse = self._saved.pop(layer)
         q, k, v = self._views(qkv)
         dq, dk, dv = self._views(dqkv)
-        K.attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, causal=True)
+        need = K.attention_bwd_scratch_bytes(batch, seq, c.n_heads)
+        if self._scratch is None or self._scratch.numel() < need:
+            self._scratch = torch.empty(need, dtype=torch.uint8, device=qkv.device)
+        K.attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, causal=True,
+                        scratch=self._scratch)
         self._lse_pool.append(lse)
 
     def reset(self) -> None:
@@ -370,6 +375,12 @@ class LlamaEngine:
         """Runs the decoder; with ``targets`` returns the mean token loss and leaves
         ``dlogits``-derived gradients of the head computed (head backward is fused into
         the loss pass so that the logits never exist in full)."""
+        out = self.forward_rows(tokens, targets, train)
+        return self.loss_rows.mean() if out is None else out
+
+    def forward_rows(self, tokens: torch.Tensor, targets: Optional[torch.Tensor], train: bool = True) -> Optional[torch.Tensor]:
+        """:meth:`forward` up to the loss of every token (in ``loss_rows``; their mean is left to the caller), or the
+        logits without ``targets``."""
         c, T, B, S = self.cfg, self.T, self.B, self.S
         L = c.n_layers
         tok = tokens.reshape(-1)
@@ -420,7 +431,7 @@ class LlamaEngine:
             if train:
                 K.linear_wgrad(self.logits, self.ws_n[sl], out=G.lm_head, accumulate=ci > 0)
                 K.linear_dgrad(self.logits, getattr(W.lm_head, "local", W.lm_head), out=self.ws_dn[sl])
-        return self.loss_rows.mean()
+        return None
 
     # -- backward --------------------------------------------------------------------------
     def backward(self, tokens: torch.Tensor) -> None:

@@ -627,13 +627,21 @@ def ref_attention_bwd(q, k, v, d_o, causal=True):
 _attn_scratch: dict = {}
 
 
+def attention_bwd_scratch_bytes(batch: int, seq_len: int, n_heads: int) -> int:
+    """Size of the ``scratch`` that :func:`attention_bwd` takes."""
+    lib = N.lib()
+    lib.ftb200_attention_bwd_scratch_bytes.restype = ctypes.c_longlong
+    return int(lib.ftb200_attention_bwd_scratch_bytes(c_int(batch), c_int(seq_len), c_int(n_heads)))
+
+
 def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor,
                   lse: torch.Tensor, dq: torch.Tensor, dk: torch.Tensor, dv: torch.Tensor, batch: int, seq_len: int,
-                  n_heads: int, n_kv_heads: int, head_dim: int, causal: bool = True) -> None:
+                  n_heads: int, n_kv_heads: int, head_dim: int, causal: bool = True,
+                  scratch: Optional[torch.Tensor] = None) -> None:
     """Backward of :func:`attention_fwd`: writes ``dq``, ``dk``, ``dv`` (2-D bf16 views like
     ``q``, ``k``, ``v``; column slices of a packed dQKV buffer are fine).  The fp32 dQ
-    accumulator lives in a per-device scratch buffer that is reused across calls on the same
-    stream."""
+    accumulator lives in ``scratch`` (bytes on the device, :func:`attention_bwd_scratch_bytes` of
+    them or more), by default a per-device buffer that is reused across calls on the same stream."""
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (o, "o"), (d_o, "d_o"), (dq, "dq"), (dk, "dk"), (dv, "dv")):
         _check_2d_bf16(t, name)
     if not q.is_cuda:
@@ -645,13 +653,15 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
         dv.copy_(gv.reshape(B * S, -1))
         return
     lib = N.lib()
-    lib.ftb200_attention_bwd_scratch_bytes.restype = ctypes.c_longlong
-    need = int(lib.ftb200_attention_bwd_scratch_bytes(c_int(batch), c_int(seq_len), c_int(n_heads)))
-    key = (q.device.index, stream_ptr().value)
-    scratch = _attn_scratch.get(key)
-    if scratch is None or scratch.numel() < need:
-        scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
-        _attn_scratch[key] = scratch
+    need = attention_bwd_scratch_bytes(batch, seq_len, n_heads)
+    if scratch is None:
+        key = (q.device.index, stream_ptr().value)
+        scratch = _attn_scratch.get(key)
+        if scratch is None or scratch.numel() < need:
+            scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
+            _attn_scratch[key] = scratch
+    elif scratch.device != q.device or scratch.dtype != torch.uint8 or scratch.numel() < need or not scratch.is_contiguous():
+        raise ValueError(f"scratch must be {need} contiguous bytes on {q.device}")
     scale = 1.0 / math.sqrt(head_dim)
     N.check(
         lib.ftb200_attention_bwd(ptr(q), ptr(k), ptr(v), ptr(o), ptr(d_o), ptr(lse), ptr(dq), ptr(dk), ptr(dv), ptr(scratch),
