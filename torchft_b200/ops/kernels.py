@@ -21,7 +21,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _native as N
-from ._native import c_float, c_int, c_ll, ptr, stream_ptr
+from ._native import c_float, c_int, c_ll, c_void_p, ptr, stream_ptr
 
 # --------------------------------------------------------------------------- status word
 
@@ -36,6 +36,44 @@ def status_word(device: torch.device) -> torch.Tensor:
         w = torch.zeros(1, dtype=torch.int32, device=device)
         _status_words[key] = w
     return w
+
+
+_status_ptrs: dict = {}
+
+
+def _status_ptr(device: torch.device) -> int:
+    at = _status_ptrs.get(device.index)
+    if at is None:
+        at = _status_ptrs[device.index] = status_word(device).data_ptr()
+    return at
+
+
+# The C functions get their argument types once and take plain numbers from then on: a ctypes object per argument and call
+# is a tenth of the host's time for a launch (the prompt pass of two layers of width 256: 257 to 299 -> 250 us).
+_ARGS = {
+    "embedding_fwd": "pppiiip", "embedding_bwd": "pppiiip", "rmsnorm_fwd": "ppppppiifp", "rmsnorm_bwd": "ppppppppiiip",
+    "rope": "ppliiilip", "swiglu_fwd": "pplip", "swiglu_bwd": "ppplip", "gemm_bf16_swiglu": "ppppiiillllpip",
+    "cross_entropy": "pppiilfip", "adamw": "ppppiplfffffipp", "sumsq": "pilpp", "clip_coef": "pfppp",
+    "attention_fwd": "pppppiiiiillllfipp", "attention_fwd2": "pppppiiiiillllfiipp",
+    "attention_bwd": "ppppppppppiiiiillllllllfipp", "gemm_bf16": "pppiiiiilllipip",
+}
+_ARGS["gemm_bf16_2cta"] = _ARGS["gemm_bf16"]
+_KIND = {"p": c_void_p, "i": c_int, "l": c_ll, "f": c_float}
+
+
+def _fn(name: str):
+    fn = getattr(N.lib(), "ftb200_" + name)
+    if fn.argtypes is None:
+        fn.argtypes = [_KIND[k] for k in _ARGS[name]]
+    return fn
+
+
+def _at(t: Optional[torch.Tensor]) -> Optional[int]:
+    return None if t is None else t.data_ptr()
+
+
+def _stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def check_status(device: torch.device) -> None:
@@ -58,9 +96,6 @@ def _check_2d_bf16(t: torch.Tensor, name: str) -> None:
 # Which GEMM kernel `gemm` launches: "2cta" (pairs of CTAs, tcgen05.mma.cta_group::2) or
 # "1cta".  Overridable per call and through the FTB200_GEMM environment variable.
 GEMM_IMPL = os.environ.get("FTB200_GEMM", "2cta")
-
-
-_GEMM_ARGS = (N.c_void_p,) * 3 + (c_int,) * 5 + (c_ll,) * 3 + (c_int, N.c_void_p, c_int, N.c_void_p)
 
 
 def gemm(
@@ -107,12 +142,9 @@ def gemm(
         out.copy_(r.to(out.dtype))
         return out
     flags = (1 if out.dtype == torch.float32 else 0) | (2 if accumulate else 0)
-    fn = N.lib().ftb200_gemm_bf16_2cta if (impl or GEMM_IMPL) == "2cta" else N.lib().ftb200_gemm_bf16
-    if fn.argtypes is None:
-        fn.argtypes = _GEMM_ARGS  # plain Python numbers from here on: no ctypes object per argument
-    rc = fn(
+    rc = _fn("gemm_bf16_2cta" if (impl or GEMM_IMPL) == "2cta" else "gemm_bf16")(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, int(a_mn_major), int(b_mn_major), a.stride(0), b.stride(0),
-        out.stride(0), flags, status_word(a.device).data_ptr(), max_ctas, stream_ptr(),
+        out.stride(0), flags, _status_ptr(a.device), max_ctas, _stream(),
     )
     N.check(rc, "gemm_bf16")
     return out
@@ -223,7 +255,7 @@ def embedding_fwd(tokens: torch.Tensor, table: torch.Tensor, out: Optional[torch
     if not table.is_cuda:
         out.copy_(table[tokens.reshape(-1)])
         return out
-    N.check(N.lib().ftb200_embedding_fwd(ptr(tokens), ptr(table), ptr(out), c_int(T), c_int(D), c_int(V), stream_ptr()),
+    N.check(_fn("embedding_fwd")(_at(tokens), _at(table), _at(out), T, D, V, _stream()),
             "embedding_fwd")
     return out
 
@@ -235,7 +267,7 @@ def embedding_bwd(tokens: torch.Tensor, dout: torch.Tensor, dtable: torch.Tensor
     if not dtable.is_cuda:
         dtable.copy_(dtable.float().index_add_(0, tokens.reshape(-1), dout.float()).to(dtable.dtype))
         return dtable
-    N.check(N.lib().ftb200_embedding_bwd(ptr(tokens), ptr(dout), ptr(dtable), c_int(T), c_int(D), c_int(V), stream_ptr()),
+    N.check(_fn("embedding_bwd")(_at(tokens), _at(dout), _at(dtable), T, D, V, _stream()),
             "embedding_bwd")
     return dtable
 
@@ -278,8 +310,7 @@ def rmsnorm_fwd(
             out.copy_(o)
         return (out if want_out else None), rstd, (h_out if res is not None else x)
     N.check(
-        N.lib().ftb200_rmsnorm_fwd(ptr(x), ptr(res), ptr(h_out), ptr(w), ptr(out if want_out else None), ptr(rstd),
-                                   c_int(T), c_int(D), c_float(eps), stream_ptr()),
+        _fn("rmsnorm_fwd")(_at(x), _at(res), _at(h_out), _at(w), _at(out if want_out else None), _at(rstd), T, D, eps, _stream()),
         "rmsnorm_fwd",
     )
     return (out if want_out else None), rstd, (h_out if res is not None else x)
@@ -320,17 +351,17 @@ def rmsnorm_bwd(
         dx.copy_(rdx)
         dw.copy_(((dw.float() if accumulate_dw else 0) + rdw).to(dw.dtype))
         return dx, dw
-    L = N.lib()
-    L.ftb200_rmsnorm_bwd_scratch_floats.restype = c_ll
-    need = int(L.ftb200_rmsnorm_bwd_scratch_floats(c_int(D)))
-    key = (x.device.index, need)
+    key = (x.device.index, D)
     scratch = _rms_scratch.get(key)
     if scratch is None:
+        L = N.lib()
+        L.ftb200_rmsnorm_bwd_scratch_floats.restype = c_ll
+        need = int(L.ftb200_rmsnorm_bwd_scratch_floats(D))
         scratch = torch.empty(need, dtype=torch.float32, device=x.device)
         _rms_scratch[key] = scratch
     N.check(
-        L.ftb200_rmsnorm_bwd(ptr(dy), ptr(x), ptr(w), ptr(rstd), ptr(dres), ptr(dx), ptr(dw), ptr(scratch), c_int(T),
-                             c_int(D), c_int(int(accumulate_dw)), stream_ptr()),
+        _fn("rmsnorm_bwd")(_at(dy), _at(x), _at(w), _at(rstd), _at(dres), _at(dx), _at(dw), _at(scratch), T, D,
+                           int(accumulate_dw), _stream()),
         "rmsnorm_bwd",
         launches=2,
     )
@@ -370,8 +401,7 @@ def rope_(buf: torch.Tensor, table: torch.Tensor, seq_len: int, n_heads: int, he
         buf.copy_(ref_rope(buf, table, seq_len, n_heads, head_dim, backward))
         return buf
     N.check(
-        N.lib().ftb200_rope(ptr(buf), ptr(table), c_ll(T), c_int(seq_len), c_int(n_heads), c_int(head_dim),
-                            c_ll(buf.stride(0)), c_int(int(backward)), stream_ptr()),
+        _fn("rope")(_at(buf), _at(table), T, seq_len, n_heads, head_dim, buf.stride(0), int(backward), _stream()),
         "rope",
     )
     return buf
@@ -395,7 +425,7 @@ def swiglu_fwd(gu: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Te
     if not gu.is_cuda:
         out.copy_(ref_swiglu_fwd(gu))
         return out
-    N.check(N.lib().ftb200_swiglu_fwd(ptr(gu), ptr(out), c_ll(T), c_int(Fd), stream_ptr()), "swiglu_fwd")
+    N.check(_fn("swiglu_fwd")(_at(gu), _at(out), T, Fd, _stream()), "swiglu_fwd")
     return out
 
 
@@ -417,7 +447,7 @@ def swiglu_bwd(ds: torch.Tensor, gu: torch.Tensor, dgu: Optional[torch.Tensor] =
     if not gu.is_cuda:
         dgu.copy_(ref_swiglu_bwd(ds, gu))
         return dgu
-    N.check(N.lib().ftb200_swiglu_bwd(ptr(ds), ptr(gu), ptr(dgu), c_ll(T), c_int(F2 // 2), stream_ptr()), "swiglu_bwd")
+    N.check(_fn("swiglu_bwd")(_at(ds), _at(gu), _at(dgu), T, F2 // 2, _stream()), "swiglu_bwd")
     return dgu
 
 
@@ -435,9 +465,9 @@ def linear_swiglu_fwd(x: torch.Tensor, w_gu: torch.Tensor, gu_out: torch.Tensor,
         gemm(x, w_gu, False, False, out=gu_out)
         swiglu_fwd(gu_out, out=s_out)
         return
-    rc = N.lib().ftb200_gemm_bf16_swiglu(
-        ptr(x), ptr(w_gu), ptr(gu_out), ptr(s_out), c_int(T), c_int(N2), c_int(Kd), c_ll(x.stride(0)), c_ll(w_gu.stride(0)),
-        c_ll(gu_out.stride(0)), c_ll(s_out.stride(0)), ptr(status_word(x.device)), c_int(0), stream_ptr())
+    rc = _fn("gemm_bf16_swiglu")(
+        _at(x), _at(w_gu), _at(gu_out), _at(s_out), T, N2, Kd, x.stride(0), w_gu.stride(0),
+        gu_out.stride(0), s_out.stride(0), _status_ptr(x.device), 0, _stream())
     N.check(rc, "gemm_bf16_swiglu")
 
 
@@ -465,8 +495,7 @@ def cross_entropy_(logits: torch.Tensor, target: torch.Tensor, grad_scale: float
             logits.copy_(g)
         return loss
     N.check(
-        N.lib().ftb200_cross_entropy(ptr(logits), ptr(target), ptr(loss), c_int(T), c_int(V), c_ll(logits.stride(0)),
-                                     c_float(grad_scale), c_int(int(grad)), stream_ptr()),
+        _fn("cross_entropy")(_at(logits), _at(target), _at(loss), T, V, logits.stride(0), grad_scale, int(grad), _stream()),
         "cross_entropy",
     )
     return loss
@@ -497,9 +526,8 @@ def adamw_(master: torch.Tensor, m: torch.Tensor, v: torch.Tensor, grad: torch.T
             param_lp.view(-1).copy_(master.view(-1).to(param_lp.dtype))
         return
     N.check(
-        N.lib().ftb200_adamw(ptr(master), ptr(m), ptr(v), ptr(grad), c_int(int(grad.dtype == torch.float32)),
-                             ptr(param_lp), c_ll(n), c_float(lr), c_float(beta1), c_float(beta2), c_float(eps),
-                             c_float(wd), c_int(step), ptr(grad_scale), stream_ptr()),
+        _fn("adamw")(_at(master), _at(m), _at(v), _at(grad), int(grad.dtype == torch.float32), _at(param_lp), n, lr, beta1,
+                     beta2, eps, wd, step, _at(grad_scale), _stream()),
         "adamw",
     )
 
@@ -509,7 +537,7 @@ def sumsq_(x: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     if not x.is_cuda:
         out.add_(x.float().pow(2).sum())
         return out
-    N.check(N.lib().ftb200_sumsq(ptr(x), c_int(int(x.dtype == torch.float32)), c_ll(x.numel()), ptr(out), stream_ptr()),
+    N.check(_fn("sumsq")(_at(x), int(x.dtype == torch.float32), x.numel(), _at(out), _stream()),
             "sumsq")
     return out
 
@@ -521,7 +549,7 @@ def clip_coef_(sumsq: torch.Tensor, max_norm: float, coef: torch.Tensor, norm_ou
             norm_out.copy_(nrm)
         coef.copy_(torch.clamp(max_norm / (nrm + 1e-6), max=1.0) if max_norm > 0 else torch.ones_like(nrm))
         return
-    N.check(N.lib().ftb200_clip_coef(ptr(sumsq), c_float(max_norm), ptr(coef), ptr(norm_out), stream_ptr()), "clip_coef")
+    N.check(_fn("clip_coef")(_at(sumsq), max_norm, _at(coef), _at(norm_out), _stream()), "clip_coef")
 
 
 # --------------------------------------------------------------------------- attention
@@ -601,18 +629,16 @@ def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int,
         # FMA pipe (8 x 2048, 32/8 heads: 303 us against 321); at head dim 128 none (475 us against 486).
         poly = int(os.environ.get("FTB200_ATTN_POLY") or ("2" if head_dim == 64 else "0"))
         N.check(
-            N.lib().ftb200_attention_fwd2(ptr(q), ptr(k), ptr(v), ptr(out), ptr(lse), c_int(batch), c_int(seq_len),
-                                          c_int(n_heads), c_int(n_kv_heads), c_int(head_dim), c_ll(q.stride(0)),
-                                          c_ll(k.stride(0)), c_ll(v.stride(0)), c_ll(out.stride(0)), c_float(scale),
-                                          c_int(int(causal)), c_int(poly), ptr(status_word(q.device)), stream_ptr()),
+            _fn("attention_fwd2")(_at(q), _at(k), _at(v), _at(out), _at(lse), batch, seq_len, n_heads, n_kv_heads, head_dim,
+                                  q.stride(0), k.stride(0), v.stride(0), out.stride(0), scale, int(causal), poly,
+                                  _status_ptr(q.device), _stream()),
             "attention_fwd2",
         )
         return
     N.check(
-        N.lib().ftb200_attention_fwd(ptr(q), ptr(k), ptr(v), ptr(out), ptr(lse), c_int(batch), c_int(seq_len), c_int(n_heads),
-                                     c_int(n_kv_heads), c_int(head_dim), c_ll(q.stride(0)), c_ll(k.stride(0)),
-                                     c_ll(v.stride(0)), c_ll(out.stride(0)), c_float(scale), c_int(int(causal)),
-                                     ptr(status_word(q.device)), stream_ptr()),
+        _fn("attention_fwd")(_at(q), _at(k), _at(v), _at(out), _at(lse), batch, seq_len, n_heads, n_kv_heads, head_dim,
+                             q.stride(0), k.stride(0), v.stride(0), out.stride(0), scale, int(causal), _status_ptr(q.device),
+                             _stream()),
         "attention_fwd",
     )
 
@@ -631,7 +657,7 @@ def attention_bwd_scratch_bytes(batch: int, seq_len: int, n_heads: int) -> int:
     """Size of the ``scratch`` that :func:`attention_bwd` takes."""
     lib = N.lib()
     lib.ftb200_attention_bwd_scratch_bytes.restype = ctypes.c_longlong
-    return int(lib.ftb200_attention_bwd_scratch_bytes(c_int(batch), c_int(seq_len), c_int(n_heads)))
+    return int(lib.ftb200_attention_bwd_scratch_bytes(batch, seq_len, n_heads))
 
 
 def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor,
@@ -655,7 +681,7 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
     lib = N.lib()
     need = attention_bwd_scratch_bytes(batch, seq_len, n_heads)
     if scratch is None:
-        key = (q.device.index, stream_ptr().value)
+        key = (q.device.index, _stream())
         scratch = _attn_scratch.get(key)
         if scratch is None or scratch.numel() < need:
             scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
@@ -664,10 +690,9 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
         raise ValueError(f"scratch must be {need} contiguous bytes on {q.device}")
     scale = 1.0 / math.sqrt(head_dim)
     N.check(
-        lib.ftb200_attention_bwd(ptr(q), ptr(k), ptr(v), ptr(o), ptr(d_o), ptr(lse), ptr(dq), ptr(dk), ptr(dv), ptr(scratch),
-                                 c_int(batch), c_int(seq_len), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim),
-                                 c_ll(q.stride(0)), c_ll(k.stride(0)), c_ll(v.stride(0)), c_ll(o.stride(0)),
-                                 c_ll(d_o.stride(0)), c_ll(dq.stride(0)), c_ll(dk.stride(0)), c_ll(dv.stride(0)),
-                                 c_float(scale), c_int(int(causal)), ptr(status_word(q.device)), stream_ptr()),
+        _fn("attention_bwd")(_at(q), _at(k), _at(v), _at(o), _at(d_o), _at(lse), _at(dq), _at(dk), _at(dv), _at(scratch),
+                             batch, seq_len, n_heads, n_kv_heads, head_dim, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
+                             d_o.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), scale, int(causal), _status_ptr(q.device),
+                             _stream()),
         "attention_bwd", launches=3,
     )
