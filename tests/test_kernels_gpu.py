@@ -152,6 +152,33 @@ def test_rmsnorm(T, D):
     assert rel_err(dw, rdw) < 2e-2
 
 
+@pytest.mark.parametrize("T", [1, 5, 149, 1300])
+@pytest.mark.parametrize("D", [8, 256, 264, 520, 1032, 2048, 2304, 8192, 8200])
+def test_rmsnorm_row_shapes(T, D):
+    """Every number of warps a row, full and with a remainder, few rows and more than the groups of a pass; beyond 8192
+    elements the forward pass reads its rows twice and the backward pass refuses.  The sums are fp32 (a few 2^-24 of sqrt(D)
+    terms), so bf16 rounding of the results is the error: at most 2^-9 of each value."""
+    torch.manual_seed(T + D)
+    x, res, dy, dres = (torch.randn(T, D, device=DEV).bfloat16() for _ in range(4))
+    w = (1 + 0.1 * torch.randn(D, device=DEV)).bfloat16()
+    h, out = torch.empty_like(x), torch.empty_like(x)
+    _, rstd, _ = K.rmsnorm_fwd(x, w, 1e-5, res=res, h_out=h, out=out)
+    assert torch.equal(h, (x.float() + res.float()).bfloat16())
+    ro, rr, _ = K.ref_rmsnorm_fwd(h, w, 1e-5)
+    assert rel_err(out, ro.float()) < 2**-8 and rel_err(rstd, rr) < 1e-6
+    assert torch.equal(K.rmsnorm_fwd(h, w, 1e-5, want_out=False)[1], rstd)
+    if D > 8192:
+        with pytest.raises(K.N.KernelError):
+            K.rmsnorm_bwd(dy, h, w, rstd, dres=dres)
+        return
+    for extra in (None, dres):
+        dw = torch.ones(D, device=DEV).bfloat16()
+        dx, _ = K.rmsnorm_bwd(dy, h, w, rstd, dres=extra, dw=dw, accumulate_dw=True)
+        hd, dyd, wd, r = h.double(), dy.double(), w.double(), rr.double().unsqueeze(-1)
+        want = r * wd * dyd - hd * (dyd * wd * hd).sum(-1, keepdim=True) * r**3 / D + (0 if extra is None else extra.double())
+        assert rel_err(dx, want) < 2**-8 and rel_err(dw, 1 + (dyd * hd * r).sum(0)) < 2**-8
+
+
 def test_rope_roundtrip_and_ref():
     torch.manual_seed(5)
     S, Hq, Hkv, Dh = 64, 4, 2, 64

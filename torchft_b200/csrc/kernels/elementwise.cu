@@ -3,6 +3,7 @@
 // are bf16 unless stated, rows are contiguous, and every row length must be a multiple
 // of 8 elements so that all traffic is 16-byte vectors.
 #include <algorithm>
+#include <type_traits>
 
 #include "ftb200_common.cuh"
 
@@ -36,10 +37,90 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ tok, const __nv
 }
 
 // ------------------------------------------------------------------ RMSNorm
-// out = x * rstd * w ;  optionally first h = x + res (written to h_out) and normalise h.
-__global__ void rmsnorm_fwd_kernel(const bf16x8* __restrict__ x, const bf16x8* __restrict__ res,
-                                   bf16x8* __restrict__ h_out, const bf16x8* __restrict__ w,
-                                   bf16x8* __restrict__ out, float* __restrict__ rstd_out, int D8, float eps) {
+// Rows are worked on by groups of TPR threads (one to eight warps), each thread with VPT vectors of 8 elements that stay in
+// registers, packed, between the reduction and the second use.
+template <int TPR>
+__device__ __forceinline__ float group_sum(float v, float* part) {
+  v = ftb200::warp_sum(v);
+  if constexpr (TPR > 32) {
+    // one barrier of the group's own: callers that come here again alternate between two sets of `part`
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+    const int g = threadIdx.x / TPR;
+    asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(TPR) : "memory");
+    v = 0.f;
+#pragma unroll
+    for (int k = 0; k < TPR / 32; ++k) v += part[g * (TPR / 32) + k];
+  }
+  return v;
+}
+
+constexpr int NORM_THREADS = 256;
+
+// out = x * rstd * w ;  optionally first h = x + res (written to h_out) and normalise h.  Bound by memory (by L2 where the
+// rows fit there): every vector is read once, all of a thread's loads are in flight together, and the 256 / TPR rows of
+// a block wait for nothing of each other's.  With a block per row, read twice around three barriers: 63.3 us for
+// 8192 x 4096 (51.8 now, 5.2 TB/s), 32.4 for 8192 x 2048 (28.0), 9.5 for 3000 x 1024 (7.8).
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(NORM_THREADS)
+rmsnorm_fwd_kernel(const bf16x8* __restrict__ x, const bf16x8* __restrict__ res, bf16x8* __restrict__ h_out,
+                   const bf16x8* __restrict__ w, bf16x8* __restrict__ out, float* __restrict__ rstd_out, int T, int D8,
+                   float eps) {
+  __shared__ float part[NORM_THREADS / 32];
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * (NORM_THREADS / TPR) + threadIdx.x / TPR;
+  if (row >= T) return;  // a whole group
+  const int i0 = threadIdx.x % TPR;
+  bf16x8 a[VPT], c[VPT];
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    const int i = i0 + v * TPR;
+    if (i < D8) {
+      a[v] = x[row * D8 + i];
+      if (res != nullptr) c[v] = res[row * D8 + i];
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    const int i = i0 + v * TPR;
+    if (i < D8) {
+      float f[8];
+      unpack8(a[v], f);
+      if (res != nullptr) {
+        float g[8];
+        unpack8(c[v], g);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] += g[e];
+        a[v] = pack8(f);
+        h_out[row * D8 + i] = a[v];
+        unpack8(a[v], f);  // normalise the rounded value that later passes will read
+      }
+      c[v] = w[i];  // on its way during the reduction
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+    }
+  }
+  ss = group_sum<TPR>(ss, part);
+  const float r = rsqrtf(ss / (8.f * D8) + eps);
+  if (i0 == 0 && rstd_out != nullptr) rstd_out[row] = r;
+  if (out == nullptr) return;
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    const int i = i0 + v * TPR;
+    if (i < D8) {
+      float f[8], g[8];
+      unpack8(a[v], f);
+      unpack8(c[v], g);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = f[e] * r * g[e];
+      out[row * D8 + i] = pack8(f);
+    }
+  }
+}
+
+// The same for rows longer than 8192 elements: a block per row, which is read twice.
+__global__ void rmsnorm_fwd_long_kernel(const bf16x8* __restrict__ x, const bf16x8* __restrict__ res,
+                                        bf16x8* __restrict__ h_out, const bf16x8* __restrict__ w,
+                                        bf16x8* __restrict__ out, float* __restrict__ rstd_out, int D8, float eps) {
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
   const bf16x8* xr = x + row * D8;
@@ -54,7 +135,7 @@ __global__ void rmsnorm_fwd_kernel(const bf16x8* __restrict__ x, const bf16x8* _
       for (int e = 0; e < 8; ++e) f[e] += g[e];
       bf16x8 hv = pack8(f);
       h_out[row * D8 + i] = hv;
-      unpack8(hv, f);  // normalise the rounded value that later passes will read
+      unpack8(hv, f);
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
@@ -74,122 +155,149 @@ __global__ void rmsnorm_fwd_kernel(const bf16x8* __restrict__ x, const bf16x8* _
   }
 }
 
+constexpr int NORM_BWD_THREADS = 512;
+
 // dx = dres + rstd*w*dy - x*rstd^3/D * sum(dy*w*x);  dw partial sums per block.
-// Each thread owns fixed 8-column groups so dw accumulates in registers across rows.
-template <int MAXV>
-__global__ void __launch_bounds__(512, MAXV == 1 ? 2 : 1) rmsnorm_bwd_kernel(const bf16x8* __restrict__ dy, const bf16x8* __restrict__ x,
-                                   const bf16x8* __restrict__ w, const float* __restrict__ rstd,
-                                   const bf16x8* __restrict__ dres, bf16x8* __restrict__ dx,
-                                   float* __restrict__ dw_partial, int T, int D8) {
-  __shared__ float scratch[66];
-  float dw_acc[MAXV][8];
+// A group keeps its columns over all its rows, so dw accumulates in registers; the groups of a block meet in shared memory
+// at the end and leave one row of partial sums.  One block per SM, 2 to 16 groups in it: what a row waits for (its loads,
+// its reduction) is covered by the rows of the other groups, which nothing ties to it.  Two rows a block and iteration around one block-wide sum, two blocks per SM, 296 rows of partial sums:
+// 8192 x 2048 45.3 us (38.0 now, both kernels), 3000 x 1024 19.4 (14.0), 2500 x 8192 60.9 (50.7), 8192 x 4096 67.8 (66.8).
+template <int TPR, int VPT>
+__global__ void __launch_bounds__(NORM_BWD_THREADS, 1)
+rmsnorm_bwd_kernel(const bf16x8* __restrict__ dy, const bf16x8* __restrict__ x, const bf16x8* __restrict__ w,
+                   const float* __restrict__ rstd, const bf16x8* __restrict__ dres, bf16x8* __restrict__ dx,
+                   float* __restrict__ dw_partial, int T, int D8) {
+  constexpr int GROUPS = NORM_BWD_THREADS / TPR;
+  __shared__ float part[2][NORM_BWD_THREADS / 32];
+  __shared__ float4 dw_groups[NORM_BWD_THREADS][2];
+  const int g = threadIdx.x / TPR, i0 = threadIdx.x % TPR;
+  float dw_acc[VPT][8];
 #pragma unroll
-  for (int v = 0; v < MAXV; ++v)
+  for (int v = 0; v < VPT; ++v)
 #pragma unroll
     for (int e = 0; e < 8; ++e) dw_acc[v][e] = 0.f;
-
-  // Two rows per iteration: their loads (dy, x and the residual gradient) are all in flight before the one
-  // block-wide reduction they share, and the rows stay in registers (packed) across it.
-  for (int64_t row0 = blockIdx.x; row0 < T; row0 += 2 * static_cast<int64_t>(gridDim.x)) {
-    const int64_t rows[2] = {row0, row0 + gridDim.x};
-    const bool live[2] = {true, rows[1] < T};
-    float r[2] = {rstd[rows[0]], live[1] ? rstd[rows[1]] : 0.f};
-    bf16x8 a[2][MAXV], b[2][MAXV], d[2][MAXV];
+  int turn = 0;
+  for (int64_t row = blockIdx.x + static_cast<int64_t>(gridDim.x) * g; row < T; row += static_cast<int64_t>(gridDim.x) * GROUPS) {
+    bf16x8 a[VPT], b[VPT], d[VPT];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int v = 0; v < VPT; ++v) {
+      const int i = i0 + v * TPR;
+      if (i < D8) {
+        a[v] = dy[row * D8 + i];
+        b[v] = x[row * D8 + i];
+        if (dres != nullptr) d[v] = dres[row * D8 + i];
+      }
+    }
+    const float r = rstd[row];
+    float dot = 0.f;
 #pragma unroll
-      for (int v = 0; v < MAXV; ++v) {
-        const int i = threadIdx.x + v * blockDim.x;
-        if (live[k] && i < D8) {
-          a[k][v] = dy[rows[k] * D8 + i];
-          b[k][v] = x[rows[k] * D8 + i];
-          if (dres != nullptr) d[k][v] = dres[rows[k] * D8 + i];
+    for (int v = 0; v < VPT; ++v) {
+      if (i0 + v * TPR < D8) {
+        float fa[8], fb[8], c[8];
+        unpack8(a[v], fa);
+        unpack8(b[v], fb);
+        unpack8(w[i0 + v * TPR], c);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          dot += fa[e] * c[e] * fb[e];
+          dw_acc[v][e] += fa[e] * fb[e] * r;
         }
       }
     }
-    float dot[2] = {0.f, 0.f};
+    dot = group_sum<TPR>(dot, part[turn]);
+    turn ^= 1;
+    const float coef = dot * r * r * r / (8.f * D8);
 #pragma unroll
-    for (int v = 0; v < MAXV; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
+    for (int v = 0; v < VPT; ++v) {
+      const int i = i0 + v * TPR;
       if (i < D8) {
-        float c[8];
-        unpack8(w[i], c);
+        float fa[8], fb[8], c[8], o[8];
+        unpack8(a[v], fa);
+        unpack8(b[v], fb);
+        unpack8(w[i0 + v * TPR], c);
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          if (live[k]) {
-            float fa[8], fb[8];
-            unpack8(a[k][v], fa);
-            unpack8(b[k][v], fb);
+        for (int e = 0; e < 8; ++e) o[e] = r * c[e] * fa[e] - fb[e] * coef;
+        if (dres != nullptr) {
+          float fd[8];
+          unpack8(d[v], fd);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              dot[k] += fa[e] * c[e] * fb[e];
-              dw_acc[v][e] += fa[e] * fb[e] * r[k];
-            }
-          }
+          for (int e = 0; e < 8; ++e) o[e] += fd[e];
         }
-      }
-    }
-    const float2 dots = ftb200::block_sum2(dot[0], dot[1], scratch);
-    const float coef[2] = {dots.x * r[0] * r[0] * r[0] / (8.f * D8), dots.y * r[1] * r[1] * r[1] / (8.f * D8)};
-#pragma unroll
-    for (int v = 0; v < MAXV; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
-      if (i < D8) {
-        float c[8];
-        unpack8(w[i], c);
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          if (live[k]) {
-            float fa[8], fb[8], o[8];
-            unpack8(a[k][v], fa);
-            unpack8(b[k][v], fb);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = r[k] * c[e] * fa[e] - fb[e] * coef[k];
-            if (dres != nullptr) {
-              float fd[8];
-              unpack8(d[k][v], fd);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) o[e] += fd[e];
-            }
-            dx[rows[k] * D8 + i] = pack8(o);
-          }
-        }
+        dx[row * D8 + i] = pack8(o);
       }
     }
   }
+  float4* dst = reinterpret_cast<float4*>(dw_partial) + static_cast<int64_t>(blockIdx.x) * (2 * D8);
 #pragma unroll
-  for (int v = 0; v < MAXV; ++v) {
-    const int i = threadIdx.x + v * blockDim.x;
-    if (i < D8) {
-      float* dst = dw_partial + (static_cast<int64_t>(blockIdx.x) * D8 + i) * 8;
+  for (int v = 0; v < VPT; ++v) {
+    if (v > 0) __syncthreads();
+    dw_groups[threadIdx.x][0] = make_float4(dw_acc[v][0], dw_acc[v][1], dw_acc[v][2], dw_acc[v][3]);
+    dw_groups[threadIdx.x][1] = make_float4(dw_acc[v][4], dw_acc[v][5], dw_acc[v][6], dw_acc[v][7]);
+    __syncthreads();
+    const int c = threadIdx.x;  // four columns of the group's 8 TPR
+    if (c < 2 * TPR && v * 2 * TPR + c < 2 * D8) {
+      float4 s = dw_groups[c >> 1][c & 1];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) dst[e] = dw_acc[v][e];
+      for (int k = 1; k < GROUPS; ++k) {
+        const float4 t = dw_groups[k * TPR + (c >> 1)][c & 1];
+        s.x += t.x;
+        s.y += t.y;
+        s.z += t.z;
+        s.w += t.w;
+      }
+      dst[v * 2 * TPR + c] = s;
     }
   }
 }
 
-// dw[c] (+)= sum_b partial[b][c].  A block owns 32 columns; its 8 warps stride over the rows (each warp
-// instruction reads one 128-byte row segment) and meet in shared memory, so a few hundred rows are a few
-// dozen independent loads per thread instead of one long serial loop.
-__global__ void colsum_partials_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw, int nblk, int D,
-                                       int accumulate) {
-  __shared__ float red[8][33];
+// dw[c] (+)= sum_b partial[b][c].  A block owns 32 columns; its 32 warps stride over the rows (each warp instruction reads
+// one 128-byte row segment) and meet in shared memory: a row of partial sums per SM is five independent loads a thread.
+__global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw,
+                                                               int nblk, int D, int accumulate) {
+  __shared__ float red[32][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
   float s = 0.f;
   if (c < D) {
-#pragma unroll 4
-    for (int b = ry; b < nblk; b += 8) s += partial[static_cast<int64_t>(b) * D + c];
+#pragma unroll 5
+    for (int b = ry; b < nblk; b += 32) s += partial[static_cast<int64_t>(b) * D + c];
   }
   red[ry][cx] = s;
   __syncthreads();
-  if (ry == 0 && c < D) {
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) t += red[k][cx];
-    if (accumulate) t += __bfloat162float(dw[c]);
-    dw[c] = __float2bfloat16(t);
-  }
+  const float t = ftb200::warp_sum(red[cx][ry]);  // warp ry: column ry of the block, lane cx: row cx of the sums
+  const int col = blockIdx.x * 32 + ry;
+  if (cx == 0 && col < D) dw[col] = __float2bfloat16(accumulate ? t + __bfloat162float(dw[col]) : t);
+}
+
+// Threads per row and vectors per thread: as few warps a row as 4 vectors a thread allow (8 loads of 16 bytes in flight in
+// the forward pass, 12 in the backward pass), up to 8 warps for 8192 elements.  With `few` rows, which leave the SMs room,
+// twice the threads and half the vectors: 64 x 1024 3.6 -> 2.8 us forward, but 3000 x 1024 7.8 -> 9.3.
+template <typename F>
+int with_row_shape(int D8, bool few, F&& f) {
+  if (few && D8 > 64 && D8 <= 128) return f(std::integral_constant<int, 64>(), std::integral_constant<int, 2>());
+  if (few && D8 > 128 && D8 <= 256) return f(std::integral_constant<int, 128>(), std::integral_constant<int, 2>());
+  if (few && D8 > 256 && D8 <= 512) return f(std::integral_constant<int, 256>(), std::integral_constant<int, 2>());
+  if (D8 <= 32) return f(std::integral_constant<int, 32>(), std::integral_constant<int, 1>());
+  if (D8 <= 64) return f(std::integral_constant<int, 32>(), std::integral_constant<int, 2>());
+  if (D8 <= 128) return f(std::integral_constant<int, 32>(), std::integral_constant<int, 4>());
+  if (D8 <= 256) return f(std::integral_constant<int, 64>(), std::integral_constant<int, 4>());
+  if (D8 <= 512) return f(std::integral_constant<int, 128>(), std::integral_constant<int, 4>());
+  if (D8 <= 1024) return f(std::integral_constant<int, 256>(), std::integral_constant<int, 4>());
+  return FTB200_E_TOOBIG;
+}
+
+// Both kernels of the backward pass; dw_partial holds at least min(T, SMs) * D floats.
+int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dw,
+                       float* dw_partial, int T, int D, int accumulate_dw, int sms, cudaStream_t st) {
+  const int D8 = D / 8;
+  return with_row_shape(D8, T <= sms, [&](auto tpr, auto vpt) {
+    constexpr int GROUPS = NORM_BWD_THREADS / tpr;
+    const int nblk = std::min((T + 3) / 4, sms);
+    rmsnorm_bwd_kernel<tpr, vpt><<<nblk, NORM_BWD_THREADS, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w,
+                                                                       rstd, (const bf16x8*)dres, (bf16x8*)dx, dw_partial, T, D8);
+    colsum_partials_kernel<<<(D + 31) / 32, 1024, 0, st>>>(dw_partial, (__nv_bfloat16*)dw, nblk, D, accumulate_dw);
+    return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+  });
 }
 
 // ------------------------------------------------------------------ RoPE (interleaved pairs)
@@ -457,9 +565,16 @@ FTB200_API int ftb200_rmsnorm_fwd(const void* x, const void* res, void* h_out, c
                                   int T, int D, float eps, cudaStream_t st) {
   if (D % 8) return FTB200_E_ALIGN;
   if (res != nullptr && h_out == nullptr) return FTB200_E_BADARG;
-  const int threads = (D / 8 >= 512) ? 512 : 256;
-  rmsnorm_fwd_kernel<<<T, threads, 0, st>>>((const bf16x8*)x, (const bf16x8*)res, (bf16x8*)h_out, (const bf16x8*)w,
-                                            (bf16x8*)out, rstd, D / 8, eps);
+  const int D8 = D / 8;
+  const int rc = with_row_shape(D8, T <= 4 * ftb200::sm_count(), [&](auto tpr, auto vpt) {
+    constexpr int ROWS = NORM_THREADS / tpr;
+    rmsnorm_fwd_kernel<tpr, vpt><<<(T + ROWS - 1) / ROWS, NORM_THREADS, 0, st>>>(
+        (const bf16x8*)x, (const bf16x8*)res, (bf16x8*)h_out, (const bf16x8*)w, (bf16x8*)out, rstd, T, D8, eps);
+    return 0;
+  });
+  if (rc != 0)
+    rmsnorm_fwd_long_kernel<<<T, 512, 0, st>>>((const bf16x8*)x, (const bf16x8*)res, (bf16x8*)h_out, (const bf16x8*)w,
+                                               (bf16x8*)out, rstd, D8, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
@@ -472,23 +587,7 @@ FTB200_API int ftb200_rmsnorm_bwd(const void* dy, const void* x, const void* w, 
                                   void* dx, void* dw, float* dw_partial, int T, int D, int accumulate_dw,
                                   cudaStream_t st) {
   if (D % 8) return FTB200_E_ALIGN;
-  const int D8 = D / 8;
-  const int threads = D8 > 256 ? 512 : 256;  // wide rows: 16 warps per block, two blocks per SM
-  const int nblk = min(T, ftb200::sm_count() * 2);
-  const int maxv = (D8 + threads - 1) / threads;
-  if (maxv <= 1)
-    rmsnorm_bwd_kernel<1><<<nblk, threads, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w, rstd,
-                                                    (const bf16x8*)dres, (bf16x8*)dx, dw_partial, T, D8);
-  else if (maxv <= 2)
-    rmsnorm_bwd_kernel<2><<<nblk, threads, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w, rstd,
-                                                    (const bf16x8*)dres, (bf16x8*)dx, dw_partial, T, D8);
-  else if (maxv <= 4)
-    rmsnorm_bwd_kernel<4><<<nblk, threads, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w, rstd,
-                                                    (const bf16x8*)dres, (bf16x8*)dx, dw_partial, T, D8);
-  else
-    return FTB200_E_TOOBIG;  // D > 8192
-  colsum_partials_kernel<<<(D + 31) / 32, 256, 0, st>>>(dw_partial, (__nv_bfloat16*)dw, nblk, D, accumulate_dw);
-  return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+  return launch_rmsnorm_bwd(dy, x, w, rstd, dres, dx, dw, dw_partial, T, D, accumulate_dw, ftb200::sm_count(), st);
 }
 
 // Rotates the first n_heads heads of every row in place.  backward != 0 applies the inverse rotation.
@@ -604,20 +703,7 @@ FTB200_API int ftb200_rmsnorm_bwd_noalloc(const void* dy, const void* x, const v
     g_noalloc_scratch_addr[dev].store(p, std::memory_order_release);
     scratch = p;
   }
-  const int D8 = D / 8;
-  const int threads = D8 > 256 ? 512 : 256;  // wide rows: 16 warps per block, two blocks per SM
-  const int maxv = (D8 + threads - 1) / threads;
-  if (maxv <= 1)
-    rmsnorm_bwd_kernel<1><<<nblk, threads, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w, rstd,
-                                                    (const bf16x8*)dres, (bf16x8*)dx, scratch, T, D8);
-  else if (maxv <= 2)
-    rmsnorm_bwd_kernel<2><<<nblk, threads, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w, rstd,
-                                                    (const bf16x8*)dres, (bf16x8*)dx, scratch, T, D8);
-  else
-    rmsnorm_bwd_kernel<4><<<nblk, threads, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w, rstd,
-                                                    (const bf16x8*)dres, (bf16x8*)dx, scratch, T, D8);
-  colsum_partials_kernel<<<(D + 31) / 32, 256, 0, st>>>(scratch, (__nv_bfloat16*)dw, nblk, D, accumulate_dw);
-  return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+  return launch_rmsnorm_bwd(dy, x, w, rstd, dres, dx, dw, scratch, T, D, accumulate_dw, sms, st);
 }
 
 // ---- checked-index debug build: status query and a self-test that records an out-of-range
