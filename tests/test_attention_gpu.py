@@ -170,6 +170,29 @@ def test_attention_bwd_tiles(B, S, Hq, Hkv, causal, scale, D):
         assert (got.float() - w).norm() <= 3 * 2**-9 * w.norm(), name
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_bwd_rotates_back(D, causal):
+    """dQ and dK of the values before the rotation: as the rotated ones turned back by a kernel of their own, which rounds once
+    more (2^-9 of each value)."""
+    B, S, Hq, Hkv = 2, 512, 4, 2
+    qkv, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=D)
+    table = K.rope_table(S, D, 10000.0, "cuda")
+    out = torch.empty(B * S, Hq * D, dtype=torch.bfloat16, device="cuda")
+    lse = torch.empty(B, Hq, S, dtype=torch.float32, device="cuda")
+    K.attention_fwd(q, k, v, B, S, Hq, Hkv, D, out, lse, causal=causal)
+    d_o = torch.randn_like(out)
+    grads = []
+    for rope in (None, table):
+        d = torch.full_like(qkv, float("nan"))
+        K.attention_bwd(q, k, v, out, d_o, lse, d[:, : Hq * D], d[:, Hq * D : (Hq + Hkv) * D], d[:, (Hq + Hkv) * D :], B, S, Hq,
+                        Hkv, D, causal=causal, rope=rope)
+        grads.append(d if rope is not None else K.rope_(d, table, S, Hq + Hkv, D, backward=True))
+    K.check_status(out.device)
+    a, b = (g.float() for g in grads)
+    assert (a - b).norm() < 2**-8 * a.norm() and torch.equal(grads[0][:, (Hq + Hkv) * D :], grads[1][:, (Hq + Hkv) * D :])
+
+
 @pytest.mark.parametrize("D,poly", [(64, None), (64, "0"), (64, "4"), (128, "0"), (128, "4")])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("key", [*range(8), 131, 200])

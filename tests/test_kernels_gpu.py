@@ -234,6 +234,76 @@ def test_cross_entropy_without_gradient(V):
     assert rel_err(logits[:2], K.ref_cross_entropy(kept, tgt.clamp(min=0), 1.0)[1][:2]) < 1e-2 and not logits[2].any()
 
 
+@pytest.mark.parametrize("T,Kd,heads,kv,Dh,S", [(300, 256, 2, 2, 128, 100), (16400, 64, 8, 2, 64, 33), (20000, 72, 4, 2, 128, 1000),
+                                               (8200, 128, 8, 4, 192, 260)])
+def test_linear_rope(T, Kd, heads, kv, Dh, S):
+    """The projection with its rotation in the epilogue against the two kernels: the same rounded values are rotated, by products
+    that the compiler may contract another way (one bf16 rounding apart at most)."""
+    torch.manual_seed(T)
+    N = (heads + 2 * kv) * Dh
+    x, w = torch.randn(T, Kd, device=DEV).bfloat16(), torch.randn(N, Kd, device=DEV).bfloat16()
+    table = K.rope_table(S, Dh, 10000.0, DEV)
+    out = torch.full((T + 1, N + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    assert T < 8000 or -(-T // 256) * -(-N // 256) > torch.cuda.get_device_properties(0).multi_processor_count  # the fused one
+    K.linear_rope_fwd(x, w, out[:T, :N], table, S, heads + kv, Dh)
+    want = K.rope_(K.linear_fwd(x, w), table, S, heads + kv, Dh)
+    assert torch.equal(out[:T, (heads + kv) * Dh : N], want[:, (heads + kv) * Dh :])
+    assert (out[:T, :N].float() - want.float()).abs().max() <= 2**-7 * want.float().abs().max()
+    assert rel_err(out[:T, :N], want) < 2**-9
+    assert bool((out[T:] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
+    K.check_status(out.device)
+
+
+@pytest.mark.parametrize("T,Kd,F", [(1, 2048, 8), (33, 2056, 40), (200, 2048, 512), (1000, 2048, 2816), (130, 4096, 1000), (300, 64, 128)])
+def test_linear_dswiglu(T, Kd, F):
+    """Down projection and activation backwards in one kernel against 64 bits: the gradient of the activation is not rounded on
+    the way, so the result's rounding (2^-9 of each value) is the whole error."""
+    torch.manual_seed(T + F)
+    dy, w = torch.randn(T, Kd, device=DEV).bfloat16(), (0.05 * torch.randn(Kd, F, device=DEV)).bfloat16()
+    buf = torch.full((T + 1, 2 * F + 8), 7.0, device=DEV, dtype=torch.bfloat16)
+    gu = torch.randn(T, 2 * F, device=DEV).bfloat16()
+    buf[:T, : 2 * F] = gu
+    ds = torch.empty(T, F, device=DEV, dtype=torch.bfloat16)
+    if Kd < 2048:  # the two kernels, which want their pairs in one piece
+        with pytest.raises(ValueError):
+            K.linear_dswiglu_(dy, w, buf[:T, : 2 * F], ds)
+        whole = gu.clone()
+        K.linear_dswiglu_(dy, w, whole, ds)
+        buf[:T, : 2 * F] = whole
+    else:
+        K.linear_dswiglu_(dy, w, buf[:T, : 2 * F], ds)
+    g, u, d = gu[:, 0::2].double(), gu[:, 1::2].double(), dy.double() @ w.double()
+    sg = torch.sigmoid(g)
+    want = torch.stack([d * u * (sg + g * sg * (1 - sg)), d * g * sg], dim=-1).reshape(T, 2 * F)
+    assert rel_err(buf[:T, : 2 * F], want) < 2**-8
+    assert bool((buf[T:] == 7.0).all()) and bool((buf[:, 2 * F :] == 7.0).all())
+    K.check_status(dy.device)
+
+
+@pytest.mark.parametrize("T,Kd,V", [(37, 128, 1000), (300, 256, 8192), (129, 64, 20008), (1050, 72, 1000), (131080, 64, 8)])
+def test_linear_cross_entropy(T, Kd, V):
+    """Head product and loss without stored logits against the two kernels: ignored targets and targets beyond the vocabulary
+    count alike, a NaN in one row stays there.  Sums of V exponentials in fp32, in another order: 1e-5."""
+    torch.manual_seed(V)
+    x, w = torch.randn(T, Kd, device=DEV).bfloat16(), (0.2 * torch.randn(V, Kd, device=DEV)).bfloat16()
+    tgt = torch.randint(0, V, (T,), device=DEV)
+    tgt[T // 3] = -1
+    if T > 2:
+        tgt[T // 2] = V + 3
+        x[T - 1, 0] = float("nan")
+    plain = K.linear_fwd(x, w)
+    want = K.cross_entropy_(plain.clone(), tgt, 0.25, grad=False)
+    loss = torch.empty(T, device=DEV)
+    K.linear_cross_entropy_(x, w, tgt, 0.25, torch.empty_like(plain), loss, grad=False)
+    K.check_status(x.device)
+    torch.testing.assert_close(loss, want, rtol=1e-5, atol=1e-5, equal_nan=True)
+    both = torch.empty_like(plain)
+    K.linear_cross_entropy_(x, w, tgt, 0.25, both, loss, grad=True)
+    torch.testing.assert_close(loss, want, rtol=1e-5, atol=1e-5, equal_nan=True)
+    assert torch.equal(K.cross_entropy_(plain, tgt, 0.25).isfinite(), loss.isfinite())
+    assert torch.equal(plain.nan_to_num(), both.nan_to_num())
+
+
 @pytest.mark.parametrize("gdt", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n", [8, 1000, 1 << 20, (1 << 20) + 3])
 def test_adamw(gdt, n):

@@ -114,8 +114,20 @@ struct BwdParams {
   __nv_bfloat16* dK;   // rows batch*seq, row stride ld_dk
   __nv_bfloat16* dV;
   long long ld_dk, ld_dv;
+  const float4* rope;  // null, or (cos, sin) pairs [seq][D / 2]: dQ and dK are rotated back
   int* status;
 };
+
+// Eight elements (four pairs) rotated back by their angles (cos, sin, cos, sin).
+__device__ __forceinline__ void rotate_back(float* f, const float4& c0, const float4& c1) {
+  const float cosv[4] = {c0.x, c0.z, c1.x, c1.z}, sinv[4] = {c0.y, c0.w, c1.y, c1.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float a = f[2 * e], b = f[2 * e + 1];
+    f[2 * e] = a * cosv[e] + b * sinv[e];
+    f[2 * e + 1] = b * cosv[e] - a * sinv[e];
+  }
+}
 
 __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -507,6 +519,10 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * c + e]);
+          if (which == 1 && p.rope != nullptr) {
+            const float4* cs = p.rope + static_cast<long long>(jb * BKV + row) * (D / 4) + g * (CW / 4) + 2 * c;
+            rotate_back(f, cs[0], cs[1]);
+          }
           reinterpret_cast<ftb200::bf16x8*>(dst)[c] = ftb200::pack8(f);
         }
       }
@@ -557,10 +573,11 @@ __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bflo
 }
 
 // dq (bf16, row stride ld) = accumulator (fp32, per 128 queries and head [D / 32][32 groups of 4 queries][32][4 queries]); a
-// thread takes 8 head-dim elements of 4 queries.
+// thread takes 8 head-dim elements of 4 queries and, with `rope`, rotates them back.
 template <int D>
 __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
-                                                                long long pieces, int n_heads, long long ld) {
+                                                                long long pieces, int n_heads, long long ld, int seq,
+                                                                const float4* __restrict__ rope) {
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= pieces) return;
   const int d8 = static_cast<int>(i % (D / 8));
@@ -578,6 +595,10 @@ __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __
     float f[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) f[e] = k == 0 ? v[e].x : k == 1 ? v[e].y : k == 2 ? v[e].z : v[e].w;
+    if (rope != nullptr) {
+      const float4* cs = rope + (row0 + k) % seq * (D / 4) + d8 * 2;
+      rotate_back(f, cs[0], cs[1]);
+    }
     *reinterpret_cast<ftb200::bf16x8*>(dq + (row0 + k) * ld + h * D + d8 * 8) = ftb200::pack8(f);
   }
 }
@@ -627,7 +648,8 @@ template <int D>
 int attention_bwd_impl(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse,
                        void* dq, void* dk, void* dv, void* scratch, int batch, int seq, int n_heads, int n_kv_heads,
                        long long ld_q, long long ld_k, long long ld_v, long long ld_o, long long ld_do, long long ld_dq,
-                       long long ld_dk, long long ld_dv, float scale, int causal, int* status, cudaStream_t stream) {
+                       long long ld_dk, long long ld_dv, float scale, int causal, const float* cos_sin, int* status,
+                       cudaStream_t stream) {
   constexpr uint32_t SMEM_BYTES = Lay<D>::SMEM_BYTES;
   const long long rows = static_cast<long long>(batch) * seq;
   float* dq_acc = reinterpret_cast<float*>(scratch);
@@ -662,11 +684,13 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   p.neg_lse2 = neg_lse2; p.neg_delta = neg_delta; p.dq_acc = dq_acc;
   p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
   p.ld_dk = ld_dk; p.ld_dv = ld_dv; p.status = status;
+  p.rope = reinterpret_cast<const float4*>(cos_sin);
   const long long grid = static_cast<long long>(batch) * n_kv_heads * (seq / BKV);
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_bwd_kernel<D><<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
   attention_dq_cast_kernel<D><<<static_cast<unsigned>((pieces / 4 + 255) / 256), 256, 0, stream>>>(
-      reinterpret_cast<const float4*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), pieces / 4, n_heads, ld_dq);
+      reinterpret_cast<const float4*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), pieces / 4, n_heads, ld_dq, seq,
+      p.rope);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
@@ -674,16 +698,19 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
 
 // q, k, v, o, d_o as in the forward pass (2-D views, row strides in elements); dq, dk, dv are
 // written (not accumulated).  lse is the forward's [batch, n_heads, seq].  scratch: at least
-// ftb200_attention_bwd_scratch_bytes, 16-byte aligned.  Head dim 64 or 128.
+// ftb200_attention_bwd_scratch_bytes, 16-byte aligned.  Head dim 64 or 128.  cos_sin: null, or fp32 [seq][head_dim / 2]
+// pairs of the angles that q and k were rotated by (pair (2i, 2i + 1) of a head by the i-th angle of its row's position):
+// dq and dk are then the gradients of the values before the rotation, rotated back in fp32 ahead of the rounding to bf16.
 FTB200_API int ftb200_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                     const float* lse, void* dq, void* dk, void* dv, void* scratch, int batch, int seq,
                                     int n_heads, int n_kv_heads, int head_dim, long long ld_q, long long ld_k,
                                     long long ld_v, long long ld_o, long long ld_do, long long ld_dq, long long ld_dk,
-                                    long long ld_dv, float scale, int causal, int* status, cudaStream_t stream) {
+                                    long long ld_dv, float scale, int causal, const float* cos_sin, int* status,
+                                    cudaStream_t stream) {
   if ((head_dim != 64 && head_dim != 128) || batch <= 0 || seq <= 0 || seq % BKV != 0 || n_heads <= 0 ||
       n_kv_heads <= 0 || n_heads % n_kv_heads != 0)
     return FTB200_E_BADARG;
-  const void* ptrs[] = {q, k, v, o, d_o, dq, dk, dv, scratch};
+  const void* ptrs[] = {q, k, v, o, d_o, dq, dk, dv, scratch, cos_sin};
   for (const void* x : ptrs)
     if (!aligned16(x)) return FTB200_E_ALIGN;
   const long long lds[] = {ld_q, ld_k, ld_v, ld_o, ld_do, ld_dq, ld_dk, ld_dv};
@@ -691,7 +718,7 @@ FTB200_API int ftb200_attention_bwd(const void* q, const void* k, const void* v,
     if (x & 7) return FTB200_E_ALIGN;
   if (head_dim == 64)
     return attention_bwd_impl<64>(q, k, v, o, d_o, lse, dq, dk, dv, scratch, batch, seq, n_heads, n_kv_heads, ld_q, ld_k,
-                                  ld_v, ld_o, ld_do, ld_dq, ld_dk, ld_dv, scale, causal, status, stream);
+                                  ld_v, ld_o, ld_do, ld_dq, ld_dk, ld_dv, scale, causal, cos_sin, status, stream);
   return attention_bwd_impl<128>(q, k, v, o, d_o, lse, dq, dk, dv, scratch, batch, seq, n_heads, n_kv_heads, ld_q, ld_k,
-                                 ld_v, ld_o, ld_do, ld_dq, ld_dk, ld_dv, scale, causal, status, stream);
+                                 ld_v, ld_o, ld_do, ld_dq, ld_dk, ld_dv, scale, causal, cos_sin, status, stream);
 }

@@ -444,6 +444,24 @@ cross_entropy_kernel(bf16x8* __restrict__ logits, const int64_t* __restrict__ ta
   for (; i < V8; i += step) put(lr[i], i);
 }
 
+// loss[row] from the maxima, sums and target values that the tiles of a product noted (ftb200_gemm_bf16_loss), a warp a row.
+__global__ void __launch_bounds__(256)
+cross_entropy_rows_kernel(const long long* __restrict__ target, const float2* __restrict__ stats,
+                          const float* __restrict__ target_value, float* __restrict__ loss, int tiles, int T, long long V) {
+  const int lane = threadIdx.x & 31;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (row >= T) return;
+  const float2* st = stats + row * tiles;
+  float mx = -INFINITY, sum = 0.f;
+  for (int i = lane; i < tiles; i += 32) mx = fmaxf(mx, st[i].x);
+  mx = ftb200::warp_max(mx);
+  const float base = mx == -INFINITY ? 0.f : mx;
+  for (int i = lane; i < tiles; i += 32) sum += st[i].y * __expf(st[i].x - base);
+  sum = ftb200::warp_sum(sum);
+  const long long tgt = target[row];
+  if (lane == 0) loss[row] = tgt >= 0 ? logf(sum) + mx - (tgt < V ? target_value[row] : 0.f) : 0.f;
+}
+
 // ------------------------------------------------------------------ AdamW (flat shard)
 // master/m/v fp32, grad bf16 or fp32, writes the bf16 working copy.  `grad_scale_dev`
 // (optional) is a device scalar multiplied into every gradient (clipping coefficient).
@@ -618,6 +636,13 @@ FTB200_API int ftb200_cross_entropy(void* logits, const int64_t* target, float* 
                                     float grad_scale, int grad, cudaStream_t st) {
   if (V % 8 || ld % 8) return FTB200_E_ALIGN;
   cross_entropy_kernel<<<T, 1024, 0, st>>>((bf16x8*)logits, target, loss, V / 8, ld / 8, grad_scale, grad);
+  return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
+}
+
+// Second half of ftb200_gemm_bf16_loss.
+int ftb200_launch_cross_entropy_rows(const long long* target, const float2* row_stats, const float* target_value, float* loss,
+                                     int tiles, int T, int V, cudaStream_t st) {
+  cross_entropy_rows_kernel<<<(T + 7) / 8, 256, 0, st>>>(target, row_stats, target_value, loss, tiles, T, V);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 

@@ -49,15 +49,29 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
 
-// A pair's tile has 256 or 128 columns; the K ring fills the same 192 KB with 6 or 8 stages.
-template <int BN_>
+// What becomes of a tile.
+enum Epilogue : int {
+  EPI_STORE = 0,    // it is stored (added, with the activation of its columns' pairs, scattered: GemmParams)
+  EPI_DSWIGLU = 1,  // it is the gradient of silu(gate) * up: the gate/up pairs it belongs to are replaced by their gradients
+  EPI_LOSS = 2,     // its rows' maximum, sum of exponentials and target value are noted; it is not stored
+  EPI_ROPE = 3,     // stored, the columns of its first heads rotated by their row's position
+};
+
+// A pair's tile has 256 or 128 columns; the K ring fills 192 KB with 6 or 8 stages.  The gradient of the activation needs
+// twice the staging area (two 64-column pieces of gate/up pairs) and leaves it 5 or 6.
+template <int BN_, int EPI>
 struct Tile {
   static constexpr int BN = BN_;        // columns per pair
   static constexpr int BNH = BN / 2;    // of B's rows, per CTA
-  static constexpr int STAGES = BN == 256 ? 6 : 8;
+  static constexpr bool DS = EPI == EPI_DSWIGLU;
+  static constexpr int STAGES = BN == 256 ? (DS ? 5 : 6) : (DS ? 6 : 8);
   static constexpr uint32_t B_BYTES = BNH * BK * 2;
   static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  static_assert(STAGES * STAGE_BYTES == 196608, "the epilogue's staging area follows the ring");
+  static constexpr uint32_t STAGE_WARP_BYTES = 32 * (DS ? 512 : 256);  // epilogue: 32 rows x 128 bf16 per warp (256)
+  static constexpr uint32_t OFF_STAGING = STAGES * STAGE_BYTES, OFF_MISC = OFF_STAGING + 4 * STAGE_WARP_BYTES;
+  static constexpr uint32_t SMEM_BYTES = OFF_MISC + 256 + 1024;
+  static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
+  static_assert(DS || OFF_STAGING == 196608, "a shared tile's exchange fills the ring");
 };
 constexpr uint32_t RING_BYTES = 196608;
 constexpr int GATHER_BLOCK = 128;  // B rows whose pieces the all-gather counts together: a CTA's half of a 256-column tile
@@ -66,10 +80,6 @@ constexpr int GATHER_WARPS = 4;  // only launched by the all-gather variant
 constexpr int NUM_THREADS_GATHER = NUM_THREADS + 32 * GATHER_WARPS;
 constexpr int GATHER_PIECE_V = 1024;  // 16-byte vectors per piece (16 KiB)
 constexpr uint32_t TMEM_COLS = 512;
-constexpr uint32_t STAGE_WARP_BYTES = 32 * 256;  // epilogue: 32 rows x 128 bf16 per warp
-constexpr uint32_t OFF_STAGING = RING_BYTES, OFF_MISC = OFF_STAGING + 4 * STAGE_WARP_BYTES;
-constexpr uint32_t SMEM_BYTES = OFF_MISC + 256 + 1024;
-static_assert(SMEM_BYTES <= 232448, "exceeds the 227 KB of shared memory a CTA can have");
 constexpr int GROUP_M = 8;  // in 256-row pair tiles (the all-gather variant uses twice that)
 
 using namespace ftb200::tc;
@@ -159,6 +169,13 @@ struct GemmParams {
   // fused SwiGLU: output columns are (gate, up) pairs; aux[row, j] = silu(C[row,2j]) * C[row,2j+1]
   void* aux;
   long long ld_aux;
+  // EPI_LOSS, per row: [tiles of a row] (maximum, sum of exponentials over it), the target's value, the target
+  float2* row_stats;
+  float* target_value;
+  const long long* target;
+  // EPI_ROPE: (cos, sin) pairs [rope_seq][head_dim / 2], columns that are rotated, row = ... * rope_seq + position
+  const float4* rope;
+  int rope_cols, rope_seq, rope_dim;
   // fused reduce-scatter epilogue: C is not written locally; every 16-byte piece of the
   // (contiguous, row-major) result goes to the rank that owns that slice of the flat
   // gradient unit, into that rank's staging area for source rank `sc_src`.
@@ -243,6 +260,20 @@ __device__ __forceinline__ uint2 silu_mul(const ftb200::bf16x8& packed) {
   return o;
 }
 
+// Four pairs rotated by their angles (cos, sin, cos, sin).
+__device__ __forceinline__ ftb200::bf16x8 rotate_pairs(const ftb200::bf16x8& x, const float4& c0, const float4& c1) {
+  float f[8];
+  ftb200::unpack8(x, f);
+  const float cosv[4] = {c0.x, c0.z, c1.x, c1.z}, sinv[4] = {c0.y, c0.w, c1.y, c1.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float a = f[2 * e], b = f[2 * e + 1];
+    f[2 * e] = a * cosv[e] - b * sinv[e];
+    f[2 * e + 1] = a * sinv[e] + b * cosv[e];
+  }
+  return ftb200::pack8(f);
+}
+
 // Asynchronous copy from this CTA's shared memory to another's, counted by a barrier there.
 __device__ __forceinline__ void copy_to_cta(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src),
@@ -258,12 +289,13 @@ constexpr int MAX_SPLIT = 4;  // 8 CTAs: the largest cluster that every part tak
 static_assert(2 * MAX_IN * CHUNK_BYTES <= RING_BYTES, "the ring holds what comes and what goes");
 
 // Clusters of two CTAs (SPLIT: of 2 S), set at the launch.
-template <int BN_, bool SPLIT>
+template <int BN_, bool SPLIT, int EPI>
 __global__ void __launch_bounds__(SPLIT ? NUM_THREADS : NUM_THREADS_GATHER, 1)
 gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                               const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux,
                               const GemmParams p) {
-  using TL = Tile<BN_>;
+  using TL = Tile<BN_, EPI>;
+  constexpr uint32_t OFF_STAGING = TL::OFF_STAGING, OFF_MISC = TL::OFF_MISC, STAGE_WARP_BYTES = TL::STAGE_WARP_BYTES;
   constexpr int BN = TL::BN, BNH = TL::BNH, STAGES = TL::STAGES;
   constexpr uint32_t STAGE_BYTES = TL::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
@@ -288,11 +320,13 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
   auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 + s); };
   const uint32_t ready_bar = bar_base + 8u * (2 * STAGES + 4), got_bar = bar_base + 8u * (2 * STAGES + 5);
+  auto pairs_bar = [&](int q, int half) { return bar_base + 8u * (2 * STAGES + 7 + 2 * q + half); };  // EPI_DSWIGLU
 
   if (warp == 0) {
     if (lane < 2 * STAGES) mbar_init(bar_base + 8u * lane, 1);                             // full, empty
     if (lane >= 16 && lane < 20) mbar_init(tfull_bar(lane - 16), lane < 18 ? 1 : 2 * 4);  // tfull, tempty (one arrival a warp)
     if (lane == 20) *abort_flag = 0;
+    if (EPI == EPI_DSWIGLU && lane >= 24) mbar_init(pairs_bar(0, lane - 24), 1);
     if (SPLIT && lane == 21) mbar_init(ready_bar, S - 1);
     if (SPLIT && lane == 22) mbar_init(got_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -300,7 +334,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     if (lane == 0) {
       prefetch_map(&tmA);
       prefetch_map(&tmB);
-      if (p.tma_out) prefetch_map(&tmC);
+      if (p.tma_out && EPI != EPI_DSWIGLU) prefetch_map(&tmC);
       if (p.tma_out && p.aux != nullptr) prefetch_map(&tmAux);
     }
     __syncwarp();
@@ -513,19 +547,102 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     int acc = 0;
     uint32_t acc_phase = 0;
     const bool vec_ok = p.out_fp32 ? ((p.ldc & 3) == 0) : ((p.ldc & 7) == 0);
+    uint32_t pairs_phase = 0;  // EPI_DSWIGLU: bit h, of half h
     for (Work w = first; have_work(w); next_work(w)) {
       if (w.t != pair_id) tile_coords(w.t, m0, n0);
+      if constexpr (EPI == EPI_DSWIGLU) {
+        // 64 columns at a time: the 128 gate/up columns they belong to come by TMA, two pieces ahead (the first two under the
+        // tile's products), are replaced in place by their gradients, and leave by TMA.
+        const int row0 = m0 + q * 32;
+        const uint32_t stg = OFF_STAGING + q * STAGE_WARP_BYTES;
+        auto inside = [&](int c) { return n0 + c * 64 < p.N && row0 < p.M; };
+        auto fetch = [&](int c) {
+          mbar_expect_tx(pairs_bar(q, c & 1), STAGE_WARP_BYTES / 2);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            tma_load_2d(smem_base + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + h * 4096, &tmAux, pairs_bar(q, c & 1),
+                        2 * (n0 + c * 64) + 64 * h, row0);
+        };
+        if (lane == 0) {
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tile before has left the staging area
+          if (inside(0)) fetch(0);
+          if (inside(1)) fetch(1);
+        }
+        __syncwarp();
+        if (!mbar_wait_warp(tfull_bar(acc), acc_phase, abort_flag)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t taddr0 = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
+        bool ok = true;
+#pragma unroll 1
+        for (int c = 0; c < BN / 64; ++c) {
+          uint32_t v[64];
+          tmem_ld32(taddr0 + c * 64, v);
+          tmem_ld32(taddr0 + c * 64 + 32, v + 32);
+          if (c > 0 && c + 1 < BN / 64 && lane == 0 && inside(c + 1)) {
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // piece c - 1 has left
+            fetch(c + 1);
+          }
+          __syncwarp();
+          tmem_wait_ld();
+          if (c + 1 == BN / 64) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), lead_cta));
+          }
+          if (!inside(c)) continue;
+          if (!mbar_wait_warp(pairs_bar(q, c & 1), (pairs_phase >> (c & 1)) & 1u, abort_flag)) {
+            ok = false;
+            break;
+          }
+          pairs_phase ^= 1u << (c & 1);
+          uint8_t* prow = smem + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + lane * 128;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            ftb200::bf16x8* at = reinterpret_cast<ftb200::bf16x8*>(prow + (j >> 3) * 4096 + (((j & 7) ^ (lane & 7)) << 4));
+            float f[8], o[8];
+            ftb200::unpack8(*at, f);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float d = __uint_as_float(v[4 * j + e]), g = f[2 * e], u = f[2 * e + 1];
+              const float sg = 1.f / (1.f + __expf(-g));
+              const float silu = g * sg;
+              o[2 * e] = d * u * (sg + silu * (1.f - sg));
+              o[2 * e + 1] = d * silu;
+            }
+            *at = ftb200::pack8(o);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              if (n0 + c * 64 + 32 * h < p.N)
+                tma_store_2d(&tmAux, smem_base + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + h * 4096, 2 * (n0 + c * 64) + 64 * h, row0);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+        if (!ok) break;
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1u;
+        }
+        continue;
+      }
       if (!mbar_wait_warp(tfull_bar(acc), acc_phase, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row = m0 + q * 32 + lane;
       const uint32_t taddr0 = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
       const uint32_t stg = OFF_STAGING + q * STAGE_WARP_BYTES;
-      if (p.tma_out && !(SPLIT && w.shared)) {
+      if (EPI == EPI_LOSS || EPI == EPI_ROPE || (p.tma_out && !(SPLIT && w.shared))) {
         // bf16 output: 64 columns at a time go, one row a thread, into a 128-byte-swizzled piece of the warp's staging area
         // and leave by TMA (which clips what lies beyond M and N), while the next 64 come out of tensor memory.  Nothing hides
         // the last tile's epilogue: 5800 cycles for 256 columns that leave a row-major staging area as row segments, 4100
         // this way, all in all 14.2 -> 12.6 us for 3000 x 1536 x 1024, 17.3 -> 14.5 us for 1024 x 1024 x 3000.
         constexpr int PIECES = BN / 64;
+        float row_max = -INFINITY, row_sum = 0.f;  // EPI_LOSS: over the tile's columns
+        long long target = -1;
+        if (EPI == EPI_LOSS && row < p.M) target = p.target[row];
+        const int rope_pos = EPI == EPI_ROPE ? (m0 + q * 32) % p.rope_seq : 0;  // of the warp's first row
         uint32_t r[2][64];
         tmem_ld32(taddr0, r[0]);
         tmem_ld32(taddr0 + 32, r[0] + 32);
@@ -543,7 +660,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
           const uint32_t* v = r[c & 1];
           const bool inside = n0 + c * 64 < p.N && m0 + q * 32 < p.M;
           // With an activation the two halves of the area are one for C and one for 64 columns of aux, which two pieces fill.
-          const bool with_aux = p.aux != nullptr;
+          const bool with_aux = EPI == EPI_STORE && p.aux != nullptr;
           const uint32_t piece = with_aux ? stg : stg + (c & 1) * (STAGE_WARP_BYTES / 2);
           if (lane == 0) {  // what was stored from this half last has been read
             if (with_aux)
@@ -563,21 +680,67 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
             *reinterpret_cast<ftb200::bf16x8*>(prow + ((j ^ (lane & 7)) << 4)) = packed;
             if (with_aux) *reinterpret_cast<uint2*>(arow + ((((c & 1) * 4 + (j >> 1)) ^ (lane & 7)) << 4) + (j & 1) * 8) = silu_mul(packed);
           }
+          if (EPI == EPI_ROPE && n0 + c * 64 < p.rope_cols) {
+            // The rounded values are rotated, as by a kernel of its own; eight lanes a row, so that the table is read in whole
+            // lines (a row a lane asks for 32 of them with every load: 3000 x 1536 x 1024 24 us).
+            __syncwarp();
+            const int seg = lane & 7, off = (n0 + c * 64) % p.rope_dim / 4 + 2 * seg;
+#pragma unroll 4
+            for (int it = 0; it < 8; ++it) {
+              const int rr = it * 4 + (lane >> 3);
+              int pos = rope_pos + rr;
+              if (pos >= p.rope_seq) pos %= p.rope_seq;
+              const float4* cs = p.rope + static_cast<long long>(pos) * (p.rope_dim / 4) + off;
+              ftb200::bf16x8* at = reinterpret_cast<ftb200::bf16x8*>(smem + piece + rr * 128 + ((seg ^ (rr & 7)) << 4));
+              *at = rotate_pairs(*at, cs[0], cs[1]);
+            }
+          }
+          if (EPI == EPI_LOSS && inside) {
+            // of the rounded values, as they are stored; columns beyond N are left out
+            const int left = p.N - (n0 + c * 64);
+            float f[8], top = row_max;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              if (8 * j < left) {  // N is a multiple of 8
+                ftb200::unpack8(*reinterpret_cast<const ftb200::bf16x8*>(prow + ((j ^ (lane & 7)) << 4)), f);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) top = fmaxf(top, f[e]);
+              }
+            }
+            const float base = top == -INFINITY ? 0.f : top;
+            row_sum *= __expf(row_max - base);
+            row_max = top;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              if (8 * j < left) {
+                ftb200::unpack8(*reinterpret_cast<const ftb200::bf16x8*>(prow + ((j ^ (lane & 7)) << 4)), f);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) row_sum += __expf(f[e] - base);
+              }
+            }
+            const long long at = target - (n0 + c * 64);
+            if (at >= 0 && at < 64 && at < left)
+              p.target_value[row] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(
+                  prow + (((static_cast<int>(at) >> 3) ^ (lane & 7)) << 4) + (at & 7) * 2));
+          }
           fence_async_smem();
           __syncwarp();
-          if (lane == 0 && inside) {
+          if (EPI != EPI_LOSS && lane == 0 && inside) {
             tma_store_2d(&tmC, smem_base + piece, n0 + c * 64, m0 + q * 32);
             if (with_aux && ((c & 1) || n0 + (c + 1) * 64 >= p.N))
               tma_store_2d(&tmAux, smem_base + stg + STAGE_WARP_BYTES / 2, (n0 + (c & ~1) * 64) >> 1, m0 + q * 32);
           }
           if (lane == 0) asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
+        if (EPI == EPI_LOSS && row < p.M)
+          p.row_stats[static_cast<long long>(row) * num_n + n0 / BN] = make_float2(row_max, row_sum);
         if (++acc == 2) {
           acc = 0;
           acc_phase ^= 1u;
         }
         continue;
       }
+      if constexpr (EPI != EPI_STORE) continue;
       auto store_chunk = [&](int c, const uint32_t* r) {  // 32 columns of the thread's row
         const int col0 = n0 + c * 32;
         if (row < p.M && col0 < p.N) {
@@ -805,6 +968,15 @@ struct ScatterSpec {
   void* const* peers = nullptr;
 };
 
+struct EpilogueSpec {
+  int kind = EPI_STORE;
+  float2* row_stats = nullptr;
+  float* target_value = nullptr;
+  const long long* target = nullptr;
+  const float4* rope = nullptr;
+  int rope_cols = 0, rope_seq = 1, rope_dim = 64;
+};
+
 struct GatherSpec {
   int world = 0;
   long long shard = 0;
@@ -813,22 +985,22 @@ struct GatherSpec {
   unsigned int* sync = nullptr;
 };
 
-template <int BN, bool SPLIT>
+template <int BN, bool SPLIT, int EPI>
 static cudaError_t prepare_2cta() {
   static std::atomic<bool> done{false};
   if (done.load(std::memory_order_acquire)) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+  const cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT, EPI>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN, EPI>::SMEM_BYTES);
   if (e == cudaSuccess) done.store(true, std::memory_order_release);
   return e;
 }
 
 static void cluster_launch(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int ctas, int pairs_per_cluster, int threads,
-                           cudaStream_t stream) {
+                           uint32_t smem, cudaStream_t stream) {
   cfg = cudaLaunchConfig_t{};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = 2 * pairs_per_cluster;
@@ -847,9 +1019,9 @@ static int resident_clusters(int split) {
   if (n == 0) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
-    cluster_launch(cfg, attr, 2 * split, split, NUM_THREADS, nullptr);
-    if (prepare_2cta<BN, true>() != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, gemm_bf16_tcgen05_2cta_kernel<BN, true>, &cfg) != cudaSuccess || n <= 0) {
+    cluster_launch(cfg, attr, 2 * split, split, NUM_THREADS, Tile<BN, EPI_STORE>::SMEM_BYTES, nullptr);
+    if (prepare_2cta<BN, true, EPI_STORE>() != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_bf16_tcgen05_2cta_kernel<BN, true, EPI_STORE>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = -1;
     }
@@ -899,7 +1071,7 @@ static TilePlan plan_tiles(int M, int N, int K, int pairs, bool may_split) {
   return best;
 }
 
-template <int BN, bool SPLIT>
+template <int BN, bool SPLIT, int EPI>
 static int launch_2cta(const void* A, const void* B, long long lda, long long ldb, int ctas, int split, int threads,
                        const GemmParams& p, cudaStream_t stream) {
   CUtensorMap tmA, tmB, tmC, tmAux;
@@ -916,23 +1088,24 @@ static int launch_2cta(const void* A, const void* B, long long lda, long long ld
   if (rc) return rc;
   tmC = tmAux = tmA;  // not used without tma_out
   if (p.tma_out) {
-    rc = encode_2d(&tmC, p.C, p.M, p.N, p.ldc, 64, 32);
-    if (rc == 0 && p.aux != nullptr) rc = encode_2d(&tmAux, p.aux, p.M, p.N / 2, p.ld_aux, 64, 32);
+    if (p.C != nullptr) rc = encode_2d(&tmC, p.C, p.M, p.N, p.ldc, 64, 32);
+    if (rc == 0 && p.aux != nullptr)
+      rc = encode_2d(&tmAux, p.aux, p.M, EPI == EPI_DSWIGLU ? 2 * p.N : p.N / 2, p.ld_aux, 64, 32);
     if (rc) return rc;
   }
-  if (prepare_2cta<BN, SPLIT>() != cudaSuccess) return FTB200_E_CUDA;
+  if (prepare_2cta<BN, SPLIT, EPI>() != cudaSuccess) return FTB200_E_CUDA;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr;
-  cluster_launch(cfg, attr, SPLIT ? ctas : std::min(2 * tiles, ctas), split, threads, stream);
-  return cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT>, tmA, tmB, tmC, tmAux, p) == cudaSuccess ? 0 : FTB200_E_CUDA;
+  cluster_launch(cfg, attr, SPLIT ? ctas : std::min(2 * tiles, ctas), split, threads, Tile<BN, EPI>::SMEM_BYTES, stream);
+  return cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT, EPI>, tmA, tmB, tmC, tmAux, p) == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, int b_mn_major,
                           long long lda, long long ldb, long long ldc, int flags, int* status, int max_ctas, void* aux,
                           long long ld_aux, cudaStream_t stream, const ScatterSpec* sc = nullptr,
-                          const GatherSpec* ga = nullptr) {
-  if (M <= 0 || N <= 0 || K <= 0 || A == nullptr || B == nullptr || (C == nullptr && sc == nullptr)) return FTB200_E_BADARG;
+                          const GatherSpec* ga = nullptr, const EpilogueSpec* ep = nullptr) {
+  if (M <= 0 || N <= 0 || K <= 0 || A == nullptr || B == nullptr || (C == nullptr && sc == nullptr && ep == nullptr)) return FTB200_E_BADARG;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
     return FTB200_E_ALIGN;
   if ((reinterpret_cast<uintptr_t>(C) & 15)) return FTB200_E_ALIGN;
@@ -947,6 +1120,13 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   p.status = status;
   p.aux = aux;
   p.ld_aux = ld_aux;
+  p.row_stats = ep != nullptr ? ep->row_stats : nullptr;
+  p.target_value = ep != nullptr ? ep->target_value : nullptr;
+  p.target = ep != nullptr ? ep->target : nullptr;
+  p.rope = ep != nullptr ? ep->rope : nullptr;
+  p.rope_cols = ep != nullptr ? ep->rope_cols : 0;
+  p.rope_seq = ep != nullptr ? ep->rope_seq : 1;
+  p.rope_dim = ep != nullptr ? ep->rope_dim : 64;
   p.sc_world = 0;
   p.sc_src = 0;
   p.sc_shard = 0;
@@ -987,16 +1167,31 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   }
   int ctas = ftb200::sm_count() & ~1;
   if (max_ctas > 0 && max_ctas < ctas) ctas = std::max(2, max_ctas & ~1);
-  if (ga != nullptr) return launch_2cta<256, false>(A, B, lda, ldb, ctas, 1, NUM_THREADS_GATHER, p, stream);
+  if (ga != nullptr) return launch_2cta<256, false, EPI_STORE>(A, B, lda, ldb, ctas, 1, NUM_THREADS_GATHER, p, stream);
+  if (ep != nullptr) {
+    p.tma_out = 1;  // the entry has looked at what TMA wants
+    const bool narrow = plan_tiles(M, N, K, ctas / 2, false).columns == 128;
+    switch (ep->kind) {
+      case EPI_DSWIGLU:
+        return narrow ? launch_2cta<128, false, EPI_DSWIGLU>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
+                      : launch_2cta<256, false, EPI_DSWIGLU>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+      case EPI_LOSS:
+        return narrow ? launch_2cta<128, false, EPI_LOSS>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
+                      : launch_2cta<256, false, EPI_LOSS>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+      default:
+        return narrow ? launch_2cta<128, false, EPI_ROPE>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
+                      : launch_2cta<256, false, EPI_ROPE>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+    }
+  }
   // scattered and activated outputs leave through the staging area, which a shared tile does not
   const TilePlan plan = plan_tiles(M, N, K, ctas / 2, sc == nullptr && aux == nullptr && max_ctas <= 0);
   p.whole = plan.whole;
   if (plan.split > 1) {
-    if (plan.columns == 128) return launch_2cta<128, true>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
-    return launch_2cta<256, true>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
+    if (plan.columns == 128) return launch_2cta<128, true, EPI_STORE>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
+    return launch_2cta<256, true, EPI_STORE>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
   }
-  if (plan.columns == 128) return launch_2cta<128, false>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
-  return launch_2cta<256, false>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+  if (plan.columns == 128) return launch_2cta<128, false, EPI_STORE>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+  return launch_2cta<256, false, EPI_STORE>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
 }
 
 FTB200_API int ftb200_gemm_bf16_2cta(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major,
@@ -1013,6 +1208,70 @@ FTB200_API int ftb200_gemm_bf16_swiglu(const void* A, const void* B, void* C, vo
                                        cudaStream_t stream) {
   if (aux == nullptr || (N % 32) || (ldc & 7) || (ld_aux & 3) || (reinterpret_cast<uintptr_t>(aux) & 7)) return FTB200_E_ALIGN;
   return gemm_2cta_impl(A, B, C, M, N, K, 0, 0, lda, ldb, ldc, 0, status, max_ctas, aux, ld_aux, stream);
+}
+
+static bool aligned16(const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; }
+
+// C[M,N] = A[M,K] . B[N,K]^T with the first `heads` heads of `head_dim` columns rotated: the pair (2i, 2i+1) of a head by the
+// angle whose (cos, sin) is cos_sin[row % seq][i], after rounding to bf16 (as ftb200_rope does it to a stored C).  head_dim a
+// multiple of 64, N and ldc of 8.
+FTB200_API int ftb200_gemm_bf16_rope(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                                     long long ldc, const float* cos_sin, int seq, int heads, int head_dim, int* status,
+                                     cudaStream_t stream) {
+  if (cos_sin == nullptr || seq <= 0 || heads < 0 || head_dim <= 0 || static_cast<long long>(heads) * head_dim > N) return FTB200_E_BADARG;
+  if (head_dim % 64 || (N & 7) || (ldc & 7) || ldc < N || !aligned16(C) || !aligned16(cos_sin)) return FTB200_E_ALIGN;
+  EpilogueSpec ep;
+  ep.kind = EPI_ROPE;
+  ep.rope = reinterpret_cast<const float4*>(cos_sin);
+  ep.rope_cols = heads * head_dim;
+  ep.rope_seq = seq;
+  ep.rope_dim = head_dim;
+  return gemm_2cta_impl(A, B, C, M, N, K, 0, 0, lda, ldb, ldc, 0, status, 0, nullptr, 0, stream, nullptr, nullptr, &ep);
+}
+
+// Backward of a gated MLP's down projection and activation: D[M,N] = dY[M,K] . W[K,N] (W row-major, as it is stored for the
+// forward product) is the gradient of silu(gate) * up and is not stored; gu [M, 2 N], the interleaved (gate, up) pairs of
+// the forward pass, is overwritten by their gradients.  N and ld_gu multiples of 8.
+FTB200_API int ftb200_gemm_bf16_dswiglu(const void* dY, const void* W, void* gu, int M, int N, int K, long long ld_dy,
+                                        long long ld_w, long long ld_gu, int* status, cudaStream_t stream) {
+  if (gu == nullptr) return FTB200_E_BADARG;
+  if ((N & 7) || (ld_gu & 7) || ld_gu < 2LL * N || !aligned16(gu)) return FTB200_E_ALIGN;
+  if (N > 0x3fffffff) return FTB200_E_TOOBIG;
+  EpilogueSpec ep;
+  ep.kind = EPI_DSWIGLU;
+  return gemm_2cta_impl(dY, W, nullptr, M, N, K, 0, 1, ld_dy, ld_w, N, 0, status, 0, gu, ld_gu, stream, nullptr, nullptr, &ep);
+}
+
+// Floats of scratch memory for ftb200_gemm_bf16_loss.
+FTB200_API long long ftb200_gemm_bf16_loss_scratch_floats(int M, int N) {
+  if (M <= 0 || N <= 0) return 0;
+  const int columns = plan_tiles(M, N, 1, ftb200::sm_count() / 2, false).columns;
+  return static_cast<long long>(M) * (2LL * ((N + columns - 1) / columns) + 1);
+}
+
+int ftb200_launch_cross_entropy_rows(const long long* target, const float2* row_stats, const float* target_value, float* loss,
+                                     int tiles, int T, int V, cudaStream_t st);
+
+// Cross-entropy of logits = A[M,K] . B[N,K]^T against target [M], which are not stored: loss[row] = logsumexp - logit of the
+// target (0 for a negative target, a target beyond N counts as logit 0), of the logits rounded to bf16.  The product's epilogue
+// notes every row's maximum, sum of exponentials and target value per tile in `scratch`
+// (ftb200_gemm_bf16_loss_scratch_floats, 8-byte aligned); a second kernel finishes the rows.  1024 x 128256 x 2048: 474 us with
+// the logits stored and read again, 346 without.  (With gradients the logits have to be stored, and reading them once instead
+// of twice gains nothing at 8192 rows: 7335 us either way at K = 4096.)  N a multiple of 8.
+FTB200_API int ftb200_gemm_bf16_loss(const void* A, const void* B, int M, int N, int K, long long lda, long long ldb,
+                                     const long long* target, float* loss, float* scratch, int* status, cudaStream_t stream) {
+  if (target == nullptr || loss == nullptr || scratch == nullptr || M <= 0 || N <= 0) return FTB200_E_BADARG;
+  if ((N & 7) || (reinterpret_cast<uintptr_t>(scratch) & 7)) return FTB200_E_ALIGN;
+  const int columns = plan_tiles(M, N, K, ftb200::sm_count() / 2, false).columns;
+  const int tiles = (N + columns - 1) / columns;
+  EpilogueSpec ep;
+  ep.kind = EPI_LOSS;
+  ep.row_stats = reinterpret_cast<float2*>(scratch);
+  ep.target_value = scratch + 2LL * M * tiles;
+  ep.target = target;
+  const int rc = gemm_2cta_impl(A, B, nullptr, M, N, K, 0, 0, lda, ldb, N, 0, status, 0, nullptr, 0, stream, nullptr, nullptr, &ep);
+  if (rc != 0) return rc;
+  return ftb200_launch_cross_entropy_rows(target, ep.row_stats, ep.target_value, loss, tiles, M, N, stream);
 }
 
 // GEMM whose epilogue is the reduce-scatter's transfer: the [M,N] result (row-major, row

@@ -152,6 +152,8 @@ class Tcgen05Attention:
     place from the packed QKV activation and dQ, dK, dV are written in place into the packed
     dQKV workspace; only the per-row log-sum-exp is saved between the passes."""
 
+    rotates_back = True  # backward() takes the rotation of q and k
+
     def __init__(self, cfg: LlamaConfig):
         self.cfg = cfg
         self._saved: Dict[int, Tuple[torch.Tensor, ...]] = {}
@@ -173,7 +175,8 @@ class Tcgen05Attention:
             self._saved[layer] = (qkv, out, lse)
         K.attention_fwd(q, k, v, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, out, lse, causal=True)
 
-    def backward(self, layer: int, dout: torch.Tensor, batch: int, seq: int, dqkv: torch.Tensor) -> None:
+    def backward(self, layer: int, dout: torch.Tensor, batch: int, seq: int, dqkv: torch.Tensor,
+                 rope: Optional[torch.Tensor] = None) -> None:
         c = self.cfg
         qkv, out, lse = self._saved.pop(layer)
         q, k, v = self._views(qkv)
@@ -182,7 +185,7 @@ class Tcgen05Attention:
         if self._scratch is None or self._scratch.numel() < need:
             self._scratch = torch.empty(need, dtype=torch.uint8, device=qkv.device)
         K.attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, causal=True,
-                        scratch=self._scratch)
+                        scratch=self._scratch, rope=rope)
         self._lse_pool.append(lse)
 
     def reset(self) -> None:
@@ -274,6 +277,7 @@ class LlamaEngine:
         self.ws_dqkv = torch.empty(T, QKV, **bf)
         self.logits = torch.empty(T // self.logit_chunks, cfg.vocab_size, **bf)
         self.loss_rows = torch.empty(T, **f32)
+        self.loss_scratch: Optional[torch.Tensor] = None  # of evaluations, kept between them
         self.rope = K.rope_table(seq_len, cfg.head_dim, cfg.rope_theta, device)
         self.kernel_launches = 0
         # The normalised inputs of the QKV and gate/up GEMMs are needed again by their weight gradients.  They are
@@ -400,8 +404,7 @@ class LlamaEngine:
             else:
                 K.rmsnorm_fwd(self.h[l - 1], W.attn_norm, c.norm_eps, res=delta, h_out=self.x[l], out=n1,
                               rstd=self.rstd1[l])
-            K.linear_fwd(n1, W.wqkv, out=self.qkv[l])
-            K.rope_(self.qkv[l], self.rope, S, c.n_heads + c.n_kv_heads, c.head_dim)
+            K.linear_rope_fwd(n1, W.wqkv, self.qkv[l], self.rope, S, c.n_heads + c.n_kv_heads, c.head_dim)
             self.attn.forward(l, self.qkv[l], B, S, self.att[l], train)
             K.linear_fwd(self.att[l], W.wo, out=self.ws_proj)
             K.rmsnorm_fwd(self.x[l], W.ffn_norm, c.norm_eps, res=self.ws_proj, h_out=self.h[l], out=n2,
@@ -424,10 +427,12 @@ class LlamaEngine:
         tgt = targets.reshape(-1)
         G = self._g(u) if train else None
         rows = T // self.logit_chunks
+        if not train and self.loss_scratch is None and self.device.type == "cuda":
+            self.loss_scratch = torch.empty(K.linear_loss_scratch_floats(rows, c.vocab_size), dtype=torch.float32, device=self.device)
         for ci in range(self.logit_chunks):
             sl = slice(ci * rows, (ci + 1) * rows)
-            K.linear_fwd(self.ws_n[sl], W.lm_head, out=self.logits)
-            K.cross_entropy_(self.logits, tgt[sl], self.grad_scale / T, loss=self.loss_rows[sl], grad=train)
+            K.linear_cross_entropy_(self.ws_n[sl], W.lm_head, tgt[sl], self.grad_scale / T, self.logits, self.loss_rows[sl],
+                                    grad=train, scratch=self.loss_scratch)
             if train:
                 K.linear_wgrad(self.logits, self.ws_n[sl], out=G.lm_head, accumulate=ci > 0)
                 K.linear_dgrad(self.logits, getattr(W.lm_head, "local", W.lm_head), out=self.ws_dn[sl])
@@ -450,8 +455,7 @@ class LlamaEngine:
             W, G = self._p(u), self._g(u)
             # ---- FFN
             self._wgrad(l, "wd", dy, self.s[l], G.wd, reads=("dy",))
-            K.linear_dgrad(dy, W.wd, out=self.ws_ds)
-            K.swiglu_bwd(self.ws_ds, self.gu[l], dgu=self.gu[l])
+            K.linear_dswiglu_(dy, W.wd, self.gu[l], self.ws_ds)
             if self.n2 is not None:
                 self._wgrad(l, "wgu", self.gu[l], self.n2[l], G.wgu, reads=())
             else:
@@ -465,8 +469,11 @@ class LlamaEngine:
             self._wgrad(l, "wo", self.ws_dh, self.att[l], G.wo, reads=("ws_dh",))
             K.linear_dgrad(self.ws_dh, W.wo, out=self.ws_dn)
             self._before_overwrite("ws_dqkv")
-            self.attn.backward(l, self.ws_dn, B, S, self.ws_dqkv)
-            K.rope_(self.ws_dqkv, self.rope, S, c.n_heads + c.n_kv_heads, c.head_dim, backward=True)
+            if getattr(self.attn, "rotates_back", False):
+                self.attn.backward(l, self.ws_dn, B, S, self.ws_dqkv, rope=self.rope)
+            else:
+                self.attn.backward(l, self.ws_dn, B, S, self.ws_dqkv)
+                K.rope_(self.ws_dqkv, self.rope, S, c.n_heads + c.n_kv_heads, c.head_dim, backward=True)
             if self.n1 is not None:
                 self._wgrad(l, "wqkv", self.ws_dqkv, self.n1[l], G.wqkv, reads=("ws_dqkv",))
             else:

@@ -53,9 +53,10 @@ def _status_ptr(device: torch.device) -> int:
 _ARGS = {
     "embedding_fwd": "pppiiip", "embedding_bwd": "pppiiip", "rmsnorm_fwd": "ppppppiifp", "rmsnorm_bwd": "ppppppppiiip",
     "rope": "ppliiilip", "swiglu_fwd": "pplip", "swiglu_bwd": "ppplip", "gemm_bf16_swiglu": "ppppiiillllpip",
+    "gemm_bf16_rope": "pppiiilllpiiipp", "gemm_bf16_dswiglu": "pppiiilllpp", "gemm_bf16_loss": "ppiiillppppp",
     "cross_entropy": "pppiilfip", "adamw": "ppppiplfffffipp", "sumsq": "pilpp", "clip_coef": "pfppp",
     "attention_fwd": "pppppiiiiillllfipp", "attention_fwd2": "pppppiiiiillllfiipp",
-    "attention_bwd": "ppppppppppiiiiillllllllfipp", "gemm_bf16": "pppiiiiilllipip",
+    "attention_bwd": "ppppppppppiiiiillllllllfippp", "gemm_bf16": "pppiiiiilllipip",
 }
 _ARGS["gemm_bf16_2cta"] = _ARGS["gemm_bf16"]
 _KIND = {"p": c_void_p, "i": c_int, "l": c_ll, "f": c_float}
@@ -439,6 +440,50 @@ def ref_swiglu_bwd(ds, gu):
     return out.to(gu.dtype)
 
 
+def linear_rope_fwd(x: torch.Tensor, w, out: torch.Tensor, table: torch.Tensor, seq_len: int, n_heads: int, head_dim: int) -> None:
+    """``out = x @ w^T`` with the first ``n_heads`` heads of its rows rotated (:func:`linear_fwd` and :func:`rope_`), in one
+    kernel where the heads are whole 64-column pieces of the product's epilogue and there are more than two waves of tiles: the
+    table's way into the last tile's epilogue is hidden by nothing.  8192 x 6144 x 4096 289 -> 256 us, 4096 x 3072 x 2048 83 -> 76;
+    1536 x 6144 x 4096 (144 tiles on 74 CTA pairs) 95 -> 96, 1024 x 3072 x 2048 34 -> 40."""
+    weight = w if not isinstance(w, GatherField) else None if w.pending else w.local
+    if (weight is None or not x.is_cuda or -(-out.shape[0] // 256) * -(-out.shape[1] // 256) <= _sm_count(x.device.index) or GEMM_IMPL != "2cta" or head_dim % 64 or out.shape[1] % 8 or out.stride(0) % 8
+            or out.data_ptr() % 16 or table.data_ptr() % 16 or out.shape[0] < 1 or out.stride(0) < out.shape[1]):
+        linear_fwd(x, w, out=out)
+        rope_(out, table, seq_len, n_heads, head_dim)
+        return
+    for t, name in ((x, "x"), (weight, "w"), (out, "out")):
+        _check_2d_bf16(t, name)
+    T, Kd = x.shape
+    if weight.shape[1] != Kd or tuple(out.shape) != (T, weight.shape[0]):
+        raise ValueError(f"shape mismatch: x {tuple(x.shape)}, w {tuple(weight.shape)}, out {tuple(out.shape)}")
+    if table.dtype != torch.float32 or not table.is_contiguous() or table.shape[0] < seq_len or tuple(table.shape[1:]) != (head_dim // 2, 2):
+        raise ValueError("table must be rope_table() of the sequence and head dim")
+    N.check(_fn("gemm_bf16_rope")(x.data_ptr(), weight.data_ptr(), out.data_ptr(), T, weight.shape[0], Kd, x.stride(0),
+                                  weight.stride(0), out.stride(0), table.data_ptr(), seq_len, n_heads, head_dim,
+                                  _status_ptr(x.device), _stream()), "gemm_bf16_rope")
+
+
+def linear_dswiglu_(dy: torch.Tensor, w: torch.Tensor, gu: torch.Tensor, ds: torch.Tensor) -> None:
+    """Backward of the down projection ``silu(gate) * up @ w^T`` into ``gu``, which holds the interleaved (gate, up) pairs and
+    receives their gradients (:func:`linear_dgrad` into ``ds`` and :func:`swiglu_bwd` in place).  On the GPU it is one kernel
+    from a width of 2048 on, and ``ds`` stays as it is: the gradient of the activation goes from the accumulator into the pairs
+    without a rounding.  A product of fewer than 32 slabs does not hide the pairs' way in and out: 3000 rows, 2816 from 1024
+    columns 31.7 -> 32.8 us; 4096 rows, 8192 from 2048 188 -> 154; 8192 rows, 14336 from 4096 758 -> 660."""
+    T, F2 = gu.shape
+    if (not dy.is_cuda or dy.shape[1] < 2048 or GEMM_IMPL != "2cta" or F2 % 16 or gu.stride(0) % 8 or gu.data_ptr() % 16 or gu.stride(0) < F2 or T < 1):
+        if not gu.is_contiguous():
+            raise ValueError("gu must be contiguous")
+        linear_dgrad(dy, w, out=ds)
+        swiglu_bwd(ds, gu, dgu=gu)
+        return
+    for t, name in ((dy, "dy"), (w, "w"), (gu, "gu")):
+        _check_2d_bf16(t, name)
+    if dy.shape[0] != T or tuple(w.shape) != (dy.shape[1], F2 // 2):
+        raise ValueError(f"shape mismatch: dy {tuple(dy.shape)}, w {tuple(w.shape)}, gu {tuple(gu.shape)}")
+    N.check(_fn("gemm_bf16_dswiglu")(dy.data_ptr(), w.data_ptr(), gu.data_ptr(), T, F2 // 2, dy.shape[1], dy.stride(0), w.stride(0),
+                                     gu.stride(0), _status_ptr(dy.device), _stream()), "gemm_bf16_dswiglu")
+
+
 def swiglu_bwd(ds: torch.Tensor, gu: torch.Tensor, dgu: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``dgu`` may alias ``gu`` (in place)."""
     T, F2 = gu.shape
@@ -498,6 +543,42 @@ def cross_entropy_(logits: torch.Tensor, target: torch.Tensor, grad_scale: float
         _fn("cross_entropy")(_at(logits), _at(target), _at(loss), T, V, logits.stride(0), grad_scale, int(grad), _stream()),
         "cross_entropy",
     )
+    return loss
+
+
+def linear_loss_scratch_floats(rows: int, vocab: int) -> int:
+    """Size of the ``scratch`` that :func:`linear_cross_entropy_` takes."""
+    lib = N.lib()
+    lib.ftb200_gemm_bf16_loss_scratch_floats.restype = c_ll
+    return int(lib.ftb200_gemm_bf16_loss_scratch_floats(rows, vocab))
+
+
+def linear_cross_entropy_(x: torch.Tensor, w, target: torch.Tensor, grad_scale: float, logits: torch.Tensor, loss: torch.Tensor,
+                          grad: bool = True, scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """:func:`cross_entropy_` of the logits ``x @ w^T``.  With ``grad`` they end as their gradient in ``logits``; without it
+    ``logits`` is a workspace that may or may not hold them afterwards: on the GPU the product's epilogue notes the rows' maxima,
+    sums and target values (in fp32 ``scratch``, :func:`linear_loss_scratch_floats` of it or more) and they are not stored.  Not
+    for fewer than 2^20 of them, where the second kernel costs more than it spares: 64 x 1024 8.7 -> 9.6 us, 750 x 8192 28 -> 24."""
+    weight = w if not isinstance(w, GatherField) else None if w.pending else w.local
+    T, Kd = x.shape
+    V = logits.shape[1]
+    if grad or weight is None or not x.is_cuda or GEMM_IMPL != "2cta" or V % 8 or T * V < 1 << 20:
+        linear_fwd(x, w, out=logits)
+        return cross_entropy_(logits, target, grad_scale, loss=loss, grad=grad)
+    for t, name in ((x, "x"), (weight, "w"), (logits, "logits")):
+        _check_2d_bf16(t, name)
+    if tuple(weight.shape) != (V, Kd) or logits.shape[0] != T or target.numel() != T or loss.numel() != T:
+        raise ValueError(f"shape mismatch: x {tuple(x.shape)}, w {tuple(weight.shape)}, logits {tuple(logits.shape)}")
+    if target.dtype != torch.int64 or not target.is_contiguous() or loss.dtype != torch.float32 or not loss.is_contiguous():
+        raise ValueError("target must be contiguous int64, loss contiguous fp32")
+    need = linear_loss_scratch_floats(T, V)
+    if scratch is None:
+        scratch = torch.empty(need, dtype=torch.float32, device=x.device)
+    elif scratch.device != x.device or scratch.dtype != torch.float32 or scratch.numel() < need or not scratch.is_contiguous():
+        raise ValueError(f"scratch must be {need} contiguous fp32 on {x.device}")
+    N.check(_fn("gemm_bf16_loss")(x.data_ptr(), weight.data_ptr(), T, V, Kd, x.stride(0), weight.stride(0), target.data_ptr(),
+                                  loss.data_ptr(), scratch.data_ptr(), _status_ptr(x.device), _stream()), "gemm_bf16_loss",
+            launches=2)
     return loss
 
 
@@ -663,11 +744,13 @@ def attention_bwd_scratch_bytes(batch: int, seq_len: int, n_heads: int) -> int:
 def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor,
                   lse: torch.Tensor, dq: torch.Tensor, dk: torch.Tensor, dv: torch.Tensor, batch: int, seq_len: int,
                   n_heads: int, n_kv_heads: int, head_dim: int, causal: bool = True,
-                  scratch: Optional[torch.Tensor] = None) -> None:
+                  scratch: Optional[torch.Tensor] = None, rope: Optional[torch.Tensor] = None) -> None:
     """Backward of :func:`attention_fwd`: writes ``dq``, ``dk``, ``dv`` (2-D bf16 views like
     ``q``, ``k``, ``v``; column slices of a packed dQKV buffer are fine).  The fp32 dQ
     accumulator lives in ``scratch`` (bytes on the device, :func:`attention_bwd_scratch_bytes` of
-    them or more), by default a per-device buffer that is reused across calls on the same stream."""
+    them or more), by default a per-device buffer that is reused across calls on the same stream.
+    With ``rope``, the table (:func:`rope_table`) that ``q`` and ``k`` were rotated by, ``dq`` and ``dk``
+    are the gradients of the values before the rotation."""
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (o, "o"), (d_o, "d_o"), (dq, "dq"), (dk, "dk"), (dv, "dv")):
         _check_2d_bf16(t, name)
     if not q.is_cuda:
@@ -677,7 +760,13 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
         dq.copy_(gq.reshape(B * S, -1))
         dk.copy_(gk.reshape(B * S, -1))
         dv.copy_(gv.reshape(B * S, -1))
+        if rope is not None:
+            dq.copy_(ref_rope(dq, rope, S, n_heads, head_dim, backward=True))
+            dk.copy_(ref_rope(dk, rope, S, n_kv_heads, head_dim, backward=True))
         return
+    if rope is not None and (rope.dtype != torch.float32 or not rope.is_contiguous() or rope.device != q.device
+                             or rope.shape[0] < seq_len or tuple(rope.shape[1:]) != (head_dim // 2, 2)):
+        raise ValueError("rope must be the table of the sequence and head dim on the device of q")
     lib = N.lib()
     need = attention_bwd_scratch_bytes(batch, seq_len, n_heads)
     if scratch is None:
@@ -692,7 +781,7 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
     N.check(
         _fn("attention_bwd")(_at(q), _at(k), _at(v), _at(o), _at(d_o), _at(lse), _at(dq), _at(dk), _at(dv), _at(scratch),
                              batch, seq_len, n_heads, n_kv_heads, head_dim, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
-                             d_o.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), scale, int(causal), _status_ptr(q.device),
-                             _stream()),
+                             d_o.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), scale, int(causal), _at(rope),
+                             _status_ptr(q.device), _stream()),
         "attention_bwd", launches=3,
     )
