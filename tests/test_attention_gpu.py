@@ -172,6 +172,42 @@ def test_attention_bwd_tiles(B, S, Hq, Hkv, causal, scale, D):
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(2, 1, 2, 1), (3, 7, 1, 1), (2, 127, 2, 2), (2, 128, 2, 1), (2, 129, 4, 2), (1, 255, 2, 1),
+                                        (3, 257, 2, 2), (2, 384, 2, 1), (2, 385, 2, 1), (3, 1000, 8, 2)])
+def test_attention_of_any_length(B, S, Hq, Hkv, causal, D):
+    """Sequences that end inside a tile, next to each other in memory: what lies behind an end (the next sequence, NaN behind
+    the last one) neither enters nor is written over.  Tolerances as for whole tiles."""
+    n = (Hq + 2 * Hkv) * D
+    whole = torch.full((B * S + 300, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+    whole[: B * S] = _qkv(B, S, Hq, Hkv, D, seed=S)[0]
+    qkv = whole[: B * S]
+    q, k, v = qkv[:, : Hq * D], qkv[:, Hq * D : (Hq + Hkv) * D], qkv[:, (Hq + Hkv) * D :]
+    out = torch.full((B * S + 300, Hq * D), 7.0, dtype=torch.bfloat16, device="cuda")
+    lse = torch.full((B * Hq * S + 300,), 7.0, device="cuda")
+    with pytest.raises(K.N.KernelError) if S % 256 and (S % 128 or D == 64) else __import__("contextlib").nullcontext():
+        K.attention_fwd(q, k, v, B, S, Hq, Hkv, D, out[: B * S].clone(), None, causal=causal)  # refused unless asked for
+    K.attention_fwd(q, k, v, B, S, Hq, Hkv, D, out[: B * S], lse[: B * Hq * S].view(B, Hq, S), causal=causal, any_length=True)
+    d_o = torch.full_like(out, float("nan"))
+    d_o[: B * S] = torch.randn(B * S, Hq * D, device="cuda")
+    d = torch.full_like(whole, 7.0)
+    K.attention_bwd(q, k, v, out[: B * S], d_o[: B * S], lse[: B * Hq * S].view(B, Hq, S), d[: B * S, : Hq * D],
+                    d[: B * S, Hq * D : (Hq + Hkv) * D], d[: B * S, (Hq + Hkv) * D :], B, S, Hq, Hkv, D, causal=causal, any_length=True)
+    K.check_status(out.device)
+    for t, rows in ((out, B * S), (d, B * S), (lse, B * Hq * S)):
+        assert bool((t[rows:] == 7.0).all())
+    q4, k4, v4, do4 = (t.reshape(B, S, -1, D) for t in (q, k, v, d_o[: B * S]))
+    ref = K.ref_attention(q4.float(), k4.float(), v4.float(), causal).reshape(B * S, Hq * D)
+    assert (out[: B * S].float() - ref).norm() < 1e-2 * ref.norm()
+    torch.testing.assert_close(lse[: B * Hq * S].view(B, Hq, S), K.ref_attention_lse(q4, k4, v4, causal), rtol=1e-3, atol=2e-3)
+    want = torch.cat([w.reshape(B * S, -1) for w in K.ref_attention_bwd(q4, k4, v4, do4, causal)], dim=1)
+    if S > 1:  # a single key has no gradient but its value's
+        for a, b in ((0, Hq), (Hq, Hq + Hkv), (Hq + Hkv, Hq + 2 * Hkv)):
+            got, w = d[: B * S, a * D : b * D].float(), want[:, a * D : b * D]
+            assert (got - w).norm() < 2e-2 * w.norm()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
 def test_attention_bwd_rotates_back(D, causal):
     """dQ and dK of the values before the rotation: as the rotated ones turned back by a kernel of their own, which rounds once
     more (2^-9 of each value)."""

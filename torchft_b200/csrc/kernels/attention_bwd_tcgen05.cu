@@ -34,6 +34,10 @@
 // same in all lanes and the MMAs' descriptors stay in uniform registers (1494 -> 1437 us, 650 -> 605 us).
 // 1 x 8192, 32/8 heads of 128: 1705 us with 64-query tiles, 1290 us (1065 TFLOP/s) with these; 8 x 2048, heads of 64: 785 -> 592 us.
 //
+// Sequences of any length: the tensor maps have the sequence as a dimension of its own, so a tile's rows beyond its end are
+// zeros.  The statistics and the dQ accumulator are laid out for whole tiles; a query beyond the end has the log-sum-exp
+// +infinity there, so its probabilities are zero, and dQ, dK and dV beyond the end are not stored.
+//
 // Every mbarrier wait is bounded; on expiry the CTA records FTB200_ST_TIMEOUT in the caller's
 // status word, frees its TMEM and returns.
 #include <cuda.h>
@@ -108,8 +112,8 @@ struct BwdParams {
   int batch, seq, n_heads, n_kv_heads;
   int causal;
   float scale, scale_log2;
-  const float* neg_lse2;   // [batch, n_heads, seq], -log2(e) times the forward's log-sum-exp
-  const float* neg_delta;  // [batch, n_heads, seq], -scale times delta
+  const float* neg_lse2;   // [batch, n_heads, whole tiles of seq], -log2(e) times the forward's log-sum-exp
+  const float* neg_delta;  // the same, -scale times delta
   float* dq_acc;           // fp32, zeroed; per 128 queries and head: [D / 32][32 groups of 4 queries][32][4 queries]
   __nv_bfloat16* dK;   // rows batch*seq, row stride ld_dk
   __nv_bfloat16* dV;
@@ -172,10 +176,9 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int bh = static_cast<int>(blockIdx.x) % per_block;
   const int b = bh / p.n_kv_heads, hk = bh % p.n_kv_heads;
   const int rep = p.n_heads / p.n_kv_heads;
-  const int n_qtiles = p.seq / BQ;
+  const int n_qtiles = (p.seq + BQ - 1) / BQ;
   const int first_q = p.causal ? jb : 0;
   const int T = rep * (n_qtiles - first_q);
-  const int kv_row0 = b * p.seq + jb * BKV;
   // tiles in order: the queries of a head that see the block, then the next head of the group
   struct TileWalk {
     int h, qt;
@@ -225,8 +228,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         mbar_expect_tx(bar(BAR_KV), 2 * TILE);
 #pragma unroll
         for (int sl = 0; sl < SLABS; ++sl) {
-          tma_load_2d(smem_base + Ly::OFF_K + sl * SLAB, &tmK, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
-          tma_load_2d(smem_base + Ly::OFF_V + sl * SLAB, &tmV, bar(BAR_KV), hk * D + 64 * sl, kv_row0);
+          tma_load_3d(smem_base + Ly::OFF_K + sl * SLAB, &tmK, bar(BAR_KV), hk * D + 64 * sl, jb * BKV, b);
+          tma_load_3d(smem_base + Ly::OFF_V + sl * SLAB, &tmV, bar(BAR_KV), hk * D + 64 * sl, jb * BKV, b);
         }
       }
       __syncwarp();
@@ -236,8 +239,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const int st = t % STAGES;
         const uint32_t was = static_cast<uint32_t>(t / STAGES) & 1u ^ 1u;
         const int dst = t % Ly::DO_STAGES;
-        const int q_row0 = b * p.seq + w.qt * BQ;
-        const long long stat_off = (static_cast<long long>(b) * p.n_heads + w.h) * p.seq + w.qt * BQ;
+        const int q0 = w.qt * BQ;
+        const long long stat_off = ((static_cast<long long>(b) * p.n_heads + w.h) * n_qtiles + w.qt) * BQ;
         const uint32_t sq = smem_base + Ly::OFF_Q + st * TILE, sdo = smem_base + Ly::OFF_DO + dst * TILE;
         const uint32_t sst = smem_base + Ly::OFF_STATS + st * STATS_BYTES;
         if (!mbar_wait_warp(bar(BAR_Q_EMPTY + st), was, abort_flag)) {
@@ -248,7 +251,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           mbar_expect_tx(bar(BAR_Q_FULL + st), TILE + STATS_BYTES);
 #pragma unroll
           for (int sl = 0; sl < SLABS; ++sl)
-            tma_load_2d(sq + sl * SLAB, &tmQ, bar(BAR_Q_FULL + st), w.h * D + 64 * sl, q_row0);
+            tma_load_3d(sq + sl * SLAB, &tmQ, bar(BAR_Q_FULL + st), w.h * D + 64 * sl, q0, b);
           bulk_load_1d(sst, p.neg_lse2 + stat_off, BQ * 4, bar(BAR_Q_FULL + st));
           bulk_load_1d(sst + BQ * 4, p.neg_delta + stat_off, BQ * 4, bar(BAR_Q_FULL + st));
         }
@@ -261,7 +264,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           mbar_expect_tx(bar(BAR_DO_FULL + dst), TILE);
 #pragma unroll
           for (int sl = 0; sl < SLABS; ++sl)
-            tma_load_2d(sdo + sl * SLAB, &tmDO, bar(BAR_DO_FULL + dst), w.h * D + 64 * sl, q_row0);
+            tma_load_3d(sdo + sl * SLAB, &tmDO, bar(BAR_DO_FULL + dst), w.h * D + 64 * sl, q0, b);
         }
         __syncwarp();
       }
@@ -407,6 +410,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     TileWalk w{hk * rep, first_q};
     const uint32_t s_addr = tmem_base + Ly::COL_S + g * CPT + lane_addr;
     const uint32_t dp_addr = tmem_base + Ly::COL_DP + g * CPT + lane_addr;
+    const bool beyond = jb * BKV + row >= p.seq;  // this key
     uint8_t* drow = smem + Ly::OFF_DS + g * SLAB + row * 128;
     for (int t = 0; t < T && ok; ++t, next_tile(w)) {
       const uint32_t odd = static_cast<uint32_t>(t) & 1u;
@@ -445,6 +449,9 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
         for (int c = 0; c < CPT; ++c)
           if (row > g * CPT + c) pe[c] = 0.f;
+      } else if (beyond) {  // no causal mask leaves it out
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) pe[c] = 0.f;
       }
       {
         uint32_t pt[CPT / 2];
@@ -509,7 +516,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint32_t col = (which == 0 ? Ly::COL_DV : Ly::COL_DK) + g * CW;
         __nv_bfloat16* base = which == 0 ? p.dV : p.dK;
         const long long ld = which == 0 ? p.ld_dv : p.ld_dk;
-        __nv_bfloat16* dst = base + static_cast<long long>(kv_row0 + row) * ld + hk * D + g * CW;
+        __nv_bfloat16* dst = base + (static_cast<long long>(b) * p.seq + jb * BKV + row) * ld + hk * D + g * CW;
         uint32_t v[CW];
 #pragma unroll
         for (int c = 0; c < CW / 32; ++c) tmem_ld32(tmem_base + col + c * 32 + lane_addr, v + c * 32);
@@ -519,6 +526,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * c + e]);
+          if (beyond) continue;
           if (which == 1 && p.rope != nullptr) {
             const float4* cs = p.rope + static_cast<long long>(jb * BKV + row) * (D / 4) + g * (CW / 4) + 2 * c;
             rotate_back(f, cs[0], cs[1]);
@@ -539,7 +547,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }
 
 // Before the main kernel, one pass over O and dO: neg_delta[b, h, s] = -scale sum_d dO O, neg_lse2 = -log2(e) lse, and the dQ
-// accumulator zeroed.  A thread takes 8 elements (16 bytes of each), D / 8 neighbouring lanes a (row, head).
+// accumulator zeroed.  A thread takes 8 elements (16 bytes of each), D / 8 neighbouring lanes a (row, head); `pieces` counts the
+// rows of whole tiles.
 template <int D>
 __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
                                                                  const __nv_bfloat16* __restrict__ d_o,
@@ -551,24 +560,30 @@ __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bflo
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool live = i < pieces;
   const int per_row = n_heads * LANES;
-  const int r = static_cast<int>((live ? i : 0) / per_row);  // batch * seq rows fit an int (the host checks)
-  const int c = static_cast<int>((live ? i : 0) - static_cast<long long>(r) * per_row);
+  const int rt = static_cast<int>((live ? i : 0) / per_row);  // rows of whole tiles fit an int (the host checks)
+  const int c = static_cast<int>((live ? i : 0) - static_cast<long long>(rt) * per_row);
+  const int seq_t = (seq + BQ - 1) / BQ * BQ;
+  const int b = rt / seq_t, pos = rt - b * seq_t;
+  const bool inside = pos < seq;
+  const long long r = static_cast<long long>(b) * seq + pos;
   float s = 0.f;
   if (live) {
+    dq_acc[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    dq_acc[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (live && inside) {
     float x[8], y[8];
     ftb200::unpack8(*reinterpret_cast<const ftb200::bf16x8*>(o + r * ld_o + c * 8), x);
     ftb200::unpack8(*reinterpret_cast<const ftb200::bf16x8*>(d_o + r * ld_do + c * 8), y);
-    dq_acc[2 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    dq_acc[2 * i + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
   }
 #pragma unroll
   for (int k = LANES / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
   if (live && c % LANES == 0) {
-    const long long at = (static_cast<long long>(r / seq) * n_heads + c / LANES) * seq + r % seq;
-    neg_delta[at] = -s * scale;
-    neg_lse2[at] = lse[at] * -1.4426950408889634f;
+    const long long bh = static_cast<long long>(b) * n_heads + c / LANES;
+    neg_delta[bh * seq_t + pos] = inside ? -s * scale : 0.f;
+    neg_lse2[bh * seq_t + pos] = inside ? lse[bh * seq + pos] * -1.4426950408889634f : -INFINITY;
   }
 }
 
@@ -585,18 +600,22 @@ __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __
   const int q4 = static_cast<int>(g & 31);
   const long long th = g >> 5;
   const int h = static_cast<int>(th % n_heads);
-  const long long row0 = th / n_heads * 128 + q4 * 4;
+  const int n_qtiles = (seq + BQ - 1) / BQ;
+  const int tile = static_cast<int>(th / n_heads);
+  const int pos0 = tile % n_qtiles * BQ + q4 * 4;  // in its sequence
+  const long long row0 = static_cast<long long>(tile / n_qtiles) * seq + pos0;
   const float4* src = acc + th * (32 * D) + (d8 >> 2) * 1024 + q4 * 32 + (d8 & 3) * 8;
   float4 v[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) v[e] = src[e];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
+    if (pos0 + k >= seq) break;
     float f[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) f[e] = k == 0 ? v[e].x : k == 1 ? v[e].y : k == 2 ? v[e].z : v[e].w;
     if (rope != nullptr) {
-      const float4* cs = rope + (row0 + k) % seq * (D / 4) + d8 * 2;
+      const float4* cs = rope + static_cast<long long>(pos0 + k) * (D / 4) + d8 * 2;
       rotate_back(f, cs[0], cs[1]);
     }
     *reinterpret_cast<ftb200::bf16x8*>(dq + (row0 + k) * ld + h * D + d8 * 8) = ftb200::pack8(f);
@@ -618,14 +637,15 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
-int encode_rows(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows) {
+// [batch, seq, cols] bf16 view with row stride ld (elements); box = 64 columns x 128 rows, 128-byte swizzle
+int encode_rows(CUtensorMap* map, const void* base, long long batch, long long seq, long long cols, long long ld) {
   auto fn = encode_fn();
   if (fn == nullptr) return FTB200_E_DRIVER;
-  cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {64u, static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), gdim, gstride, box, estr,
+  cuuint64_t gdim[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(seq), static_cast<cuuint64_t>(batch)};
+  cuuint64_t gstride[2] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(seq) * ld * 2};
+  cuuint32_t box[3] = {64u, 128u, 1u};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : FTB200_E_DRIVER;
@@ -638,7 +658,7 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 // Scratch the backward pass needs, in bytes: fp32 dQ accumulator, -scale delta, -log2(e) lse.
 // (sized for head dim 128; enough for 64 as well)
 FTB200_API long long ftb200_attention_bwd_scratch_bytes(int batch, int seq, int n_heads) {
-  const long long rows = static_cast<long long>(batch) * seq;
+  const long long rows = static_cast<long long>(batch) * ((static_cast<long long>(seq) + BQ - 1) / BQ * BQ);
   return rows * n_heads * 128 * 4 + 2 * rows * n_heads * 4;
 }
 
@@ -651,16 +671,17 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
                        long long ld_dk, long long ld_dv, float scale, int causal, const float* cos_sin, int* status,
                        cudaStream_t stream) {
   constexpr uint32_t SMEM_BYTES = Lay<D>::SMEM_BYTES;
-  const long long rows = static_cast<long long>(batch) * seq;
+  const long long tiles = (static_cast<long long>(seq) + BQ - 1) / BQ;
+  const long long rows = batch * tiles * BQ;
   float* dq_acc = reinterpret_cast<float*>(scratch);
   float* neg_delta = dq_acc + rows * n_heads * D;
   float* neg_lse2 = neg_delta + rows * n_heads;
   if (rows > 0x7fffffffLL) return FTB200_E_TOOBIG;
   CUtensorMap tq, tk, tv, tdo;
-  int rc = encode_rows(&tq, q, rows, static_cast<long long>(n_heads) * D, ld_q, BQ);
-  if (rc == 0) rc = encode_rows(&tdo, d_o, rows, static_cast<long long>(n_heads) * D, ld_do, BQ);
-  if (rc == 0) rc = encode_rows(&tk, k, rows, static_cast<long long>(n_kv_heads) * D, ld_k, BKV);
-  if (rc == 0) rc = encode_rows(&tv, v, rows, static_cast<long long>(n_kv_heads) * D, ld_v, BKV);
+  int rc = encode_rows(&tq, q, batch, seq, static_cast<long long>(n_heads) * D, ld_q);
+  if (rc == 0) rc = encode_rows(&tdo, d_o, batch, seq, static_cast<long long>(n_heads) * D, ld_do);
+  if (rc == 0) rc = encode_rows(&tk, k, batch, seq, static_cast<long long>(n_kv_heads) * D, ld_k);
+  if (rc == 0) rc = encode_rows(&tv, v, batch, seq, static_cast<long long>(n_kv_heads) * D, ld_v);
   if (rc != 0) return rc;
   static bool attr_set = false;
   if (!attr_set) {
@@ -685,7 +706,7 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
   p.ld_dk = ld_dk; p.ld_dv = ld_dv; p.status = status;
   p.rope = reinterpret_cast<const float4*>(cos_sin);
-  const long long grid = static_cast<long long>(batch) * n_kv_heads * (seq / BKV);
+  const long long grid = static_cast<long long>(batch) * n_kv_heads * tiles;
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_bwd_kernel<D><<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
   attention_dq_cast_kernel<D><<<static_cast<unsigned>((pieces / 4 + 255) / 256), 256, 0, stream>>>(
@@ -707,7 +728,7 @@ FTB200_API int ftb200_attention_bwd(const void* q, const void* k, const void* v,
                                     long long ld_v, long long ld_o, long long ld_do, long long ld_dq, long long ld_dk,
                                     long long ld_dv, float scale, int causal, const float* cos_sin, int* status,
                                     cudaStream_t stream) {
-  if ((head_dim != 64 && head_dim != 128) || batch <= 0 || seq <= 0 || seq % BKV != 0 || n_heads <= 0 ||
+  if ((head_dim != 64 && head_dim != 128) || batch <= 0 || seq <= 0 || n_heads <= 0 ||
       n_kv_heads <= 0 || n_heads % n_kv_heads != 0)
     return FTB200_E_BADARG;
   const void* ptrs[] = {q, k, v, o, d_o, dq, dk, dv, scratch, cos_sin};

@@ -29,6 +29,9 @@
 // Measured, 1 x 8192, 32/8 heads of 128: 630 -> 475 us (1157 TFLOP/s); 8 x 2048, heads of 64:
 // 379 -> 303 us.
 //
+// Sequences of any length: the tensor maps have the sequence as a dimension of its own, so a tile's rows beyond its end are
+// zeros (not the next sequence's); keys there are masked, queries there are not stored.
+//
 // Every mbarrier wait is bounded; on expiry the CTA records FTB200_ST_TIMEOUT in the caller's
 // status word, frees its TMEM and returns.
 #include <cuda.h>
@@ -109,16 +112,17 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   auto bar = [&](int i) { return bar_base + 8u * i; };
 
   // heavy (late) query blocks first: with a causal mask their work is largest
-  const int n_qpairs = p.seq / (BQ * TILES);
+  const int n_qpairs = (p.seq + BQ * TILES - 1) / (BQ * TILES);
   const int per_block = p.batch * p.n_heads;
   const int qp = n_qpairs - 1 - static_cast<int>(blockIdx.x) / per_block;
   const int bh = static_cast<int>(blockIdx.x) % per_block;
   const int b = bh / p.n_heads, h = bh % p.n_heads;
   const int hk = h / (p.n_heads / p.n_kv_heads);
   // key blocks seen by tile 0 and tile 1
-  const int n_kv1 = p.causal ? qp * TILES + 2 : p.seq / BKV;
-  const int n_kv0 = p.causal ? n_kv1 - 1 : n_kv1;
-  const int q_row0 = b * p.seq + qp * BQ * TILES;
+  const int n_blocks = (p.seq + BKV - 1) / BKV;
+  const int n_kv0 = p.causal ? qp * TILES + 1 : n_blocks;
+  const int n_kv1 = p.causal ? min(qp * TILES + 2, n_blocks) : n_blocks;
+  const int q0 = qp * BQ * TILES;  // first query in its sequence
 
   if (threadIdx.x == 0) {
     for (int t = 0; t < TILES; ++t) {
@@ -157,7 +161,7 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const uint32_t sq = smem_base + C::OFF_Q + t * C::TILE_BYTES;
         mbar_expect_tx(bar(BAR_Q_FULL + t), C::TILE_BYTES);
         for (int s = 0; s < C::SLABS; ++s)
-          tma_load_2d(sq + s * C::SLAB_BYTES, &tmQ, bar(BAR_Q_FULL + t), h * D + s * 64, q_row0 + t * BQ);
+          tma_load_3d(sq + s * C::SLAB_BYTES, &tmQ, bar(BAR_Q_FULL + t), h * D + s * 64, q0 + t * BQ, b);
       }
       bool ok = true;
       for (int j = 0; j < n_kv1 && ok; ++j) {
@@ -169,10 +173,10 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         const uint32_t sk = smem_base + C::OFF_KV + st * 2 * C::TILE_BYTES;
         const uint32_t sv = sk + C::TILE_BYTES;
-        const int kv_row0 = b * p.seq + j * BKV;
+        const int kv0 = j * BKV;
         if (elect_one()) {
           mbar_expect_tx(bar(BAR_K_FULL + st), C::TILE_BYTES);
-          for (int s = 0; s < C::SLABS; ++s) tma_load_2d(sk + s * C::SLAB_BYTES, &tmK, bar(BAR_K_FULL + st), hk * D + s * 64, kv_row0);
+          for (int s = 0; s < C::SLABS; ++s) tma_load_3d(sk + s * C::SLAB_BYTES, &tmK, bar(BAR_K_FULL + st), hk * D + s * 64, kv0, b);
         }
         __syncwarp();
         if (!mbar_wait_warp(bar(BAR_V_EMPTY + st), (use & 1u) ^ 1u, abort_flag)) {
@@ -181,7 +185,7 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         if (elect_one()) {
           mbar_expect_tx(bar(BAR_V_FULL + st), C::TILE_BYTES);
-          for (int s = 0; s < C::SLABS; ++s) tma_load_2d(sv + s * C::SLAB_BYTES, &tmV, bar(BAR_V_FULL + st), hk * D + s * 64, kv_row0);
+          for (int s = 0; s < C::SLABS; ++s) tma_load_3d(sv + s * C::SLAB_BYTES, &tmV, bar(BAR_V_FULL + st), hk * D + s * 64, kv0, b);
         }
         __syncwarp();
       }
@@ -326,6 +330,11 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
         for (int c = 0; c < BKV; ++c)
           if (c > row) sv[c] = __float_as_uint(-INFINITY);
+      } else if (!p.causal && (j + 1) * BKV > p.seq) {  // keys beyond the sequence's end
+        const int left = p.seq - j * BKV;
+#pragma unroll
+        for (int c = 0; c < BKV; ++c)
+          if (c >= left) sv[c] = __float_as_uint(-INFINITY);
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -406,8 +415,9 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (ok && mbar_wait_warp(bar(BAR_O_DONE + t), static_cast<uint32_t>(n_kv - 1) & 1u, abort_flag)) {
       tc_fence_after();
       const float inv = 1.f / l_sum;
-      const long long grow = static_cast<long long>(q_row0 + t * BQ + row);
-      __nv_bfloat16* dst = p.O + grow * p.ld_o + h * D;
+      const int query = q0 + t * BQ + row;
+      const bool stored = query < p.seq;
+      __nv_bfloat16* dst = p.O + (static_cast<long long>(b) * p.seq + query) * p.ld_o + h * D;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t ov[32];
@@ -418,11 +428,11 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           float f[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(ov[8 * q4 + e]) * inv;
-          reinterpret_cast<ftb200::bf16x8*>(dst + c * 32)[q4] = ftb200::pack8(f);
+          if (stored) reinterpret_cast<ftb200::bf16x8*>(dst + c * 32)[q4] = ftb200::pack8(f);
         }
       }
-      if (p.lse != nullptr) {
-        p.lse[(static_cast<long long>(b) * p.n_heads + h) * p.seq + qp * BQ * TILES + t * BQ + row] =
+      if (p.lse != nullptr && stored) {
+        p.lse[(static_cast<long long>(b) * p.n_heads + h) * p.seq + query] =
             (m_used * p.scale_log2 + log2f(l_sum)) * 0.6931471805599453f;
       }
     }
@@ -452,15 +462,15 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn2() {
   return fn;
 }
 
-// [rows, cols] bf16 view with row stride ld (elements); box = 64 columns x 128 rows, 128-byte swizzle
-int encode_rows2(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld) {
+// [batch, seq, cols] bf16 view with row stride ld (elements); box = 64 columns x 128 rows, 128-byte swizzle
+int encode_rows2(CUtensorMap* map, const void* base, long long batch, long long seq, long long cols, long long ld) {
   auto fn = encode_fn2();
   if (fn == nullptr) return FTB200_E_DRIVER;
-  cuuint64_t gdim[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t gstride[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {64u, 128u};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), gdim, gstride, box, estr,
+  cuuint64_t gdim[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(seq), static_cast<cuuint64_t>(batch)};
+  cuuint64_t gstride[2] = {static_cast<cuuint64_t>(ld) * 2, static_cast<cuuint64_t>(seq) * ld * 2};
+  cuuint32_t box[3] = {64u, 128u, 1u};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : FTB200_E_DRIVER;
@@ -489,13 +499,13 @@ int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
 
 // q: [batch*seq, n_heads*head_dim] view with row stride ld_q; k, v: [batch*seq, n_kv_heads*head_dim] views with
 // row strides ld_k, ld_v; o: [batch*seq, n_heads*head_dim] with row stride ld_o.  lse (may be null):
-// [batch, n_heads, seq] fp32.  head_dim 64 or 128; seq must be a multiple of 256.  poly: how many of every
+// [batch, n_heads, seq] fp32.  head_dim 64 or 128, any seq.  poly: how many of every
 // eight exponentials are computed on the FMA pipe (0, 2 or 4).
 FTB200_API int ftb200_attention_fwd2(const void* q, const void* k, const void* v, void* o, float* lse, int batch, int seq,
                                      int n_heads, int n_kv_heads, int head_dim, long long ld_q, long long ld_k,
                                      long long ld_v, long long ld_o, float scale, int causal, int poly, int* status,
                                      cudaStream_t stream) {
-  if ((head_dim != 64 && head_dim != 128) || batch <= 0 || seq <= 0 || seq % (BQ * TILES) != 0 || n_heads <= 0 ||
+  if ((head_dim != 64 && head_dim != 128) || batch <= 0 || seq <= 0 || n_heads <= 0 ||
       n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || (poly != 0 && poly != 2 && poly != 4))
     return FTB200_E_BADARG;
   auto aligned16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
@@ -503,16 +513,15 @@ FTB200_API int ftb200_attention_fwd2(const void* q, const void* k, const void* v
       (ld_o & 7))
     return FTB200_E_ALIGN;
   CUtensorMap tq, tk, tv;
-  const long long rows = static_cast<long long>(batch) * seq;
-  int rc = encode_rows2(&tq, q, rows, static_cast<long long>(n_heads) * head_dim, ld_q);
-  if (rc == 0) rc = encode_rows2(&tk, k, rows, static_cast<long long>(n_kv_heads) * head_dim, ld_k);
-  if (rc == 0) rc = encode_rows2(&tv, v, rows, static_cast<long long>(n_kv_heads) * head_dim, ld_v);
+  int rc = encode_rows2(&tq, q, batch, seq, static_cast<long long>(n_heads) * head_dim, ld_q);
+  if (rc == 0) rc = encode_rows2(&tk, k, batch, seq, static_cast<long long>(n_kv_heads) * head_dim, ld_k);
+  if (rc == 0) rc = encode_rows2(&tv, v, batch, seq, static_cast<long long>(n_kv_heads) * head_dim, ld_v);
   if (rc != 0) return rc;
   Attn2Params p;
   p.batch = batch; p.seq = seq; p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.causal = causal;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.O = reinterpret_cast<__nv_bfloat16*>(o); p.ld_o = ld_o; p.lse = lse; p.status = status;
-  const long long grid = static_cast<long long>(batch) * n_heads * (seq / (BQ * TILES));
+  const long long grid = static_cast<long long>(batch) * n_heads * ((static_cast<long long>(seq) + BQ * TILES - 1) / (BQ * TILES));
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   if (head_dim == 128) {
     if (poly == 0) return launch_fwd2<128, 0>(tq, tk, tv, p, grid, stream);

@@ -173,7 +173,7 @@ class Tcgen05Attention:
             lse = self._lse_pool.pop() if self._lse_pool else torch.empty(batch, c.n_heads, seq, dtype=torch.float32,
                                                                           device=qkv.device)
             self._saved[layer] = (qkv, out, lse)
-        K.attention_fwd(q, k, v, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, out, lse, causal=True)
+        K.attention_fwd(q, k, v, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, out, lse, causal=True, any_length=True)
 
     def backward(self, layer: int, dout: torch.Tensor, batch: int, seq: int, dqkv: torch.Tensor,
                  rope: Optional[torch.Tensor] = None) -> None:
@@ -185,7 +185,7 @@ class Tcgen05Attention:
         if self._scratch is None or self._scratch.numel() < need:
             self._scratch = torch.empty(need, dtype=torch.uint8, device=qkv.device)
         K.attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, causal=True,
-                        scratch=self._scratch, rope=rope)
+                        scratch=self._scratch, rope=rope, any_length=True)
         self._lse_pool.append(lse)
 
     def reset(self) -> None:
@@ -196,14 +196,17 @@ class Tcgen05Attention:
 
 def make_attention(cfg: LlamaConfig, seq_len: int, device: torch.device, kind: Optional[str] = None):
     """``kind``: "tcgen05" (hand-written kernels; CUDA, head dim 128 and a sequence that is a multiple of 128,
-    or head dim 64 and a multiple of 256), "sdpa" (library), or None for tcgen05 where it applies.  The environment variable
-    ``FTB200_ATTENTION`` overrides None."""
+    or head dim 64 and a multiple of 256), "sdpa" (library), or None for tcgen05 there and wherever else the sequence is longer
+    than a tile (128): the library's kernels want four transposing copies and an autograd graph around them (four layers of
+    width 1024, 3 x 1000 tokens: a step of 2845 us against 2309).  The environment variable ``FTB200_ATTENTION`` overrides
+    None."""
     kind = kind or os.environ.get("FTB200_ATTENTION") or "auto"
     ok = device.type == "cuda" and K.attention_supported(seq_len, cfg.head_dim)
     if kind == "tcgen05" and not ok:
         raise ValueError("tcgen05 attention needs CUDA and head_dim 128 with seq_len % 128 == 0 or head_dim 64 with "
                          "seq_len % 256 == 0")
-    if kind == "tcgen05" or (kind == "auto" and ok):
+    longer = device.type == "cuda" and cfg.head_dim in (64, 128) and seq_len > 128
+    if kind == "tcgen05" or (kind == "auto" and (ok or longer)):
         return Tcgen05Attention(cfg)
     return SdpaAttention(cfg)
 

@@ -686,11 +686,12 @@ def _two_query_tiles(batch: int, seq_len: int, n_heads: int, sms: int) -> bool:
 
 def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int, seq_len: int, n_heads: int,
                   n_kv_heads: int, head_dim: int, out: torch.Tensor, lse: Optional[torch.Tensor] = None,
-                  causal: bool = True) -> None:
+                  causal: bool = True, any_length: bool = False) -> None:
     """Causal GQA attention forward.  ``q`` ``[batch*seq, n_heads*head_dim]`` and ``k``/``v``
     ``[batch*seq, n_kv_heads*head_dim]`` are 2-D bf16 views (column slices of the packed QKV
     activation are fine), ``out`` ``[batch*seq, n_heads*head_dim]``, ``lse`` ``[batch, n_heads,
-    seq]`` fp32 (saved for the backward pass)."""
+    seq]`` fp32 (saved for the backward pass).  Sequence lengths are those of :func:`attention_supported`; ``any_length``
+    takes every other one as well (of head dims 64 and 128)."""
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (out, "out")):
         _check_2d_bf16(t, name)
     if not q.is_cuda:
@@ -702,6 +703,10 @@ def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, batch: int,
         return
     scale = 1.0 / math.sqrt(head_dim)
     impl = os.environ.get("FTB200_ATTN_FWD", "auto")
+    if seq_len % 256 and (head_dim != 128 or seq_len % 128 or impl == "pair"):
+        if not any_length:
+            N.check(-1, "attention_fwd")
+        impl = "pair"  # the other kernel takes whole tiles only
     if impl == "auto":
         impl = "pair" if _two_query_tiles(batch, seq_len, n_heads, _sm_count(q.device.index)) else "single"
     if impl == "pair" or head_dim != 128:
@@ -744,13 +749,14 @@ def attention_bwd_scratch_bytes(batch: int, seq_len: int, n_heads: int) -> int:
 def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor,
                   lse: torch.Tensor, dq: torch.Tensor, dk: torch.Tensor, dv: torch.Tensor, batch: int, seq_len: int,
                   n_heads: int, n_kv_heads: int, head_dim: int, causal: bool = True,
-                  scratch: Optional[torch.Tensor] = None, rope: Optional[torch.Tensor] = None) -> None:
+                  scratch: Optional[torch.Tensor] = None, rope: Optional[torch.Tensor] = None, any_length: bool = False) -> None:
     """Backward of :func:`attention_fwd`: writes ``dq``, ``dk``, ``dv`` (2-D bf16 views like
     ``q``, ``k``, ``v``; column slices of a packed dQKV buffer are fine).  The fp32 dQ
     accumulator lives in ``scratch`` (bytes on the device, :func:`attention_bwd_scratch_bytes` of
     them or more), by default a per-device buffer that is reused across calls on the same stream.
     With ``rope``, the table (:func:`rope_table`) that ``q`` and ``k`` were rotated by, ``dq`` and ``dk``
-    are the gradients of the values before the rotation."""
+    are the gradients of the values before the rotation.  Sequences are a multiple of 128 or, with
+    ``any_length``, of any length."""
     for t, name in ((q, "q"), (k, "k"), (v, "v"), (o, "o"), (d_o, "d_o"), (dq, "dq"), (dk, "dk"), (dv, "dv")):
         _check_2d_bf16(t, name)
     if not q.is_cuda:
@@ -764,6 +770,8 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
             dq.copy_(ref_rope(dq, rope, S, n_heads, head_dim, backward=True))
             dk.copy_(ref_rope(dk, rope, S, n_kv_heads, head_dim, backward=True))
         return
+    if seq_len % 128 and not any_length:
+        N.check(-1, "attention_bwd")
     if rope is not None and (rope.dtype != torch.float32 or not rope.is_contiguous() or rope.device != q.device
                              or rope.shape[0] < seq_len or tuple(rope.shape[1:]) != (head_dim // 2, 2)):
         raise ValueError("rope must be the table of the sequence and head dim on the device of q")
