@@ -90,7 +90,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + OFF_MISC + 196);
   float* xchg = reinterpret_cast<float*>(smem + OFF_MISC + 256);  // [parity][group][row]
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_base = smem_u32(bars);
@@ -131,7 +131,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
