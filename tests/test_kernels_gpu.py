@@ -82,6 +82,26 @@ def test_gemm_split_last_wave(a_mn, b_mn, M, N, K_):
     K.check_status(out.device)
 
 
+@pytest.mark.parametrize("N", [1, 2, 17, 1000, 8192])
+@pytest.mark.parametrize("K_", [8, 72, 256, 1024, 1032, 4104])
+def test_gemm_one_row(N, K_):
+    """A single row reads the other operand once, by a kernel of its own; the remainders of its lanes and rows, a row stride.
+    fp32 sums: bf16 rounding of the result (2^-9 of each value) is the error.  Transposed operands, fp32 results and
+    accumulation stay with the tiles."""
+    torch.manual_seed(N + K_)
+    a, b = torch.randn(1, K_, device=DEV).bfloat16(), torch.randn(N + 1, K_ + 8, device=DEV).bfloat16()[:N, :K_]
+    ref = a.double() @ b.double().t()
+    out = torch.full((2, N + 4), 7.0, device=DEV, dtype=torch.bfloat16)
+    K.gemm(a, b, out=out[:1, :N])
+    assert ((out[0, :N].double() - ref[0]).abs() <= 2**-8 * ref[0].abs() + 1e-4).all()
+    assert bool((out[1] == 7.0).all()) and bool((out[0, N:] == 7.0).all())
+    acc = torch.ones(1, N, device=DEV, dtype=torch.float32)
+    K.gemm(a, b, out=acc, accumulate=True)
+    # K products and the one summed in fp32, in any order: K 2^-24 of the sum of their magnitudes at most
+    assert ((acc.double() - 1 - ref).abs() <= (K_ + 1) * 2**-24 * (1 + a.double().abs() @ b.double().abs().t())).all()
+    K.check_status(a.device)
+
+
 @pytest.mark.parametrize("M", [1, 33, 160, 257])
 @pytest.mark.parametrize("N", [8, 72, 200, 328, 12])
 def test_gemm_store_edges(M, N):
