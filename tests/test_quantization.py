@@ -230,6 +230,28 @@ def test_list_kernels_match_flat_kernels_gpu(numels, dtype):
         Q.fused_dequantize_from_fp8([leaf], Q.fused_quantize_into_fp8([leaf], world)[0], world)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("head", [0, 1, 8, 2048, 2049])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_list_kernel_encodes_special_values_gpu(dtype, head):
+    """Parts of 2048 elements that lie in one tensor are encoded from their packed values: the same bytes as the flat kernel
+    gives, for NaN, infinities, negative zero, the smallest and largest numbers and blocks of zeros, whether the part begins
+    on a 16-byte boundary, a tensor's end lies in it or not."""
+    g = torch.Generator(device="cuda").manual_seed(head)
+    x = torch.randn(3 * 2048 + 77, generator=g, device="cuda", dtype=dtype)
+    x[:128] = 0.0
+    x[130], x[300], x[301], x[500], x[700] = float("nan"), float("inf"), -float("inf"), -0.0, torch.finfo(dtype).tiny
+    x[900], x[1100:1228], x[2100], x[5000] = torch.finfo(dtype).max, float("nan"), torch.finfo(dtype).tiny / 8, -torch.finfo(dtype).max
+    lead = torch.randn(head, generator=g, device="cuda", dtype=dtype)
+    ts = ([lead] if head else []) + [x]
+    buf, (n,) = Q.fused_quantize_into_fp8(ts, 2)
+    flat = torch.zeros(n, dtype=dtype, device="cuda")
+    flat[: head + x.numel()] = torch.cat(ts)
+    want = Q.quantize_into(flat, torch.empty_like(buf))
+    assert torch.equal(buf, want)
+
+
+
 def test_a_buffer_that_is_too_short_is_refused():
     """A buffer packed for fewer ranks (less padding), cut short, or of another type, before anything reads it."""
     ts = [torch.randn(1000), torch.randn(77)]
