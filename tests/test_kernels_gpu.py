@@ -254,26 +254,6 @@ def test_cross_entropy_without_gradient(V):
     assert rel_err(logits[:2], K.ref_cross_entropy(kept, tgt.clamp(min=0), 1.0)[1][:2]) < 1e-2 and not logits[2].any()
 
 
-@pytest.mark.parametrize("T,Kd,heads,kv,Dh,S", [(300, 256, 2, 2, 128, 100), (16400, 64, 8, 2, 64, 33), (20000, 72, 4, 2, 128, 1000),
-                                               (8200, 128, 8, 4, 192, 260)])
-def test_linear_rope(T, Kd, heads, kv, Dh, S):
-    """The projection with its rotation in the epilogue against the two kernels: the same rounded values are rotated, by products
-    that the compiler may contract another way (one bf16 rounding apart at most)."""
-    torch.manual_seed(T)
-    N = (heads + 2 * kv) * Dh
-    x, w = torch.randn(T, Kd, device=DEV).bfloat16(), torch.randn(N, Kd, device=DEV).bfloat16()
-    table = K.rope_table(S, Dh, 10000.0, DEV)
-    out = torch.full((T + 1, N + 8), 7.0, device=DEV, dtype=torch.bfloat16)
-    assert T < 8000 or -(-T // 256) * -(-N // 256) > torch.cuda.get_device_properties(0).multi_processor_count  # the fused one
-    K.linear_rope_fwd(x, w, out[:T, :N], table, S, heads + kv, Dh)
-    want = K.rope_(K.linear_fwd(x, w), table, S, heads + kv, Dh)
-    assert torch.equal(out[:T, (heads + kv) * Dh : N], want[:, (heads + kv) * Dh :])
-    assert (out[:T, :N].float() - want.float()).abs().max() <= 2**-7 * want.float().abs().max()
-    assert rel_err(out[:T, :N], want) < 2**-9
-    assert bool((out[T:] == 7.0).all()) and bool((out[:, N:] == 7.0).all())
-    K.check_status(out.device)
-
-
 @pytest.mark.parametrize("T,Kd,F", [(1, 2048, 8), (33, 2056, 40), (200, 2048, 512), (1000, 2048, 2816), (130, 4096, 1000), (300, 64, 128)])
 def test_linear_dswiglu(T, Kd, F):
     """Down projection and activation backwards in one kernel against 64 bits: the gradient of the activation is not rounded on

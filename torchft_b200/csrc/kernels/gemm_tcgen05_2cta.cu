@@ -54,7 +54,6 @@ enum Epilogue : int {
   EPI_STORE = 0,    // it is stored (added, with the activation of its columns' pairs, scattered: GemmParams)
   EPI_DSWIGLU = 1,  // it is the gradient of silu(gate) * up: the gate/up pairs it belongs to are replaced by their gradients
   EPI_LOSS = 2,     // its rows' maximum, sum of exponentials and target value are noted; it is not stored
-  EPI_ROPE = 3,     // stored, the columns of its first heads rotated by their row's position
 };
 
 // A pair's tile has 256 or 128 columns; the K ring fills 192 KB with 6 or 8 stages.  The gradient of the activation needs
@@ -173,9 +172,6 @@ struct GemmParams {
   float2* row_stats;
   float* target_value;
   const long long* target;
-  // EPI_ROPE: (cos, sin) pairs [rope_seq][head_dim / 2], columns that are rotated, row = ... * rope_seq + position
-  const float4* rope;
-  int rope_cols, rope_seq, rope_dim;
   // fused reduce-scatter epilogue: C is not written locally; every 16-byte piece of the
   // (contiguous, row-major) result goes to the rank that owns that slice of the flat
   // gradient unit, into that rank's staging area for source rank `sc_src`.
@@ -258,20 +254,6 @@ __device__ __forceinline__ uint2 silu_mul(const ftb200::bf16x8& packed) {
   o.x = *reinterpret_cast<uint32_t*>(&lo);
   o.y = *reinterpret_cast<uint32_t*>(&hi);
   return o;
-}
-
-// Four pairs rotated by their angles (cos, sin, cos, sin).
-__device__ __forceinline__ ftb200::bf16x8 rotate_pairs(const ftb200::bf16x8& x, const float4& c0, const float4& c1) {
-  float f[8];
-  ftb200::unpack8(x, f);
-  const float cosv[4] = {c0.x, c0.z, c1.x, c1.z}, sinv[4] = {c0.y, c0.w, c1.y, c1.w};
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float a = f[2 * e], b = f[2 * e + 1];
-    f[2 * e] = a * cosv[e] - b * sinv[e];
-    f[2 * e + 1] = a * sinv[e] + b * cosv[e];
-  }
-  return ftb200::pack8(f);
 }
 
 // Asynchronous copy from this CTA's shared memory to another's, counted by a barrier there.
@@ -633,7 +615,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       const int row = m0 + q * 32 + lane;
       const uint32_t taddr0 = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
       const uint32_t stg = OFF_STAGING + q * STAGE_WARP_BYTES;
-      if (EPI == EPI_LOSS || EPI == EPI_ROPE || (p.tma_out && !(SPLIT && w.shared))) {
+      if (EPI == EPI_LOSS || (p.tma_out && !(SPLIT && w.shared))) {
         // bf16 output: 64 columns at a time go, one row a thread, into a 128-byte-swizzled piece of the warp's staging area
         // and leave by TMA (which clips what lies beyond M and N), while the next 64 come out of tensor memory.  Nothing hides
         // the last tile's epilogue: 5800 cycles for 256 columns that leave a row-major staging area as row segments, 4100
@@ -642,7 +624,6 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         float row_max = -INFINITY, row_sum = 0.f;  // EPI_LOSS: over the tile's columns
         long long target = -1;
         if (EPI == EPI_LOSS && row < p.M) target = p.target[row];
-        const int rope_pos = EPI == EPI_ROPE ? (m0 + q * 32) % p.rope_seq : 0;  // of the warp's first row
         uint32_t r[2][64];
         tmem_ld32(taddr0, r[0]);
         tmem_ld32(taddr0 + 32, r[0] + 32);
@@ -679,21 +660,6 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
             const ftb200::bf16x8 packed = ftb200::pack8(f);
             *reinterpret_cast<ftb200::bf16x8*>(prow + ((j ^ (lane & 7)) << 4)) = packed;
             if (with_aux) *reinterpret_cast<uint2*>(arow + ((((c & 1) * 4 + (j >> 1)) ^ (lane & 7)) << 4) + (j & 1) * 8) = silu_mul(packed);
-          }
-          if (EPI == EPI_ROPE && n0 + c * 64 < p.rope_cols) {
-            // The rounded values are rotated, as by a kernel of its own; eight lanes a row, so that the table is read in whole
-            // lines (a row a lane asks for 32 of them with every load: 3000 x 1536 x 1024 24 us).
-            __syncwarp();
-            const int seg = lane & 7, off = (n0 + c * 64) % p.rope_dim / 4 + 2 * seg;
-#pragma unroll 4
-            for (int it = 0; it < 8; ++it) {
-              const int rr = it * 4 + (lane >> 3);
-              int pos = rope_pos + rr;
-              if (pos >= p.rope_seq) pos %= p.rope_seq;
-              const float4* cs = p.rope + static_cast<long long>(pos) * (p.rope_dim / 4) + off;
-              ftb200::bf16x8* at = reinterpret_cast<ftb200::bf16x8*>(smem + piece + rr * 128 + ((seg ^ (rr & 7)) << 4));
-              *at = rotate_pairs(*at, cs[0], cs[1]);
-            }
           }
           if (EPI == EPI_LOSS && inside) {
             // of the rounded values, as they are stored; columns beyond N are left out
@@ -1021,8 +987,6 @@ struct EpilogueSpec {
   float2* row_stats = nullptr;
   float* target_value = nullptr;
   const long long* target = nullptr;
-  const float4* rope = nullptr;
-  int rope_cols = 0, rope_seq = 1, rope_dim = 64;
 };
 
 struct GatherSpec {
@@ -1179,10 +1143,6 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   p.row_stats = ep != nullptr ? ep->row_stats : nullptr;
   p.target_value = ep != nullptr ? ep->target_value : nullptr;
   p.target = ep != nullptr ? ep->target : nullptr;
-  p.rope = ep != nullptr ? ep->rope : nullptr;
-  p.rope_cols = ep != nullptr ? ep->rope_cols : 0;
-  p.rope_seq = ep != nullptr ? ep->rope_seq : 1;
-  p.rope_dim = ep != nullptr ? ep->rope_dim : 64;
   p.sc_world = 0;
   p.sc_src = 0;
   p.sc_shard = 0;
@@ -1227,17 +1187,11 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   if (ep != nullptr) {
     p.tma_out = 1;  // the entry has looked at what TMA wants
     const bool narrow = plan_tiles(M, N, K, ctas / 2, false).columns == 128;
-    switch (ep->kind) {
-      case EPI_DSWIGLU:
-        return narrow ? launch_2cta<128, false, EPI_DSWIGLU>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
-                      : launch_2cta<256, false, EPI_DSWIGLU>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
-      case EPI_LOSS:
-        return narrow ? launch_2cta<128, false, EPI_LOSS>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
-                      : launch_2cta<256, false, EPI_LOSS>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
-      default:
-        return narrow ? launch_2cta<128, false, EPI_ROPE>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
-                      : launch_2cta<256, false, EPI_ROPE>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
-    }
+    if (ep->kind == EPI_DSWIGLU)
+      return narrow ? launch_2cta<128, false, EPI_DSWIGLU>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
+                    : launch_2cta<256, false, EPI_DSWIGLU>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+    return narrow ? launch_2cta<128, false, EPI_LOSS>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
+                  : launch_2cta<256, false, EPI_LOSS>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
   }
   // scattered and activated outputs leave through the staging area, which a shared tile does not
   const TilePlan plan = plan_tiles(M, N, K, ctas / 2, sc == nullptr && aux == nullptr && max_ctas <= 0);
@@ -1267,23 +1221,6 @@ FTB200_API int ftb200_gemm_bf16_swiglu(const void* A, const void* B, void* C, vo
 }
 
 static bool aligned16(const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; }
-
-// C[M,N] = A[M,K] . B[N,K]^T with the first `heads` heads of `head_dim` columns rotated: the pair (2i, 2i+1) of a head by the
-// angle whose (cos, sin) is cos_sin[row % seq][i], after rounding to bf16 (as ftb200_rope does it to a stored C).  head_dim a
-// multiple of 64, N and ldc of 8.
-FTB200_API int ftb200_gemm_bf16_rope(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
-                                     long long ldc, const float* cos_sin, int seq, int heads, int head_dim, int* status,
-                                     cudaStream_t stream) {
-  if (cos_sin == nullptr || seq <= 0 || heads < 0 || head_dim <= 0 || static_cast<long long>(heads) * head_dim > N) return FTB200_E_BADARG;
-  if (head_dim % 64 || (N & 7) || (ldc & 7) || ldc < N || !aligned16(C) || !aligned16(cos_sin)) return FTB200_E_ALIGN;
-  EpilogueSpec ep;
-  ep.kind = EPI_ROPE;
-  ep.rope = reinterpret_cast<const float4*>(cos_sin);
-  ep.rope_cols = heads * head_dim;
-  ep.rope_seq = seq;
-  ep.rope_dim = head_dim;
-  return gemm_2cta_impl(A, B, C, M, N, K, 0, 0, lda, ldb, ldc, 0, status, 0, nullptr, 0, stream, nullptr, nullptr, &ep);
-}
 
 // Backward of a gated MLP's down projection and activation: D[M,N] = dY[M,K] . W[K,N] (W row-major, as it is stored for the
 // forward product) is the gradient of silu(gate) * up and is not stored; gu [M, 2 N], the interleaved (gate, up) pairs of

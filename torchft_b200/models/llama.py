@@ -407,7 +407,8 @@ class LlamaEngine:
             else:
                 K.rmsnorm_fwd(self.h[l - 1], W.attn_norm, c.norm_eps, res=delta, h_out=self.x[l], out=n1,
                               rstd=self.rstd1[l])
-            K.linear_rope_fwd(n1, W.wqkv, self.qkv[l], self.rope, S, c.n_heads + c.n_kv_heads, c.head_dim)
+            K.linear_fwd(n1, W.wqkv, out=self.qkv[l])
+            K.rope_(self.qkv[l], self.rope, S, c.n_heads + c.n_kv_heads, c.head_dim)
             self.attn.forward(l, self.qkv[l], B, S, self.att[l], train)
             K.linear_fwd(self.att[l], W.wo, out=self.ws_proj)
             K.rmsnorm_fwd(self.x[l], W.ffn_norm, c.norm_eps, res=self.ws_proj, h_out=self.h[l], out=n2,

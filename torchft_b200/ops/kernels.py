@@ -53,7 +53,7 @@ def _status_ptr(device: torch.device) -> int:
 _ARGS = {
     "embedding_fwd": "pppiiip", "embedding_bwd": "pppiiip", "rmsnorm_fwd": "ppppppiifp", "rmsnorm_bwd": "ppppppppiiip",
     "rope": "ppliiilip", "swiglu_fwd": "pplip", "swiglu_bwd": "ppplip", "gemm_bf16_swiglu": "ppppiiillllpip",
-    "gemm_bf16_rope": "pppiiilllpiiipp", "gemm_bf16_dswiglu": "pppiiilllpp", "gemm_bf16_loss": "ppiiillppppp",
+    "gemm_bf16_dswiglu": "pppiiilllpp", "gemm_bf16_loss": "ppiiillppppp",
     "cross_entropy": "pppiilfip", "adamw": "ppppiplfffffipp", "sumsq": "pilpp", "clip_coef": "pfppp",
     "attention_fwd": "pppppiiiiillllfipp", "attention_fwd2": "pppppiiiiillllfiipp",
     "attention_bwd": "ppppppppppiiiiillllllllfippp", "gemm_bf16": "pppiiiiilllipip",
@@ -438,29 +438,6 @@ def ref_swiglu_bwd(ds, gu):
     out[:, 0::2] = d * u * (sg + silu * (1 - sg))
     out[:, 1::2] = d * silu
     return out.to(gu.dtype)
-
-
-def linear_rope_fwd(x: torch.Tensor, w, out: torch.Tensor, table: torch.Tensor, seq_len: int, n_heads: int, head_dim: int) -> None:
-    """``out = x @ w^T`` with the first ``n_heads`` heads of its rows rotated (:func:`linear_fwd` and :func:`rope_`), in one
-    kernel where the heads are whole 64-column pieces of the product's epilogue and there are more than two waves of tiles: the
-    table's way into the last tile's epilogue is hidden by nothing.  8192 x 6144 x 4096 289 -> 256 us, 4096 x 3072 x 2048 83 -> 76;
-    1536 x 6144 x 4096 (144 tiles on 74 CTA pairs) 95 -> 96, 1024 x 3072 x 2048 34 -> 40."""
-    weight = w if not isinstance(w, GatherField) else None if w.pending else w.local
-    if (weight is None or not x.is_cuda or -(-out.shape[0] // 256) * -(-out.shape[1] // 256) <= _sm_count(x.device.index) or GEMM_IMPL != "2cta" or head_dim % 64 or out.shape[1] % 8 or out.stride(0) % 8
-            or out.data_ptr() % 16 or table.data_ptr() % 16 or out.shape[0] < 1 or out.stride(0) < out.shape[1]):
-        linear_fwd(x, w, out=out)
-        rope_(out, table, seq_len, n_heads, head_dim)
-        return
-    for t, name in ((x, "x"), (weight, "w"), (out, "out")):
-        _check_2d_bf16(t, name)
-    T, Kd = x.shape
-    if weight.shape[1] != Kd or tuple(out.shape) != (T, weight.shape[0]):
-        raise ValueError(f"shape mismatch: x {tuple(x.shape)}, w {tuple(weight.shape)}, out {tuple(out.shape)}")
-    if table.dtype != torch.float32 or not table.is_contiguous() or table.shape[0] < seq_len or tuple(table.shape[1:]) != (head_dim // 2, 2):
-        raise ValueError("table must be rope_table() of the sequence and head dim")
-    N.check(_fn("gemm_bf16_rope")(x.data_ptr(), weight.data_ptr(), out.data_ptr(), T, weight.shape[0], Kd, x.stride(0),
-                                  weight.stride(0), out.stride(0), table.data_ptr(), seq_len, n_heads, head_dim,
-                                  _status_ptr(x.device), _stream()), "gemm_bf16_rope")
 
 
 def linear_dswiglu_(dy: torch.Tensor, w: torch.Tensor, gu: torch.Tensor, ds: torch.Tensor) -> None:
