@@ -229,6 +229,33 @@ def test_attention_bwd_rotates_back(D, causal):
     assert (a - b).norm() < 2**-8 * a.norm() and torch.equal(grads[0][:, (Hq + Hkv) * D :], grads[1][:, (Hq + Hkv) * D :])
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("S,Hq,Hkv", [(1, 2, 1), (129, 3, 1), (256, 7, 1), (300, 12, 2), (1000, 8, 2), (1280, 6, 1)])
+def test_attention_bwd_shares_heads(S, Hq, Hkv, causal, D):
+    """A batch that leaves SMs idle shares the heads of a group out, one beyond a block a SM does not: the same sums in another
+    order in fp32 (far below a rounding to bf16, which may then fall to the other side: 2^-8 of the value)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = sms // ((S + 127) // 128 * Hkv) + 1
+    qkv, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=S + D)
+    table = K.rope_table(S, D, 10000.0, "cuda")
+    out = torch.empty(B * S, Hq * D, dtype=torch.bfloat16, device="cuda")
+    lse = torch.empty(B, Hq, S, dtype=torch.float32, device="cuda")
+    K.attention_fwd(q, k, v, B, S, Hq, Hkv, D, out, lse, causal=causal, any_length=True)
+    d_o = torch.randn_like(out)
+    a, b = Hq * D, (Hq + Hkv) * D
+    grads = []
+    for n in (B, 1):
+        d = torch.full_like(qkv, 7.0)
+        K.attention_bwd(q, k, v, out, d_o, lse, d[:, :a], d[:, a:b], d[:, b:], n, S, Hq, Hkv, D, causal=causal, rope=table,
+                        any_length=True)
+        grads.append(d[:S].float())
+        assert bool((d[n * S :] == 7).all())
+    K.check_status(out.device)
+    for lo, hi in ((0, a), (a, b), (b, qkv.shape[1])):
+        assert (grads[0][:, lo:hi] - grads[1][:, lo:hi]).norm() <= 2**-8 * grads[0][:, lo:hi].norm() + 1e-6 * d_o.float()[:S].norm()
+
+
 @pytest.mark.parametrize("D,poly", [(64, None), (64, "0"), (64, "4"), (128, "0"), (128, "4")])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("key", [*range(8), 131, 200])

@@ -1,8 +1,8 @@
 // Causal grouped-query attention, backward pass, on the 5th-generation tensor cores.
 //
 // One CTA owns one (batch, kv head, 128-key block) and walks over every query head of the
-// group and every 128-query tile that can see the block.  Scores are formed transposed, keys on
-// the TMEM lanes and queries on the columns, so every MMA has M = 128:
+// group (where that would leave SMs idle, over a share of them: head_split) and every 128-query tile that can
+// see the block.  Scores are formed transposed, keys on the TMEM lanes and queries on the columns, so every MMA has M = 128:
 //
 //   S^T  = K  Q^T            [keys x q]      A = K   (K-major)      B = Q   (K-major)
 //   dP^T = V  dO^T           [keys x q]      A = V   (K-major)      B = dO  (K-major)
@@ -118,6 +118,8 @@ struct BwdParams {
   __nv_bfloat16* dK;   // rows batch*seq, row stride ld_dk
   __nv_bfloat16* dV;
   long long ld_dk, ld_dv;
+  int split;           // CTAs that share the query heads of a kv head
+  float4* dkv_part;    // split > 1: their dV and dK, fp32, per (batch, kv head, key block, share) [2][D / 4][128 keys][4]
   const float4* rope;  // null, or (cos, sin) pairs [seq][D / 2]: dQ and dK are rotated back
   int* status;
 };
@@ -171,11 +173,13 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
 
   // early key blocks see the most queries under a causal mask: schedule them first
-  const int per_block = p.batch * p.n_kv_heads;
+  const int per_block = p.batch * p.n_kv_heads * p.split;
   const int jb = static_cast<int>(blockIdx.x) / per_block;
-  const int bh = static_cast<int>(blockIdx.x) % per_block;
+  const int share = static_cast<int>(blockIdx.x) % p.split;
+  const int bh = static_cast<int>(blockIdx.x) % per_block / p.split;
   const int b = bh / p.n_kv_heads, hk = bh % p.n_kv_heads;
-  const int rep = p.n_heads / p.n_kv_heads;
+  const int rep = p.n_heads / p.n_kv_heads / p.split;  // of this CTA
+  const int h0 = (hk * p.split + share) * rep;
   const int n_qtiles = (p.seq + BQ - 1) / BQ;
   const int first_q = p.causal ? jb : 0;
   const int T = rep * (n_qtiles - first_q);
@@ -234,7 +238,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       __syncwarp();
       bool ok = true;
-      TileWalk w{hk * rep, first_q};
+      TileWalk w{h0, first_q};
       for (int t = 0; t < T && ok; ++t, next_tile(w)) {
         const int st = t % STAGES;
         const uint32_t was = static_cast<uint32_t>(t / STAGES) & 1u ^ 1u;
@@ -361,7 +365,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const bool mine = quarter * 32 < D;  // head dim 64: only lanes 0..63 of dQ^T are real
     const uint32_t off = Ly::OFF_DQ + quarter * 2 * DQ_PART_BYTES;
     constexpr int PER = BQ / 4 / DQ_PARTS;  // groups of four queries in a part
-    TileWalk w{hk * rep, first_q};
+    TileWalk w{h0, first_q};
     for (int u = 0; u < T; ++u, next_tile(w)) {
       if (!mbar_wait_warp(bar(BAR_DQ_FULL), static_cast<uint32_t>(u) & 1u, abort_flag)) break;
       tc_fence_after();
@@ -407,7 +411,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     bool ok = true;
     const unsigned long long scale2 = f2_pack(p.scale_log2, p.scale_log2), dscale2 = f2_pack(p.scale, p.scale);
-    TileWalk w{hk * rep, first_q};
+    TileWalk w{h0, first_q};
     const uint32_t s_addr = tmem_base + Ly::COL_S + g * CPT + lane_addr;
     const uint32_t dp_addr = tmem_base + Ly::COL_DP + g * CPT + lane_addr;
     const bool beyond = jb * BKV + row >= p.seq;  // this key
@@ -521,6 +525,15 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
         for (int c = 0; c < CW / 32; ++c) tmem_ld32(tmem_base + col + c * 32 + lane_addr, v + c * 32);
         tmem_wait_ld();
+        if (p.split > 1) {
+          float4* part = p.dkv_part + ((static_cast<long long>(bh) * n_qtiles + jb) * p.split + share) * (2 * D / 4 * BKV) +
+                         (which * D / 4 + g * CW / 4) * BKV + row;
+#pragma unroll
+          for (int c = 0; c < CW / 4; ++c)
+            part[c * BKV] = make_float4(__uint_as_float(v[4 * c]), __uint_as_float(v[4 * c + 1]), __uint_as_float(v[4 * c + 2]),
+                                        __uint_as_float(v[4 * c + 3]));
+          continue;
+        }
 #pragma unroll
         for (int c = 0; c < CW / 8; ++c) {
           float f[8];
@@ -589,7 +602,7 @@ __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bflo
 
 // dq (bf16, row stride ld) = accumulator (fp32, per 128 queries and head [D / 32][32 groups of 4 queries][32][4 queries]),
 // rotated back with `rope`.  A warp takes 64 head-dim elements, two a lane, of CAST_GROUPS groups of four queries: 512
-// consecutive bytes a half warp and load, 128 a warp and store.  (Eight elements of a group a lane: 47 us for 8 x 2048, 32 heads
+// consecutive bytes a half warp and load, 128 a warp and store.  (Eight elements of a group a lane: 44 us for 8 x 2048, 32 heads
 // of 64, against 27.)
 constexpr int CAST_GROUPS = 4;
 
@@ -636,6 +649,55 @@ __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __
   }
 }
 
+// dK and dV of a key block (bf16) from the shares' sums, added in their order; dK is rotated back with `rope`.  A block takes 32
+// head-dim elements of dV (blockIdx.y < D / 32) or dK, a thread 16 of them of one key.
+template <int D>
+__global__ void __launch_bounds__(256) attention_dkv_cast_kernel(const float4* __restrict__ part, const BwdParams p) {
+  const int tiles = (p.seq + BKV - 1) / BKV;
+  const int bh = static_cast<int>(blockIdx.x) / tiles, jb = static_cast<int>(blockIdx.x) % tiles;
+  const int which = static_cast<int>(blockIdx.y) / (D / 32);
+  const int key = threadIdx.x >> 1, d0 = static_cast<int>(blockIdx.y) % (D / 32) * 32 + (threadIdx.x & 1) * 16;
+  const int pos = jb * BKV + key;
+  if (pos >= p.seq) return;
+  const float4* src = part + static_cast<long long>(blockIdx.x) * p.split * (2 * D / 4 * BKV) + (which * D / 4 + d0 / 4) * BKV + key;
+  float f[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) f[e] = 0.f;
+  for (int s = 0; s < p.split; ++s, src += 2 * D / 4 * BKV) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float4 x = src[c * BKV];
+      f[4 * c] += x.x;
+      f[4 * c + 1] += x.y;
+      f[4 * c + 2] += x.z;
+      f[4 * c + 3] += x.w;
+    }
+  }
+  if (which == 1 && p.rope != nullptr) {
+    const float4* cs = p.rope + static_cast<long long>(pos) * (D / 4) + d0 / 4;
+    rotate_back(f, cs[0], cs[1]);
+    rotate_back(f + 8, cs[2], cs[3]);
+  }
+  const int b = bh / p.n_kv_heads, hk = bh % p.n_kv_heads;
+  __nv_bfloat16* dst = (which == 0 ? p.dV : p.dK) + (static_cast<long long>(b) * p.seq + pos) * (which == 0 ? p.ld_dv : p.ld_dk) + hk * D + d0;
+  reinterpret_cast<ftb200::bf16x8*>(dst)[0] = ftb200::pack8(f);
+  reinterpret_cast<ftb200::bf16x8*>(dst)[1] = ftb200::pack8(f + 8);
+}
+
+// How many CTAs share the query heads of a kv head: one where every SM has a CTA anyway, else as many as divide the heads and stay
+// at four CTAs a SM.  The CTA of the first key block walks over all of a head's tiles, so its heads are the longest chain; what
+// sharing costs is dK and dV in fp32, written and read once more.  Whole pass, us: 3 x 1000, 8/2 heads of 128 (48 CTAs) 102 -> 48;
+// 1 x 1024, 8/2 of 128 (16) 92 -> 37; 1 x 1536, 32/8 of 128 (96) 146 -> 99; 2 x 2048, 16/4 of 128 (128) 188 -> 144; 1 x 2048,
+// 32/8 of 64 (128) 133 -> 98.  Beyond one CTA a SM it loses: 2 x 2048, 32/8 of 128 (256) 222 -> 238.
+int head_split(long long ctas, int rep) {
+  const int sms = ftb200::sm_count();
+  int split = 1;
+  if (ctas <= sms)
+    for (int s = 2; s <= rep; ++s)
+      if (rep % s == 0 && ctas * s <= 4LL * sms) split = s;
+  return split;
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static bool tried = false;
@@ -669,11 +731,14 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 }  // namespace
 
-// Scratch the backward pass needs, in bytes: fp32 dQ accumulator, -scale delta, -log2(e) lse.
-// (sized for head dim 128; enough for 64 as well)
-FTB200_API long long ftb200_attention_bwd_scratch_bytes(int batch, int seq, int n_heads) {
-  const long long rows = static_cast<long long>(batch) * ((static_cast<long long>(seq) + BQ - 1) / BQ * BQ);
-  return rows * n_heads * 128 * 4 + 2 * rows * n_heads * 4;
+// Scratch the backward pass needs, in bytes: fp32 dQ accumulator, -scale delta, -log2(e) lse, and the shares' dV and dK where the
+// query heads are shared out.  (sized for head dim 128; enough for 64 as well)
+FTB200_API long long ftb200_attention_bwd_scratch_bytes(int batch, int seq, int n_heads, int n_kv_heads) {
+  if (batch <= 0 || seq <= 0 || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads != 0) return 0;
+  const long long tiles = (static_cast<long long>(seq) + BQ - 1) / BQ, rows = batch * tiles * BQ;
+  const long long ctas = batch * tiles * n_kv_heads;
+  const int split = head_split(ctas, n_heads / n_kv_heads);
+  return rows * n_heads * 128 * 4 + 2 * rows * n_heads * 4 + (split > 1 ? ctas * split * (2 * 128 * BKV * 4) : 0);
 }
 
 namespace {
@@ -690,6 +755,7 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   float* dq_acc = reinterpret_cast<float*>(scratch);
   float* neg_delta = dq_acc + rows * n_heads * D;
   float* neg_lse2 = neg_delta + rows * n_heads;
+  const int split = head_split(batch * tiles * n_kv_heads, n_heads / n_kv_heads);
   if (rows > 0x7fffffffLL) return FTB200_E_TOOBIG;
   CUtensorMap tq, tk, tv, tdo;
   int rc = encode_rows(&tq, q, batch, seq, static_cast<long long>(n_heads) * D, ld_q);
@@ -720,13 +786,17 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   p.dK = reinterpret_cast<__nv_bfloat16*>(dk); p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
   p.ld_dk = ld_dk; p.ld_dv = ld_dv; p.status = status;
   p.rope = reinterpret_cast<const float4*>(cos_sin);
-  const long long grid = static_cast<long long>(batch) * n_kv_heads * tiles;
+  p.split = split;
+  p.dkv_part = reinterpret_cast<float4*>(neg_lse2 + rows * n_heads);
+  const long long grid = static_cast<long long>(batch) * n_kv_heads * tiles * split;
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
   attention_bwd_kernel<D><<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
   const long long cast_warps = batch * tiles * n_heads * (D / 64) * (32 / CAST_GROUPS);
   attention_dq_cast_kernel<D><<<static_cast<unsigned>((cast_warps + 7) / 8), 256, 0, stream>>>(
       reinterpret_cast<const float4*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), cast_warps, n_heads, ld_dq, seq,
       reinterpret_cast<const float2*>(cos_sin));
+  if (split > 1)
+    attention_dkv_cast_kernel<D><<<dim3(static_cast<unsigned>(batch * n_kv_heads * tiles), 2 * D / 32), 256, 0, stream>>>(p.dkv_part, p);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 

@@ -181,7 +181,7 @@ class Tcgen05Attention:
         qkv, out, lse = self._saved.pop(layer)
         q, k, v = self._views(qkv)
         dq, dk, dv = self._views(dqkv)
-        need = K.attention_bwd_scratch_bytes(batch, seq, c.n_heads)
+        need = K.attention_bwd_scratch_bytes(batch, seq, c.n_heads, c.n_kv_heads)
         if self._scratch is None or self._scratch.numel() < need:
             self._scratch = torch.empty(need, dtype=torch.uint8, device=qkv.device)
         K.attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, causal=True,

@@ -716,11 +716,11 @@ def ref_attention_bwd(q, k, v, d_o, causal=True):
 _attn_scratch: dict = {}
 
 
-def attention_bwd_scratch_bytes(batch: int, seq_len: int, n_heads: int) -> int:
+def attention_bwd_scratch_bytes(batch: int, seq_len: int, n_heads: int, n_kv_heads: int) -> int:
     """Size of the ``scratch`` that :func:`attention_bwd` takes."""
     lib = N.lib()
     lib.ftb200_attention_bwd_scratch_bytes.restype = ctypes.c_longlong
-    return int(lib.ftb200_attention_bwd_scratch_bytes(batch, seq_len, n_heads))
+    return int(lib.ftb200_attention_bwd_scratch_bytes(batch, seq_len, n_heads, n_kv_heads))
 
 
 def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Tensor, d_o: torch.Tensor,
@@ -753,7 +753,7 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
                              or rope.shape[0] < seq_len or tuple(rope.shape[1:]) != (head_dim // 2, 2)):
         raise ValueError("rope must be the table of the sequence and head dim on the device of q")
     lib = N.lib()
-    need = attention_bwd_scratch_bytes(batch, seq_len, n_heads)
+    need = attention_bwd_scratch_bytes(batch, seq_len, n_heads, n_kv_heads)
     if scratch is None:
         key = (q.device.index, _stream())
         scratch = _attn_scratch.get(key)
@@ -768,5 +768,6 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
                              batch, seq_len, n_heads, n_kv_heads, head_dim, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
                              d_o.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), scale, int(causal), _at(rope),
                              _status_ptr(q.device), _stream()),
-        "attention_bwd", launches=3,
+        # a fourth kernel where the scratch has room for dK and dV of shared heads
+        "attention_bwd", launches=3 + (need > batch * -(-seq_len // 128) * 128 * n_heads * (128 * 4 + 8)),
     )
