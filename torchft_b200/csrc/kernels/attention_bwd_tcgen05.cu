@@ -168,6 +168,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   // tiles have to start at their swizzle atom; there is no room to move them up to it
   if ((smem_base & 1023u) != 0) {
+    ftb200::wait_for_previous();
     if (threadIdx.x == 0 && p.status != nullptr) atomicExch(p.status, FTB200_ST_BOUNDS);
     return;
   }
@@ -224,6 +225,8 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
+  ftb200::wait_for_previous();
+
   if (warp < 4) {
     regs_dec<ISSUE_REGS>();
     if (warp == 0) {
@@ -272,6 +275,7 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
         __syncwarp();
       }
+      ftb200::start_next();
       if (!ok) {
         const uint64_t t0 = ftb200::globaltimer_ns();
         while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -563,12 +567,14 @@ attention_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // accumulator zeroed.  A thread takes 8 elements (16 bytes of each), D / 8 neighbouring lanes a (row, head); `pieces` counts the
 // rows of whole tiles.
 template <int D>
-__global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o,
-                                                                 const __nv_bfloat16* __restrict__ d_o,
-                                                                 const float* __restrict__ lse, float* __restrict__ neg_lse2,
-                                                                 float* __restrict__ neg_delta, float4* __restrict__ dq_acc,
+__global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bfloat16* o,
+                                                                 const __nv_bfloat16* d_o,
+                                                                 const float* lse, float* neg_lse2,
+                                                                 float* neg_delta, float4* dq_acc,
                                                                  int seq, int n_heads, long long pieces, long long ld_o,
                                                                  long long ld_do, float scale) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   constexpr int LANES = D / 8;
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool live = i < pieces;
@@ -607,9 +613,11 @@ __global__ void __launch_bounds__(256) attention_bwd_prep_kernel(const __nv_bflo
 constexpr int CAST_GROUPS = 4;
 
 template <int D>
-__global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
+__global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* acc, __nv_bfloat16* dq,
                                                                 long long warps, int n_heads, long long ld, int seq,
-                                                                const float2* __restrict__ rope) {
+                                                                const float2* rope) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   constexpr int PER_HEAD = (D / 64) * (32 / CAST_GROUPS);  // warps per tile and head
   const long long wi = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (wi >= warps) return;
@@ -652,7 +660,9 @@ __global__ void __launch_bounds__(256) attention_dq_cast_kernel(const float4* __
 // dK and dV of a key block (bf16) from the shares' sums, added in their order; dK is rotated back with `rope`.  A block takes 32
 // head-dim elements of dV (blockIdx.y < D / 32) or dK, a thread 16 of them of one key.
 template <int D>
-__global__ void __launch_bounds__(256) attention_dkv_cast_kernel(const float4* __restrict__ part, const BwdParams p) {
+__global__ void __launch_bounds__(256) attention_dkv_cast_kernel(const float4* part, const BwdParams p) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int tiles = (p.seq + BKV - 1) / BKV;
   const int bh = static_cast<int>(blockIdx.x) / tiles, jb = static_cast<int>(blockIdx.x) % tiles;
   const int which = static_cast<int>(blockIdx.y) / (D / 32);
@@ -776,7 +786,7 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   }
   const long long pieces = rows * n_heads * (D / 8);
   if ((pieces + 255) / 256 > 0x7fffffffLL) return FTB200_E_TOOBIG;
-  attention_bwd_prep_kernel<D><<<static_cast<unsigned>((pieces + 255) / 256), 256, 0, stream>>>(
+  ftb200::launch_after(attention_bwd_prep_kernel<D>, static_cast<unsigned>((pieces + 255) / 256), 256, 0, stream,
       reinterpret_cast<const __nv_bfloat16*>(o), reinterpret_cast<const __nv_bfloat16*>(d_o), lse, neg_lse2, neg_delta,
       reinterpret_cast<float4*>(dq_acc), seq, n_heads, pieces, ld_o, ld_do, scale);
   BwdParams p;
@@ -790,13 +800,15 @@ int attention_bwd_impl(const void* q, const void* k, const void* v, const void* 
   p.dkv_part = reinterpret_cast<float4*>(neg_lse2 + rows * n_heads);
   const long long grid = static_cast<long long>(batch) * n_kv_heads * tiles * split;
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
-  attention_bwd_kernel<D><<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p);
+  ftb200::launch_after(attention_bwd_kernel<D>, static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream, tq, tk, tv, tdo,
+      p);
   const long long cast_warps = batch * tiles * n_heads * (D / 64) * (32 / CAST_GROUPS);
-  attention_dq_cast_kernel<D><<<static_cast<unsigned>((cast_warps + 7) / 8), 256, 0, stream>>>(
+  ftb200::launch_after(attention_dq_cast_kernel<D>, static_cast<unsigned>((cast_warps + 7) / 8), 256, 0, stream,
       reinterpret_cast<const float4*>(dq_acc), reinterpret_cast<__nv_bfloat16*>(dq), cast_warps, n_heads, ld_dq, seq,
       reinterpret_cast<const float2*>(cos_sin));
   if (split > 1)
-    attention_dkv_cast_kernel<D><<<dim3(static_cast<unsigned>(batch * n_kv_heads * tiles), 2 * D / 32), 256, 0, stream>>>(p.dkv_part, p);
+    ftb200::launch_after(attention_dkv_cast_kernel<D>, dim3(static_cast<unsigned>(batch * n_kv_heads * tiles), 2 * D / 32),
+        256, 0, stream, p.dkv_part, p);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 

@@ -154,6 +154,8 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
+  ftb200::wait_for_previous();
+
   if (warp < 4) {
     regs_dec<ISSUE_REGS>();
     if (warp == 0) {
@@ -190,6 +192,7 @@ attention_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         __syncwarp();
       }
+      ftb200::start_next();
       if (!ok) {
         // copies in flight land in this CTA's shared memory: give them time before the CTA exits
         const uint64_t t0 = ftb200::globaltimer_ns();
@@ -492,7 +495,8 @@ int launch_fwd2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap&
     if (attr.numRegs < LAUNCH_REGS) return FTB200_E_REGS;
     attr_set = true;
   }
-  attention_fwd2_kernel<D, POLY><<<static_cast<unsigned>(grid), NUM_THREADS, Cfg<D>::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  ftb200::launch_after(attention_fwd2_kernel<D, POLY>, static_cast<unsigned>(grid), NUM_THREADS, Cfg<D>::SMEM_BYTES, stream,
+      tq, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 

@@ -14,8 +14,10 @@ using ftb200::unpack8;
 namespace {
 
 // ------------------------------------------------------------------ embedding
-__global__ void embedding_fwd_kernel(const int64_t* __restrict__ tok, const bf16x8* __restrict__ table,
-                                     bf16x8* __restrict__ out, int T, int D8, int V) {
+__global__ void embedding_fwd_kernel(const int64_t* tok, const bf16x8* table,
+                                     bf16x8* out, int T, int D8, int V) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int t = blockIdx.x;
   if (t >= T) return;
   int64_t id = tok[t];
@@ -25,8 +27,10 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ tok, const bf16
   for (int i = threadIdx.x; i < D8; i += blockDim.x) dst[i] = src[i];
 }
 
-__global__ void embedding_bwd_kernel(const int64_t* __restrict__ tok, const __nv_bfloat162* __restrict__ dout,
-                                     __nv_bfloat162* __restrict__ dtable, int T, int D2, int V) {
+__global__ void embedding_bwd_kernel(const int64_t* tok, const __nv_bfloat162* dout,
+                                     __nv_bfloat162* dtable, int T, int D2, int V) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int t = blockIdx.x;
   if (t >= T) return;
   int64_t id = tok[t];
@@ -62,9 +66,11 @@ constexpr int NORM_THREADS = 256;
 // 8192 x 4096 (51.8 now, 5.2 TB/s), 32.4 for 8192 x 2048 (28.0), 9.5 for 3000 x 1024 (7.8).
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
-rmsnorm_fwd_kernel(const bf16x8* __restrict__ x, const bf16x8* __restrict__ res, bf16x8* __restrict__ h_out,
-                   const bf16x8* __restrict__ w, bf16x8* __restrict__ out, float* __restrict__ rstd_out, int T, int D8,
+rmsnorm_fwd_kernel(const bf16x8* x, const bf16x8* res, bf16x8* h_out,
+                   const bf16x8* w, bf16x8* out, float* rstd_out, int T, int D8,
                    float eps) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   __shared__ float part[NORM_THREADS / 32];
   const int64_t row = static_cast<int64_t>(blockIdx.x) * (NORM_THREADS / TPR) + threadIdx.x / TPR;
   if (row >= T) return;  // a whole group
@@ -118,9 +124,11 @@ rmsnorm_fwd_kernel(const bf16x8* __restrict__ x, const bf16x8* __restrict__ res,
 }
 
 // The same for rows longer than 8192 elements: a block per row, which is read twice.
-__global__ void rmsnorm_fwd_long_kernel(const bf16x8* __restrict__ x, const bf16x8* __restrict__ res,
-                                        bf16x8* __restrict__ h_out, const bf16x8* __restrict__ w,
-                                        bf16x8* __restrict__ out, float* __restrict__ rstd_out, int D8, float eps) {
+__global__ void rmsnorm_fwd_long_kernel(const bf16x8* x, const bf16x8* res,
+                                        bf16x8* h_out, const bf16x8* w,
+                                        bf16x8* out, float* rstd_out, int D8, float eps) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
   const bf16x8* xr = x + row * D8;
@@ -164,9 +172,11 @@ constexpr int NORM_BWD_THREADS = 512;
 // 8192 x 2048 45.3 us (38.0 now, both kernels), 3000 x 1024 19.4 (14.0), 2500 x 8192 60.9 (50.7), 8192 x 4096 67.8 (66.8).
 template <int TPR, int VPT>
 __global__ void __launch_bounds__(NORM_BWD_THREADS, 1)
-rmsnorm_bwd_kernel(const bf16x8* __restrict__ dy, const bf16x8* __restrict__ x, const bf16x8* __restrict__ w,
-                   const float* __restrict__ rstd, const bf16x8* __restrict__ dres, bf16x8* __restrict__ dx,
-                   float* __restrict__ dw_partial, int T, int D8) {
+rmsnorm_bwd_kernel(const bf16x8* dy, const bf16x8* x, const bf16x8* w,
+                   const float* rstd, const bf16x8* dres, bf16x8* dx,
+                   float* dw_partial, int T, int D8) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   constexpr int GROUPS = NORM_BWD_THREADS / TPR;
   __shared__ float part[2][NORM_BWD_THREADS / 32];
   __shared__ float4 dw_groups[NORM_BWD_THREADS][2];
@@ -252,8 +262,10 @@ rmsnorm_bwd_kernel(const bf16x8* __restrict__ dy, const bf16x8* __restrict__ x, 
 
 // dw[c] (+)= sum_b partial[b][c].  A block owns 32 columns; its 32 warps stride over the rows (each warp instruction reads
 // one 128-byte row segment) and meet in shared memory: a row of partial sums per SM is five independent loads a thread.
-__global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw,
+__global__ void __launch_bounds__(1024) colsum_partials_kernel(const float* partial, __nv_bfloat16* dw,
                                                                int nblk, int D, int accumulate) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   __shared__ float red[32][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -293,9 +305,10 @@ int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float
   return with_row_shape(D8, T <= sms, [&](auto tpr, auto vpt) {
     constexpr int GROUPS = NORM_BWD_THREADS / tpr;
     const int nblk = std::min((T + 3) / 4, sms);
-    rmsnorm_bwd_kernel<tpr, vpt><<<nblk, NORM_BWD_THREADS, 0, st>>>((const bf16x8*)dy, (const bf16x8*)x, (const bf16x8*)w,
-                                                                       rstd, (const bf16x8*)dres, (bf16x8*)dx, dw_partial, T, D8);
-    colsum_partials_kernel<<<(D + 31) / 32, 1024, 0, st>>>(dw_partial, (__nv_bfloat16*)dw, nblk, D, accumulate_dw);
+    ftb200::launch_after(rmsnorm_bwd_kernel<tpr, vpt>, nblk, NORM_BWD_THREADS, 0, st, (const bf16x8*)dy, (const bf16x8*)x,
+        (const bf16x8*)w, rstd, (const bf16x8*)dres, (bf16x8*)dx, dw_partial, T, D8);
+    ftb200::launch_after(colsum_partials_kernel, (D + 31) / 32, 1024, 0, st, dw_partial, (__nv_bfloat16*)dw, nblk, D,
+        accumulate_dw);
     return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
   });
 }
@@ -304,8 +317,10 @@ int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float
 // buf rows are [n_rot_heads * Dh | untouched tail]; cs = [S, Dh/2] of (cos, sin).
 // One thread rotates 8 consecutive elements (4 pairs): one 16-byte load/store of data and
 // two 16-byte loads of the table.
-__global__ void rope_kernel(bf16x8* __restrict__ buf, const float4* __restrict__ cs, int64_t T, int S, int n_heads,
+__global__ void rope_kernel(bf16x8* buf, const float4* cs, int64_t T, int S, int n_heads,
                             int Dh8, int64_t row_stride8, float sin_sign) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t per_row = static_cast<int64_t>(n_heads) * Dh8;
   if (idx >= T * per_row) return;
@@ -341,7 +356,9 @@ __device__ __forceinline__ void store4_bf16(__nv_bfloat16* p, const float* f) {
   *reinterpret_cast<uint2*>(p) = o;
 }
 
-__global__ void swiglu_fwd_kernel(const bf16x8* __restrict__ gu, __nv_bfloat16* __restrict__ out, int64_t n8) {
+__global__ void swiglu_fwd_kernel(const bf16x8* gu, __nv_bfloat16* out, int64_t n8) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= n8) return;
   float f[8], o[4];
@@ -352,7 +369,9 @@ __global__ void swiglu_fwd_kernel(const bf16x8* __restrict__ gu, __nv_bfloat16* 
 }
 
 // dgu pair = (ds * u * dsilu(g), ds * silu(g))   (may alias gu: in place)
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ ds, const bf16x8* gu, bf16x8* dgu, int64_t n8) {
+__global__ void swiglu_bwd_kernel(const __nv_bfloat16* ds, const bf16x8* gu, bf16x8* dgu, int64_t n8) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= n8) return;
   float f[8], o[8];
@@ -379,8 +398,10 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ ds, const bf
 constexpr int CE_LOADS = 2;
 
 __global__ void __launch_bounds__(1024, 2)
-cross_entropy_kernel(bf16x8* __restrict__ logits, const int64_t* __restrict__ target, float* __restrict__ loss, int V8,
+cross_entropy_kernel(bf16x8* logits, const int64_t* target, float* loss, int V8,
                      int64_t ld8, float grad_scale, int grad) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
   bf16x8* lr = logits + row * ld8;
@@ -446,8 +467,10 @@ cross_entropy_kernel(bf16x8* __restrict__ logits, const int64_t* __restrict__ ta
 
 // loss[row] from the maxima, sums and target values that the tiles of a product noted (ftb200_gemm_bf16_loss), a warp a row.
 __global__ void __launch_bounds__(256)
-cross_entropy_rows_kernel(const long long* __restrict__ target, const float2* __restrict__ stats,
-                          const float* __restrict__ target_value, float* __restrict__ loss, int tiles, int T, long long V) {
+cross_entropy_rows_kernel(const long long* target, const float2* stats,
+                          const float* target_value, float* loss, int tiles, int T, long long V) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= T) return;
@@ -525,7 +548,9 @@ __global__ void adamw_kernel(float* __restrict__ master, float* __restrict__ m, 
 
 // sum of squares of a bf16 (or fp32) buffer, accumulated into *out with one atomic per block.
 template <typename G>
-__global__ void sumsq_kernel(const G* __restrict__ x, int64_t n, float* __restrict__ out) {
+__global__ void sumsq_kernel(const G* x, int64_t n, float* out) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   __shared__ float scratch[33];
   float s = 0.f;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -550,8 +575,10 @@ __global__ void sumsq_kernel(const G* __restrict__ x, int64_t n, float* __restri
 }
 
 // coef = min(1, max_norm / (sqrt(sumsq) + 1e-6)); also stores the norm.
-__global__ void clip_coef_kernel(const float* __restrict__ sumsq, float max_norm, float* __restrict__ coef,
-                                 float* __restrict__ norm_out) {
+__global__ void clip_coef_kernel(const float* sumsq, float max_norm, float* coef,
+                                 float* norm_out) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const float nrm = sqrtf(*sumsq);
   if (norm_out) *norm_out = nrm;
   *coef = (max_norm > 0.f) ? fminf(1.f, max_norm / (nrm + 1e-6f)) : 1.f;
@@ -567,14 +594,15 @@ int grid_for(int64_t work_items, int block) {
 FTB200_API int ftb200_embedding_fwd(const int64_t* tok, const void* table, void* out, int T, int D, int V,
                                     cudaStream_t st) {
   if (D % 8) return FTB200_E_ALIGN;
-  embedding_fwd_kernel<<<T, 256, 0, st>>>(tok, (const bf16x8*)table, (bf16x8*)out, T, D / 8, V);
+  ftb200::launch_after(embedding_fwd_kernel, T, 256, 0, st, tok, (const bf16x8*)table, (bf16x8*)out, T, D / 8, V);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 FTB200_API int ftb200_embedding_bwd(const int64_t* tok, const void* dout, void* dtable, int T, int D, int V,
                                     cudaStream_t st) {
   if (D % 8) return FTB200_E_ALIGN;
-  embedding_bwd_kernel<<<T, 256, 0, st>>>(tok, (const __nv_bfloat162*)dout, (__nv_bfloat162*)dtable, T, D / 2, V);
+  ftb200::launch_after(embedding_bwd_kernel, T, 256, 0, st, tok, (const __nv_bfloat162*)dout, (__nv_bfloat162*)dtable, T,
+      D / 2, V);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
@@ -586,13 +614,13 @@ FTB200_API int ftb200_rmsnorm_fwd(const void* x, const void* res, void* h_out, c
   const int D8 = D / 8;
   const int rc = with_row_shape(D8, T <= 4 * ftb200::sm_count(), [&](auto tpr, auto vpt) {
     constexpr int ROWS = NORM_THREADS / tpr;
-    rmsnorm_fwd_kernel<tpr, vpt><<<(T + ROWS - 1) / ROWS, NORM_THREADS, 0, st>>>(
-        (const bf16x8*)x, (const bf16x8*)res, (bf16x8*)h_out, (const bf16x8*)w, (bf16x8*)out, rstd, T, D8, eps);
+    ftb200::launch_after(rmsnorm_fwd_kernel<tpr, vpt>, (T + ROWS - 1) / ROWS, NORM_THREADS, 0, st, (const bf16x8*)x,
+        (const bf16x8*)res, (bf16x8*)h_out, (const bf16x8*)w, (bf16x8*)out, rstd, T, D8, eps);
     return 0;
   });
   if (rc != 0)
-    rmsnorm_fwd_long_kernel<<<T, 512, 0, st>>>((const bf16x8*)x, (const bf16x8*)res, (bf16x8*)h_out, (const bf16x8*)w,
-                                               (bf16x8*)out, rstd, D8, eps);
+    ftb200::launch_after(rmsnorm_fwd_long_kernel, T, 512, 0, st, (const bf16x8*)x, (const bf16x8*)res, (bf16x8*)h_out,
+        (const bf16x8*)w, (bf16x8*)out, rstd, D8, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
@@ -613,36 +641,37 @@ FTB200_API int ftb200_rope(void* buf, const float* cos_sin, long long T, int S, 
                            long long row_stride, int backward, cudaStream_t st) {
   if (head_dim % 8 || row_stride % 8 || (reinterpret_cast<uintptr_t>(buf) & 15)) return FTB200_E_ALIGN;
   const int64_t total = T * n_heads * (head_dim / 8);
-  rope_kernel<<<grid_for(total, 256), 256, 0, st>>>((bf16x8*)buf, (const float4*)cos_sin, T, S, n_heads, head_dim / 8,
-                                                    row_stride / 8, backward ? -1.f : 1.f);
+  ftb200::launch_after(rope_kernel, grid_for(total, 256), 256, 0, st, (bf16x8*)buf, (const float4*)cos_sin, T, S, n_heads,
+      head_dim / 8, row_stride / 8, backward ? -1.f : 1.f);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 FTB200_API int ftb200_swiglu_fwd(const void* gu, void* out, long long T, int F, cudaStream_t st) {
   if (F % 4) return FTB200_E_ALIGN;
   const int64_t n8 = T * (F / 4);
-  swiglu_fwd_kernel<<<grid_for(n8, 256), 256, 0, st>>>((const bf16x8*)gu, (__nv_bfloat16*)out, n8);
+  ftb200::launch_after(swiglu_fwd_kernel, grid_for(n8, 256), 256, 0, st, (const bf16x8*)gu, (__nv_bfloat16*)out, n8);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 FTB200_API int ftb200_swiglu_bwd(const void* ds, const void* gu, void* dgu, long long T, int F, cudaStream_t st) {
   if (F % 4) return FTB200_E_ALIGN;
   const int64_t n8 = T * (F / 4);
-  swiglu_bwd_kernel<<<grid_for(n8, 256), 256, 0, st>>>((const __nv_bfloat16*)ds, (const bf16x8*)gu, (bf16x8*)dgu, n8);
+  ftb200::launch_after(swiglu_bwd_kernel, grid_for(n8, 256), 256, 0, st, (const __nv_bfloat16*)ds, (const bf16x8*)gu,
+      (bf16x8*)dgu, n8);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 FTB200_API int ftb200_cross_entropy(void* logits, const int64_t* target, float* loss, int T, int V, long long ld,
                                     float grad_scale, int grad, cudaStream_t st) {
   if (V % 8 || ld % 8) return FTB200_E_ALIGN;
-  cross_entropy_kernel<<<T, 1024, 0, st>>>((bf16x8*)logits, target, loss, V / 8, ld / 8, grad_scale, grad);
+  ftb200::launch_after(cross_entropy_kernel, T, 1024, 0, st, (bf16x8*)logits, target, loss, V / 8, ld / 8, grad_scale, grad);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 // Second half of ftb200_gemm_bf16_loss.
 int ftb200_launch_cross_entropy_rows(const long long* target, const float2* row_stats, const float* target_value, float* loss,
                                      int tiles, int T, int V, cudaStream_t st) {
-  cross_entropy_rows_kernel<<<(T + 7) / 8, 256, 0, st>>>(target, row_stats, target_value, loss, tiles, T, V);
+  ftb200::launch_after(cross_entropy_rows_kernel, (T + 7) / 8, 256, 0, st, target, row_stats, target_value, loss, tiles, T, V);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
@@ -675,14 +704,14 @@ FTB200_API int ftb200_sumsq(const void* x, int is_fp32, long long n, float* out,
   if (reinterpret_cast<uintptr_t>(x) & 15) return FTB200_E_ALIGN;
   const int blocks = static_cast<int>(std::min<long long>((n / 8 + 255) / 256 + 1, ftb200::sm_count() * 8LL));
   if (is_fp32)
-    sumsq_kernel<float><<<blocks, 256, 0, st>>>((const float*)x, n, out);
+    ftb200::launch_after(sumsq_kernel<float>, blocks, 256, 0, st, (const float*)x, n, out);
   else
-    sumsq_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)x, n, out);
+    ftb200::launch_after(sumsq_kernel<__nv_bfloat16>, blocks, 256, 0, st, (const __nv_bfloat16*)x, n, out);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
 FTB200_API int ftb200_clip_coef(const float* sumsq, float max_norm, float* coef, float* norm_out, cudaStream_t st) {
-  clip_coef_kernel<<<1, 1, 0, st>>>(sumsq, max_norm, coef, norm_out);
+  ftb200::launch_after(clip_coef_kernel, 1, 1, 0, st, sumsq, max_norm, coef, norm_out);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 

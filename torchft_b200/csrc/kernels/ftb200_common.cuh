@@ -168,6 +168,35 @@ __device__ __forceinline__ bf16x8 pack8(const float* f) {
   return p;
 }
 
+// Kernels of a step follow one another every few microseconds, and a launch that waits for the whole of the one before leaves the
+// chip empty while it is set up (barriers, tensor maps, tensor memory, the launch itself: about 2 us).  So they are launched
+// (launch_after) as dependents that may become resident while the kernel before them on the stream drains:
+//  * such a kernel calls wait_for_previous in every thread before it touches global memory or returns.  It returns when the
+//    kernel before has ended and its writes are visible, and since that one waited likewise, when all before it have;
+//  * start_next says that the one behind may become resident.  It is called after wait_for_previous (so no more than one
+//    kernel waits on the chip) by at least a thread of every CTA that lives long, and holds back nothing else;
+//  * their pointers are not __restrict__: a read-only load of a kernel's whole life may not see what was written during it.
+// Kernels that wait for other GPUs are launched as usual and do not call start_next.  Neither does AdamW wait: its 250 us and more
+// gain nothing.  A step of two layers on 256 tokens (79 launches, a graph) 369 -> 310 us; of four layers of width 1024 on
+// 3 x 1000 tokens 2138 -> 1982; the evaluation of a 16-layer model 10.4 -> 10.0 ms.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... Params, class... Args>
+void launch_after(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // cudaGetLastError tells
+}
+
 inline int sm_count() {
   static int n = 0;
   if (n == 0) {

@@ -372,6 +372,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   cluster_sync_relaxed();  // the partner's barriers exist (they were fenced) before anything signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  ftb200::wait_for_previous();
 
   if (warp == 0) {
     // ---------------- TMA producer (both CTAs) ----------------
@@ -421,6 +422,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         }
       }
     }
+    if (p.ga_world == 0 && p.sc_world == 0) ftb200::start_next();
     if (!ok) {
       const uint64_t t0 = ftb200::globaltimer_ns();
       while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -901,8 +903,10 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
 constexpr int GEMV_ROWS = 2, GEMV_LOADS = 4, GEMV_THREADS = 256;
 
 __global__ void __launch_bounds__(GEMV_THREADS)
-gemv_bf16_kernel(const ftb200::bf16x8* __restrict__ a, const ftb200::bf16x8* __restrict__ B, __nv_bfloat16* __restrict__ C, int N,
+gemv_bf16_kernel(const ftb200::bf16x8* a, const ftb200::bf16x8* B, __nv_bfloat16* C, int N,
                  int K8, long long ldb8) {
+  ftb200::wait_for_previous();
+  ftb200::start_next();
   const int lane = threadIdx.x & 31;
   const int n0 = (static_cast<int>(blockIdx.x) * (GEMV_THREADS / 32) + (threadIdx.x >> 5)) * GEMV_ROWS;
   if (n0 >= N) return;
@@ -1007,18 +1011,19 @@ static cudaError_t prepare_2cta() {
   return e;
 }
 
-static void cluster_launch(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr, int ctas, int pairs_per_cluster, int threads,
+// attrs: room for two.
+static void cluster_launch(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attrs, int ctas, int pairs_per_cluster, int threads,
                            uint32_t smem, cudaStream_t stream) {
   cfg = cudaLaunchConfig_t{};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2 * pairs_per_cluster;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = 2 * pairs_per_cluster;
+  attrs[0].val.clusterDim.y = 1;
+  attrs[0].val.clusterDim.z = 1;
+  cfg.attrs = attrs;
   cfg.numAttrs = 1;
 }
 
@@ -1030,8 +1035,8 @@ static int resident_clusters(int split) {
   int n = known[split].load(std::memory_order_relaxed);
   if (n == 0) {
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr;
-    cluster_launch(cfg, attr, 2 * split, split, NUM_THREADS, Tile<BN, EPI_STORE>::SMEM_BYTES, nullptr);
+    cudaLaunchAttribute attrs[2];
+    cluster_launch(cfg, attrs, 2 * split, split, NUM_THREADS, Tile<BN, EPI_STORE>::SMEM_BYTES, nullptr);
     if (prepare_2cta<BN, true, EPI_STORE>() != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, gemm_bf16_tcgen05_2cta_kernel<BN, true, EPI_STORE>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
@@ -1108,9 +1113,16 @@ static int launch_2cta(const void* A, const void* B, long long lda, long long ld
   if (prepare_2cta<BN, SPLIT, EPI>() != cudaSuccess) return FTB200_E_CUDA;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr;
-  cluster_launch(cfg, attr, SPLIT ? ctas : std::min(2 * tiles, ctas), split, threads, Tile<BN, EPI>::SMEM_BYTES, stream);
-  return cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT, EPI>, tmA, tmB, tmC, tmAux, p) == cudaSuccess ? 0 : FTB200_E_CUDA;
+  cudaLaunchAttribute attrs[2];
+  cluster_launch(cfg, attrs, SPLIT ? ctas : std::min(2 * tiles, ctas), split, threads, Tile<BN, EPI>::SMEM_BYTES, stream);
+  if (p.ga_world == 0 && p.sc_world == 0) {  // as ftb200::launch_after does
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
+  return cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_2cta_kernel<BN, SPLIT, EPI>, tmA, tmB, tmC, tmAux, p) == cudaSuccess
+             ? 0
+             : FTB200_E_CUDA;
 }
 
 static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, int K, int a_mn_major, int b_mn_major,
@@ -1124,7 +1136,7 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   if (M == 1 && !a_mn_major && !b_mn_major && flags == 0 && (K & 7) == 0 && aux == nullptr && sc == nullptr && ga == nullptr &&
       ep == nullptr && max_ctas <= 0) {
     constexpr int PER_BLOCK = GEMV_ROWS * GEMV_THREADS / 32;
-    gemv_bf16_kernel<<<(N + PER_BLOCK - 1) / PER_BLOCK, GEMV_THREADS, 0, stream>>>(
+    ftb200::launch_after(gemv_bf16_kernel, (N + PER_BLOCK - 1) / PER_BLOCK, GEMV_THREADS, 0, stream,
         reinterpret_cast<const ftb200::bf16x8*>(A), reinterpret_cast<const ftb200::bf16x8*>(B),
         reinterpret_cast<__nv_bfloat16*>(C), N, K / 8, ldb / 8);
     return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
