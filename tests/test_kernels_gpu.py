@@ -239,6 +239,24 @@ def test_cross_entropy(T, V):
     assert rel_err(logits, rg) < 1e-2
 
 
+@pytest.mark.parametrize("V", [8, 4088, 4096, 4104, 4 * 4096 - 8, 4 * 4096, 4 * 4096 + 8, 7 * 4096 + 2000])
+def test_cross_entropy_row_lengths(V):
+    """Rows that end inside a thread's batch of loads, targets at both ends.  A gradient rounds to bf16 (8
+    significant bits: half a unit of the last is up to 2^-8 of the value) after a handful of fp32 operations on numbers of at
+    most 1 (2^-20 of them, the exponential's error included)."""
+    T = 5
+    wide = torch.randn(T, V + 16, device="cuda").mul_(4).bfloat16()
+    logits = wide[:, :V]
+    tgt = torch.tensor([0, V - 1, -1, V // 2, 7], device="cuda")
+    x = logits.double()
+    loss = K.cross_entropy_(logits, tgt, 0.5)
+    onehot = torch.nn.functional.one_hot(tgt.clamp(min=0), V).double()
+    want = (x.softmax(-1) - onehot) * 0.5 * (tgt >= 0)[:, None]
+    assert bool(((logits.double() - want).abs() <= 2**-8 * want.abs() + 2**-20).all())
+    ref = (x.logsumexp(-1) - (x * onehot).sum(-1)) * (tgt >= 0)
+    assert bool(((loss.double() - ref).abs() <= 2**-18 * (1 + x.abs().amax(-1))).all())
+
+
 @pytest.mark.parametrize("V", [8, 8 * 1024, 8 * 1024 + 8, 8 * 3 * 1024 - 8, 128256])
 def test_cross_entropy_without_gradient(V):
     """One to several vectors per thread, with remainders; the logits stay as they are and the loss is the same number."""

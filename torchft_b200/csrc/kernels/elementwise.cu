@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "ftb200_common.cuh"
+#include "tcgen05_helpers.cuh"
 
 using ftb200::bf16x8;
 using ftb200::pack8;
@@ -393,19 +394,31 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* ds, const bf16x8* gu, bf1
 
 // ------------------------------------------------------------------ cross-entropy
 // One block per row.  loss[row] = logsumexp(row) - row[target]; with `grad` the row is overwritten in place by
-// (softmax - onehot) * grad_scale, without it it is only read.  Bound by memory and, next to it, by the exponential
-// unit; CE_LOADS loads in flight per thread and two blocks per SM.
-constexpr int CE_LOADS = 2;
+// (softmax - onehot) * grad_scale, without it it is only read.  Bound by memory: a row is read from DRAM and written once, and
+// read a second time from the L2, last pieces first (they are the likeliest still there) and, like the writes, without a claim to
+// stay.  The exponential unit (two an element) and the issue slots come next, hence packed pairs, no one-hot test outside
+// the target's vector, and blocks of 512: three on an SM are seldom all in the same pass, and have the registers for four loads
+// in flight.  8192 x 128256 1015 -> 778 us (5.4 TB/s), 4096 x 50304 221 -> 156, 1024 x 32000 45 -> 35, 750 x 8192 18 -> 14;
+// in blocks of 1024, two loads, 769, 172, 35, 16; first pieces first 847, 176, 39, 16.
+constexpr int CE_LOADS = 4, CE_THREADS = 512;
 
-__global__ void __launch_bounds__(1024, 2)
-cross_entropy_kernel(bf16x8* logits, const int64_t* target, float* loss, int V8,
-                     int64_t ld8, float grad_scale, int grad) {
+__global__ void __launch_bounds__(CE_THREADS, 3)
+cross_entropy_kernel(bf16x8* logits, const int64_t* target, float* loss, int V8, int64_t ld8, float grad_scale, int grad) {
+  using namespace ftb200::tc;
   ftb200::wait_for_previous();
   ftb200::start_next();
   __shared__ float scratch[33];
   const int64_t row = blockIdx.x;
   bf16x8* lr = logits + row * ld8;
-  float mx = -INFINITY, sum = 0.f;
+  const unsigned long long log2e = f2_pack(1.4426950408889634f, 1.4426950408889634f);
+  // exp(x + d) of two
+  auto exp_of = [&](float x0, float x1, unsigned long long d) {
+    float y0, y1;
+    f2_unpack(f2_mul(f2_add(f2_pack(x0, x1), d), log2e), y0, y1);
+    return f2_pack(exp2f(y0), exp2f(y1));
+  };
+  float mx = -INFINITY;
+  unsigned long long sum2 = 0ull;
   auto take = [&](const bf16x8& v) {
     float f[8];
     unpack8(v, f);
@@ -413,22 +426,26 @@ cross_entropy_kernel(bf16x8* logits, const int64_t* target, float* loss, int V8,
 #pragma unroll
     for (int e = 1; e < 8; ++e) cm = fmaxf(cm, f[e]);
     if (cm > mx) {
-      sum *= __expf(mx - cm);
+      const float a = __expf(mx - cm);
+      sum2 = f2_mul(sum2, f2_pack(a, a));
       mx = cm;
     }
+    const unsigned long long neg_mx = f2_pack(-mx, -mx);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) sum += __expf(f[e] - mx);
+    for (int e = 0; e < 8; e += 2) sum2 = f2_add(sum2, exp_of(f[e], f[e + 1], neg_mx));
   };
-  const int step = blockDim.x;
   int i = threadIdx.x;
-  for (; i + (CE_LOADS - 1) * step < V8; i += CE_LOADS * step) {
+  for (; i + (CE_LOADS - 1) * CE_THREADS < V8; i += CE_LOADS * CE_THREADS) {
     bf16x8 v[CE_LOADS];
 #pragma unroll
-    for (int u = 0; u < CE_LOADS; ++u) v[u] = lr[i + u * step];
+    for (int u = 0; u < CE_LOADS; ++u) v[u] = lr[i + u * CE_THREADS];
 #pragma unroll
     for (int u = 0; u < CE_LOADS; ++u) take(v[u]);
   }
-  for (; i < V8; i += step) take(lr[i]);
+  for (; i < V8; i += CE_THREADS) take(lr[i]);
+  float sum, sum_odd;
+  f2_unpack(sum2, sum, sum_odd);
+  sum += sum_odd;
   const float gmx = ftb200::block_max(mx, scratch);
   sum *= __expf(mx - gmx);
   const float gsum = ftb200::block_sum(sum, scratch);
@@ -436,33 +453,40 @@ cross_entropy_kernel(bf16x8* logits, const int64_t* target, float* loss, int V8,
   if (tgt >= 0) (void)FTB_IN_RANGE(tgt, 8 * static_cast<int64_t>(V8));  // negative targets mean "ignore"
   (void)FTB_IN_RANGE(V8 - 1, ld8);                                        // a row must fit inside its stride
   const float inv = 1.f / gsum;
+  const bool inside = tgt >= 0 && tgt < 8 * static_cast<int64_t>(V8);
   if (threadIdx.x == 0) {
     const __nv_bfloat16* flat = reinterpret_cast<const __nv_bfloat16*>(lr);
-    const float xt = (tgt >= 0 && tgt < 8 * static_cast<int64_t>(V8)) ? __bfloat162float(flat[tgt]) : 0.f;
-    loss[row] = (tgt >= 0) ? (logf(gsum) + gmx - xt) : 0.f;
+    loss[row] = (tgt >= 0) ? (logf(gsum) + gmx - (inside ? __bfloat162float(flat[tgt]) : 0.f)) : 0.f;
   }
   if (!grad) return;
   __syncthreads();  // the target logit is read before any thread overwrites it
   const float gs = (tgt >= 0) ? grad_scale : 0.f;
-  auto put = [&](const bf16x8& v, int at) {
+  const int tgt8 = inside ? static_cast<int>(tgt >> 3) : -1, tgt_e = static_cast<int>(tgt & 7);
+  const unsigned long long neg_gmx = f2_pack(-gmx, -gmx), scale2 = f2_pack(inv * gs, inv * gs);
+  auto put = [&](const uint4& raw, int at) {
     float f[8];
-    unpack8(v, f);
+    unpack8(*reinterpret_cast<const bf16x8*>(&raw), f);
+    if (at != tgt8) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float pr = __expf(f[e] - gmx) * inv;
-      if (static_cast<int64_t>(at) * 8 + e == tgt) pr -= 1.f;
-      f[e] = pr * gs;
+      for (int e = 0; e < 8; e += 2) f2_unpack(f2_mul(exp_of(f[e], f[e + 1], neg_gmx), scale2), f[e], f[e + 1]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = (__expf(f[e] - gmx) * inv - (e == tgt_e ? 1.f : 0.f)) * gs;
     }
-    lr[at] = pack8(f);
+    const bf16x8 out = pack8(f);
+    __stcs(reinterpret_cast<uint4*>(lr + at), *reinterpret_cast<const uint4*>(&out));
   };
-  for (i = threadIdx.x; i + (CE_LOADS - 1) * step < V8; i += CE_LOADS * step) {
-    bf16x8 v[CE_LOADS];
+  const uint4* src = reinterpret_cast<const uint4*>(lr);
+  if (static_cast<int>(threadIdx.x) >= V8) return;
+  i = threadIdx.x + (V8 - 1 - static_cast<int>(threadIdx.x)) / CE_THREADS * CE_THREADS;  // this thread's last
+  for (; i - (CE_LOADS - 1) * CE_THREADS >= 0; i -= CE_LOADS * CE_THREADS) {
+    uint4 v[CE_LOADS];
 #pragma unroll
-    for (int u = 0; u < CE_LOADS; ++u) v[u] = lr[i + u * step];
+    for (int u = 0; u < CE_LOADS; ++u) v[u] = __ldcs(src + i - u * CE_THREADS);
 #pragma unroll
-    for (int u = 0; u < CE_LOADS; ++u) put(v[u], i + u * step);
+    for (int u = 0; u < CE_LOADS; ++u) put(v[u], i - u * CE_THREADS);
   }
-  for (; i < V8; i += step) put(lr[i], i);
+  for (; i >= 0; i -= CE_THREADS) put(__ldcs(src + i), i);
 }
 
 // loss[row] from the maxima, sums and target values that the tiles of a product noted (ftb200_gemm_bf16_loss), a warp a row.
@@ -664,7 +688,7 @@ FTB200_API int ftb200_swiglu_bwd(const void* ds, const void* gu, void* dgu, long
 FTB200_API int ftb200_cross_entropy(void* logits, const int64_t* target, float* loss, int T, int V, long long ld,
                                     float grad_scale, int grad, cudaStream_t st) {
   if (V % 8 || ld % 8) return FTB200_E_ALIGN;
-  ftb200::launch_after(cross_entropy_kernel, T, 1024, 0, st, (bf16x8*)logits, target, loss, V / 8, ld / 8, grad_scale, grad);
+  ftb200::launch_after(cross_entropy_kernel, T, CE_THREADS, 0, st, (bf16x8*)logits, target, loss, V / 8, ld / 8, grad_scale, grad);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
 
