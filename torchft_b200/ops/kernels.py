@@ -768,6 +768,5 @@ def attention_bwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, o: torch.Te
                              batch, seq_len, n_heads, n_kv_heads, head_dim, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
                              d_o.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), scale, int(causal), _at(rope),
                              _status_ptr(q.device), _stream()),
-        # a fourth kernel where the scratch has room for dK and dV of shared heads
-        "attention_bwd", launches=3 + (need > batch * -(-seq_len // 128) * 128 * n_heads * (128 * 4 + 8)),
+        "attention_bwd", launches=3,
     )
