@@ -82,6 +82,24 @@ def test_gemm_split_last_wave(a_mn, b_mn, M, N, K_):
     K.check_status(out.device)
 
 
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (True, True)])
+@pytest.mark.parametrize("M,N,K_", [(8, 8, 64), (40, 72, 200), (256, 128, 64), (264, 136, 72), (296, 520, 264), (8192, 1024, 752),
+                                    (1024, 264, 3000), (752, 1024, 8200), (5000, 2056, 64)])
+def test_gemm_adds_to_bf16(M, N, K_, a_mn, b_mn):
+    """What C holds comes and goes by TMA, shared tiles excepted: the sum with the fp32 product, rounded once, to the bit, and
+    nothing beyond M and N."""
+    torch.manual_seed(M + N)
+    a = torch.randn((K_, M) if a_mn else (M, K_), device=DEV).bfloat16()
+    b = torch.randn((K_, N) if b_mn else (N, K_), device=DEV).bfloat16()
+    product = K.gemm(a, b, a_mn, b_mn, out_dtype=torch.float32)
+    out = (torch.randn(M + 3, N + 16, device=DEV) * K_**0.5).bfloat16()
+    want = out.clone()
+    want[:M, 8 : N + 8] = (want[:M, 8 : N + 8].float() + product).bfloat16()
+    K.gemm(a, b, a_mn, b_mn, out=out[:M, 8 : N + 8], accumulate=True)
+    K.check_status(out.device)
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("N", [1, 2, 17, 1000, 8192])
 @pytest.mark.parametrize("K_", [8, 72, 256, 1024, 1032, 4104])
 def test_gemm_one_row(N, K_):

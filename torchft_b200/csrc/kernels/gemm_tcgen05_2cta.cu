@@ -51,9 +51,10 @@ constexpr uint32_t A_BYTES = BM * BK * 2;
 
 // What becomes of a tile.
 enum Epilogue : int {
-  EPI_STORE = 0,    // it is stored (added, with the activation of its columns' pairs, scattered: GemmParams)
+  EPI_STORE = 0,    // it is stored (added to fp32 or rows that TMA does not take, with the activation of its columns' pairs, scattered: GemmParams)
   EPI_DSWIGLU = 1,  // it is the gradient of silu(gate) * up: the gate/up pairs it belongs to are replaced by their gradients
   EPI_LOSS = 2,     // its rows' maximum, sum of exponentials and target value are noted; it is not stored
+  EPI_ADD = 3,      // it is added to what bf16 C holds
 };
 
 // A pair's tile has 256 or 128 columns; the K ring fills 192 KB with 6 or 8 stages.  The gradient of the activation needs
@@ -302,13 +303,13 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
   auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + s); };
   auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 + s); };
   const uint32_t ready_bar = bar_base + 8u * (2 * STAGES + 4), got_bar = bar_base + 8u * (2 * STAGES + 5);
-  auto pairs_bar = [&](int q, int half) { return bar_base + 8u * (2 * STAGES + 7 + 2 * q + half); };  // EPI_DSWIGLU
+  auto pairs_bar = [&](int q, int half) { return bar_base + 8u * (2 * STAGES + 7 + 2 * q + half); };  // EPI_DSWIGLU, EPI_ADD
 
   if (warp == 0) {
     if (lane < 2 * STAGES) mbar_init(bar_base + 8u * lane, 1);                             // full, empty
     if (lane >= 16 && lane < 20) mbar_init(tfull_bar(lane - 16), lane < 18 ? 1 : 2 * 4);  // tfull, tempty (one arrival a warp)
     if (lane == 20) *abort_flag = 0;
-    if (EPI == EPI_DSWIGLU && lane >= 24) mbar_init(pairs_bar(0, lane - 24), 1);
+    if ((EPI == EPI_DSWIGLU || EPI == EPI_ADD) && lane >= 24) mbar_init(pairs_bar(0, lane - 24), 1);
     if (SPLIT && lane == 21) mbar_init(ready_bar, S - 1);
     if (SPLIT && lane == 22) mbar_init(got_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -531,21 +532,25 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
     int acc = 0;
     uint32_t acc_phase = 0;
     const bool vec_ok = p.out_fp32 ? ((p.ldc & 3) == 0) : ((p.ldc & 7) == 0);
-    uint32_t pairs_phase = 0;  // EPI_DSWIGLU: bit h, of half h
+    uint32_t pairs_phase = 0;  // EPI_DSWIGLU, EPI_ADD: bit h, of half h
     for (Work w = first; have_work(w); next_work(w)) {
       if (w.t != pair_id) tile_coords(w.t, m0, n0);
-      if constexpr (EPI == EPI_DSWIGLU) {
-        // 64 columns at a time: the 128 gate/up columns they belong to come by TMA, two pieces ahead (the first two under the
-        // tile's products), are replaced in place by their gradients, and leave by TMA.
+      if (EPI == EPI_DSWIGLU || (EPI == EPI_ADD && !(SPLIT && w.shared))) {
+        // 64 columns at a time: the 128 gate/up columns they belong to (EPI_ADD: what C holds there) come by TMA, two pieces ahead
+        // (the first two under the tile's products), are replaced in place by their gradients (the sums), and leave by TMA.
+        // A thread that reads its row of C piece by piece where it writes it waits for memory 32 times in a row: 8192 x 1024 x
+        // 750 added to C 63.5 -> 24.6 us (stored: 20.5), 1024 x 256 x 64 20.5 -> 10.2, 128256 x 2048 x 2048 1546 -> 695.
+        constexpr int BOXES = EPI == EPI_DSWIGLU ? 2 : 1;  // 64 columns each, of a piece
+        const CUtensorMap* map = EPI == EPI_DSWIGLU ? &tmAux : &tmC;
         const int row0 = m0 + q * 32;
         const uint32_t stg = OFF_STAGING + q * STAGE_WARP_BYTES;
         auto inside = [&](int c) { return n0 + c * 64 < p.N && row0 < p.M; };
         auto fetch = [&](int c) {
           mbar_expect_tx(pairs_bar(q, c & 1), STAGE_WARP_BYTES / 2);
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
-            tma_load_2d(smem_base + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + h * 4096, &tmAux, pairs_bar(q, c & 1),
-                        2 * (n0 + c * 64) + 64 * h, row0);
+          for (int h = 0; h < BOXES; ++h)
+            tma_load_2d(smem_base + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + h * 4096, map, pairs_bar(q, c & 1),
+                        BOXES * (n0 + c * 64) + 64 * h, row0);
         };
         if (lane == 0) {
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the tile before has left the staging area
@@ -581,10 +586,16 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
           pairs_phase ^= 1u << (c & 1);
           uint8_t* prow = smem + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + lane * 128;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
+          for (int j = 0; j < 8 * BOXES; ++j) {
             ftb200::bf16x8* at = reinterpret_cast<ftb200::bf16x8*>(prow + (j >> 3) * 4096 + (((j & 7) ^ (lane & 7)) << 4));
             float f[8], o[8];
             ftb200::unpack8(*at, f);
+            if (EPI == EPI_ADD) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(v[(8 * j + e) & 63]) + f[e];
+              *at = ftb200::pack8(o);
+              continue;
+            }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float d = __uint_as_float(v[4 * j + e]), g = f[2 * e], u = f[2 * e + 1];
@@ -599,9 +610,10 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
           __syncwarp();
           if (lane == 0) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+            for (int h = 0; h < BOXES; ++h)
               if (n0 + c * 64 + 32 * h < p.N)
-                tma_store_2d(&tmAux, smem_base + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + h * 4096, 2 * (n0 + c * 64) + 64 * h, row0);
+                tma_store_2d(map, smem_base + stg + (c & 1) * (STAGE_WARP_BYTES / 2) + h * 4096, BOXES * (n0 + c * 64) + 64 * h,
+                             row0);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         }
@@ -617,7 +629,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       const int row = m0 + q * 32 + lane;
       const uint32_t taddr0 = tmem_base + acc * BN + (static_cast<uint32_t>(q * 32) << 16);
       const uint32_t stg = OFF_STAGING + q * STAGE_WARP_BYTES;
-      if (EPI == EPI_LOSS || (p.tma_out && !(SPLIT && w.shared))) {
+      if (EPI == EPI_LOSS || (EPI == EPI_STORE && p.tma_out && !(SPLIT && w.shared))) {
         // bf16 output: 64 columns at a time go, one row a thread, into a 128-byte-swizzled piece of the warp's staging area
         // and leave by TMA (which clips what lies beyond M and N), while the next 64 come out of tensor memory.  Nothing hides
         // the last tile's epilogue: 5800 cycles for 256 columns that leave a row-major staging area as row segments, 4100
@@ -708,7 +720,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
         }
         continue;
       }
-      if constexpr (EPI != EPI_STORE) continue;
+      if constexpr (EPI != EPI_STORE && !(EPI == EPI_ADD && SPLIT)) continue;
       auto store_chunk = [&](int c, const uint32_t* r) {  // 32 columns of the thread's row
         const int col0 = n0 + c * 32;
         if (row < p.M && col0 < p.N) {
@@ -738,6 +750,11 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
           } else {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(row) * p.ldc + col0;
             if (full) {
+              ftb200::bf16x8 old[4];
+              if (EPI == EPI_ADD) {  // all on their way before the first store
+#pragma unroll
+                for (int j = 0; j < 4; ++j) old[j] = reinterpret_cast<const ftb200::bf16x8*>(dst)[j];
+              }
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 float f[8];
@@ -745,7 +762,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
                 for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * j + e]);
                 if (p.accumulate) {
                   float o[8];
-                  ftb200::unpack8(reinterpret_cast<const ftb200::bf16x8*>(dst)[j], o);
+                  ftb200::unpack8(EPI == EPI_ADD ? old[j] : reinterpret_cast<const ftb200::bf16x8*>(dst)[j], o);
 #pragma unroll
                   for (int e = 0; e < 8; ++e) f[e] += o[e];
                 }
@@ -1167,9 +1184,11 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
     p.sc_off = sc->off;
     for (int i = 0; i < sc->world && i < 8; ++i) p.sc_peers[i] = sc->peers[i];
   }
-  // TMA wants 16-byte rows; what else comes (fp32, accumulation, other strides) takes the general path of the epilogue
-  p.tma_out = sc == nullptr && !p.out_fp32 && !p.accumulate && (ldc & 7) == 0 && ldc >= N && (N & 7) == 0 &&
+  // TMA wants 16-byte rows; what else comes (fp32, other strides) takes the general path of the epilogue
+  p.tma_out = sc == nullptr && !p.out_fp32 && (ldc & 7) == 0 && ldc >= N && (N & 7) == 0 &&
               (aux == nullptr || ((ld_aux & 7) == 0 && ld_aux >= N / 2 && (reinterpret_cast<uintptr_t>(aux) & 15) == 0));
+  const bool add = p.tma_out && p.accumulate && ga == nullptr && aux == nullptr;
+  if (p.accumulate && !add) p.tma_out = 0;
   p.group_m = GROUP_M;
   p.whole = 0;
   p.ga_world = 0;
@@ -1208,6 +1227,13 @@ static int gemm_2cta_impl(const void* A, const void* B, void* C, int M, int N, i
   // scattered and activated outputs leave through the staging area, which a shared tile does not
   const TilePlan plan = plan_tiles(M, N, K, ctas / 2, sc == nullptr && aux == nullptr && max_ctas <= 0);
   p.whole = plan.whole;
+  if (add) {
+    if (plan.split > 1)
+      return plan.columns == 128 ? launch_2cta<128, true, EPI_ADD>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream)
+                                 : launch_2cta<256, true, EPI_ADD>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
+    return plan.columns == 128 ? launch_2cta<128, false, EPI_ADD>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream)
+                               : launch_2cta<256, false, EPI_ADD>(A, B, lda, ldb, ctas, 1, NUM_THREADS, p, stream);
+  }
   if (plan.split > 1) {
     if (plan.columns == 128) return launch_2cta<128, true, EPI_STORE>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
     return launch_2cta<256, true, EPI_STORE>(A, B, lda, ldb, plan.ctas, plan.split, NUM_THREADS, p, stream);
