@@ -12,36 +12,37 @@ class _Chain:
     """Forward and backward kernels in turn, each reading what the one before wrote, many writing what earlier ones read.
     Sequences of one key block: every sum has one order."""
 
-    def __init__(self, batch, seq, dim, ffn, seed=0):
+    def __init__(self, batch, seq, dim, ffn, head=64, seed=0):
         g = torch.Generator(device="cuda").manual_seed(seed)
         T, D, F = batch * seq, dim, ffn
         r = lambda *shape: (torch.randn(*shape, device="cuda", generator=g) * 0.1).bfloat16()  # noqa: E731
         e = lambda *shape: torch.zeros(*shape, device="cuda", dtype=torch.bfloat16)  # noqa: E731
-        self.sizes = batch, seq, dim
+        self.sizes = batch, seq, dim, head
         self.x, self.h, self.w, self.wq, self.wo, self.wu, self.wd = (r(T, D), r(T, D), r(D) + 1, r(3 * D, D), r(D, D), r(2 * F, D),
                                                                       r(D, F))
         self.n, self.qkv, self.dqkv, self.gu, self.act, self.d, self.out = (e(T, D), e(T, 3 * D), e(T, 3 * D), e(T, 2 * F), e(T, F),
                                                                             e(T, D), e(T, D))
         self.dwq, self.dw = e(3 * D, D), e(D)
-        self.rstd, self.lse = torch.zeros(T, device="cuda"), torch.zeros(batch, D // 64, seq, device="cuda")
-        self.table = K.rope_table(seq, 64, 10000.0, "cuda")
+        self.rstd, self.lse = torch.zeros(T, device="cuda"), torch.zeros(batch, D // head, seq, device="cuda")
+        self.table = K.rope_table(seq, head, 10000.0, "cuda")
         torch.cuda.synchronize()
 
     def step(self, between=lambda: None, side=None):
-        (B, S, D), H = self.sizes, self.sizes[2] // 64
+        B, S, D, hd = self.sizes
+        H = D // hd
         views = lambda t: (t[:, :D], t[:, D : 2 * D], t[:, 2 * D :])  # noqa: E731
         main = torch.cuda.current_stream()
         side = side or main
         for launch in (
             lambda: K.rmsnorm_fwd(self.x, self.w, res=self.h, h_out=self.h, out=self.n, rstd=self.rstd),
             lambda: K.linear_fwd(self.n, self.wq, self.qkv),
-            lambda: K.rope_(self.qkv, self.table, S, 2 * H, 64),
-            lambda: K.attention_fwd(*views(self.qkv), B, S, H, H, 64, self.out, self.lse, any_length=True),
+            lambda: K.rope_(self.qkv, self.table, S, 2 * H, hd),
+            lambda: K.attention_fwd(*views(self.qkv), B, S, H, H, hd, self.out, self.lse, any_length=True),
             lambda: K.linear_fwd(self.out, self.wo, self.d),
             lambda: K.linear_fwd(self.d, self.wu, self.gu),
             lambda: K.swiglu_fwd(self.gu, self.act),
             lambda: K.linear_fwd(self.act, self.wd, self.d),
-            lambda: K.attention_bwd(*views(self.qkv), self.out, self.d, self.lse, *views(self.dqkv), B, S, H, H, 64, rope=self.table,
+            lambda: K.attention_bwd(*views(self.qkv), self.out, self.d, self.lse, *views(self.dqkv), B, S, H, H, hd, rope=self.table,
                                     any_length=True),
         ):
             launch()
@@ -64,7 +65,7 @@ class _Chain:
 
 
 @pytest.mark.parametrize("how", ["stream", "two streams", "graph"])
-@pytest.mark.parametrize("sizes", [(1, 32, 64, 128), (5, 100, 256, 512), (16, 128, 512, 1536)])
+@pytest.mark.parametrize("sizes", [(1, 32, 64, 128), (5, 100, 256, 512), (16, 128, 512, 1536), (9, 128, 512, 1024, 128)])
 def test_results_are_those_of_launches_one_by_one(sizes, how):
     STEPS = 8
     apart, run = _Chain(*sizes), _Chain(*sizes)

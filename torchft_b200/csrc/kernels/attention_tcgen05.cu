@@ -132,6 +132,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  ftb200::wait_for_previous();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -163,6 +164,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmK,
       }
       __syncwarp();
     }
+    ftb200::start_next();
     if (!ok) {
       const uint64_t t0 = ftb200::globaltimer_ns();
       while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
@@ -436,6 +438,6 @@ FTB200_API int ftb200_attention_fwd(const void* q, const void* k, const void* v,
   p.ld_o = ld_o; p.O = reinterpret_cast<__nv_bfloat16*>(o); p.lse = lse; p.status = status;
   const long long grid = static_cast<long long>(batch) * n_heads * (seq / BQ);
   if (grid > 0x7fffffffLL) return FTB200_E_TOOBIG;
-  attention_fwd_kernel<<<static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream>>>(tk, tv, p);
+  ftb200::launch_after(attention_fwd_kernel, static_cast<unsigned>(grid), NUM_THREADS, SMEM_BYTES, stream, tk, tv, p);
   return cudaGetLastError() == cudaSuccess ? 0 : FTB200_E_CUDA;
 }
