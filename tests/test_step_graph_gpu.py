@@ -70,3 +70,31 @@ def test_graph_step_leaves_hooks_and_strangers_alone():
     tr.g_flat.zero_()
     outer.replay()
     assert (tr.g_flat.float() - want).norm() < 0.03 * want.norm()
+
+
+def test_graph_step_after_passes_without_a_backward():
+    """Losses measured with the engine's default argument, which trains, between the steps: the captured step's tensors are
+    still its own.  Tensors of the log-sum-exps' size that are made afterwards keep their values, and gradients are those of
+    launches one by one (atomic sums of dQ and the embedding gradient in another order: the bound of the step's test)."""
+    cfg, dev, B, S = CONFIGS["llama-tiny"], torch.device("cuda", 0), 1, 256
+    trs = [ShardedLlamaTrainer(cfg, B, S, dev, seed=5, step_graph=on) for on in (False, True)]
+    for step in range(6):
+        tok, tgt = _batch(cfg, B, S, step)
+        for tr in trs:
+            tr.train_step(tok, tgt)
+        assert (trs[1]._step_graph.graph is not None) == (step not in (0, 4))
+        a, b = (tr.g_flat.float() for tr in trs)
+        assert (a - b).norm() < 0.03 * a.norm(), step
+        for tr in trs:
+            for _ in range(3):
+                tr.engine.forward(tok, tgt)
+        others = [torch.full((B, cfg.n_heads, S), 7.0, device=dev) for _ in range(8 * cfg.n_layers)]
+        trs[1].forward_backward(tok, tgt)
+        trs[0].forward_backward(tok, tgt)
+        assert all(bool((t == 7.0).all()) for t in others), step
+        if step == 3:
+            trs[1].engine.rope = trs[1].engine.rope.clone()
+            trs[1].train_step(tok, tgt)  # as usual: what it reads is elsewhere now
+            assert trs[1]._step_graph.graph is None
+            trs[0].train_step(tok, tgt)
+            trs[1].engine.rope = trs[1].engine.rope.clone()

@@ -157,7 +157,7 @@ class Tcgen05Attention:
     def __init__(self, cfg: LlamaConfig):
         self.cfg = cfg
         self._saved: Dict[int, Tuple[torch.Tensor, ...]] = {}
-        self._lse_pool: List[torch.Tensor] = []
+        self._lse: Dict[int, torch.Tensor] = {}  # per layer, kept: a captured pass has the addresses in it
         self._scratch: Optional[torch.Tensor] = None  # of the backward pass, kept between calls
 
     def _views(self, qkv: torch.Tensor):
@@ -170,8 +170,9 @@ class Tcgen05Attention:
         q, k, v = self._views(qkv)
         lse = None
         if need_grad:
-            lse = self._lse_pool.pop() if self._lse_pool else torch.empty(batch, c.n_heads, seq, dtype=torch.float32,
-                                                                          device=qkv.device)
+            lse = self._lse.get(layer)
+            if lse is None or lse.shape != (batch, c.n_heads, seq) or lse.device != qkv.device:
+                lse = self._lse[layer] = torch.empty(batch, c.n_heads, seq, dtype=torch.float32, device=qkv.device)
             self._saved[layer] = (qkv, out, lse)
         K.attention_fwd(q, k, v, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, out, lse, causal=True, any_length=True)
 
@@ -186,11 +187,8 @@ class Tcgen05Attention:
             self._scratch = torch.empty(need, dtype=torch.uint8, device=qkv.device)
         K.attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, batch, seq, c.n_heads, c.n_kv_heads, c.head_dim, causal=True,
                         scratch=self._scratch, rope=rope, any_length=True)
-        self._lse_pool.append(lse)
 
     def reset(self) -> None:
-        for _, _, lse in self._saved.values():
-            self._lse_pool.append(lse)
         self._saved.clear()
 
 

@@ -53,13 +53,15 @@ class _StepGraph:
     Everything the passes touch belongs to the trainer and its engine and stays where it is from step to step (parameters,
     gradients, activations, workspaces), except the token ids, which are copied into buffers that the graph reads, and the
     mean of the losses, which is formed outside so that every step returns a tensor of its own.  The first step runs as
-    usual (it allocates what is kept and loads the kernels), the second is captured.  What is baked into the graph and can be
-    changed from outside is compared at every step (:meth:`_state`); after a change there is another first step."""
+    usual (it allocates what is kept and loads the kernels), the second is captured.  The graph's owner holds a reference to
+    every tensor whose address is baked into it, so that a replay never meets freed memory, and what can be changed from
+    outside, those addresses among it, is compared at every step (:meth:`_state`); after a change there is another first step."""
 
     def __init__(self, trainer: "ShardedLlamaTrainer") -> None:
         self.tr = trainer
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self.state: Optional[tuple] = None
+        self.tensors: List[torch.Tensor] = []  # those of the state
         self.launches = 0
         self.failed = False
         eng = trainer.engine
@@ -72,11 +74,25 @@ class _StepGraph:
                 and eng.grad_done == tr._grad_done and eng.grad_fields is None and eng.fwd_fields is None
                 and not {"forward", "forward_rows", "backward"} & (vars(eng).keys() | vars(attn).keys()))
 
-    def _state(self) -> tuple:
+    def _tensors(self) -> List[torch.Tensor]:
+        """The tensors that the passes work on: parameters, gradients and whatever the engine and the attention keep."""
         tr, eng = self.tr, self.tr.engine
-        units = [t.data_ptr() for ts in (tr.p_full, tr.g_shard) for t in ts]
-        return (id(eng), id(eng.attn), eng.grad_scale, eng.logit_chunks, eng.param_unit, eng.grad_unit, eng.wstream, K.GEMM_IMPL,
-                os.environ.get("FTB200_ATTN_FWD"), os.environ.get("FTB200_ATTN_POLY"), *units)
+        found = [*tr.p_full, *tr.g_shard]
+        for owner in (eng, eng.attn):
+            for name, value in vars(owner).items():
+                if isinstance(value, torch.Tensor):
+                    if name != "loss_scratch":  # comes with the first evaluation, which alone uses it
+                        found.append(value)
+                elif isinstance(value, (list, dict)):
+                    values = value.values() if isinstance(value, dict) else value
+                    found.extend(t for t in values if isinstance(t, torch.Tensor))
+        return found
+
+    def _state(self, tensors: List[torch.Tensor]) -> tuple:
+        eng = self.tr.engine
+        return (eng, eng.attn, eng.B, eng.S, eng.T, eng.grad_scale, eng.logit_chunks, eng.param_unit, eng.grad_unit, eng.wstream,
+                K.GEMM_IMPL, os.environ.get("FTB200_ATTN_FWD"), os.environ.get("FTB200_ATTN_POLY"), *vars(eng.cfg).values(),
+                *vars(eng.attn.cfg).values(), *[t.data_ptr() for t in tensors])
 
     def run(self, tokens: torch.Tensor, targets: torch.Tensor) -> bool:
         """One forward and backward pass through the graph, or False: the caller runs them itself."""
@@ -85,9 +101,7 @@ class _StepGraph:
         for t, own in ((tokens, self.tokens), (targets, self.targets)):
             if t.device != own.device or t.dtype != own.dtype or t.numel() != own.numel():
                 return False
-        state = self._state()
-        if state != self.state:
-            self.state, self.graph = state, None
+        if self._state(self._tensors()) != self.state:
             return False
         self.tokens.view(-1).copy_(tokens.reshape(-1))
         self.targets.view(-1).copy_(targets.reshape(-1))
@@ -96,6 +110,13 @@ class _StepGraph:
         self.graph.replay()
         N.launch_count += self.launches
         return True
+
+    def ran_without(self) -> None:
+        """A step has run as usual: what the next one finds unchanged may be captured."""
+        tensors = self._tensors()
+        state = self._state(tensors)
+        if state != self.state:
+            self.state, self.tensors, self.graph = state, tensors, None
 
     def _capture(self) -> bool:
         eng, current = self.tr.engine, torch.cuda.current_stream(self.tr.device)
@@ -490,6 +511,8 @@ class ShardedLlamaTrainer:
             return self.engine.loss_rows.mean()
         loss = self.engine.forward(tokens, targets, train=True)
         self.engine.backward(tokens)
+        if self._step_graph is not None:
+            self._step_graph.ran_without()
         return loss
 
     def _finish_comm(self) -> None:
