@@ -80,3 +80,50 @@ def test_a_change_is_seen_and_the_old_tensors_stay(change):
     gc.collect()
     assert old() is not None
     assert graph._state(graph._tensors()) != graph.state
+
+
+class _Hooked(ShardedLlamaTrainer):
+    def _grad_done(self, u):
+        super()._grad_done(u)
+
+
+class _Buffers(ShardedLlamaTrainer):
+    def _grad_buf(self, u):
+        return super()._grad_buf(u)
+
+
+class _Steps(ShardedLlamaTrainer):
+    def forward_backward(self, tokens, targets):  # runs around the graph, not in it
+        return super().forward_backward(tokens, targets)
+
+
+def _attention(cls):
+    def change(tr):
+        tr.engine.attn.__class__ = cls
+
+    return change
+
+
+class _Backward(Tcgen05Attention):
+    def backward(self, layer, dout, batch, seq, dqkv, rope=None):
+        super().backward(layer, dout, batch, seq, dqkv, rope)
+
+
+@pytest.mark.parametrize("cls,change,own", [
+    (ShardedLlamaTrainer, lambda tr: None, True),
+    (_Steps, lambda tr: None, True),
+    (_Hooked, lambda tr: None, False),
+    (_Buffers, lambda tr: None, False),
+    (ShardedLlamaTrainer, _attention(_Backward), False),
+    (ShardedLlamaTrainer, lambda tr: setattr(tr, "manager", object()), False),
+    (ShardedLlamaTrainer, lambda tr: setattr(tr, "_replica_allreduce", lambda u: None), False),
+    (ShardedLlamaTrainer, lambda tr: setattr(tr.engine, "grad_done", lambda u: None), False),
+    (ShardedLlamaTrainer, lambda tr: setattr(tr.engine, "_wgrad", lambda *a, **k: None), False),
+    (ShardedLlamaTrainer, lambda tr: setattr(tr.engine, "forward_rows", lambda *a, **k: None), False),
+    (ShardedLlamaTrainer, lambda tr: setattr(tr.engine.attn, "forward", lambda *a: None), False),
+])
+def test_host_code_of_others_is_not_left_out(cls, change, own):
+    tr = _trainer(cls)
+    graph = _StepGraph(tr)
+    change(tr)
+    assert graph._own_code() == own

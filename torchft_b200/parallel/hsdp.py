@@ -67,12 +67,19 @@ class _StepGraph:
         eng = trainer.engine
         self.tokens, self.targets = (torch.empty(eng.B, eng.S, dtype=torch.int64, device=trainer.device) for _ in range(2))
 
+    # what a step calls of the trainer while it is captured
+    _HOOKS = ("_before_unit", "_grad_done", "_param_unit", "_grad_unit", "_grad_buf", "_replica_allreduce")
+
     def _own_code(self) -> bool:
-        """Whether a step runs nothing on the host but the trainer's and the engine's own code (a graph would leave it out)."""
+        """Whether a step runs nothing on the host but the trainer's and the engine's own code (a graph would leave it out):
+        no subclass's, nothing in an object's attributes that hides a method, no manager or shard group given later."""
         tr, eng, attn = self.tr, self.tr.engine, self.tr.engine.attn
-        return (type(eng) is LlamaEngine and type(attn) is Tcgen05Attention and eng.before_unit == tr._before_unit
-                and eng.grad_done == tr._grad_done and eng.grad_fields is None and eng.fwd_fields is None
-                and not {"forward", "forward_rows", "backward"} & (vars(eng).keys() | vars(attn).keys()))
+        return (type(eng) is LlamaEngine and type(attn) is Tcgen05Attention
+                and all(getattr(type(tr), n) is getattr(ShardedLlamaTrainer, n) for n in self._HOOKS)
+                and not any(hasattr(type(o), n) for o in (tr, eng, attn) for n in vars(o))
+                and eng.before_unit == tr._before_unit and eng.grad_done == tr._grad_done
+                and eng.param_unit == tr._param_unit and eng.grad_unit == tr._grad_unit
+                and eng.grad_fields is None and eng.fwd_fields is None and tr.manager is None and tr.comm.size == 1)
 
     def _tensors(self) -> List[torch.Tensor]:
         """The tensors that the passes work on: parameters, gradients and whatever the engine and the attention keep."""
@@ -90,8 +97,8 @@ class _StepGraph:
 
     def _state(self, tensors: List[torch.Tensor]) -> tuple:
         eng = self.tr.engine
-        return (eng, eng.attn, eng.B, eng.S, eng.T, eng.grad_scale, eng.logit_chunks, eng.param_unit, eng.grad_unit, eng.wstream,
-                K.GEMM_IMPL, os.environ.get("FTB200_ATTN_FWD"), os.environ.get("FTB200_ATTN_POLY"), *vars(eng.cfg).values(),
+        return (eng, eng.attn, eng.B, eng.S, eng.T, eng.grad_scale, eng.logit_chunks, eng.wstream, K.GEMM_IMPL,
+                os.environ.get("FTB200_ATTN_FWD"), os.environ.get("FTB200_ATTN_POLY"), *vars(eng.cfg).values(),
                 *vars(eng.attn.cfg).values(), *[t.data_ptr() for t in tensors])
 
     def run(self, tokens: torch.Tensor, targets: torch.Tensor) -> bool:
