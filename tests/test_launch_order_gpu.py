@@ -90,3 +90,26 @@ def test_results_are_those_of_launches_one_by_one(sizes, how):
     for name, want in apart.state().items():
         assert bool(want.isfinite().all()), name
         assert torch.equal(want, got[name]), name
+
+
+def test_norm_gradients_on_two_streams():
+    """Backward passes of norms of one width on two streams at once give what they give one after the other: no sum has
+    another order, so to the bit."""
+    T, D, N = 2048, 1024, 40
+    g = torch.Generator(device="cuda").manual_seed(3)
+    sides = []
+    for _ in range(2):
+        dy, x = (torch.randn(T, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+        sides.append((dy, x, torch.ones(D, device="cuda").bfloat16(), torch.rand(T, device="cuda", generator=g) + 0.5))
+    want = [K.rmsnorm_bwd(*s) for s in sides]
+    out = [[(torch.empty_like(s[1]), torch.empty_like(s[2])) for _ in range(N)] for s in sides]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in sides]
+    for i in range(N):
+        for s, st, o in zip(sides, streams, out):
+            with torch.cuda.stream(st):
+                K.rmsnorm_bwd(*s, dx=o[i][0], dw=o[i][1])
+    torch.cuda.synchronize()
+    for (dx, dw), o in zip(want, out):
+        for got_dx, got_dw in o:
+            assert torch.equal(got_dx, dx) and torch.equal(got_dw, dw)

@@ -278,6 +278,8 @@ class LlamaEngine:
         self.ws_dqkv = torch.empty(T, QKV, **bf)
         self.logits = torch.empty(T // self.logit_chunks, cfg.vocab_size, **bf)
         self.loss_rows = torch.empty(T, **f32)
+        # partial sums of the norm weights' gradients
+        self.norm_scratch = torch.empty(K.rmsnorm_bwd_scratch_floats(D), **f32) if device.type == "cuda" else None
         self.loss_scratch: Optional[torch.Tensor] = None  # of evaluations, kept between them
         self.rope = K.rope_table(seq_len, cfg.head_dim, cfg.rope_theta, device)
         self.kernel_launches = 0
@@ -448,7 +450,8 @@ class LlamaEngine:
         L = c.n_layers
         u = L + 1
         W, G = self._p(u), self._g(u)
-        K.rmsnorm_bwd(self.ws_dn, self.x[L], W.final_norm, self.rstd1[L], dres=None, dx=self.ws_dy, dw=G.final_norm)
+        K.rmsnorm_bwd(self.ws_dn, self.x[L], W.final_norm, self.rstd1[L], dres=None, dx=self.ws_dy, dw=G.final_norm,
+                      scratch=self.norm_scratch)
         self.grad_done(u)
         dy = self.ws_dy
         for l in reversed(range(L)):
@@ -466,7 +469,8 @@ class LlamaEngine:
                 self._wgrad(l, "wgu", self.gu[l], self.ws_n2, G.wgu, reads=("ws_n2",))
             K.linear_dgrad(self.gu[l], W.wgu, out=self.ws_dn)
             self._before_overwrite("ws_dh", "grad_done")
-            K.rmsnorm_bwd(self.ws_dn, self.h[l], W.ffn_norm, self.rstd2[l], dres=dy, dx=self.ws_dh, dw=G.ffn_norm)
+            K.rmsnorm_bwd(self.ws_dn, self.h[l], W.ffn_norm, self.rstd2[l], dres=dy, dx=self.ws_dh, dw=G.ffn_norm,
+                          scratch=self.norm_scratch)
             # ---- attention
             self._wgrad(l, "wo", self.ws_dh, self.att[l], G.wo, reads=("ws_dh",))
             K.linear_dgrad(self.ws_dh, W.wo, out=self.ws_dn)
@@ -485,7 +489,7 @@ class LlamaEngine:
             K.linear_dgrad(self.ws_dqkv, W.wqkv, out=self.ws_dn)
             self._before_overwrite("dy")
             K.rmsnorm_bwd(self.ws_dn, self.x[l], W.attn_norm, self.rstd1[l], dres=self.ws_dh, dx=self.ws_dy,
-                          dw=G.attn_norm)
+                          dw=G.attn_norm, scratch=self.norm_scratch)
             self._grad_done_after_wgrads(u)
             dy = self.ws_dy
         self.before_unit(0, True)

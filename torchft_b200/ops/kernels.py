@@ -332,6 +332,13 @@ def ref_rmsnorm_bwd(dy, x, w, rstd, dres=None):
 _rms_scratch: dict = {}
 
 
+def rmsnorm_bwd_scratch_floats(dim: int) -> int:
+    """Size of the ``scratch`` that :func:`rmsnorm_bwd` takes."""
+    lib = N.lib()
+    lib.ftb200_rmsnorm_bwd_scratch_floats.restype = c_ll
+    return int(lib.ftb200_rmsnorm_bwd_scratch_floats(dim))
+
+
 def rmsnorm_bwd(
     dy: torch.Tensor,
     x: torch.Tensor,
@@ -341,7 +348,11 @@ def rmsnorm_bwd(
     dx: Optional[torch.Tensor] = None,
     dw: Optional[torch.Tensor] = None,
     accumulate_dw: bool = False,
+    scratch: Optional[torch.Tensor] = None,
 ) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``(dx, dw)`` of :func:`rmsnorm_fwd`.  The partial sums of ``dw`` lie in ``scratch`` (fp32 on the device,
+    :func:`rmsnorm_bwd_scratch_floats` of them or more) between the two kernels, by default in a buffer of the current stream's
+    that is reused across calls."""
     T, D = x.shape
     if dx is None:
         dx = torch.empty_like(x)
@@ -352,14 +363,14 @@ def rmsnorm_bwd(
         dx.copy_(rdx)
         dw.copy_(((dw.float() if accumulate_dw else 0) + rdw).to(dw.dtype))
         return dx, dw
-    key = (x.device.index, D)
-    scratch = _rms_scratch.get(key)
     if scratch is None:
-        L = N.lib()
-        L.ftb200_rmsnorm_bwd_scratch_floats.restype = c_ll
-        need = int(L.ftb200_rmsnorm_bwd_scratch_floats(D))
-        scratch = torch.empty(need, dtype=torch.float32, device=x.device)
-        _rms_scratch[key] = scratch
+        key = (x.device.index, _stream(), D)
+        scratch = _rms_scratch.get(key)
+        if scratch is None:
+            scratch = _rms_scratch[key] = torch.empty(rmsnorm_bwd_scratch_floats(D), dtype=torch.float32, device=x.device)
+    elif (scratch.device != x.device or scratch.dtype != torch.float32 or not scratch.is_contiguous()
+          or scratch.numel() < rmsnorm_bwd_scratch_floats(D) or scratch.data_ptr() % 16):
+        raise ValueError(f"scratch must be {rmsnorm_bwd_scratch_floats(D)} contiguous fp32 on {x.device}")
     N.check(
         _fn("rmsnorm_bwd")(_at(dy), _at(x), _at(w), _at(rstd), _at(dres), _at(dx), _at(dw), _at(scratch), T, D,
                            int(accumulate_dw), _stream()),
