@@ -1,7 +1,7 @@
 """The explicit forward/backward engine must match autograd on the same weights."""
 import torch
 
-from torchft_b200.models.llama import LLAMA_TINY, TorchLlama
+from torchft_b200.models.llama import LLAMA_TINY, Tcgen05Attention, TorchLlama
 from torchft_b200.parallel.hsdp import ShardedLlamaTrainer
 
 
@@ -123,3 +123,45 @@ def test_forward_attention_kernel_follows_the_number_of_sms():
         assert _two_query_tiles(1, 256, sms // 2 + 1, sms)
         assert _two_query_tiles(sms, 256, 1, sms) and not _two_query_tiles(sms, 128, 2, sms)
         assert not _two_query_tiles(4, 384, sms, sms)
+
+
+def _with_own_backward(attn):
+    own = attn.backward
+    attn.backward = lambda layer, dout, batch, seq, dqkv: own(layer, dout, batch, seq, dqkv)
+    return attn
+
+
+class _OwnBackward(Tcgen05Attention):
+    def backward(self, layer, dout, batch, seq, dqkv):
+        super().backward(layer, dout, batch, seq, dqkv)
+
+
+class _Mixin:
+    def backward(self, layer, dout, batch, seq, dqkv):
+        Tcgen05Attention.backward(self, layer, dout, batch, seq, dqkv)
+
+
+class _Mixed(_Mixin, Tcgen05Attention):
+    pass
+
+
+class _OwnRotation(Tcgen05Attention):
+    rotates_back = True
+
+    def backward(self, layer, dout, batch, seq, dqkv, rope=None):
+        assert rope is not None
+        super().backward(layer, dout, batch, seq, dqkv, rope)
+
+
+def test_an_attention_with_a_backward_of_its_own_is_not_asked_to_rotate():
+    """A subclass's (or an instance's) backward() of five arguments gets five; the engine rotates its dQ and dK back."""
+    cfg, B, S = LLAMA_TINY, 2, 16
+    tokens, targets = torch.randint(0, cfg.vocab_size, (2, B, S), generator=torch.Generator().manual_seed(5))
+    grads = []
+    for attn in (Tcgen05Attention(cfg), _OwnRotation(cfg), _OwnBackward(cfg), _Mixed(cfg),
+                  _with_own_backward(Tcgen05Attention(cfg))):
+        tr = ShardedLlamaTrainer(cfg, B, S, torch.device("cpu"), logit_chunks=1, seed=11, attention=attn)
+        tr.forward_backward(tokens, targets)
+        grads.append(tr.g_flat.float())
+    for g in grads[1:]:  # dQ and dK are rounded once more where they are rotated apart
+        assert (g - grads[0]).norm() < 0.01 * grads[0].norm()

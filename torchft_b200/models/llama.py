@@ -154,6 +154,13 @@ class Tcgen05Attention:
 
     rotates_back = True  # backward() takes the rotation of q and k
 
+    def __init_subclass__(cls, **kwargs) -> None:
+        super().__init_subclass__(**kwargs)
+        # whoever brings a backward() of its own says itself whether it takes the rotation
+        by = next(c for c in cls.__mro__ if {"backward", "rotates_back"} & vars(c).keys())
+        if "rotates_back" not in vars(by):
+            cls.rotates_back = False
+
     def __init__(self, cfg: LlamaConfig):
         self.cfg = cfg
         self._saved: Dict[int, Tuple[torch.Tensor, ...]] = {}
@@ -475,7 +482,7 @@ class LlamaEngine:
             self._wgrad(l, "wo", self.ws_dh, self.att[l], G.wo, reads=("ws_dh",))
             K.linear_dgrad(self.ws_dh, W.wo, out=self.ws_dn)
             self._before_overwrite("ws_dqkv")
-            if getattr(self.attn, "rotates_back", False):
+            if getattr(self.attn, "rotates_back", False) and "backward" not in getattr(self.attn, "__dict__", ()):
                 self.attn.backward(l, self.ws_dn, B, S, self.ws_dqkv, rope=self.rope)
             else:
                 self.attn.backward(l, self.ws_dn, B, S, self.ws_dqkv)
