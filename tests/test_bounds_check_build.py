@@ -31,6 +31,15 @@ tok = torch.tensor([1, 2, V + 7, 3], device=dev)
 emb = K.embedding_fwd(tok, table)
 torch.cuda.synchronize()
 out["embedding"] = (N.bounds_status(), bool(torch.equal(emb[2], table[0])), bool(torch.equal(emb[1], table[2])))
+# a target beyond the vocabulary, whether the logits are stored or not (64 x 16384 of them are not)
+for T, V in ((64, 1024), (64, 16384)):
+    x, head = torch.randn(T, 64, device=dev).bfloat16(), torch.randn(V, 64, device=dev).bfloat16()
+    tgt = torch.randint(0, V, (T,), device=dev)
+    tgt[5], tgt[6] = V + 9, -100
+    loss, logits = torch.empty(T, device=dev), torch.zeros(T, V, device=dev).bfloat16()
+    K.linear_cross_entropy_(x, head, tgt, 1.0, logits, loss, grad=False)
+    torch.cuda.synchronize()
+    out[f"target_{V}"] = (N.bounds_status(), bool(logits.any()))
 # a warp that waits on an mbarrier in vain sees the abort flag of its CTA
 ns = torch.zeros(1, dtype=torch.int64, device=dev)
 assert lib.ftb200_wait_selftest(N.ptr(ns), N.stream_ptr()) == 0
@@ -59,6 +68,8 @@ def test_checked_build_records_and_skips():
     assert res["out_of_range"] == [0, [4, 5]]
     assert res["cleared"] == [0, 0]
     assert res["embedding"] == [[4, 64 + 7], True, True]
+    assert res["target_1024"] == [[4, 1024 + 9], True]
+    assert res["target_16384"] == [[4, 16384 + 9], False]
     # 64 failed polls of about 2 us each lie between two looks at the flag; a factor of four over that
     assert 0 <= res["gave_up_ns"] < 512_000, res["gave_up_ns"]
     assert res["clean"] == [0, 0]

@@ -506,7 +506,10 @@ cross_entropy_rows_kernel(const long long* target, const float2* stats,
   for (int i = lane; i < tiles; i += 32) sum += st[i].y * __expf(st[i].x - base);
   sum = ftb200::warp_sum(sum);
   const long long tgt = target[row];
-  if (lane == 0) loss[row] = tgt >= 0 ? logf(sum) + mx - (tgt < V ? target_value[row] : 0.f) : 0.f;
+  if (lane == 0) {
+    if (tgt >= 0) (void)FTB_IN_RANGE(tgt, V);
+    loss[row] = tgt >= 0 ? logf(sum) + mx - (tgt < V ? target_value[row] : 0.f) : 0.f;
+  }
 }
 
 // ------------------------------------------------------------------ AdamW (flat shard)
