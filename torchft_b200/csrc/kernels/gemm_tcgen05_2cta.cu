@@ -217,6 +217,12 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   }
 }
 
+// After a wait that ran out: copies in flight land in shared memory, so the CTA stays until they have.
+__device__ __forceinline__ void sleep_200us() {
+  const uint64_t t0 = ftb200::globaltimer_ns();
+  while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+}
+
 // Bounded wait until *p >= want (device-scope acquire).
 __device__ __forceinline__ bool count_wait(const unsigned int* p, unsigned int want, volatile int* abort_flag) {
   const uint64_t t0 = ftb200::globaltimer_ns();
@@ -424,10 +430,7 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       }
     }
     if (p.ga_world == 0 && p.sc_world == 0) ftb200::start_next();
-    if (!ok) {
-      const uint64_t t0 = ftb200::globaltimer_ns();
-      while (ftb200::globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-    }
+    if (!ok) sleep_200us();
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
@@ -901,12 +904,19 @@ gemm_bf16_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __g
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // no store reads the staging area any more
+    if (*abort_flag) sleep_200us();  // this warp's loads and copies that nobody waited for have ended then
+    __syncwarp();
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag && p.status != nullptr) atomicExch(p.status, FTB200_ST_TIMEOUT);
   cluster_sync_relaxed();  // no CTA retires while another may still touch its barriers, operands or ring
+  // what another pair copied into this CTA's ring may still be on its way if this one has given up waiting for it
+  if (SPLIT) {
+    if (*abort_flag) sleep_200us();
+    __syncwarp();
+  }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -1081,7 +1091,7 @@ struct TilePlan {
 // 1536 x 4096 x 28672 290 -> 240, 3072 x 2048 x 8192 84 -> 77, 750 x 1024 x 8192 30 -> 25, 77 x 4096 x 14336 52 -> 44; where the
 // estimate says no: 500 x 4096 x 4096 20 -> 27, 1536 x 1024 x 3000 15 -> 22, 1000 x 2048 x 2048 13 -> 20.
 static TilePlan plan_tiles(int M, int N, int K, int pairs, bool may_split) {
-    constexpr float NARROW = 0.7f, SPLIT_COST = 32.f;
+  constexpr float NARROW = 0.7f, SPLIT_COST = 32.f;
   const int rows = (M + 2 * BM - 1) / (2 * BM), slabs = (K + BK - 1) / BK;
   const int wide = rows * ((N + 255) / 256), narrow = rows * ((N + 127) / 128);
   TilePlan best{narrow <= pairs ? 128 : 256, 1, 0, 2 * pairs};
