@@ -1,7 +1,10 @@
 """The explicit forward/backward engine must match autograd on the same weights."""
+import dataclasses
+
+import pytest
 import torch
 
-from torchft_b200.models.llama import LLAMA_TINY, Tcgen05Attention, TorchLlama
+from torchft_b200.models.llama import LLAMA_TINY, SdpaAttention, Tcgen05Attention, TorchLlama, make_attention
 from torchft_b200.parallel.hsdp import ShardedLlamaTrainer
 
 
@@ -165,3 +168,23 @@ def test_an_attention_with_a_backward_of_its_own_is_not_asked_to_rotate():
         grads.append(tr.g_flat.float())
     for g in grads[1:]:  # dQ and dK are rounded once more where they are rotated apart
         assert (g - grads[0]).norm() < 0.01 * grads[0].norm()
+
+
+@pytest.mark.parametrize("head_dim,seq,auto,explicit", [
+    (128, 128, True, True), (128, 100, False, True), (128, 129, True, True), (64, 128, False, True), (64, 129, True, True),
+    (64, 256, True, True), (64, 1, False, True), (32, 256, False, False), (96, 1024, False, False)])
+def test_attention_kernels_are_chosen_by_length_and_taken_at_any(monkeypatch, head_dim, seq, auto, explicit):
+    """Left to itself the choice depends on the length; asked for, the kernels are taken wherever they run."""
+    monkeypatch.delenv("FTB200_ATTENTION", raising=False)
+    cfg, cuda = dataclasses.replace(LLAMA_TINY, dim=2 * head_dim, n_heads=2, n_kv_heads=1), torch.device("cuda")
+    assert isinstance(make_attention(cfg, seq, cuda), Tcgen05Attention) == auto
+    if explicit:
+        assert isinstance(make_attention(cfg, seq, cuda, "tcgen05"), Tcgen05Attention)
+        monkeypatch.setenv("FTB200_ATTENTION", "tcgen05")
+        assert isinstance(make_attention(cfg, seq, cuda), Tcgen05Attention)
+        assert isinstance(make_attention(cfg, seq, cuda, "sdpa"), SdpaAttention)
+    else:
+        with pytest.raises(ValueError):
+            make_attention(cfg, seq, cuda, "tcgen05")
+    with pytest.raises(ValueError):
+        make_attention(cfg, seq, torch.device("cpu"), "tcgen05")

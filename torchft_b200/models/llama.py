@@ -200,18 +200,15 @@ class Tcgen05Attention:
 
 
 def make_attention(cfg: LlamaConfig, seq_len: int, device: torch.device, kind: Optional[str] = None):
-    """``kind``: "tcgen05" (hand-written kernels; CUDA, head dim 128 and a sequence that is a multiple of 128,
-    or head dim 64 and a multiple of 256), "sdpa" (library), or None for tcgen05 there and wherever else the sequence is longer
-    than a tile (128): the library's kernels want four transposing copies and an autograd graph around them (four layers of
-    width 1024, 3 x 1000 tokens: a step of 2845 us against 2309).  The environment variable ``FTB200_ATTENTION`` overrides
-    None."""
+    """``kind``: "tcgen05" (hand-written kernels; CUDA and head dim 64 or 128, any sequence length), "sdpa" (library), or None:
+    tcgen05 for these head dims where the sequence is longer than a tile (128) or a whole number of tiles (a multiple of 128, 256 at head dim 64).  The
+    library's kernels want four transposing copies and an autograd graph around them (four layers of width 1024, 3 x 1000 tokens: a
+    step of 2845 us against 2309).  The environment variable ``FTB200_ATTENTION`` overrides None."""
     kind = kind or os.environ.get("FTB200_ATTENTION") or "auto"
-    ok = device.type == "cuda" and K.attention_supported(seq_len, cfg.head_dim)
-    if kind == "tcgen05" and not ok:
-        raise ValueError("tcgen05 attention needs CUDA and head_dim 128 with seq_len % 128 == 0 or head_dim 64 with "
-                         "seq_len % 256 == 0")
-    longer = device.type == "cuda" and cfg.head_dim in (64, 128) and seq_len > 128
-    if kind == "tcgen05" or (kind == "auto" and (ok or longer)):
+    takes = device.type == "cuda" and cfg.head_dim in (64, 128)
+    if kind == "tcgen05" and not takes:
+        raise ValueError("tcgen05 attention needs CUDA and a head dim of 64 or 128")
+    if kind == "tcgen05" or (kind == "auto" and takes and (seq_len > 128 or K.attention_supported(seq_len, cfg.head_dim))):
         return Tcgen05Attention(cfg)
     return SdpaAttention(cfg)
 
