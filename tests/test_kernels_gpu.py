@@ -275,19 +275,6 @@ def test_cross_entropy_row_lengths(V):
     assert bool(((loss.double() - ref).abs() <= 2**-18 * (1 + x.abs().amax(-1))).all())
 
 
-@pytest.mark.parametrize("V", [16, 4096 + 16])
-def test_cross_entropy_gradients_below_the_normal_numbers(V):
-    """A token e^-88 to e^-91 as likely as the largest has a gradient of 2^-127 to 2^-132, a subnormal bf16 number: at most half
-    a unit of 2^-133 from 64 bits, and 2^-16 of the value for an exponent of 127 that is rounded to 24 bits, not zero."""
-    logits = torch.full((4, V), -120.0, device=DEV).bfloat16()
-    logits[:, 0] = 0.0  # the target is in the first vector, which is worked out apart
-    logits[:, 8:] = torch.tensor([-88.0, -88.5, -89.0, -89.5, -90.0, -90.5, -91.0, -100.0], device=DEV).repeat((V - 8) // 8)
-    want = logits.double().softmax(-1)[:, 8:]
-    K.cross_entropy_(logits, torch.zeros(4, dtype=torch.int64, device=DEV), 1.0)
-    got = logits[:, 8:].double()
-    assert bool(((got - want).abs() <= 2.0**-134 + 2**-16 * want).all()) and bool((got[:, :7] > 0).all())
-
-
 @pytest.mark.parametrize("V", [8, 8 * 1024, 8 * 1024 + 8, 8 * 3 * 1024 - 8, 128256])
 def test_cross_entropy_without_gradient(V):
     """One to several vectors per thread, with remainders; the logits stay as they are and the loss is the same number."""

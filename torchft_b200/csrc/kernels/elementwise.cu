@@ -468,7 +468,7 @@ cross_entropy_kernel(bf16x8* logits, const int64_t* target, float* loss, int V8,
     unpack8(*reinterpret_cast<const bf16x8*>(&raw), f);
     if (at != tgt8) {
 #pragma unroll
-      for (int e = 0; e < 8; e += 2) f2_unpack(f2_mul_subnormal(exp_of(f[e], f[e + 1], neg_gmx), scale2), f[e], f[e + 1]);
+      for (int e = 0; e < 8; e += 2) f2_unpack(f2_mul(exp_of(f[e], f[e + 1], neg_gmx), scale2), f[e], f[e + 1]);
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] = (__expf(f[e] - gmx) * inv - (e == tgt_e ? 1.f : 0.f)) * gs;

@@ -245,12 +245,6 @@ __device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsig
   asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// The same with subnormal numbers, for results that are kept.
-__device__ __forceinline__ unsigned long long f2_mul_subnormal(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 
 // max(a, b), NaN if either is (fmaxf would drop it).
 __device__ __forceinline__ float max_nan(float a, float b) {
