@@ -113,3 +113,68 @@ def test_norm_gradients_on_two_streams():
     for (dx, dw), o in zip(want, out):
         for got_dx, got_dw in o:
             assert torch.equal(got_dx, dx) and torch.equal(got_dw, dw)
+
+
+class _Engine:
+    """The engine's order around a workspace that two streams use: a kernel of one stream writes it and the other's next kernel, a
+    dependent of the one before it there, waits for nothing but an event; then the first stream's next dependent overwrites what
+    the other reads, again behind an event alone."""
+
+    B, S, D, HD = 64, 128, 1024, 64
+
+    def __init__(self, steps):
+        g = torch.Generator(device="cuda").manual_seed(1)
+        T, D = self.B * self.S, self.D
+        r = lambda *shape: (torch.randn(*shape, device="cuda", generator=g) * 0.1).bfloat16()  # noqa: E731
+        self.w, self.wo, self.wq, self.qkv, self.dqkv, self.d = r(D) + 1, r(D, D), r(3 * D, D), r(T, 3 * D), r(T, 3 * D), r(T, D)
+        self.n, self.out, self.dout = (torch.zeros_like(self.d) for _ in range(3))
+        self.lse = torch.zeros(self.B, D // self.HD, self.S, device="cuda")
+        self.dw = [torch.zeros(3 * D, D, device="cuda", dtype=torch.bfloat16) for _ in range(steps)]
+        views, H = self.views(self.qkv), D // self.HD
+        K.attention_fwd(*views, self.B, self.S, H, H, self.HD, self.out, self.lse, any_length=True)
+        torch.cuda.synchronize()
+
+    def views(self, t):
+        return t[:, : self.D], t[:, self.D : 2 * self.D], t[:, 2 * self.D :]
+
+    def run(self, side=None, product=True, between=lambda: None):
+        main, H = torch.cuda.current_stream(), self.D // self.HD
+        side = side or main
+        for dw in self.dw:
+            K.rmsnorm_fwd(self.d, self.w, out=self.n)
+            between()
+            ready = main.record_event()
+            with torch.cuda.stream(side):
+                side.wait_event(ready)
+                K.linear_wgrad(self.dqkv, self.n, out=dw)
+                between()
+                done = side.record_event()
+            if product:
+                K.linear_fwd(self.n, self.wo, out=self.dout)
+                between()
+            main.wait_event(done)
+            K.attention_bwd(*self.views(self.qkv), self.out, self.dout if product else self.d, self.lse, *self.views(self.dqkv), self.B,
+                            self.S, H, H, self.HD, any_length=True)
+            between()
+            K.linear_dgrad(self.dqkv, self.wq, out=self.d)
+            between()
+
+
+@pytest.mark.parametrize("product", [True, False])
+@pytest.mark.parametrize("graph", [False, True])
+def test_dependents_behind_an_event_alone(graph, product):
+    """Sequences of one key block: every sum has one order, so the results are those of launches one by one, to the bit."""
+    apart, run, side = _Engine(6), _Engine(6), torch.cuda.Stream()
+    apart.run(None, product, torch.cuda.synchronize)
+    if graph:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            run.run(side, product)
+        g.replay()
+    else:
+        run.run(side, product)
+    torch.cuda.synchronize()
+    K.check_status(run.d.device)
+    for i, (want, got) in enumerate(zip(apart.dw, run.dw)):
+        assert bool(want.isfinite().all()) and bool(want.any()) and torch.equal(want, got), i
+    assert torch.equal(apart.dqkv, run.dqkv) and torch.equal(apart.d, run.d)
