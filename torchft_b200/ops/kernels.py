@@ -332,6 +332,7 @@ def ref_rmsnorm_bwd(dy, x, w, rstd, dres=None):
 _rms_scratch: dict = {}
 
 
+@functools.lru_cache(maxsize=256)
 def rmsnorm_bwd_scratch_floats(dim: int) -> int:
     """Size of the ``scratch`` that :func:`rmsnorm_bwd` takes."""
     lib = N.lib()

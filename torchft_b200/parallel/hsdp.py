@@ -108,7 +108,7 @@ class _StepGraph:
         for t, own in ((tokens, self.tokens), (targets, self.targets)):
             if t.device != own.device or t.dtype != own.dtype or t.numel() != own.numel():
                 return False
-        if self._state(self._tensors()) != self.state:
+        if self.state is None or self._state(self._tensors()) != self.state:
             return False
         self.tokens.view(-1).copy_(tokens.reshape(-1))
         self.targets.view(-1).copy_(targets.reshape(-1))
