@@ -40,6 +40,7 @@ def main() -> None:
     ap.add_argument("--seed", type=int, default=0)
     ap.add_argument("--hold-step", type=int, default=10 ** 9,
                     help="from this step on keep training until a second group has been seen, then stop at a multiple of 5")
+    ap.add_argument("--meet", default="", help="directory in which the ranks of both groups wait for each other before they train")
     a = ap.parse_args()
     world = 2
     dist.init_process_group("gloo", init_method=f"tcp://127.0.0.1:{a.init_port}", rank=a.rank, world_size=world)
@@ -84,6 +85,12 @@ def main() -> None:
         inner.state[p]["momentum_buffer"] = torch.zeros_like(p)
     holder.update(model=model, opt=inner)
     opt = Optimizer(manager, inner)
+
+    if a.meet:  # a group that is up long before the other would be past the step at which that one leaves
+        open(os.path.join(a.meet, f"{a.group}-{a.rank}"), "w").close()
+        deadline = time.monotonic() + 120
+        while len(os.listdir(a.meet)) < 2 * world and time.monotonic() < deadline:
+            time.sleep(0.01)
 
     rejoined = False
     while True:

@@ -24,13 +24,13 @@ def _free_port() -> int:
     return p
 
 
-def _spawn_group(group, lighthouse, steps, exit_at=-1, seed=0, hold=10 ** 9):
+def _spawn_group(group, lighthouse, steps, exit_at=-1, seed=0, hold=10 ** 9, meet=""):
     init_port, store_port = _free_port(), _free_port()
     env = dict(os.environ, OMP_NUM_THREADS="1")
     return [subprocess.Popen(
         [sys.executable, WORKER, "--group", str(group), "--rank", str(r), "--init-port", str(init_port), "--store-port",
          str(store_port), "--lighthouse", lighthouse, "--steps", str(steps), "--exit-at-step", str(exit_at), "--seed", str(seed),
-         "--hold-step", str(hold)],
+         "--hold-step", str(hold), "--meet", str(meet)],
         stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True, env=env) for r in range(2)]
 
 
@@ -107,13 +107,13 @@ def test_fsdp2_groups_agree_after_init_sync_and_training():
 
 
 @pytest.mark.timeout(600)
-def test_fsdp2_group_leaves_and_heals():
+def test_fsdp2_group_leaves_and_heals(tmp_path):
     lh = LighthouseServer("[::]:0", 1, join_timeout_ms=300, quorum_tick_ms=20, heartbeat_timeout_ms=1000)
     addr = "http://127.0.0.1:" + lh.address().rsplit(":", 1)[1]
     procs = []
     try:
-        g0 = _spawn_group(0, addr, 10, seed=0, hold=5)
-        g1 = _spawn_group(1, addr, 10, exit_at=3, seed=1)
+        g0 = _spawn_group(0, addr, 10, seed=0, hold=5, meet=tmp_path)
+        g1 = _spawn_group(1, addr, 10, exit_at=3, seed=1, meet=tmp_path)
         procs = g0 + g1
         assert [p.wait(timeout=180) for p in g1] == [17, 17]
         time.sleep(0.5)
