@@ -153,7 +153,8 @@ def test_attention_bwd_matches_reference(B, S, Hq, Hkv, causal, D):
 ])
 def test_attention_bwd_tiles(B, S, Hq, Hkv, causal, scale, D):
     """Tiles of 128 queries at the edges of the walk over them.  Three roundings to bf16 lie on the way of every
-    gradient (probabilities or dS, the forward's O behind delta, the result), each at most 2^-9 of its value."""
+    gradient (probabilities or dS, the forward's O behind delta, the result), each at most 2^-8 of a value and less
+    than 2^-9 in norm."""
     qkv, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=S + D, scale=scale)
     out = torch.empty(B * S, Hq * D, dtype=torch.bfloat16, device="cuda")
     lse = torch.empty(B, Hq, S, dtype=torch.float32, device="cuda")
@@ -210,7 +211,7 @@ def test_attention_of_any_length(B, S, Hq, Hkv, causal, D):
 @pytest.mark.parametrize("causal", [True, False])
 def test_attention_bwd_rotates_back(D, causal):
     """dQ and dK of the values before the rotation: as the rotated ones turned back by a kernel of their own, which rounds once
-    more (2^-9 of each value)."""
+    more (at most 2^-8 of each value)."""
     B, S, Hq, Hkv = 2, 512, 4, 2
     qkv, q, k, v = _qkv(B, S, Hq, Hkv, D, seed=D)
     table = K.rope_table(S, D, 10000.0, "cuda")

@@ -104,7 +104,7 @@ def test_gemm_adds_to_bf16(M, N, K_, a_mn, b_mn):
 @pytest.mark.parametrize("K_", [8, 72, 256, 1024, 1032, 4104])
 def test_gemm_one_row(N, K_):
     """A single row reads the other operand once, by a kernel of its own; the remainders of its lanes and rows, a row stride.
-    fp32 sums: bf16 rounding of the result (2^-9 of each value) is the error.  Transposed operands, fp32 results and
+    fp32 sums: bf16 rounding of the result (at most 2^-8 of each value) is the error.  Transposed operands, fp32 results and
     accumulation stay with the tiles."""
     torch.manual_seed(N + K_)
     a, b = torch.randn(1, K_, device=DEV).bfloat16(), torch.randn(N + 1, K_ + 8, device=DEV).bfloat16()[:N, :K_]
@@ -195,7 +195,7 @@ def test_rmsnorm(T, D):
 def test_rmsnorm_row_shapes(T, D):
     """Every number of warps a row, full and with a remainder, few rows and more than the groups of a pass; beyond 8192
     elements the forward pass reads its rows twice and the backward pass refuses.  The sums are fp32 (a few 2^-24 of sqrt(D)
-    terms), so bf16 rounding of the results is the error: at most 2^-9 of each value."""
+    terms), so bf16 rounding of the results is the error: at most 2^-8 of each value."""
     torch.manual_seed(T + D)
     x, res, dy, dres = (torch.randn(T, D, device=DEV).bfloat16() for _ in range(4))
     w = (1 + 0.1 * torch.randn(D, device=DEV)).bfloat16()
@@ -293,7 +293,7 @@ def test_cross_entropy_without_gradient(V):
 @pytest.mark.parametrize("T,Kd,F", [(1, 2048, 8), (33, 2056, 40), (200, 2048, 512), (1000, 2048, 2816), (130, 4096, 1000), (300, 64, 128)])
 def test_linear_dswiglu(T, Kd, F):
     """Down projection and activation backwards in one kernel against 64 bits: the gradient of the activation is not rounded on
-    the way, so the result's rounding (2^-9 of each value) is the whole error."""
+    the way, so the result's rounding (at most 2^-8 of each value) is the whole error."""
     torch.manual_seed(T + F)
     dy, w = torch.randn(T, Kd, device=DEV).bfloat16(), (0.05 * torch.randn(Kd, F, device=DEV)).bfloat16()
     buf = torch.full((T + 1, 2 * F + 8), 7.0, device=DEV, dtype=torch.bfloat16)

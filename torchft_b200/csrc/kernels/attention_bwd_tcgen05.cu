@@ -14,8 +14,8 @@
 // P^T and dS^T go back, as packed bf16, into the TMEM columns their scores came from and are the
 // A operands of the dV and dK MMAs straight from tensor memory; dS^T is also written to shared
 // memory (128-byte swizzle) as the MN-major B operand of the dQ^T MMA.  dK and dV stay in TMEM for the
-// whole CTA; dQ^T is drained every tile and added to an fp32 accumulator in global memory (four
-// queries of a head-dim element per reduction, 512 consecutive bytes per warp instruction).
+// whole CTA; dQ^T is drained every tile: a drain warp puts its 32 head-dim elements into shared memory, a quarter of the queries
+// at a time, and each quarter is added to an fp32 accumulator in global memory by one bulk reduction of 4 KB.
 //
 // Warps: 0 = TMA (K, V once; Q with lse and delta, dO per tile), 1 = MMA issue, 4..7 = dQ drain, 8..15 = softmax (two
 // threads per key, 64 queries each; together they store dK, dV at the end).  Issue order of a tile t:
@@ -29,7 +29,9 @@
 // for dS^T and the statistics, whose second half then takes 2570 cycles instead of 1020 (800 with no reductions at all).  A
 // tile takes 3750 cycles: 4890 with red.v4, 3250 with no reductions, 2600 for its 40 MMAs, 2048 + 1000 for what they, the
 // TMA and the softmax move through shared memory at 128 bytes a cycle.  dO has one stage there, as the staging of dQ^T takes
-// the second one's place.  At head dim 64 it is the chain of the softmax, 2830 cycles a tile.
+// the second one's place.  At head dim 64 it is the chain of the softmax, 2830 cycles a tile
+// (the slope over one CTA's chain of 32, 64 and 128 tiles).  Starts, ends and the last wave included a tile costs an SM 4210
+// cycles at 1 x 8192 and 3650 at 8 x 2048, heads of 64.
 // The warp's index and the TMEM base are read from lane 0 (shfl): then the branch and the addresses are known to be the
 // same in all lanes and the MMAs' descriptors stay in uniform registers (1494 -> 1437 us, 650 -> 605 us).
 // 1 x 8192, 32/8 heads of 128: 1705 us with 64-query tiles, 1290 us (1065 TFLOP/s) with these; 8 x 2048, heads of 64: 785 -> 592 us.

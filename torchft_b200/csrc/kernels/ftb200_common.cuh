@@ -177,7 +177,7 @@ __device__ __forceinline__ bf16x8 pack8(const float* f) {
 //    kernel waits on the chip) by at least a thread of every CTA that lives long, and holds back nothing else;
 //  * their pointers are not __restrict__: a read-only load of a kernel's whole life may not see what was written during it.
 // Kernels that wait for other GPUs are launched as usual and do not call start_next.  Neither does AdamW wait: its 250 us and more
-// gain nothing.  A step of two layers on 256 tokens (79 launches, a graph) 369 -> 310 us; of four layers of width 1024 on
+// gain nothing.  A step of two layers on 256 tokens (a graph) 369 -> 310 us; of four layers of width 1024 on
 // 3 x 1000 tokens 2138 -> 1982; the evaluation of a 16-layer model 10.4 -> 10.0 ms.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

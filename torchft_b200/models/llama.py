@@ -202,8 +202,8 @@ class Tcgen05Attention:
 def make_attention(cfg: LlamaConfig, seq_len: int, device: torch.device, kind: Optional[str] = None):
     """``kind``: "tcgen05" (hand-written kernels; CUDA and head dim 64 or 128, any sequence length), "sdpa" (library), or None:
     tcgen05 for these head dims where the sequence is longer than a tile (128) or a whole number of tiles (a multiple of 128, 256 at head dim 64).  The
-    library's kernels want four transposing copies and an autograd graph around them (four layers of width 1024, 3 x 1000 tokens: a
-    step of 2845 us against 2309).  The environment variable ``FTB200_ATTENTION`` overrides None."""
+    library's kernels want four transposing copies and an autograd graph around them (four layers of width 1024, 3 x 1000 tokens,
+    launched one by one: a step of 2833 us against 1864).  The environment variable ``FTB200_ATTENTION`` overrides None."""
     kind = kind or os.environ.get("FTB200_ATTENTION") or "auto"
     takes = device.type == "cuda" and cfg.head_dim in (64, 128)
     if kind == "tcgen05" and not takes:
@@ -383,9 +383,10 @@ class LlamaEngine:
 
     # -- forward ---------------------------------------------------------------------------
     def forward(self, tokens: torch.Tensor, targets: Optional[torch.Tensor], train: bool = True) -> torch.Tensor:
-        """Runs the decoder; with ``targets`` returns the mean token loss and leaves
+        """Runs the decoder; with ``targets`` returns the mean token loss and, with ``train``, leaves
         ``dlogits``-derived gradients of the head computed (head backward is fused into
-        the loss pass so that the logits never exist in full)."""
+        the loss pass so that the logits never exist in full).  ``logits`` is a workspace of these passes: after a training pass
+        it holds the last chunk's gradients, after an evaluation the logits or nothing of use."""
         out = self.forward_rows(tokens, targets, train)
         return self.loss_rows.mean() if out is None else out
 

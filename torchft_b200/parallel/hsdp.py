@@ -305,10 +305,12 @@ class ShardedLlamaTrainer:
         )
         self._mark_params_written()
         # Forward and backward pass as one CUDA graph.  The GPU works on the passes of a small model for less time than the
-        # host needs for their launches (77 of them, 430 us against 1130, for two layers of width 256 and 256 tokens), so
-        # the second step on captures them and the following ones launch the graph.  By default where a step is less than
-        # 4 TFLOP: at 1 TFLOP (four layers of width 1024, 3000 tokens) host and GPU take about as long, at 25 the host is
-        # ahead by 20 ms.  Only without a shard group and a manager: their hooks run host code in every step.
+        # host needs for their launches, so the second step on captures them and the following ones launch the graph.  By
+        # default where a step is less than 4 TFLOP.  Step without and with the graph, us: two layers of width 256 on 256
+        # tokens (0.002 TFLOP) 1179 and 251, on 4096 (0.05) 1235 and 424; of width 1024, two layers on 512 (0.1) 1170 and 675,
+        # four on 1000 (0.35) 2296 and 1268, four on 3000 (1.0) 2411 and 1856; from there on the GPU is the slower one and the two
+        # differ by less than 1 % (2.4 TFLOP 6359 and 6342, 4.3 6111 and 6074, 12.8 15129 and 15135), only the host is free sooner.
+        # Only without a shard group and a manager: their hooks run host code in every step.
         if step_graph is None:
             step_graph = cfg.flops_per_token(seq_len) * batch * seq_len < 4e12
         self._step_graph = (_StepGraph(self) if step_graph and self.cuda and ws == 1 and manager is None
